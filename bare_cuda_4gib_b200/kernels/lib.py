@@ -248,12 +248,33 @@ def add_rmsnorm(residual: torch.Tensor, delta: Optional[Partials], weight: torch
         stream if stream is not None else stream_handle()), "add_rmsnorm")
 
 
+_matmul_f32 = None
+
+
+def _matmul_f32_lib():
+    global _matmul_f32
+    if _matmul_f32 is None:
+        l = build.load_library("matmul_f32.cu")
+        P, I, L = c_void_p, c_int, c_longlong
+        l.llm_matmul_f32.argtypes = [P, P, P, I, I, I, L, L, I, P]
+        l.llm_matmul_f32.restype = c_int
+        _matmul_f32 = l
+    return _matmul_f32
+
+
 def matmul_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, m: int, stream=None) -> None:
-    """out[:m] = a[:m] @ w.T with w stored [out features, in features]."""
+    """out[:m] = a[:m] @ w.T with w stored [out features, in features].  All float32 with 16-byte aligned rows (every
+    product of the 32-bit run) goes to the kernel that is made for it, anything else to the general one."""
     _dev(a, w, out)
     n, k = w.shape
     if a.shape[-1] != k or out.shape[-1] != n or a.stride(-1) != 1 or out.stride(-1) != 1 or not w.is_contiguous():
         raise KernelLaunchError(f"matmul_plain: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)}")
+    if (a.dtype == w.dtype == out.dtype == torch.float32 and k > 0 and k % 4 == 0 and a.stride(-2) % 4 == 0
+            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+        _check(_matmul_f32_lib().llm_matmul_f32(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, a.stride(-2),
+                                                out.stride(-2), sm_count(), stream if stream is not None else stream_handle()),
+               "matmul_f32")
+        return
     _check(plain().lib.llm_matmul_plain(a.data_ptr(), dtype_code(a.dtype), w.data_ptr(), dtype_code(w.dtype),
                                         out.data_ptr(), dtype_code(out.dtype), m, n, k, a.stride(-2),
                                         out.stride(-2), stream if stream is not None else stream_handle()),

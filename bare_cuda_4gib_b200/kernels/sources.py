@@ -7,7 +7,7 @@ DIFF_ATTENTION_SIZES = ((16, 16), (64, 128), (128, 256))
 
 
 def all_libraries():
-    jobs = [("plain_kernels.cu", ()), ("gemm_tcgen05.cu", ()), ("gemv_fused.cu", ()), ("stream_kernels.cu", ()),
+    jobs = [("plain_kernels.cu", ()), ("matmul_f32.cu", ()), ("gemm_tcgen05.cu", ()), ("gemv_fused.cu", ()), ("stream_kernels.cu", ()),
             ("linear_attention.cu", ()), ("biased_attention.cu", ()), ("sandwich_norm.cu", ()), ("head_prepare.cu", ()),
             ("latent_attention.cu", ()), ("mlstm.cu", ()), ("diff_attention.cu", ()), ("moe.cu", ()),
             ("gated_sandwich.cu", ()), ("mamba2.cu", ()),
