@@ -1,6 +1,7 @@
 """The CUDA libraries of the engine: (source file, -D flags) pairs.  A model compiles what it
 needs at first use; `all_libraries()` is everything, for the build check."""
 
+ATTENTION_F32_HEAD_DIMS = (64, 128)
 ATTENTION_HEAD_DIMS = (16, 32, 48, 64, 80, 96, 112, 128)
 # (entries of one map, value entries) of differential attention on the tensor cores, as the presets have them
 DIFF_ATTENTION_SIZES = ((16, 16), (64, 128), (128, 256))
@@ -21,6 +22,7 @@ def all_libraries():
     # value heads of their own size and capped scores, as the Gurolix and Fuzazen presets have them
     jobs += [("attention_mma.cu", ("-DHEAD_DIM=16", "-DV_DIM=32")), ("attention_mma.cu", ("-DHEAD_DIM=128", "-DV_DIM=64")), ("attention_mma.cu", ("-DHEAD_DIM=128", "-DV_DIM=64", "-DSCORE_CAP")),
              ("attention_mma.cu", ("-DHEAD_DIM=128", "-DSCORE_CAP")), ("attention_mma.cu", ("-DHEAD_DIM=16", "-DV_DIM=32", "-DSCORE_CAP"))]
+    jobs += [("attention_f32.cu", (f"-DHEAD_DIM={d}",)) for d in ATTENTION_F32_HEAD_DIMS]
     jobs += [("attention_tcgen05.cu", (f"-DHEAD_DIM={d}",)) for d in (64, 128)]
     jobs += [("attention_decode.cu", (f"-DHEAD_DIM={d}",)) for d in (64, 128)]
     jobs += [("diff_attention.cu", (f"-DDA_DQ={d}", f"-DDA_DV={v}")) for d, v in DIFF_ATTENTION_SIZES]

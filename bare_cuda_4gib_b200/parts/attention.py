@@ -102,8 +102,8 @@ class Attention(Part):
             from ..kernels import attention as fast
             fast.run(ctx, self.fast, q, out, call.cache, self.scale, window)
         else:
-            K.attention_plain(q, out, call.cache, ctx.positions, ctx.row_seq, self.heads, n,
-                              self.scale, window, ctx.stream)
+            from ..kernels import attention_f32
+            attention_f32.run(ctx, q, out, call.cache, self.heads, self.scale, window)
         residual = getattr(ctx, "residual", None)
         return self.o.forward(ctx, out, n, torch.float32, "attn_proj", allow_partials=True,
                               epilogue=K.AddTo(residual, getattr(ctx, "following_norm", None)) if residual is not None else None)
@@ -200,7 +200,8 @@ class GatedAttention(Part):
             from ..kernels import attention as fast
             fast.run(ctx, self.fast, q, out, call.cache, self.scale, window)
         else:
-            K.attention_plain(q, out, call.cache, ctx.positions, ctx.row_seq, self.heads, n, self.scale, window, ctx.stream)
+            from ..kernels import attention_f32
+            attention_f32.run(ctx, q, out, call.cache, self.heads, self.scale, window)
         HP.sigmoid_gate(ctx, out, u[:, u.shape[1] - qd:], n)
         return self.o.forward(ctx, out, n, torch.float32, "attn_proj", allow_partials=True)
 

@@ -1,5 +1,7 @@
-"""The kernels of the 32-bit run alone: the float32 product against float64, at the edges of their tiles,
+"""The kernels of the 32-bit run alone: the float32 product and attention against float64, at the edges of their tiles,
 and against themselves under other cuts of the same rows (a sum's order hangs on the operation's sizes only)."""
+
+import types
 
 import pytest
 import torch
@@ -39,3 +41,72 @@ def test_matmul_f32_strided_rows_and_bad_values():
     assert torch.equal(got.nan_to_num(7.0, 8.0, 9.0), clean.nan_to_num(7.0, 8.0, 9.0))
     bad = ~torch.isfinite(got).all(-1)
     assert bad.nonzero().flatten().tolist() == [7, 9]        # a row's values stay in that row
+
+
+class _Attention:
+    """Requests of (tokens of the step, keys) over pages in random order."""
+
+    def __init__(self, dim, kv_heads, group, seqs, window, page):
+        self.dim, self.kv_heads, self.group, self.window, self.page, self.seqs = dim, kv_heads, group, window, page, seqs
+        blocks = -(-max(kv for _, kv in seqs) // page)
+        self.elems = 2 * kv_heads * page * dim
+        self.pool = torch.full((len(seqs) * blocks + 2, self.elems), float("nan"), device=DEV)    # pages nobody holds
+        table = torch.full((len(seqs), blocks), -1, dtype=torch.int32)
+        order = torch.randperm(self.pool.shape[0]).tolist()
+        for s, (_, kv) in enumerate(seqs):
+            for b in range(-(-kv // page)):
+                table[s, b] = order.pop()
+                self.pool[table[s, b]] = torch.randn(self.elems, device=DEV)
+        self.table = table.to(DEV)
+        self.q = torch.randn(sum(q for q, _ in seqs), kv_heads * group * dim, device=DEV)
+        self.at = [sum(q for q, _ in seqs[:s]) for s in range(len(seqs))]
+
+    def run(self, parts):
+        """`parts`: (request, first token of its step, tokens); what the kernel gives for them as one step."""
+        from bare_cuda_4gib_b200.kernels import attention_f32, lib as K
+        ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        ctx, lens = types.SimpleNamespace(), [n for _, _, n in parts]
+        kv = [self.seqs[s][1] - self.seqs[s][0] + first + n for s, first, n in parts]
+        ctx.host_q_len, ctx.n_seqs, ctx.max_q_len, ctx.n_tokens, ctx.stream = lens, len(parts), max(lens), sum(lens), K.stream_handle()
+        ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len = ints([sum(lens[:i]) for i in range(len(lens))]), ints(lens), ints(kv)
+        table = self.table[[s for s, _, _ in parts]].contiguous()
+        view = K.CacheView(self.pool.data_ptr(), self.pool.data_ptr() + self.elems // 2 * 4, table, self.elems, table.stride(0),
+                           self.page, self.kv_heads, self.dim, torch.float32)
+        q = torch.cat([self.q[self.at[s] + first: self.at[s] + first + n] for s, first, n in parts])
+        out = torch.full_like(q, float("nan"))
+        assert attention_f32.takes(q, out, view)
+        attention_f32.run(ctx, q, out, view, self.kv_heads * self.group, self.dim ** -0.5, self.window)
+        return out
+
+    def want(self):
+        rows = []
+        for s, (n, kv) in enumerate(self.seqs):
+            held = self.table[s, : -(-kv // self.page)].long()
+            both = self.pool[held].view(-1, 2, self.kv_heads, self.page, self.dim).double()
+            k, v = (both[:, i].permute(1, 0, 2, 3).reshape(self.kv_heads, -1, self.dim)[:, :kv] for i in (0, 1))
+            q = self.q[self.at[s]: self.at[s] + n].double().view(n, self.kv_heads, self.group, self.dim)
+            i, j = (kv - n + torch.arange(n, device=DEV))[:, None], torch.arange(kv, device=DEV)[None]
+            hidden = (j > i) | (i - j >= self.window) if self.window else j > i
+            w = (torch.einsum("tkgd,kjd->kgtj", q, k) * self.dim ** -0.5).masked_fill(hidden, -float("inf")).softmax(-1)
+            rows.append(torch.einsum("kgtj,kjd->tkgd", w, v).reshape(n, -1))
+        return torch.cat(rows)
+
+
+@pytest.mark.parametrize("dim,kv_heads,group,page,window,seqs", [
+    (64, 2, 8, 64, 0, [(1, 300), (1, 1), (70, 70), (1, 64), (2, 65)]),
+    (64, 2, 1, 32, 0, [(3, 70), (9, 64), (8, 8), (90, 200)]),            # at most and over eight rows of a request
+    (64, 1, 3, 16, 40, [(3, 70), (1, 2100), (65, 129)]),                 # a window; more spans than a cluster holds at once
+    (128, 2, 4, 64, 0, [(1, 1100), (2, 127), (33, 128)]),
+    (128, 1, 16, 32, 100, [(1, 333), (50, 90)]),                         # more than eight heads to a key head
+])
+def test_attention_f32(dim, kv_heads, group, page, window, seqs):
+    torch.manual_seed(dim + group)
+    case = _Attention(dim, kv_heads, group, seqs, window, page)
+    whole, want = case.run([(s, 0, n) for s, (n, _) in enumerate(seqs)]), case.want()
+    # scores of size ~ 4 carry dim / 2 + 2 roundings, which the exponential passes on; 64 values and a join a span follow
+    bound = (4 * (dim / 2 + 2) + 2 * 64 + 3 * (max(kv for _, kv in seqs) / 64 + 1)) * EPS
+    assert ((whole.double() - want).abs() <= bound * want.abs().max()).all()
+    for tail in (1, 2, 7):                   # the last tokens of every request alone, as later steps would bring them
+        parts = [(s, max(0, n - tail), min(n, tail)) for s, (n, _) in enumerate(seqs)]
+        rows = torch.cat([whole[case.at[s] + f: case.at[s] + f + n] for s, f, n in parts])
+        assert torch.equal(case.run(parts), rows), tail
