@@ -89,11 +89,29 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ residual, const TD* __res
   }
 }
 
-// The same with 16-byte accesses: float32 delta, bfloat16 weight and output, hidden a multiple of 4.
-// A thread keeps its elements in registers (at most 4 float4: hidden <= 16 * blockDim.x).
+// Four neighbouring values.
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  uint2 raw;
+  raw.x = *reinterpret_cast<const uint32_t*>(&a);
+  raw.y = *reinterpret_cast<const uint32_t*>(&b);
+  *reinterpret_cast<uint2*>(p) = raw;
+}
+
+// The same with 16-byte accesses: float32 delta, hidden a multiple of 4.  A thread keeps its elements in
+// registers (at most 4 float4: hidden <= 16 * blockDim.x).  Bound by the trip to memory: with few float32 rows of 2,048
+// the loop of single loads above took 8.0 us a launch, this takes 4.4.
+template <typename TW, typename TO>
 __global__ void add_rmsnorm_vec_kernel(float* __restrict__ residual, const float* __restrict__ delta,
                                        int n_partials, long long partial_stride,
-                                       const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ out,
+                                       const TW* __restrict__ weight, TO* __restrict__ out,
                                        const int32_t* __restrict__ row_index, int hidden, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -126,20 +144,13 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ residual, const float
   const float total = block_sum(sq, scratch);
   const float scale = 1.0f / sqrtf(total / (float)hidden + eps);
   if (out) {
-    uint2* dst = reinterpret_cast<uint2*>(out + (long long)r * hidden);
+    TO* dst = out + (long long)r * hidden;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int i = threadIdx.x + j * blockDim.x;
       if (i < n4) {
-        const uint2 wraw = reinterpret_cast<const uint2*>(weight)[i];
-        const __nv_bfloat162 w01 = *reinterpret_cast<const __nv_bfloat162*>(&wraw.x);
-        const __nv_bfloat162 w23 = *reinterpret_cast<const __nv_bfloat162*>(&wraw.y);
-        __nv_bfloat162 o01 = __floats2bfloat162_rn(v[j].x * scale * __low2float(w01), v[j].y * scale * __high2float(w01));
-        __nv_bfloat162 o23 = __floats2bfloat162_rn(v[j].z * scale * __low2float(w23), v[j].w * scale * __high2float(w23));
-        uint2 o;
-        o.x = *reinterpret_cast<uint32_t*>(&o01);
-        o.y = *reinterpret_cast<uint32_t*>(&o23);
-        dst[i] = o;
+        const float4 w = load4(weight + 4 * i);
+        store4(dst + 4 * i, make_float4(v[j].x * scale * w.x, v[j].y * scale * w.y, v[j].z * scale * w.z, v[j].w * scale * w.w));
       }
     }
   }
@@ -236,6 +247,14 @@ static int add_rmsnorm_out(float* residual, const void* delta, int n_partials,
   return launch_status();
 }
 
+// Threads of the vector kernel for rows of n4 float4: at most two a thread when wide, four at most.
+static int norm_vec_threads(int n4) {
+  int threads = 128;
+  while (threads < 1024 && threads * 2 <= n4) threads *= 2;
+  while (threads * 4 < n4) threads *= 2;
+  return threads;
+}
+
 extern "C" int llm_add_rmsnorm(float* residual, const void* delta, int delta_dtype, int n_partials,
                                long long partial_stride, const void* weight, int weight_dtype,
                                void* out, int out_dtype, const int32_t* row_index, int rows,
@@ -258,11 +277,17 @@ extern "C" int llm_add_rmsnorm(float* residual, const void* delta, int delta_dty
                       partial_stride, (const __nv_bfloat16*)weight, (__nv_bfloat16*)out, row_index, rows, hidden, eps);
       return launch_status();
     }
-    int threads = 128;
-    while (threads < 1024 && threads * 2 <= n4) threads *= 2;   // <= 2 float4 per thread when wide
-    while (threads * 4 < n4) threads *= 2;
-    launch_kernel(add_rmsnorm_vec_kernel, rows, threads, 0, stream, residual, (const float*)delta, n_partials,
-                  partial_stride, (const __nv_bfloat16*)weight, (__nv_bfloat16*)out, row_index, hidden, eps);
+    launch_kernel(add_rmsnorm_vec_kernel<__nv_bfloat16, __nv_bfloat16>, rows, norm_vec_threads(n4), 0, stream, residual,
+                  (const float*)delta, n_partials, partial_stride, (const __nv_bfloat16*)weight, (__nv_bfloat16*)out,
+                  row_index, hidden, eps);
+    return launch_status();
+  }
+  // the 32-bit run's: a block per row whatever the number of rows, so that a row's sums keep their order
+  if (delta_dtype == DT_F32 && weight_dtype == DT_F32 && (out == nullptr || out_dtype == DT_F32) && hidden % 4 == 0 &&
+      hidden <= 16 * 1024 && aligned16(residual) && aligned16(delta) && partial_stride % 4 == 0 && aligned16(weight) &&
+      aligned16(out)) {
+    launch_kernel(add_rmsnorm_vec_kernel<float, float>, rows, norm_vec_threads(hidden / 4), 0, stream, residual,
+                  (const float*)delta, n_partials, partial_stride, (const float*)weight, (float*)out, row_index, hidden, eps);
     return launch_status();
   }
   if (delta_dtype == DT_F32 && weight_dtype == DT_F32)

@@ -110,3 +110,18 @@ def test_attention_f32(dim, kv_heads, group, page, window, seqs):
         parts = [(s, max(0, n - tail), min(n, tail)) for s, (n, _) in enumerate(seqs)]
         rows = torch.cat([whole[case.at[s] + f: case.at[s] + f + n] for s, f, n in parts])
         assert torch.equal(case.run(parts), rows), tail
+
+
+@pytest.mark.parametrize("rows,hidden,partials", [(1, 64, 1), (3, 2048, 2), (300, 4100, 1), (2, 2050, 1)])
+def test_add_rmsnorm_f32(rows, hidden, partials):
+    from bare_cuda_4gib_b200.kernels import lib as K
+    torch.manual_seed(hidden)
+    x, w = torch.randn(rows, hidden, device=DEV), 1.0 + 0.1 * torch.randn(hidden, device=DEV)
+    delta = torch.randn(partials, rows, hidden, device=DEV)
+    residual, out = x.clone(), torch.empty(rows, hidden, device=DEV)
+    K.add_rmsnorm(residual, K.Partials(delta if partials > 1 else delta[0], partials), w, out, 1e-5, rows)
+    want = x.double() + delta.double().sum(0)
+    normed = want / torch.sqrt((want * want).mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert ((residual.double() - want).abs() <= (partials + 1) * 2 * EPS * (x.abs() + delta.abs().sum(0)).double()).all()
+    # the sum of squares adds up at most 16 terms a thread and 10 levels of the block, the factor rounds four times more
+    assert ((out.double() - normed).abs() <= ((16 + 10) / 2 + 6 + 2 * partials) * 2 * EPS * normed.abs() + 1e-6).all()
