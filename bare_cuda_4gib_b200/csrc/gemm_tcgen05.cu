@@ -860,6 +860,415 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The product for a few dozen tokens with the work around it fused in (the counterpart of gemv_fused.cu,
+// whose input no longer fits in shared memory there).  With weights on the MMA rows a product of
+// a layer has 16 to 90 tiles, too few to draw HBM's bandwidth, so K has to be split; and split over
+// independent blocks it leaves partial sums that further kernels add up (norm, rotation: three more launches a
+// layer, 4 to 6 us each).  Here the blocks that share a tile's K range are a cluster: each turns its
+// accumulator over to the others in slices (bulk copies through distributed shared memory), so block r
+// ends up with all parts of slice r, adds them in the order of the blocks and finishes the outputs:
+//   CL_STORE   plain store
+//   CL_ADD     residual[t, f] += result, and what the next norm's product needs (see RowsExtra)
+//   CL_SWIGLU  w = [gate; up]: act(gate) * up
+//   CL_ROPE    w = [Wq; Wk; Wv]: q and k rotated by position, q to `out`, k and v into the paged cache
+// Rows of a tile go by pairs (a feature and its rotation partner, a gate row and its up row): a slice is
+// half = 64 / cluster pairs, first all their first members, then the second ones.  Without pairs the two
+// members are simply neighbouring runs.
+// Two blocks share an SM (112 KB of shared memory each), so that a kernel's weights are on their way while
+// the kernel before it still runs on the other half.  What bounds it: the chain wait for the input - first tile - last
+// product - exchange - stores, which is why eight warps share the epilogue.  (Storing the slices straight from registers into
+// the other blocks' shared memory, 16 bytes a lane, measured slower: 9.5 against 8.0 us for 64 tokens x 2,048 x 2,048.)
+enum { CL_STORE = 0, CL_ADD = 1, CL_SWIGLU = 2, CL_ROPE = 3 };
+constexpr int CL_MAX_TOKENS = 64;
+constexpr int CL_EPI_WARPS = 8, CL_EPI = CL_EPI_WARPS * 32, CL_THREADS = 64 + CL_EPI;
+constexpr int ERR_TIMEOUT_CLUSTER = 4;
+
+struct ClusterArgs {
+  int bn, stages, stage_bytes, tmem_cols;
+  uint32_t idesc;
+  unsigned long long wait_ns;
+  int pair_span;                // a row's partner lies this far behind it, rows come in groups of twice this many
+  int n_tokens, n_features, k_blocks, k_per_block, up_row_offset;
+  const float* sq_in;           // parts of the input rows' sums of squares (null: the input is what it is)
+  int sq_items;
+  long long sq_stride;
+  float norm_width, eps;
+  void* out;                    // CL_ADD: the float32 residual stream; CL_ROPE: q
+  int out_is_f32;
+  long long ld_out;
+  __nv_bfloat16* pre_x;
+  long long pre_x_stride;
+  const void* pre_w;
+  int pre_w_dtype;
+  float* pre_sq;                // [slice][pre_sq_stride]
+  long long pre_sq_stride;
+  PagedCache cache;
+  const int32_t* positions;
+  const int32_t* row_seq;
+  const float* inv_freq;
+  int q_heads, write_cache;
+  int* error_word;
+};
+
+// The cluster's barrier in two halves: a thread arrives, later waits, then may arrive again.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+__device__ __forceinline__ uint32_t peer_address(uint32_t smem_addr, int rank) {
+  uint32_t at;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_addr), "r"(rank));
+  return at;
+}
+
+template <int N>
+__device__ __forceinline__ void load_run(const float* from, float (&v)[N]) {
+  if (N == 4) {
+    const float4 x = *reinterpret_cast<const float4*>(from);
+    v[0] = x.x, v[1] = x.y, v[N - 2] = x.z, v[N - 1] = x.w;
+  } else {
+    const float2 x = *reinterpret_cast<const float2*>(from);
+    v[0] = x.x, v[1] = x.y;
+  }
+}
+
+// 4 or 2 neighbouring values.
+template <int N>
+__device__ __forceinline__ void store_run(float* to, const float (&v)[N]) {
+  if (N == 4) *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+  else *reinterpret_cast<float2*>(to) = make_float2(v[0], v[1]);
+}
+template <int N>
+__device__ __forceinline__ void store_run(__nv_bfloat16* to, const float (&v)[N]) {
+  __nv_bfloat162 b[N / 2];
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) b[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+  if (N == 4) *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<uint32_t*>(&b[0]), *reinterpret_cast<uint32_t*>(&b[N / 2 - 1]));
+  else *reinterpret_cast<uint32_t*>(to) = *reinterpret_cast<uint32_t*>(&b[0]);
+}
+
+template <int EPI, int C>
+__global__ void __launch_bounds__(CL_THREADS, 2)
+gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a) {
+  constexpr int HALF = 64 / C, ROWS = 2 * HALF;       // pairs and rows of a slice
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int slot = a.bn * ROWS + 8;                                                 // floats of a slice (8 more keep slices on other banks)
+  float* received = reinterpret_cast<float*>(smem + a.stages * a.stage_bytes);      // [C][bn][ROWS], a slice `slot` apart
+  float* sq_part = received + C * slot;                                             // [CL_EPI_WARPS][bn]
+  float* scale_s = sq_part + CL_EPI_WARPS * a.bn;                                   // [bn]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(scale_s + a.bn);
+  uint64_t* empty_bar = full_bar + a.stages;
+  uint64_t* acc_bar = empty_bar + a.stages;
+  uint64_t* received_bar = acc_bar + 1;
+  uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(received_bar + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = blockIdx.x % C, tile = blockIdx.x / C;
+  constexpr int TILE_OUT = EPI == CL_SWIGLU ? BM / 2 : BM;
+  const int f0 = tile * TILE_OUT;
+  const int kb_begin = rank * a.k_per_block, n_kb = max(0, min(a.k_blocks, kb_begin + a.k_per_block) - kb_begin);
+
+  auto issue_weights = [&](int i, int s) {
+    uint8_t* stage = smem + s * a.stage_bytes;
+    mbar_expect_tx(&full_bar[s], a.stage_bytes);
+    const int k0 = (kb_begin + i) * BK;
+    tma_load_2d(stage, &map_w, &full_bar[s], k0, f0);      // CL_SWIGLU: the box has 64 rows
+    if (EPI == CL_SWIGLU) tma_load_2d(stage + A_BYTES / 2, &map_w, &full_bar[s], k0, a.up_row_offset + f0);
+  };
+  auto issue_activations = [&](int i, int s) {
+    tma_load_2d(smem + s * a.stage_bytes + A_BYTES, &map_a, &full_bar[s], (kb_begin + i) * BK, 0);
+  };
+  const int n_early = min(n_kb, a.stages);
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(acc_bar, 1);
+    mbar_init(received_bar, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_expect_tx(received_bar, (uint32_t)(C * a.n_tokens * ROWS * 4));
+    for (int i = 0; i < n_early; ++i) issue_weights(i, i);   // overlaps the tail of the kernel before
+    pdl_wait();
+    for (int i = 0; i < n_early; ++i) issue_activations(i, i);
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)),
+                 "r"(a.tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  pdl_wait();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  cluster_arrive();        // this block has its barriers
+  const uint32_t tmem_base = *tmem_base_slot;
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- TMA producer (two lanes share a stage's copies)
+    if (lane < 2) {
+      int armed = n_early;
+      int s = n_early == a.stages ? 0 : n_early;
+      uint32_t phase = n_early == a.stages ? 1 : 0;
+      for (int i = n_early; i < n_kb; ++i) {
+        if (!mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, a.wait_ns)) {
+          *abort_flag = 1;
+          atomicCAS(a.error_word, 0, ERR_TIMEOUT_PRODUCER);
+          break;
+        }
+        if (lane == 1) issue_activations(i, s);
+        else issue_weights(i, s);
+        armed = i + 1;
+        if (++s == a.stages) { s = 0; phase ^= 1; }
+      }
+      if (lane == 0 && *abort_flag) {
+        // copies already issued still land in shared memory: wait for them (bounded) before leaving
+        for (int i = max(0, armed - a.stages); i < armed; ++i) {
+          const unsigned long long start = global_timer();
+          while (!mbar_try_wait(&full_bar[i % a.stages], (i / a.stages) & 1) && global_timer() - start < a.wait_ns / 10) {
+          }
+        }
+      }
+    }
+    __syncwarp();
+    cluster_wait();
+    cluster_arrive();
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issuer
+    if (lane == 0) {
+      int s = 0;
+      uint32_t phase = 0;
+      const uint32_t smem_base = smem_u32(smem);
+      for (int i = 0; i < n_kb; ++i) {
+        if (!mbar_wait(&full_bar[s], phase, abort_flag, a.wait_ns)) {
+          *abort_flag = 1;
+          atomicCAS(a.error_word, 0, ERR_TIMEOUT_MMA);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t desc_a = smem_desc_sw128(smem_base + s * a.stage_bytes);
+        const uint64_t desc_b = smem_desc_sw128(smem_base + s * a.stage_bytes + A_BYTES);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k) {
+          const uint64_t koff = (uint64_t)((k * UMMA_K * 2) >> 4);
+          umma_bf16(tmem_base, desc_a + koff, desc_b + koff, a.idesc, (i > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit(&empty_bar[s]);
+        if (++s == a.stages) { s = 0; phase ^= 1; }
+      }
+      umma_commit(acc_bar);
+    }
+    __syncwarp();
+    cluster_wait();
+    cluster_arrive();
+  } else {
+    // ---------------------------------------------------------------- epilogue (warps 2..9)
+    const int e = threadIdx.x - 64, ew = warp - 2, quad = warp & 3;   // quad: the tensor-memory lanes 32 quad .. of this warp
+    // What does not depend on the accumulator comes first: the norm's factor per token ...
+    if (a.sq_in) {
+      float sq[2] = {0.0f, 0.0f};
+#pragma unroll 16
+      for (int i = ew; i < a.sq_items; i += CL_EPI_WARPS)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (lane + 32 * j < a.n_tokens) sq[j] += a.sq_in[(long long)i * a.sq_stride + lane + 32 * j];
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (lane + 32 * j < a.n_tokens) sq_part[ew * a.bn + lane + 32 * j] = sq[j];
+      asm volatile("bar.sync 1, %0;" ::"n"(CL_EPI) : "memory");
+      if (e < a.n_tokens) {
+        float total = 0.0f;
+#pragma unroll
+        for (int i = 0; i < CL_EPI_WARPS; ++i) total += sq_part[i * a.bn + e];
+        scale_s[e] = 1.0f / sqrtf(total / a.norm_width + a.eps);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(CL_EPI) : "memory");
+    }
+    // ... and what the thread's first output needs.  A thread owns RUN neighbouring features of a token, with pairs their
+    // partners too; a token's threads are neighbouring lanes.
+    constexpr bool PAIRED = EPI == CL_SWIGLU || EPI == CL_ROPE;
+    constexpr int RUN = EPI == CL_ROPE ? 2 : 4, PER_TOKEN = (PAIRED ? HALF : ROWS) / RUN, TOKEN_STEP = CL_EPI / PER_TOKEN;
+    static_assert(PER_TOKEN <= 32, "a token's threads lie in one warp");
+    const int at = e % PER_TOKEN * RUN, first_token = e / PER_TOKEN;     // first row of the slice that the thread owns
+    const int f_plain = f0 + rank * ROWS + at;                           // CL_ADD, CL_STORE: its feature
+    float old[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pre_w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float rot_c[2] = {1.0f, 1.0f}, rot_s[2] = {0.0f, 0.0f};
+    const int dim = a.cache.head_dim, span = max(dim / 2, 1), first_pair = tile * 64 + rank * HALF + at;
+    const int head = first_pair / span, entry = first_pair % span;       // CL_ROPE: of [q; k; v]
+    const bool turned = EPI == CL_ROPE && a.inv_freq && head < a.q_heads + a.cache.kv_heads;
+    if (EPI == CL_ADD && f_plain + 4 <= a.n_features) {
+      if (first_token < a.n_tokens) {
+        const float4 o = *reinterpret_cast<const float4*>(static_cast<const float*>(a.out) + (long long)first_token * a.ld_out + f_plain);
+        old[0] = o.x, old[1] = o.y, old[2] = o.z, old[3] = o.w;
+      }
+      if (a.pre_x) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          pre_w[j] = a.pre_w_dtype == DT_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.pre_w)[f_plain + j])
+                                              : static_cast<const float*>(a.pre_w)[f_plain + j];
+      }
+    }
+    if (turned && first_token < a.n_tokens)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) sincosf((float)a.positions[first_token] * a.inv_freq[entry + j], &rot_s[j], &rot_c[j]);
+
+    bool ok = mbar_wait(acc_bar, 0, abort_flag, a.wait_ns);
+    if (!ok) {
+      *abort_flag = 1;
+      atomicCAS(a.error_word, 0, ERR_TIMEOUT_EPILOGUE);
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Two groups of four warps take half of the tokens each: the accumulator, cut into slices, into the pipeline's
+    // stages (idle by now), then one bulk copy to every block of the cluster.
+    const int part = ew / 4, part_tokens = (a.bn / 2 + 15) / 16 * 16, t_begin = part * part_tokens;
+    const int t_end = min(a.n_tokens, t_begin + part_tokens);
+    float* outgoing = reinterpret_cast<float*>(smem);
+    if (ok) {
+      const int row = quad * 32 + lane, in_group = row % (2 * a.pair_span);
+      const int pair = row / (2 * a.pair_span) * a.pair_span + in_group % a.pair_span;
+      float* mine = outgoing + pair / HALF * slot + pair % HALF + (in_group >= a.pair_span ? HALF : 0);
+      const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+#pragma unroll 1
+      for (int c0 = t_begin; c0 < t_end; c0 += 16) {
+        uint32_t v[16];
+        if (n_kb > 0) {
+          tmem_load16(lane_base + c0, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) mine[(c0 + j) * ROWS] = __uint_as_float(v[j]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    cluster_wait();          // the others have their barriers
+    asm volatile("bar.sync %0, 128;" ::"r"(2 + part) : "memory");
+    if (ok && t_end > t_begin && ew % 4 == 0 && lane < C) {      // a lane per receiver
+      const uint32_t bytes = (uint32_t)(t_end - t_begin) * ROWS * 4;
+      const uint32_t to = peer_address(smem_u32(received + rank * slot + t_begin * ROWS), lane);
+      asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                   ::"r"(to), "r"(smem_u32(outgoing + lane * slot + t_begin * ROWS)), "r"(bytes),
+                     "r"(peer_address(smem_u32(received_bar), lane)) : "memory");
+    }
+    if (ok) {
+      ok = mbar_wait(received_bar, 0, abort_flag, a.wait_ns);
+      if (!ok) atomicCAS(a.error_word, 0, ERR_TIMEOUT_CLUSTER);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    cluster_arrive();        // what was sent here has come (or this thread has given up)
+    if (ok) {
+      auto summed = [&](int t, int r, float (&v)[RUN]) {      // rows r .. of the slice, the parts added in the order of the blocks
+        float part_of[C][RUN];
+#pragma unroll
+        for (int q = 0; q < C; ++q) load_run(received + q * slot + t * ROWS + r, part_of[q]);
+#pragma unroll
+        for (int j = 0; j < RUN; ++j) v[j] = part_of[0][j];
+#pragma unroll
+        for (int q = 1; q < C; ++q)
+#pragma unroll
+          for (int j = 0; j < RUN; ++j) v[j] += part_of[q][j];
+        if (a.sq_in) {
+          const float f = scale_s[t];
+#pragma unroll
+          for (int j = 0; j < RUN; ++j) v[j] *= f;
+        }
+      };
+      const int rounds = (a.n_tokens + TOKEN_STEP - 1) / TOKEN_STEP;
+#pragma unroll 1
+      for (int i = 0; i < rounds; ++i) {
+        const int t = first_token + i * TOKEN_STEP;
+        const bool there = t < a.n_tokens;
+        float v[RUN];
+        if (EPI == CL_ADD || EPI == CL_STORE) {
+          float sq = 0.0f;
+          if (there && f_plain + 4 <= a.n_features) {         // (the width is a multiple of four)
+            summed(t, at, v);
+            const long long where = (long long)t * a.ld_out + f_plain;
+            if (EPI == CL_STORE) {
+              if (a.out_is_f32) store_run(static_cast<float*>(a.out) + where, v);
+              else store_run(static_cast<__nv_bfloat16*>(a.out) + where, v);
+            } else {
+              float* res = static_cast<float*>(a.out) + where;
+              if (i > 0) {
+                const float4 o = *reinterpret_cast<const float4*>(res);
+                old[0] = o.x, old[1] = o.y, old[2] = o.z, old[3] = o.w;
+              }
+#pragma unroll
+              for (int j = 0; j < RUN; ++j) v[j] += old[j];
+              store_run(res, v);
+              if (a.pre_x) {
+                float w[RUN];
+#pragma unroll
+                for (int j = 0; j < RUN; ++j) w[j] = v[j] * pre_w[j], sq += v[j] * v[j];
+                store_run(a.pre_x + (long long)t * a.pre_x_stride + f_plain, w);
+              }
+            }
+          }
+          if (EPI == CL_ADD && a.pre_x) {
+#pragma unroll
+            for (int o = 1; o < PER_TOKEN; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            if (at == 0 && there) a.pre_sq[(long long)(tile * C + rank) * a.pre_sq_stride + t] = sq;
+          }
+        } else if (there) {
+          float u[RUN];
+          summed(t, at, v);
+          summed(t, HALF + at, u);
+          if (EPI == CL_SWIGLU) {
+            const int f = f0 + rank * HALF + at;
+            if (f + RUN > a.n_features) continue;
+#pragma unroll
+            for (int j = 0; j < RUN; ++j) v[j] = glu_pair(v[j], u[j]);
+            if (a.out_is_f32) store_run(static_cast<float*>(a.out) + (long long)t * a.ld_out + f, v);
+            else store_run(static_cast<__nv_bfloat16*>(a.out) + (long long)t * a.ld_out + f, v);
+          } else if (head < a.q_heads + 2 * a.cache.kv_heads) {     // CL_ROPE: RUN pairs of one head
+            const int pos = a.positions[t];
+            if (turned) {
+#pragma unroll
+              for (int j = 0; j < RUN; ++j) {
+                if (i > 0) sincosf((float)pos * a.inv_freq[entry + j], &rot_s[j], &rot_c[j]);
+                const float lo = v[j], hi = u[j];
+                v[j] = lo * rot_c[j] - hi * rot_s[j];
+                u[j] = hi * rot_c[j] + lo * rot_s[j];
+              }
+            }
+            __nv_bfloat16* to = nullptr;
+            if (head < a.q_heads) {
+              to = static_cast<__nv_bfloat16*>(a.out) + (long long)t * a.ld_out + (long long)head * dim;
+            } else if (a.write_cache) {
+              const bool is_v = head >= a.q_heads + a.cache.kv_heads;
+              const long long off = cache_offset(a.cache, a.row_seq[t], pos, head - a.q_heads - (is_v ? a.cache.kv_heads : 0));
+              if (off >= 0) to = static_cast<__nv_bfloat16*>(is_v ? a.cache.v : a.cache.k) + off;
+            }
+            if (to) {
+              store_run(to + entry, v);
+              store_run(to + entry + span, u);
+            }
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+
+  cluster_wait();          // no block leaves while slices of it are on their way
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(a.tmem_cols)
+                 : "memory");
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -922,6 +1331,57 @@ int launch_persistent(int bn, const CUtensorMap* map_w, const CUtensorMap* map_a
   launch_kernel(kern, grid, NUM_THREADS, smem, stream, g, *map_w, *map_a, out, out_is_f32, n_tokens, n_features,
                 (K + BK - 1) / BK, ld_out, up_row_offset, f_tiles, t_tiles, ex, error_word);
   return launch_status();
+}
+
+// How a cluster product lays out a block: as many stages as let two blocks share an SM.
+static bool cluster_layout(int bn, int k_per_block, int& stages, size_t& smem) {
+  const size_t fixed = (size_t)(128 * bn + 8 * 8) * 4 + (size_t)(CL_EPI_WARPS + 1) * bn * 4 + (2 * MAX_STAGES + 2) * 8 + 16 + 1024;
+  const size_t stage = A_BYTES + (size_t)bn * BK * 2, budget = 112 * 1024;
+  stages = (int)((budget - fixed) / stage);
+  if (stages > k_per_block) stages = k_per_block;
+  if (stages > MAX_STAGES) stages = MAX_STAGES;
+  smem = fixed + stages * stage;
+  const size_t outgoing = (size_t)(128 * bn + 8 * 8) * 4;        // the outgoing slices lie in the stages
+  while (stages * stage < outgoing) ++stages;
+  smem = fixed + stages * stage;
+  return smem <= budget && (stages >= 2 || stages >= k_per_block);
+}
+
+template <int EPI, int C>
+int launch_cluster(const ClusterArgs& a, size_t smem, int tiles, const CUtensorMap& map_w, const CUtensorMap& map_a, cudaStream_t stream) {
+  auto kern = gemm_cluster_kernel<EPI, C>;
+  static size_t configured = 0;
+  if (smem > configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return launch_status();
+    configured = smem;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * C);
+  cfg.blockDim = dim3(CL_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, kern, a, map_w, map_a);
+  return launch_status();
+}
+
+template <int EPI>
+int launch_cluster_of(int cluster, const ClusterArgs& a, size_t smem, int tiles, const CUtensorMap& mw, const CUtensorMap& ma, cudaStream_t stream) {
+  switch (cluster) {
+    case 1: return launch_cluster<EPI, 1>(a, smem, tiles, mw, ma, stream);
+    case 2: return launch_cluster<EPI, 2>(a, smem, tiles, mw, ma, stream);
+    case 4: return launch_cluster<EPI, 4>(a, smem, tiles, mw, ma, stream);
+    case 8: return launch_cluster<EPI, 8>(a, smem, tiles, mw, ma, stream);
+  }
+  return ERR_BAD_SIZE;
 }
 
 }  // namespace
@@ -1066,4 +1526,71 @@ extern "C" int llm_gemm_bf16(const void* map_w, const void* map_a, void* out, in
   GEMM_CASE(1, 1);
   return ERR_BAD_SIZE;
 #undef GEMM_CASE
+}
+
+// The product of a few dozen tokens with its ends fused in (see gemm_cluster_kernel): `cluster` (1, 2, 4 or 8)
+// blocks share a tile of 128 weight rows.  map_w's box has 128 rows (64 for CL_SWIGLU), map_a's bn rows, bn the
+// tokens rounded up to a multiple of 16.  `pair_span` (CL_ROPE: head_dim / 2).  CL_ADD: out is the float32 residual
+// stream; pre_x, pre_w, pre_sq as for llm_gemm_bf16, with one row of parts per slice of 128 / cluster rows.
+extern "C" int llm_gemm_cluster(const void* map_w, const void* map_a, int epi, int cluster, int bn, int n_tokens, int n_features,
+                                int K, void* out, int out_dtype, long long ld_out, int up_row_offset, const float* sq_in,
+                                int sq_items, long long sq_stride, float norm_width, float eps, void* pre_x, long long pre_x_stride,
+                                const void* pre_w, int pre_w_dtype, float* pre_sq, long long pre_sq_stride, void* k_base,
+                                void* v_base, const int32_t* block_table, long long page_stride, int table_stride,
+                                int page_tokens, int kv_heads, int head_dim, const int32_t* positions, const int32_t* row_seq,
+                                const float* inv_freq, int q_heads, int write_cache, int* error_word, cudaStream_t stream) {
+  if (n_tokens <= 0 || n_features <= 0) return 0;
+  if (n_tokens > CL_MAX_TOKENS || bn < 16 || bn > CL_MAX_TOKENS || bn % 16 || n_tokens > bn || K <= 0 || n_features % 4) return ERR_BAD_SIZE;
+  if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ERR_BAD_SIZE;
+  if (out_dtype != DT_F32 && out_dtype != DT_BF16) return ERR_BAD_DTYPE;
+  if ((reinterpret_cast<uintptr_t>(out) & 15) || ld_out % 4) return ERR_BAD_ALIGN;
+  ClusterArgs a = {};
+  a.bn = bn, a.pair_span = 64 / cluster;
+  a.stage_bytes = A_BYTES + bn * BK * 2;
+  a.tmem_cols = 32;
+  while (a.tmem_cols < bn) a.tmem_cols *= 2;
+  a.idesc = instr_desc_bf16(BM, bn);
+  a.wait_ns = g_wait_ns;
+  a.k_blocks = (K + BK - 1) / BK;
+  a.k_per_block = (a.k_blocks + cluster - 1) / cluster;
+  size_t smem = 0;
+  if (!cluster_layout(bn, a.k_per_block, a.stages, smem)) return ERR_BAD_SIZE;
+  a.n_tokens = n_tokens, a.n_features = n_features, a.up_row_offset = up_row_offset;
+  if (sq_in) {
+    if (sq_items < 1 || sq_stride < n_tokens || !(norm_width > 0.0f)) return ERR_BAD_SIZE;
+    a.sq_in = sq_in, a.sq_items = sq_items, a.sq_stride = sq_stride, a.norm_width = norm_width, a.eps = eps;
+  }
+  a.out = out, a.out_is_f32 = out_dtype == DT_F32 ? 1 : 0, a.ld_out = ld_out;
+  a.error_word = error_word;
+  CUtensorMap mw, ma;
+  memcpy(&mw, map_w, sizeof(CUtensorMap));
+  memcpy(&ma, map_a, sizeof(CUtensorMap));
+  int rows = n_features;
+  switch (epi) {
+    case CL_STORE:
+      return launch_cluster_of<CL_STORE>(cluster, a, smem, (rows + BM - 1) / BM, mw, ma, stream);
+    case CL_ADD:
+      if (out_dtype != DT_F32) return ERR_BAD_DTYPE;
+      if (pre_x) {
+        if (!pre_w || !pre_sq || pre_sq_stride < n_tokens || pre_x_stride % 4) return ERR_BAD_SIZE;
+        if ((reinterpret_cast<uintptr_t>(pre_w) & 15) || (reinterpret_cast<uintptr_t>(pre_x) & 7)) return ERR_BAD_ALIGN;
+        if (pre_w_dtype != DT_F32 && pre_w_dtype != DT_BF16) return ERR_BAD_DTYPE;
+        a.pre_x = static_cast<__nv_bfloat16*>(pre_x), a.pre_x_stride = pre_x_stride, a.pre_w = pre_w;
+        a.pre_w_dtype = pre_w_dtype, a.pre_sq = pre_sq, a.pre_sq_stride = pre_sq_stride;
+      }
+      return launch_cluster_of<CL_ADD>(cluster, a, smem, (rows + BM - 1) / BM, mw, ma, stream);
+    case CL_SWIGLU:
+      if (up_row_offset < n_features) return ERR_BAD_SIZE;
+      a.pair_span = 64;
+      return launch_cluster_of<CL_SWIGLU>(cluster, a, smem, (rows + 63) / 64, mw, ma, stream);
+    case CL_ROPE:
+      if (out_dtype != DT_BF16 || head_dim < 8 || head_dim % 8 || 128 % head_dim || (q_heads + 2 * kv_heads) * head_dim != n_features)
+        return ERR_BAD_SIZE;
+      if ((reinterpret_cast<uintptr_t>(k_base) | reinterpret_cast<uintptr_t>(v_base)) & 7 || page_stride % 4) return ERR_BAD_ALIGN;
+      a.pair_span = head_dim / 2;
+      a.cache = PagedCache{k_base, v_base, block_table, page_stride, table_stride, page_tokens, kv_heads, head_dim};
+      a.positions = positions, a.row_seq = row_seq, a.inv_freq = inv_freq, a.q_heads = q_heads, a.write_cache = write_cache;
+      return launch_cluster_of<CL_ROPE>(cluster, a, smem, (rows + BM - 1) / BM, mw, ma, stream);
+  }
+  return ERR_BAD_SIZE;
 }

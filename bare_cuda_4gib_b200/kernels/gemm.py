@@ -12,7 +12,7 @@ import torch
 
 from ..errors import KernelLaunchError
 from . import build
-from .lib import DT_BF16, DT_F32, AddTo, glu_defines, LazyNorm, Partials, Prenormed, _check, _ptr, sm_count
+from .lib import DT_BF16, DT_F32, AddTo, glu_defines, LazyNorm, Partials, Prenormed, RotateAndCache, _check, _ptr, sm_count
 
 BM, BK = 128, 64
 SPLIT_MAX_ROWS = 256          # steps with more rows never split K
@@ -32,6 +32,9 @@ def lib(activation: str = "silu"):
         l.llm_gemm_bf16.restype = c_int
         l.llm_gemm_grouped_bf16.argtypes = [P, P, P, I, I, I, I, L, I, I, I, I, P, P, P, P, P, P]
         l.llm_gemm_grouped_bf16.restype = c_int
+        l.llm_gemm_cluster.argtypes = [P, P, I, I, I, I, I, I, P, I, L, I, P, I, L, F, F, P, L, P, I, P, L, P, P, P, L, I, I, I, I,
+                                       P, P, P, I, I, P, P]
+        l.llm_gemm_cluster.restype = c_int
         _lib = _libs[activation] = l
     return _lib
 
@@ -52,7 +55,7 @@ def check_errors() -> None:
             role = {1: "gemm TMA producer", 2: "gemm MMA issuer", 3: "gemm epilogue", 11: "attention loader",
                     12: "attention MMA issuer", 13: "attention softmax",
                     14: "attention (shared memory not 1024-byte aligned)", 21: "few-token product, producer",
-                    22: "few-token product, consumer", 31: "decode attention"}.get(code, f"code {code}")
+                    22: "few-token product, consumer", 4: "gemm cluster exchange", 31: "decode attention"}.get(code, f"code {code}")
             raise KernelLaunchError(f"a kernel gave up ({role}): a bounded wait ran out; the result is invalid")
 
 
@@ -268,3 +271,90 @@ def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
                            out.stride(-2), stride, splits, bn, 0, 0, 0, 0, *NO_EXTRA, err.data_ptr(), ctx.stream),
            "gemm_tcgen05")
     return Partials(out, splits)
+
+
+# ------------------------------------------------------------------ a few dozen tokens, ends fused in
+CL_STORE, CL_ADD, CL_SWIGLU, CL_ROPE = 0, 1, 2, 3
+# Measured, a whole step of TinyLlama's 22 layers, product + norm + rotation kernels against this: 25 rows 1,187 -> 989 us,
+# 32 rows 1,221 -> 1,011, 48 rows 1,338 -> 1,141, 64 rows 1,379 -> 1,245; with a tile of 96 or 128 tokens a block's shared
+# memory fills an SM and the step is slower (96 rows 1,513 -> 1,971, 128 rows 1,600 -> 3,084).
+CLUSTER_MAX_ROWS = 64
+# With so few rows that the few-token product (gemv.py) takes the layer's other products, what comes here is a down
+# projection whose input does not fit beside its ring.  A small one gains (12 rows x 2,048 x 5,632, 23 MB: the step 904 -> 873 us),
+# a large one is bound by its weights, which the split product's deeper ring streams faster (8 rows x 4,096 x 14,336, 117 MB:
+# 18.0 us and a norm kernel of 4.3 against 23.5).
+CLUSTER_FEW_ROWS, CLUSTER_FEW_BYTES = 24, 64 << 20
+
+
+def cluster_size(n_tiles: int, k: int) -> int:
+    """Blocks that share a tile's K range: as many (1, 2, 4, 8) as two blocks an SM and two 64-wide K blocks each allow."""
+    c = 8
+    while c > 1 and (n_tiles * c > 2 * sm_count() or -(-k // BK) < 2 * c):
+        c //= 2
+    return c
+
+
+def cluster_kind(plan: GemmPlan, rows: int, out_dtype, swiglu: bool, epilogue) -> Optional[int]:
+    """Which of the cluster product's ends a call asks for, None where the kernel does not take it."""
+    if not 0 < rows <= CLUSTER_MAX_ROWS or plan.n % 8 or (rows <= CLUSTER_FEW_ROWS and 2 * plan.n * plan.k > CLUSTER_FEW_BYTES):
+        return None
+    if swiglu:
+        return CL_SWIGLU
+    if isinstance(epilogue, AddTo):
+        r = epilogue.residual
+        fits = (r.dtype == torch.float32 and r.shape[-1] == plan.n and r.stride(-1) == 1 and r.stride(0) % 4 == 0
+                and r.data_ptr() % 16 == 0)
+        return CL_ADD if fits else None
+    if isinstance(epilogue, RotateAndCache):
+        c, q = epilogue.cache, epilogue.q_out
+        fits = (c.dtype == q.dtype == torch.bfloat16 and c.v_dim == c.head_dim and c.head_dim % 8 == 0 and 128 % c.head_dim == 0
+                and (epilogue.q_heads + 2 * c.kv_heads) * c.head_dim == plan.n and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0
+                and (c.k_ptr | c.v_ptr) % 8 == 0 and c.page_stride % 4 == 0)
+        return CL_ROPE if fits else None
+    return None
+
+
+def run_cluster(ctx, plan: GemmPlan, kind: int, a, rows: int, out_dtype: torch.dtype, buffer: str, epilogue=None,
+                activation: str = "silu") -> Optional[Partials]:
+    """The product with the end that `cluster_kind` named; None comes back where the epilogue consumed the result."""
+    extra_in = NO_EXTRA[:5]
+    if isinstance(a, LazyNorm):
+        pre = a.prenormed
+        if pre is None or a.row_index is not None:
+            a = a.materialize()
+        else:
+            extra_in = (pre.sq.data_ptr(), pre.items, pre.sq.stride(0), float(pre.x.shape[-1]), a.eps)
+            a = pre.x
+    ctx.prenormed = None
+    if a.dtype != torch.bfloat16 or a.stride(-1) != 1 or a.shape[-1] != plan.k or a.data_ptr() % 16 or a.stride(0) % 8:
+        raise KernelLaunchError(f"gemm_cluster: activations {tuple(a.shape)} {a.dtype} do not fit weight [{plan.n}, {plan.k}]")
+    n_out = plan.n // 2 if kind == CL_SWIGLU else plan.n
+    tiles = -(-n_out // (BM // 2 if kind == CL_SWIGLU else BM))
+    cluster = cluster_size(tiles, plan.k)
+    bn = -(-rows // 16) * 16
+    pre = None
+    extra_out, rope = (0, 0, 0, 0, 0, 0), (0, 0, 0, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0)
+    if kind == CL_ADD:
+        out = epilogue.residual
+        then = epilogue.then_norm
+        if then is not None and then.tensors["weight"].data_ptr() % 16 == 0 and then.tensors["weight"].dtype in (torch.float32, torch.bfloat16):
+            w, slices = then.tensors["weight"], tiles * cluster
+            pre_x = ctx.ws.get("prenormed.cluster.x", (rows, n_out), torch.bfloat16, max_rows=CLUSTER_MAX_ROWS)
+            pre_sq = ctx.ws.get("prenormed.cluster.sq", (slices, CLUSTER_MAX_ROWS), torch.float32, max_rows=slices)
+            extra_out = (pre_x.data_ptr(), pre_x.stride(0), w.data_ptr(), DT_BF16 if w.dtype == torch.bfloat16 else DT_F32,
+                         pre_sq.data_ptr(), pre_sq.stride(0))
+            pre = Prenormed(then, pre_x, pre_sq, slices)
+    elif kind == CL_ROPE:
+        c, out = epilogue.cache, epilogue.q_out
+        rope = (c.k_ptr, c.v_ptr, c.block_table.data_ptr(), c.page_stride, c.table_stride, c.page_tokens, c.kv_heads, c.head_dim,
+                epilogue.positions.data_ptr(), epilogue.row_seq.data_ptr(), _ptr(epilogue.inv_freq), epilogue.q_heads,
+                1 if epilogue.write_cache else 0)
+    else:
+        out = ctx.ws.get(buffer, (rows, n_out), out_dtype)
+    _check(lib(activation if kind == CL_SWIGLU else "silu").llm_gemm_cluster(
+        ctypes.addressof(plan.weight_map(BM // 2 if kind == CL_SWIGLU else BM)), ctypes.addressof(plan.act_map(a, bn)), kind,
+        cluster, bn, rows, n_out, plan.k, out.data_ptr(), DT_BF16 if out.dtype == torch.bfloat16 else DT_F32, out.stride(0),
+        n_out if kind == CL_SWIGLU else 0, *extra_in, *extra_out, *rope, error_word(a.device).data_ptr(), ctx.stream),
+        "gemm_cluster")
+    ctx.prenormed = pre
+    return None if kind in (CL_ADD, CL_ROPE) else Partials(out)

@@ -49,6 +49,9 @@ class Linear:
                 return gemv.run(ctx, self.weight, a, rows, out_dtype, buffer, swiglu, epilogue, activation)
         if self.fast is not None and ctx.use_fast_gemm:
             from ..kernels import gemm
+            kind = gemm.cluster_kind(self.fast, rows, out_dtype, swiglu, epilogue)
+            if kind is not None:
+                return gemm.run_cluster(ctx, self.fast, kind, a, rows, out_dtype, buffer, epilogue, activation)
             return gemm.run(ctx, self.fast, a, rows, out_dtype, buffer, allow_partials, swiglu, epilogue, activation)
         a = K.materialize(a)
         if swiglu:

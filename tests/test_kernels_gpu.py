@@ -375,6 +375,80 @@ def test_gemm_tcgen05_swiglu(m, inter, k):
     _close(res.tensor, want, 2 ** -7, 1e-3)
 
 
+@pytest.mark.parametrize("rows,n,k", [(1, 128, 64), (16, 136, 72), (17, 2048, 2048), (33, 2560, 200), (48, 320, 5632), (63, 1000, 1024),
+                                      (64, 2048, 5632), (8, 2048, 14336), (25, 72, 1088)])
+@pytest.mark.parametrize("prenormed", [False, True])
+def test_gemm_cluster_adds_prepares_and_gates(rows, n, k, prenormed):
+    """The product whose blocks exchange their parts through distributed shared memory: into the residual stream with the
+    next norm prepared, and gated, from a plain input and from one that a product before it prepared."""
+    from bare_cuda_4gib_b200.kernels import gemm
+    from bare_cuda_4gib_b200.kernels import lib as K
+    torch.manual_seed(rows + n)
+    ctx, eps = _ctx(), 1e-5
+    a = ctx.ws.get("a", (rows, k), torch.bfloat16)
+    a.copy_(torch.randn(rows, k, device=DEV))
+    x, xd = a, a.double()
+    if prenormed:
+        parts = torch.rand(5, rows + 3, device=DEV) * k
+        x = K.LazyNorm(ctx, None, None, eps, rows, None, "normed", K.Prenormed(None, a, parts, 5))
+        xd = xd * torch.rsqrt(parts[:, :rows].double().sum(0) / k + eps)[:, None]
+    w = (torch.randn(n, k, device=DEV) / math.sqrt(k)).to(torch.bfloat16)
+    plan, full = gemm.plan_for(w), xd @ w.double().t()
+    size = (xd.abs() @ w.double().abs().t()).max().item()
+    residual, norm = torch.randn(rows + 2, n, device=DEV), _RowNorm(1 + 0.3 * torch.randn(n, device=DEV), eps)
+    before = residual.double().clone()
+    kind = gemm.cluster_kind(plan, rows, torch.float32, False, K.AddTo(residual, norm))
+    assert kind == gemm.CL_ADD
+    assert gemm.run_cluster(ctx, plan, kind, x, rows, torch.float32, "out", K.AddTo(residual, norm)) is None
+    gemm.check_errors()
+    before[:rows] += full
+    _close(residual, before, 1e-5, 2 ** -20 * size)        # float32 sums in the tensor core: 2^-22 a step, a few steps deep
+    pre, now = ctx.prenormed, residual[:rows].double()
+    _close(pre.x[:rows].float(), now * norm.tensors["weight"].double(), 2 ** -8, 1e-6)
+    _close(pre.sq[: pre.items, :rows].double().sum(0), now.square().sum(-1), 1e-5, 1e-5)
+    inter = n // 2
+    if inter % 8 == 0:
+        kind = gemm.cluster_kind(plan, rows, torch.bfloat16, True, None)
+        got = gemm.run_cluster(ctx, plan, kind, x, rows, torch.bfloat16, "act").tensor
+        gemm.check_errors()
+        gate, up = full[:, :inter], full[:, inter:]
+        _close(got, gate / (1 + torch.exp(-gate)) * up, 2 ** -8, 1e-4 + 2 ** -18 * size)
+
+
+@pytest.mark.parametrize("rows,heads,kv_heads,d,rotate", [(25, 8, 2, 64, True), (64, 3, 1, 128, True), (40, 5, 2, 32, True), (33, 2, 1, 8, False)])
+def test_gemm_cluster_rotates_and_writes_the_cache(rows, heads, kv_heads, d, rotate):
+    from bare_cuda_4gib_b200.kernels import gemm
+    from bare_cuda_4gib_b200.kernels import lib as K
+    torch.manual_seed(rows + d)
+    ctx, k = _ctx(), 320
+    a = ctx.ws.get("a", (rows, k), torch.bfloat16)
+    a.copy_(torch.randn(rows, k, device=DEV))
+    n = (heads + 2 * kv_heads) * d
+    w = (torch.randn(n, k, device=DEV) / math.sqrt(k)).to(torch.bfloat16)
+    page, storage = 16, None
+    storage, table, view = _paged_cache(kv_heads, d, page, 24, torch.bfloat16)
+    table[0, :6] = torch.randperm(24, device=DEV)[:6].int()
+    seq = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    pos = torch.arange(7, 7 + rows, dtype=torch.int32, device=DEV)
+    inv = 1.0 / 10000.0 ** (torch.arange(d // 2, device=DEV).float() * 2 / d) if rotate else None
+    q = torch.full((rows, heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+    end = K.RotateAndCache(q, view, pos, seq, inv, heads, True)
+    plan = gemm.plan_for(w)
+    kind = gemm.cluster_kind(plan, rows, torch.float32, False, end)
+    assert kind == gemm.CL_ROPE
+    assert gemm.run_cluster(ctx, plan, kind, a, rows, torch.float32, "qkv", end) is None
+    gemm.check_errors()
+    full = (a.double() @ w.double().t()).view(rows, heads + 2 * kv_heads, d)
+    turned = _rope_ref(full[:, : heads + kv_heads], pos, inv) if rotate else full[:, : heads + kv_heads]
+    _close(q.float().view(rows, heads, d), turned[:, :heads], 2 ** -8, 1e-3)
+    pages = storage.view(24, 2, kv_heads, page, d)
+    for t in range(rows):
+        p = int(pos[t])
+        held = pages[int(table[0, p // page]), :, :, p % page].float()
+        _close(held[0], turned[t, heads:], 2 ** -8, 1e-3)
+        _close(held[1], full[t, heads + kv_heads:], 2 ** -8, 1e-3)
+
+
 def test_a_bounded_wait_runs_out_and_the_kernel_returns():
     """Every wait inside the pipelined kernels has a limit.  Here one is seen to run out: with the
     test hooks of the GEMM library the producer arms one stage's barrier and issues no copy for it,
