@@ -10,7 +10,7 @@ import ctypes
 import math
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
-from typing import Dict, Optional
+from typing import Dict, Optional, Tuple
 
 import numpy as np
 import torch
@@ -23,8 +23,14 @@ KEY_BLOCK = 64
 COUNTER_WORDS = 4096          # per-tile split counters at the start of the scratch (see the kernel)
 _libs: Dict[int, object] = {}
 _tc_libs: Dict[int, object] = {}
-_decode_libs: Dict[int, object] = {}
+_decode_libs: Dict[Tuple[int, bool], object] = {}
 TC_HEAD_DIMS = (64, 128)      # head sizes the tcgen05 prefill kernel and the decode kernel are built for
+HALF_KEY_BLOCKS = ("-DDECODE_KEY_BLOCK=32",)
+# At head size 64 a step with many tiles takes twice the blocks with key blocks of half the size: a block needs 40 KB instead of
+# 73, so five share an SM, and a long request's keys are on twice as many warps.  A decode step of TinyLlama's 22 layers at
+# 2,000 positions (500 to 2,000): batch 64 1,701 -> 1,638 us (1,631 -> 1,556), batch 32 1,219 -> 1,185 (1,189 -> 1,146); at
+# batch 16 (8 blocks a tile then) it is slower (400 positions: 874 -> 944 us).
+HALF_BLOCKS_MAX_SPLITS = 4
 DECODE_MAX_TILES = 65535 // 4 # (tiles x kv heads) up to which the cluster decode kernel runs
 
 
@@ -82,11 +88,11 @@ def tc_lib(head_dim: int):
     return l
 
 
-def decode_lib(head_dim: int):
-    """The cluster decode kernel's library for this head size."""
-    l = _decode_libs.get(head_dim)
+def decode_lib(head_dim: int, half_blocks: bool = False):
+    """The cluster decode kernel's library for this head size; `half_blocks`: with key blocks of 32 positions at head size 64."""
+    l = _decode_libs.get((head_dim, half_blocks))
     if l is None:
-        l = build.load_library("attention_decode.cu", defines(head_dim))
+        l = build.load_library("attention_decode.cu", defines(head_dim) + (HALF_KEY_BLOCKS if half_blocks else ()))
         P, I, L, F = c_void_p, c_int, c_longlong, c_float
         l.llm_attention_decode.argtypes = [P, P, L, I, P, P, P, P, P, L, I, I, I, I, P, P, P, P, P, I, I, I, I, F, I, I, P, P, L,
                                            P, P]
@@ -95,7 +101,7 @@ def decode_lib(head_dim: int):
         l.llm_attention_decode_pool_map.restype = c_int
         l.llm_attention_decode_key_block.restype = c_int
         l.key_block = int(l.llm_attention_decode_key_block())
-        _decode_libs[head_dim] = l
+        _decode_libs[head_dim, half_blocks] = l
     return l
 
 
@@ -121,10 +127,11 @@ class AttentionPlan:
         if head_dim in TC_HEAD_DIMS and not distance_bias and not self.general:
             self.tc = tc_lib(head_dim)
             self.prefill_rows = int(self.tc.llm_attention_tc_rows())
-        self.decode = None
+        self.decode = self.decode_half = None
         if head_dim in TC_HEAD_DIMS and not distance_bias and not self.general \
                 and not os.environ.get("BARE_CUDA_B200_NO_DECODE_ATTENTION"):
             self.decode = decode_lib(head_dim)
+            self.decode_half = decode_lib(head_dim, True) if head_dim == 64 else None
         self._host = None
         self._dev = None
         self._scratch = None
@@ -141,14 +148,14 @@ class AttentionPlan:
             n = min(n, self.chunk // block if whole else -(-(self.chunk + q_len - 2) // block) + 1)
         return n
 
-    def decode_map(self, cache: CacheView):
-        """The decode kernel's tensor map over a cache group's pool (boxes of at most 64 rows)."""
-        box_rows = math.gcd(self.decode.key_block, cache.page_tokens)
+    def decode_map(self, cache: CacheView, library):
+        """The decode kernel's tensor map over a cache group's pool (boxes of at most a key block)."""
+        box_rows = math.gcd(library.key_block, cache.page_tokens)
         key = (cache.pool_ptr, cache.pool_elems, box_rows)
         m = self._decode_maps.get(key)
         if m is None:
             m = (ctypes.c_ubyte * 128)()
-            _check(self.decode.llm_attention_decode_pool_map(ctypes.addressof(m), cache.pool_ptr,
+            _check(library.llm_attention_decode_pool_map(ctypes.addressof(m), cache.pool_ptr,
                                                              cache.pool_elems // self.head_dim, box_rows),
                    "attention decode pool map")
             self._decode_maps[key] = m
@@ -251,7 +258,7 @@ def step_tiles(ctx, plan: AttentionPlan):
             n_splits = min(key_blocks, int(os.environ["BARE_CUDA_B200_ATTN_SPLITS"]))
         if n_tiles * plan.kv_heads > COUNTER_WORDS:
             n_splits = 1
-    dec_splits = dec_slots = 0
+    dec_splits = dec_slots = half = 0
     if use_decode:
         # The cluster decode kernel: up to 8 blocks of 4 warps share a tile, a warp keeps one key
         # block in flight.  Measured at a context of 2,048 (batches 8 to 64): the kernel is fastest
@@ -268,7 +275,9 @@ def step_tiles(ctx, plan: AttentionPlan):
         dec_slots = 1
         if os.environ.get("BARE_CUDA_B200_ATTN_SPLITS"):     # experiments only
             dec_splits = max(1, min(8, int(os.environ["BARE_CUDA_B200_ATTN_SPLITS"])))
-    out = (dev[:n_tiles], dev[n_tiles: 2 * n_tiles], n_tiles, rows_per_tile, n_splits, dec_splits, dec_slots)
+        elif plan.decode_half is not None and 2 * dec_splits <= HALF_BLOCKS_MAX_SPLITS and 4 * dec_splits < most:
+            half, dec_splits = 1, 2 * dec_splits
+    out = (dev[:n_tiles], dev[n_tiles: 2 * n_tiles], n_tiles, rows_per_tile, n_splits, dec_splits, dec_slots, half)
     ctx.extras[key] = out
     return out
 
@@ -288,7 +297,7 @@ def run(ctx, plan: AttentionPlan, q: torch.Tensor, out: torch.Tensor, cache: Cac
     more = (extras or AttentionExtras()).arguments(plan.heads, q.dtype)
     if plan.distance_bias and extras:
         raise KernelLaunchError("attention_mma (distance bias): the variant takes no blocks of positions, sink or gate")
-    tile_seq, tile_index, n_tiles, rows_per_tile, n_splits, dec_splits, dec_slots = step_tiles(ctx, plan)
+    tile_seq, tile_index, n_tiles, rows_per_tile, n_splits, dec_splits, dec_slots, half = step_tiles(ctx, plan)
     if plan.distance_bias:
         scratch_ptr = 0
         if n_splits > 1:
@@ -303,8 +312,9 @@ def run(ctx, plan: AttentionPlan, q: torch.Tensor, out: torch.Tensor, cache: Cac
         return
     if dec_splits and plan.decode_usable(cache):
         from . import gemm
-        pool_map, box_rows = plan.decode_map(cache)
-        _check(plan.decode.llm_attention_decode(
+        library = plan.decode_half if half else plan.decode
+        pool_map, box_rows = plan.decode_map(cache, library)
+        _check(library.llm_attention_decode(
             ctypes.addressof(pool_map), cache.pool_ptr, cache.pool_elems // plan.head_dim, box_rows, q.data_ptr(),
             out.data_ptr(), cache.k_ptr, cache.v_ptr, cache.block_table.data_ptr(), cache.page_stride,
             cache.table_stride, cache.page_tokens, cache.kv_heads, cache.head_dim, ctx.seq_q_start.data_ptr(),

@@ -25,5 +25,6 @@ def all_libraries():
     jobs += [("attention_f32.cu", (f"-DHEAD_DIM={d}",)) for d in ATTENTION_F32_HEAD_DIMS]
     jobs += [("attention_tcgen05.cu", (f"-DHEAD_DIM={d}",)) for d in (64, 128)]
     jobs += [("attention_decode.cu", (f"-DHEAD_DIM={d}",)) for d in (64, 128)]
+    jobs += [("attention_decode.cu", ("-DHEAD_DIM=64", "-DDECODE_KEY_BLOCK=32"))]
     jobs += [("diff_attention.cu", (f"-DDA_DQ={d}", f"-DDA_DV={v}")) for d, v in DIFF_ATTENTION_SIZES]
     return jobs

@@ -776,6 +776,19 @@ def test_attention_decode_cluster(heads, kv_heads, d, page, splits, monkeypatch)
     _close(got, want, 2 ** -7, 4e-3)
 
 
+@pytest.mark.parametrize("heads,kv_heads,page,window,count", [(32, 4, 64, 0, 40), (8, 4, 16, 0, 75), (16, 8, 32, 100, 20), (4, 4, 8, 0, 160)])
+def test_attention_decode_half_key_blocks(heads, kv_heads, page, window, count):
+    """Steps with many tiles take key blocks of 32 positions: lengths around their edges, and few tokens beside single ones."""
+    from bare_cuda_4gib_b200.kernels import attention as fast
+    lens = [1, 31, 32, 33, 63, 64, 65, 129, 500, 900]
+    most = 16 // (heads // kv_heads)
+    seqs = [(min(1 + i % most, lens[i % 10]), lens[i % 10]) for i in range(count)]
+    got, want, ctx = _attention_case(seqs, heads, kv_heads, 64, page, window, 11)
+    tiles = [v for k, v in ctx.extras.items() if isinstance(k, tuple) and k[0] == "attention_tiles"]
+    assert tiles[0][7] == 1 and tiles[0][5] <= fast.HALF_BLOCKS_MAX_SPLITS
+    _close(got, want, 2 ** -7, 1e-2)
+
+
 def test_attention_decode_two_tokens_window_and_far_key(monkeypatch):
     # two tokens per request still fit the 16 packed rows of a tile when the group has at most 8 heads
     got, want, ctx = _attention_case([(2, 300), (2, 2), (1, 77), (2, 1030)], 16, 2, 64, 16, 0, seed=11)
