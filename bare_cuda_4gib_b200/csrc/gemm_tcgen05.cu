@@ -24,6 +24,7 @@
 // gate in lanes 0..63 and up in lanes 64..127; the two epilogue warps that own the up lanes hand
 // their values over through shared memory.  ORIENT 1 loads BN/2 gate rows and the matching BN/2
 // up rows as one N operand, so a thread finds gate in column c and up in column BN/2 + c.
+// MODE 2 (ORIENT 1): w is [Wq; Wk; Wv] and the epilogue turns heads and writes the cache (see HeadsExtra).
 //
 // Warps: 0 = TMA producer, 1 = tensor memory allocation + MMA issue, 2..5 = epilogue.
 // Every wait on an mbarrier is bounded: after about a second without progress the thread sets
@@ -175,6 +176,18 @@ struct RowsExtra {
   const float* row_weight;
 };
 
+// What the epilogue of a [q; k; v] product needs (MODE 2; `out` is q, bfloat16): q and k heads turned by `turn`
+// [dim / 2][stride] (cosine, sine) pairs, k and v into the paged cache.  Tiles hold whole heads, and a half head is a
+// multiple of 16.  `turn` null: q and k are not turned.
+struct HeadsExtra {
+  int dim, q_heads, write_cache;
+  const float2* turn;
+  long long stride;             // tokens lie next to one another: a warp's lanes are tokens
+  PagedCache cache;
+  const int32_t* positions;
+  const int32_t* row_seq;
+};
+
 constexpr int STAGING_BYTES = 4 * 32 * 32 * 4;   // per epilogue warp 32 rows of 32 float32, for the adding epilogue
 
 // The factor of the norm that the input rows were prepared for (1 without one).
@@ -195,7 +208,7 @@ template <int MODE, int DEPTH, typename Wait>
 __device__ __forceinline__ void epilogue_tokens_on_rows(uint32_t lane_base, int BN, int F_TILE, int f0, int f_tile_index,
                                                         int t_first, int lane, bool have_acc, void* out, int out_is_f32,
                                                         long long ld_out, int n_tokens, int n_features,
-                                                        const RowsExtra& ex, float* staging, Wait&& wait_acc) {
+                                                        const RowsExtra& ex, const HeadsExtra& hx, float* staging, Wait&& wait_acc) {
   float* out_f32 = reinterpret_cast<float*>(out);
   __nv_bfloat16* out_bf16 = reinterpret_cast<__nv_bfloat16*>(out);
   if (MODE == 0 && out_is_f32 == 2 && ex.pre_x) {
@@ -302,6 +315,66 @@ __device__ __forceinline__ void epilogue_tokens_on_rows(uint32_t lane_base, int 
     if (ex.row_weight) rs *= ex.row_weight[t_out];
   }
   if (!wait_acc()) return;
+  if (MODE == 2) {
+    // ---- heads turned and put where attention reads them: a thread has a token's whole heads in its row of the
+    // accumulator, so both halves of a pair meet here.  The angles' cosines and sines come from a table that the step
+    // makes once for all its layers (precise sincosf: too much to repeat for every head).
+    const int half = hx.dim / 2;
+    const bool live = t < n_tokens;
+    const int seq = live ? hx.row_seq[t] : 0, pos = live ? hx.positions[t] : 0;
+#pragma unroll 1
+    for (int h0 = 0; h0 < F_TILE; h0 += hx.dim) {
+      if (f0 + h0 >= n_features) break;   // uniform across the block
+      const int head = (f0 + h0) / hx.dim;
+      const bool is_q = head < hx.q_heads, is_v = head >= hx.q_heads + hx.cache.kv_heads;
+      __nv_bfloat16* dst = nullptr;
+      if (live && is_q) {
+        dst = out_bf16 + (long long)t * ld_out + (long long)head * hx.dim;
+      } else if (live && hx.write_cache) {
+        const long long at = cache_offset(hx.cache, seq, pos, head - hx.q_heads - (is_v ? hx.cache.kv_heads : 0));
+        if (at >= 0) dst = static_cast<__nv_bfloat16*>(is_v ? hx.cache.v : hx.cache.k) + at;
+      }
+#pragma unroll 1
+      for (int p0 = 0; p0 < half; p0 += 16) {
+        float2 cs[16];
+        const bool turned = dst && !is_v && hx.turn;
+        if (turned)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) cs[j] = hx.turn[(p0 + j) * hx.stride + t];
+        uint32_t g[16], u[16];
+        if (have_acc) {
+          tmem_load16(lane_base + h0 + p0, g);
+          tmem_load16(lane_base + h0 + half + p0, u);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) g[j] = u[j] = 0u;
+        }
+        if (!dst) continue;
+        uint32_t lo[8], hi[8];
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          float a0 = __uint_as_float(g[j]) * rs, b0 = __uint_as_float(u[j]) * rs;
+          float a1 = __uint_as_float(g[j + 1]) * rs, b1 = __uint_as_float(u[j + 1]) * rs;
+          if (turned) {
+            const float x0 = a0, y0 = b0, x1 = a1, y1 = b1;
+            a0 = x0 * cs[j].x - y0 * cs[j].y, b0 = y0 * cs[j].x + x0 * cs[j].y;
+            a1 = x1 * cs[j + 1].x - y1 * cs[j + 1].y, b1 = y1 * cs[j + 1].x + x1 * cs[j + 1].y;
+          }
+          const __nv_bfloat162 l2 = __floats2bfloat162_rn(a0, a1), h2 = __floats2bfloat162_rn(b0, b1);
+          lo[j / 2] = *reinterpret_cast<const uint32_t*>(&l2);
+          hi[j / 2] = *reinterpret_cast<const uint32_t*>(&h2);
+        }
+        uint4* to = reinterpret_cast<uint4*>(dst + p0);
+        to[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        to[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+        to = reinterpret_cast<uint4*>(dst + half + p0);
+        to[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        to[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+      }
+    }
+    return;
+  }
   const bool vec_ok = out_is_f32 ? (ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out_f32) & 15) == 0)
                                  : (ld_out % 8 == 0 && (reinterpret_cast<uintptr_t>(out_bf16) & 15) == 0);
 #pragma unroll 1
@@ -429,7 +502,7 @@ __global__ void __launch_bounds__(NUM_THREADS, BLOCKS_PER_SM)
 gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                     void* __restrict__ out, int out_is_f32, int n_tokens, int n_features, int k_blocks,
                     int k_blocks_per_split, long long ld_out, long long partial_stride, int up_row_offset,
-                    const RowsExtra ex, int* __restrict__ error_word) {
+                    const RowsExtra ex, const HeadsExtra hx, int* __restrict__ error_word) {
   const int BN = geo.bn;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -598,7 +671,7 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
       epilogue_tokens_on_rows<MODE, BLOCKS_PER_SM == 1 ? 4 : 1>(
           lane_base, BN, F_TILE, f0, blockIdx.x, t0 + quad * 32, lane, n_kb > 0,
           out_is_f32 ? static_cast<void*>(out_f32) : static_cast<void*>(out_bf16), out_is_f32, ld_out, n_tokens, n_features,
-          ex, reinterpret_cast<float*>(smem) + quad * (32 * 32), wait_acc);
+          ex, hx, reinterpret_cast<float*>(smem) + quad * (32 * 32), wait_acc);
     } else if (wait_acc()) {
       if (ORIENT == 0 && MODE == 1) {
         // lanes 0..63 hold gate, lanes 64..127 up, for the block's 64 output features: the up warps
@@ -697,7 +770,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_w,
                                const __grid_constant__ CUtensorMap map_a, void* __restrict__ out, int out_is_f32,
                                int n_tokens, int n_features, int n_kb, long long ld_out, int up_row_offset,
-                               int f_tiles, int t_tiles, const RowsExtra ex, int* __restrict__ error_word) {
+                               int f_tiles, int t_tiles, const RowsExtra ex, const HeadsExtra hx, int* __restrict__ error_word) {
   const int BN = geo.bn;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -841,7 +914,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
       };
       const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * ACC_COLS;
       epilogue_tokens_on_rows<MODE, 2>(lane_base, BN, F_TILE, f0, tile / t_tiles, t0 + quad * 32, lane, n_kb > 0, out, out_is_f32,
-                                       ld_out, n_tokens, n_features, ex,
+                                       ld_out, n_tokens, n_features, ex, hx,
                                        reinterpret_cast<float*>(smem + geo.stages * geo.stage_bytes + 256) + quad * (32 * 32),
                                        wait_acc);
       if (!ok) break;
@@ -1288,7 +1361,7 @@ EncodeTiledFn encode_tiled_fn() {
 template <int MODE, int ORIENT, int BLOCKS_PER_SM>
 int launch(int bn, const CUtensorMap* map_w, const CUtensorMap* map_a, void* out, int out_is_f32, int n_tokens,
            int n_features, int K, long long ld_out, long long partial_stride, int splits, int up_row_offset,
-           const RowsExtra& ex, int* error_word, cudaStream_t stream) {
+           const RowsExtra& ex, const HeadsExtra& hx, int* error_word, cudaStream_t stream) {
   const Geometry g = make_geometry(bn, MODE, ORIENT, BLOCKS_PER_SM);
   if (g.stages < 1 || g.tmem_cols * BLOCKS_PER_SM > 512) return ERR_BAD_SIZE;
   auto kern = gemm_tcgen05_kernel<MODE, ORIENT, BLOCKS_PER_SM>;
@@ -1306,13 +1379,13 @@ int launch(int bn, const CUtensorMap* map_w, const CUtensorMap* map_a, void* out
   dim3 grid((n_features + f_tile - 1) / f_tile, (n_tokens + t_tile - 1) / t_tile, splits);
   if (grid.y > 65535 || grid.z > 65535) return ERR_BAD_SIZE;
   launch_kernel(kern, grid, NUM_THREADS, smem, stream, g, *map_w, *map_a, out, out_is_f32, n_tokens, n_features,
-                k_blocks, per_split, ld_out, partial_stride, up_row_offset, ex, error_word);
+                k_blocks, per_split, ld_out, partial_stride, up_row_offset, ex, hx, error_word);
   return launch_status();
 }
 
 template <int MODE>
 int launch_persistent(int bn, const CUtensorMap* map_w, const CUtensorMap* map_a, void* out, int out_is_f32, int n_tokens,
-                      int n_features, int K, long long ld_out, int up_row_offset, const RowsExtra& ex, int* error_word,
+                      int n_features, int K, long long ld_out, int up_row_offset, const RowsExtra& ex, const HeadsExtra& hx, int* error_word,
                       cudaStream_t stream) {
   const Geometry g = make_geometry(bn, MODE, 1, 1);
   if (g.stages < 2 || g.tmem_cols > ACC_COLS) return ERR_BAD_SIZE;
@@ -1329,7 +1402,7 @@ int launch_persistent(int bn, const CUtensorMap* map_w, const CUtensorMap* map_a
   const long long tiles = (long long)f_tiles * t_tiles;
   const int grid = tiles < sm_count() ? (int)tiles : sm_count();
   launch_kernel(kern, grid, NUM_THREADS, smem, stream, g, *map_w, *map_a, out, out_is_f32, n_tokens, n_features,
-                (K + BK - 1) / BK, ld_out, up_row_offset, f_tiles, t_tiles, ex, error_word);
+                (K + BK - 1) / BK, ld_out, up_row_offset, f_tiles, t_tiles, ex, hx, error_word);
   return launch_status();
 }
 
@@ -1425,6 +1498,7 @@ extern "C" int llm_gemm_grouped_bf16(const void* map_w, const void* map_a, void*
   memcpy(&mw, map_w, sizeof(CUtensorMap));
   memcpy(&ma, map_a, sizeof(CUtensorMap));
   RowsExtra ex = {};
+  const HeadsExtra hx = {};
   ex.group_tiles = tiles, ex.group_n_tiles = n_tiles, ex.group_w_rows = group_w_rows;
   ex.row_map = row_map, ex.row_weight = row_weight;
   const int f32 = out_dtype == DT_F32 ? 1 : 0;
@@ -1436,9 +1510,9 @@ extern "C" int llm_gemm_grouped_bf16(const void* map_w, const void* map_a, void*
 #define GROUPED_CASE(MODE_)                                                                                           \
   if (mode == MODE_)                                                                                                  \
     return pair ? launch<MODE_, 1, 2>(bn, &mw, &ma, out, f32, rows_bound, n_features, K, ld_out, 0, 1, up_row_offset, \
-                                      ex, error_word, stream)                                                         \
+                                      ex, hx, error_word, stream)                                                         \
                 : launch<MODE_, 1, 1>(bn, &mw, &ma, out, f32, rows_bound, n_features, K, ld_out, 0, 1, up_row_offset, \
-                                      ex, error_word, stream)
+                                      ex, hx, error_word, stream)
   GROUPED_CASE(0);
   GROUPED_CASE(1);
   return ERR_BAD_SIZE;
@@ -1467,12 +1541,12 @@ extern "C" void llm_gemm_test_hooks(long long wait_ns, int drop_k_block) {
 // factor per row, 1 / sqrt(sum of the parts / norm_width + eps), is applied to the sums;
 // `pre_x` (with accumulate): the kernel also writes pre_x[t, f] = bfloat16(out[t, f] * pre_w[f]) and
 // pre_sq[feature tile][t] = that tile's part of the row's sum of squares (ceil(n_features / bn) tiles).
-extern "C" int llm_gemm_bf16(const void* map_w, const void* map_a, void* out, int out_dtype, int n_tokens,
-                             int n_features, int K, long long ld_out, long long partial_stride, int splits,
-                             int bn, int mode, int orient, int up_row_offset, int accumulate, const float* sq_in,
-                             int sq_items, long long sq_stride, float norm_width, float eps, void* pre_x,
-                             long long pre_x_stride, const void* pre_w, int pre_w_dtype, float* pre_sq,
-                             long long pre_sq_stride, int* error_word, cudaStream_t stream) {
+static int gemm_bf16(const void* map_w, const void* map_a, void* out, int out_dtype, int n_tokens,
+                     int n_features, int K, long long ld_out, long long partial_stride, int splits,
+                     int bn, int mode, int orient, int up_row_offset, int accumulate, const float* sq_in,
+                     int sq_items, long long sq_stride, float norm_width, float eps, void* pre_x,
+                     long long pre_x_stride, const void* pre_w, int pre_w_dtype, float* pre_sq,
+                     long long pre_sq_stride, const HeadsExtra& hx, int* error_word, cudaStream_t stream) {
   if (n_tokens <= 0 || n_features <= 0) return 0;
   if (K <= 0 || splits <= 0 || (mode == 1 && splits != 1)) return ERR_BAD_SIZE;
   if (splits > 1 && out_dtype != DT_F32) return ERR_BAD_DTYPE;
@@ -1511,21 +1585,78 @@ extern "C" int llm_gemm_bf16(const void* map_w, const void* map_a, void* out, in
     // wide tiles: a stage of a narrow tile is shorter on the tensor core than the one issuing
     // thread's round of waiting for it, issuing its instructions and committing, and then two
     // blocks per SM with an issuing thread each are faster.
-    if (mode == 0) return launch_persistent<0>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, error_word, stream);
-    return launch_persistent<1>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, error_word, stream);
+    if (hx.dim) return launch_persistent<2>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, hx, error_word, stream);
+    if (mode == 0) return launch_persistent<0>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, hx, error_word, stream);
+    return launch_persistent<1>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, hx, error_word, stream);
   }
 #define GEMM_CASE(MODE_, ORIENT_)                                                                            \
   if (mode == MODE_ && orient == ORIENT_)                                                                    \
     return pair ? launch<MODE_, ORIENT_, 2>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out,           \
-                                            partial_stride, splits, up_row_offset, ex, error_word, stream)  \
+                                            partial_stride, splits, up_row_offset, ex, hx, error_word, stream)  \
                 : launch<MODE_, ORIENT_, 1>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out,           \
-                                            partial_stride, splits, up_row_offset, ex, error_word, stream)
+                                            partial_stride, splits, up_row_offset, ex, hx, error_word, stream)
+  if (hx.dim)
+    return pair ? launch<2, 1, 2>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, 0, 1, 0, ex, hx, error_word, stream)
+                : launch<2, 1, 1>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, 0, 1, 0, ex, hx, error_word, stream);
   GEMM_CASE(0, 0);
   GEMM_CASE(1, 0);
   GEMM_CASE(0, 1);
   GEMM_CASE(1, 1);
   return ERR_BAD_SIZE;
 #undef GEMM_CASE
+}
+
+extern "C" int llm_gemm_bf16(const void* map_w, const void* map_a, void* out, int out_dtype, int n_tokens,
+                             int n_features, int K, long long ld_out, long long partial_stride, int splits,
+                             int bn, int mode, int orient, int up_row_offset, int accumulate, const float* sq_in,
+                             int sq_items, long long sq_stride, float norm_width, float eps, void* pre_x,
+                             long long pre_x_stride, const void* pre_w, int pre_w_dtype, float* pre_sq,
+                             long long pre_sq_stride, int* error_word, cudaStream_t stream) {
+  return gemm_bf16(map_w, map_a, out, out_dtype, n_tokens, n_features, K, ld_out, partial_stride, splits, bn, mode, orient,
+                   up_row_offset, accumulate, sq_in, sq_items, sq_stride, norm_width, eps, pre_x, pre_x_stride, pre_w,
+                   pre_w_dtype, pre_sq, pre_sq_stride, HeadsExtra{}, error_word, stream);
+}
+
+// The [q; k; v] product of many tokens (orient 1, no split) whose epilogue turns q and k heads by `turn`
+// [head_dim / 2][turn_stride] (cosine, sine; null: not at all), writes q to `q_out` [token][q_stride] and k and v into the paged
+// cache.  bn is a multiple of head_dim, head_dim of 32.
+extern "C" int llm_gemm_qkv(const void* map_w, const void* map_a, void* q_out, int n_tokens, int K, long long q_stride, int bn,
+                            const float* sq_in, int sq_items, long long sq_stride, float norm_width, float eps, const float* turn,
+                            long long turn_stride, void* k_base, void* v_base, const int32_t* block_table, long long page_stride, int table_stride,
+                            int page_tokens, int kv_heads, int head_dim, const int32_t* positions, const int32_t* row_seq,
+                            int q_heads, int write_cache, int* error_word, cudaStream_t stream) {
+  if (head_dim < 32 || head_dim % 32 || bn % head_dim || (turn && turn_stride < n_tokens) || q_stride % 8 || page_stride % 8) return ERR_BAD_SIZE;
+  if ((reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_base) | reinterpret_cast<uintptr_t>(v_base) |
+       reinterpret_cast<uintptr_t>(turn)) & 15)
+    return ERR_BAD_ALIGN;
+  HeadsExtra hx = {};
+  hx.dim = head_dim, hx.q_heads = q_heads, hx.write_cache = write_cache, hx.turn = reinterpret_cast<const float2*>(turn);
+  hx.stride = turn_stride;
+  hx.cache = PagedCache{k_base, v_base, block_table, page_stride, table_stride, page_tokens, kv_heads, head_dim};
+  hx.positions = positions, hx.row_seq = row_seq;
+  return gemm_bf16(map_w, map_a, q_out, DT_BF16, n_tokens, (q_heads + 2 * kv_heads) * head_dim, K, q_stride, 0, 1, bn, 0, 1, 0, 0,
+                   sq_in, sq_items, sq_stride, norm_width, eps, nullptr, 0, nullptr, DT_F32, nullptr, 0, hx, error_word, stream);
+}
+
+// turn[p][t] = (cosine, sine) of positions[t] * inv_freq[p], a float32 product and the precise functions.
+__global__ void turn_table_kernel(const int32_t* __restrict__ positions, const float* __restrict__ inv_freq, float2* __restrict__ turn,
+                                  long long stride, int n_tokens) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.y;
+  if (t >= n_tokens) return;
+  float2 v;
+  sincosf((float)positions[t] * inv_freq[p], &v.y, &v.x);
+  turn[p * stride + t] = v;
+}
+
+extern "C" int llm_turn_table(const int32_t* positions, const float* inv_freq, float* turn, long long stride, int n_tokens, int half,
+                              cudaStream_t stream) {
+  if (n_tokens <= 0) return 0;
+  if (half <= 0 || half > 65535 || stride < n_tokens) return ERR_BAD_SIZE;
+  launch_kernel(turn_table_kernel, dim3((n_tokens + 255) / 256, half), 256, 0, stream, positions, inv_freq,
+                reinterpret_cast<float2*>(turn), stride, n_tokens);
+  return launch_status();
 }
 
 // The product of a few dozen tokens with its ends fused in (see gemm_cluster_kernel): `cluster` (1, 2, 4 or 8)

@@ -35,6 +35,10 @@ def lib(activation: str = "silu"):
         l.llm_gemm_cluster.argtypes = [P, P, I, I, I, I, I, I, P, I, L, I, P, I, L, F, F, P, L, P, I, P, L, P, P, P, L, I, I, I, I,
                                        P, P, P, I, I, P, P]
         l.llm_gemm_cluster.restype = c_int
+        l.llm_gemm_qkv.argtypes = [P, P, P, I, I, L, I, P, I, L, F, F, P, L, P, P, P, L, I, I, I, I, P, P, I, I, P, P]
+        l.llm_gemm_qkv.restype = c_int
+        l.llm_turn_table.argtypes = [P, P, P, L, I, I, P]
+        l.llm_turn_table.restype = c_int
         _lib = _libs[activation] = l
     return _lib
 
@@ -149,28 +153,41 @@ TOKENS_ON_ROWS_ABOVE = 240    # steps with more rows put 128 tokens on the MMA r
 SWIGLU_TOKENS_ON_ROWS_ABOVE = 60
 
 
-def feature_tile(rows: int, n_out: int, swiglu: bool) -> int:
+def tile_cost(rows: int, n_out: int, bn: int, swiglu: bool) -> float:
+    """What a product in tiles of `bn` weight rows takes, in tiles of 256 (see `feature_tile`)."""
+    tiles = -(-rows // BM) * -(-n_out // (bn // 2 if swiglu else bn))
+    cost = -(-tiles // sm_count()) * (bn / 256.0 + 0.12)
+    return cost * 0.88 if bn >= 192 and tiles > sm_count() else cost
+
+
+def whole_heads_pay(rows: int, n_out: int, end: RotateAndCache) -> bool:
+    """Whether turning heads in the product beats a kernel behind it: its tiles have to hold whole heads, which must not
+    cost more than the best tile does."""
+    d = end.cache.head_dim
+    return tile_cost(rows, n_out, feature_tile(rows, n_out, False, d), False) <= tile_cost(rows, n_out, feature_tile(rows, n_out, False), False)
+
+
+def feature_tile(rows: int, n_out: int, swiglu: bool, multiple: int = 0) -> int:
     """Orientation 1: how many weight rows a tile takes (a multiple of 16 up to 256; of 32 with
     SwiGLU, whose tile is half gate rows and half up rows).  Every SM works through
     ceil(tiles / SMs) tiles and a tile's time grows with its width, so the product of the two is
     minimised; a small fixed cost per tile breaks ties towards wider tiles.  Wide tiles (192 rows
     and more) of a product with more tiles than SMs run in the persistent kernel, whose tiles
-    measured about an eighth cheaper (no pipeline refill per tile, the epilogue off the critical path)."""
+    measured about an eighth cheaper (no pipeline refill per tile, the epilogue off the critical path).
+    `multiple`: the tile has to be a multiple of this (whole heads)."""
     forced = os.environ.get("BARE_CUDA_B200_GEMM_BN")     # experiments only
-    if forced:
+    if forced and not multiple:
         return int(forced)
     step = 32 if swiglu else 16
     best, best_cost = 256, None
     for bn in range(256, 63, -step):
+        if multiple and bn % multiple:
+            continue
         # between 160 and 256 a tile is too big for two blocks per SM with three stages each, yet
         # more than one tile per SM needs that overlap: only SwiGLU tiles (two stages) use the range
         if not swiglu and 160 < bn < 256:
             continue
-        out_per_tile = bn // 2 if swiglu else bn
-        tiles = -(-rows // BM) * -(-n_out // out_per_tile)
-        cost = -(-tiles // sm_count()) * (bn / 256.0 + 0.12)
-        if bn >= 192 and tiles > sm_count():
-            cost *= 0.88
+        cost = tile_cost(rows, n_out, bn, swiglu)
         if best_cost is None or cost < best_cost - 1e-9:
             best, best_cost = bn, cost
     return best
@@ -184,6 +201,31 @@ def takes_prenormed(rows: int, swiglu: bool) -> bool:
     factor per row (tokens on the MMA rows), so that the product can take a `LazyNorm` that a
     product before it prepared."""
     return rows > (SWIGLU_TOKENS_ON_ROWS_ABOVE if swiglu else TOKENS_ON_ROWS_ABOVE)
+
+
+def turns(end: RotateAndCache, n_out: int) -> bool:
+    """Whether the many-token product's epilogue can turn the heads and write the cache: angles that the step's layers
+    share, whole heads to a tile, 16-byte stores everywhere."""
+    c, q = end.cache, end.q_out
+    return ((end.inv_freq is None or end.angles is not None) and c.dtype == q.dtype == torch.bfloat16 and c.v_dim == c.head_dim and c.head_dim in (32, 64, 128, 256)
+            and (end.q_heads + 2 * c.kv_heads) * c.head_dim == n_out and q.stride(0) % 8 == 0 and c.page_stride % 8 == 0
+            and (q.data_ptr() | c.k_ptr | c.v_ptr) % 16 == 0)
+
+
+def turn_table(ctx, l, end: RotateAndCache, rows: int) -> Tuple[int, int]:
+    """The step's table of (cosine, sine) pairs for these angles (address, row stride), made by the first layer that asks
+    for it."""
+    if end.inv_freq is None:
+        return 0, 0
+    half = end.cache.head_dim // 2
+    key = ("turn_table", end.angles, half)
+    table = ctx.extras.get(key)
+    if table is None:
+        table = ctx.ws.get(f"turn_table {end.angles}", (half, 2 * ctx.ws.max_rows), torch.float32, max_rows=half)
+        _check(l.llm_turn_table(end.positions.data_ptr(), end.inv_freq.data_ptr(), table.data_ptr(), ctx.ws.max_rows, rows, half,
+                                ctx.stream), "turn_table")
+        ctx.extras[key] = table
+    return table.data_ptr(), ctx.ws.max_rows
 
 
 def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
@@ -211,6 +253,15 @@ def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
     code = DT_BF16 if out_dtype == torch.bfloat16 else DT_F32
     if takes_prenormed(rows, swiglu):
         n_out = plan.n // 2 if swiglu else plan.n
+        if isinstance(epilogue, RotateAndCache) and not swiglu and turns(epilogue, n_out) and whole_heads_pay(rows, n_out, epilogue):
+            c, q = epilogue.cache, epilogue.q_out
+            bn = feature_tile(rows, n_out, False, c.head_dim)
+            _check(l.llm_gemm_qkv(ctypes.addressof(plan.weight_map(bn)), ctypes.addressof(plan.act_map(a, BM)), q.data_ptr(), rows,
+                                  plan.k, q.stride(0), bn, *extra_in, *turn_table(ctx, l, epilogue, rows), c.k_ptr, c.v_ptr,
+                                  c.block_table.data_ptr(), c.page_stride, c.table_stride, c.page_tokens, c.kv_heads, c.head_dim,
+                                  epilogue.positions.data_ptr(), epilogue.row_seq.data_ptr(), epilogue.q_heads,
+                                  1 if epilogue.write_cache else 0, err.data_ptr(), ctx.stream), "gemm_tcgen05 (q, k, v)")
+            return None
         bn = feature_tile(rows, n_out, swiglu)
         extra_out = NO_EXTRA[5:]
         out, then = None, None

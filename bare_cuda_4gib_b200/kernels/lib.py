@@ -197,9 +197,10 @@ class RotateAndCache:
     """Asks the [q; k; v] product to rotate q and k by position, write q to `q_out` and put k and
     v into the cache (what `rope_cache_write` does as a kernel of its own)."""
 
-    __slots__ = ("q_out", "cache", "positions", "row_seq", "inv_freq", "q_heads", "write_cache")
+    __slots__ = ("q_out", "cache", "positions", "row_seq", "inv_freq", "q_heads", "write_cache", "angles")
 
-    def __init__(self, q_out, cache, positions, row_seq, inv_freq, q_heads, write_cache):
+    def __init__(self, q_out, cache, positions, row_seq, inv_freq, q_heads, write_cache, angles=None):
+        self.angles = angles        # what `inv_freq` was made from: layers that agree in it share a step's table of angles
         self.q_out, self.cache, self.positions, self.row_seq = q_out, cache, positions, row_seq
         self.inv_freq, self.q_heads, self.write_cache = inv_freq, q_heads, write_cache
 

@@ -23,6 +23,7 @@ class RotaryPositions(Part):
         d, theta = int(self.params["head_dim"]), float(self.params["theta"])
         exponent = torch.arange(d // 2, dtype=torch.float32) * 2.0 / d
         self.inv_freq = (1.0 / (theta ** exponent)).to(device)
+        self.angles = ("rope", theta, d)      # layers that agree in these have the same angles
 
     def fused_rotation(self):
         """Inverse frequencies for kernels that rotate q and k themselves."""

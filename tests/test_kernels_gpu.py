@@ -449,6 +449,53 @@ def test_gemm_cluster_rotates_and_writes_the_cache(rows, heads, kv_heads, d, rot
         _close(held[1], full[t, heads + kv_heads:], 2 ** -8, 1e-3)
 
 
+@pytest.mark.parametrize("rows,heads,kv_heads,d,rotate", [(241, 5, 1, 64, True), (300, 3, 2, 128, True), (1300, 32, 4, 64, True), (270, 9, 1, 32, True),
+                                                          (257, 2, 1, 256, False), (2048, 16, 16, 128, True)])
+@pytest.mark.parametrize("prenormed", [False, True])
+def test_gemm_many_tokens_rotates_and_writes_the_cache(rows, heads, kv_heads, d, rotate, prenormed, monkeypatch):
+    from bare_cuda_4gib_b200.kernels import gemm
+    from bare_cuda_4gib_b200.kernels import lib as K
+    monkeypatch.setattr(gemm, "whole_heads_pay", lambda *sizes: True)      # whatever the tiles cost at this size
+    torch.manual_seed(rows + d)
+    ctx, k, eps = _ctx(), 200, 1e-5
+    ctx.extras = {}
+    a = ctx.ws.get("a", (rows, k), torch.bfloat16)
+    a.copy_(torch.randn(rows, k, device=DEV))
+    x, xd = a, a.double()
+    if prenormed:
+        parts = torch.rand(3, rows + 5, device=DEV) * k
+        x = K.LazyNorm(ctx, None, None, eps, rows, None, "normed", K.Prenormed(None, a, parts, 3))
+        xd = xd * torch.rsqrt(parts[:, :rows].double().sum(0) / k + eps)[:, None]
+    n, page = (heads + 2 * kv_heads) * d, 64
+    w = (torch.randn(n, k, device=DEV) / math.sqrt(k)).to(torch.bfloat16)
+    blocks = -(-(rows + 7) // page)
+    elems = 2 * kv_heads * page * d
+    storage = torch.zeros(blocks + 3, elems, device=DEV, dtype=torch.bfloat16)
+    table = torch.full((2, blocks + 1), -1, dtype=torch.int32, device=DEV)
+    table[1, :blocks] = torch.randperm(blocks + 3, device=DEV)[:blocks].int()
+    table[1, 0] = -1                                      # a page that is not held: nothing is written there
+    view = K.CacheView(storage.data_ptr(), storage.data_ptr() + elems, table, elems, table.stride(0), page, kv_heads, d, torch.bfloat16)
+    seq = torch.ones(rows, dtype=torch.int32, device=DEV)
+    pos = torch.arange(7, 7 + rows, dtype=torch.int32, device=DEV)
+    inv = 1.0 / 10000.0 ** (torch.arange(d // 2, device=DEV).float() * 2 / d) if rotate else None
+    q = torch.full((rows, heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+    end = K.RotateAndCache(q, view, pos, seq, inv, heads, True, ("rope", 10000.0, d))
+    assert gemm.turns(end, n)
+    assert gemm.run(ctx, gemm.plan_for(w), x, rows, torch.bfloat16, "qkv", True, False, end) is None
+    gemm.check_errors()
+    full = (xd @ w.double().t()).view(rows, heads + 2 * kv_heads, d)
+    turned = _rope_ref(full[:, : heads + kv_heads], pos, inv) if rotate else full[:, : heads + kv_heads]
+    _close(q.float().view(rows, heads, d), turned[:, :heads], 2 ** -8, 1e-3)
+    held = table[1, (pos // page).long()].long()
+    got = storage.view(-1, 2, kv_heads, page, d)[held.clamp(min=0), :, :, (pos % page).long()].float()
+    there = held >= 0
+    _close(got[there, 0], turned[there, heads:], 2 ** -8, 1e-3)
+    _close(got[there, 1], full[there, heads + kv_heads:], 2 ** -8, 1e-3)
+    used = torch.zeros(storage.shape[0], dtype=torch.bool, device=DEV)
+    used[held[there]] = True
+    assert not storage[~used].any()
+
+
 def test_a_bounded_wait_runs_out_and_the_kernel_returns():
     """Every wait inside the pipelined kernels has a limit.  Here one is seen to run out: with the
     test hooks of the GEMM library the producer arms one stage's barrier and issues no copy for it,
