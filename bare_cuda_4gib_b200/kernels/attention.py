@@ -216,6 +216,50 @@ def plan_for(head_dim: int, heads: int, kv_heads: int, distance_bias: bool = Fal
     return AttentionPlan(head_dim, heads, kv_heads, distance_bias, v_dim, softcap, window, chunk)
 
 
+def few_beside_prompts(plan: AttentionPlan, q_len, kv_len) -> list:
+    """In a step with prompt portions: the requests (at most 16 packed rows each) that a launch of the decode kernel takes,
+    if that pays.  In the prefill kernel such a request's tile of 128 rows walks through all of its keys alone, so long
+    contexts beside short portions make the launch as long as the longest of them; the decode kernel deals a
+    request's keys out.  In blocks of 128 keys (about 2 us each) a launch takes its longest tile, or what two tiles to an SM
+    leave for each place; the second launch takes about 8 us.  (24 requests of 100 to 1,500 positions beside three portions
+    of 200 to 389 tokens: 29.5 us a layer in one launch, 22.4 in two; the step 3,373 -> 3,248 us.)"""
+    if plan.tc is None or plan.decode is None:
+        return []
+    few = [s for s, q in enumerate(q_len) if q * plan.group <= 16]
+    if not few or len(few) == len(q_len) or len(few) * plan.kv_heads > DECODE_MAX_TILES:
+        return []
+    tiles = [-(-q * plan.group // plan.prefill_rows) for q in q_len]
+    blocks = [plan.key_blocks(kv, q, 128) for q, kv in zip(q_len, kv_len)]
+    chosen = set(few)
+
+    def launch(which):
+        return max(max(blocks[s] for s in which), sum(blocks[s] * tiles[s] for s in which) * plan.kv_heads / (2 * sm_count()))
+
+    rest = [s for s in range(len(q_len)) if s not in chosen]
+    return few if launch(range(len(q_len))) - launch(rest) >= 4 else []
+
+
+def decode_blocks(plan: AttentionPlan, n_tiles: int, max_q_len: int) -> Tuple[int, int]:
+    """How many blocks of the cluster decode kernel share a tile, and whether with key blocks of half the size.
+
+    Up to 8 blocks of 4 warps share a tile, a warp keeps one key block in flight.  Measured at a context of 2,048 (batches 8
+    to 64): the kernel is fastest with about two blocks per SM in all, and with a power of two of them per tile (batch 64:
+    26.7 us with one block per tile, 32 with two or four; batch 32: 13.4 us with two, 20.9 / 16.1 with one / four; batch 16:
+    8.5 us with four, 12.1 / 12.6 with two / eight).  The number does not depend on the context length (a short context
+    leaves some warps without a key block), so a captured graph of the step stays valid while the requests grow.  Key blocks
+    of half the size: see HALF_BLOCKS_MAX_SPLITS."""
+    splits = 1
+    # where a window or a block of positions bounds the keys: no more blocks of four warps than have a key block each
+    most = plan.key_blocks(1 << 30, max_q_len, plan.decode.key_block)
+    while splits < 8 and 4 * splits < most and n_tiles * plan.kv_heads * splits * 2 <= 2 * sm_count():
+        splits *= 2
+    if os.environ.get("BARE_CUDA_B200_ATTN_SPLITS"):     # experiments only
+        return max(1, min(8, int(os.environ["BARE_CUDA_B200_ATTN_SPLITS"]))), 0
+    if plan.decode_half is not None and 2 * splits <= HALF_BLOCKS_MAX_SPLITS and 4 * splits < most:
+        return 2 * splits, 1
+    return splits, 0
+
+
 def step_tiles(ctx, plan: AttentionPlan):
     """The step's row tiles for this head grouping: built once per step and shared by all layers."""
     key = ("attention_tiles", plan.group, plan.kv_heads, plan.head_dim, plan.distance_bias, plan.prefill_rows,
@@ -225,16 +269,21 @@ def step_tiles(ctx, plan: AttentionPlan):
         return cached
     g = plan.group
     rows_per_tile = 16 if ctx.max_q_len * g <= 16 else plan.prefill_rows
-    counts = [-(-q * g // rows_per_tile) for q in ctx.host_q_len]
+    # requests whose rows the decode kernel takes although others of the step bring a prompt
+    few = few_beside_prompts(plan, ctx.host_q_len, ctx.host_kv_len) if rows_per_tile != 16 else []
+    apart = set(few)
+    counts = [0 if s in apart else -(-q * g // rows_per_tile) for s, q in enumerate(ctx.host_q_len)]
     pad = ctx.pad_seqs if rows_per_tile == 16 else 0     # padded decode steps keep a fixed grid
-    n_tiles = sum(counts) + pad
-    host, dev = plan.buffers(ctx, n_tiles, ctx.token_ids.device)
+    n_tiles, n_few = sum(counts) + pad, len(few)
+    host, dev = plan.buffers(ctx, n_tiles + n_few, ctx.token_ids.device)
     h = host.numpy()
     at = 0
     for s, c in enumerate(counts):
         h[at: at + c] = s
         h[n_tiles + at: n_tiles + at + c] = np.arange(c, dtype=np.int32)
         at += c
+    h[2 * n_tiles: 2 * n_tiles + n_few] = few
+    h[2 * n_tiles + n_few: 2 * (n_tiles + n_few)] = 0        # one tile of 16 rows each
     if plan.chunk and rows_per_tile != 16:
         # the kernels start the last tile first: without blocks of positions it is the one that sees the most
         # keys, with them the tiles are sorted by what they see
@@ -246,7 +295,7 @@ def step_tiles(ctx, plan: AttentionPlan):
         h[:at], h[n_tiles: n_tiles + at] = seq[order], index[order]
     h[at: n_tiles] = -1
     h[n_tiles + at: 2 * n_tiles] = 0
-    dev[: 2 * n_tiles].copy_(host[: 2 * n_tiles], non_blocking=True)
+    dev[: 2 * (n_tiles + n_few)].copy_(host[: 2 * (n_tiles + n_few)], non_blocking=True)
     plan.sent()
     n_splits = 1
     use_decode = rows_per_tile == 16 and plan.decode is not None and n_tiles * plan.kv_heads <= DECODE_MAX_TILES
@@ -258,26 +307,9 @@ def step_tiles(ctx, plan: AttentionPlan):
             n_splits = min(key_blocks, int(os.environ["BARE_CUDA_B200_ATTN_SPLITS"]))
         if n_tiles * plan.kv_heads > COUNTER_WORDS:
             n_splits = 1
-    dec_splits = dec_slots = half = 0
-    if use_decode:
-        # The cluster decode kernel: up to 8 blocks of 4 warps share a tile, a warp keeps one key
-        # block in flight.  Measured at a context of 2,048 (batches 8 to 64): the kernel is fastest
-        # with about two blocks per SM in all, and with a power of two of them per tile (batch 64:
-        # 26.7 us with one block per tile, 32 with two or four; batch 32: 13.4 us with two, 20.9 / 16.1 with
-        # one / four; batch 16: 8.5 us with four, 12.1 / 12.6 with two / eight).  The number does not depend
-        # on the context length (a short context leaves some warps without a key block), so a captured
-        # graph of the step stays valid while the requests grow.
-        dec_splits = 1
-        # where a window or a block of positions bounds the keys: no more blocks of four warps than have a key block each
-        most = plan.key_blocks(1 << 30, ctx.max_q_len, plan.decode.key_block)
-        while dec_splits < 8 and 4 * dec_splits < most and n_tiles * plan.kv_heads * dec_splits * 2 <= 2 * sm_count():
-            dec_splits *= 2
-        dec_slots = 1
-        if os.environ.get("BARE_CUDA_B200_ATTN_SPLITS"):     # experiments only
-            dec_splits = max(1, min(8, int(os.environ["BARE_CUDA_B200_ATTN_SPLITS"])))
-        elif plan.decode_half is not None and 2 * dec_splits <= HALF_BLOCKS_MAX_SPLITS and 4 * dec_splits < most:
-            half, dec_splits = 1, 2 * dec_splits
-    out = (dev[:n_tiles], dev[n_tiles: 2 * n_tiles], n_tiles, rows_per_tile, n_splits, dec_splits, dec_slots, half)
+    dec_splits, half = decode_blocks(plan, n_tiles, ctx.max_q_len) if use_decode else (0, 0)
+    few_splits, few_half = decode_blocks(plan, n_few, max(ctx.host_q_len[s] for s in few)) if few else (0, 0)
+    out = (dev[:n_tiles], dev[n_tiles: 2 * n_tiles], n_tiles, rows_per_tile, n_splits, dec_splits, half, n_few, few_splits, few_half)
     ctx.extras[key] = out
     return out
 
@@ -297,7 +329,7 @@ def run(ctx, plan: AttentionPlan, q: torch.Tensor, out: torch.Tensor, cache: Cac
     more = (extras or AttentionExtras()).arguments(plan.heads, q.dtype)
     if plan.distance_bias and extras:
         raise KernelLaunchError("attention_mma (distance bias): the variant takes no blocks of positions, sink or gate")
-    tile_seq, tile_index, n_tiles, rows_per_tile, n_splits, dec_splits, dec_slots, half = step_tiles(ctx, plan)
+    tile_seq, tile_index, n_tiles, rows_per_tile, n_splits, dec_splits, half, n_few, few_splits, few_half = step_tiles(ctx, plan)
     if plan.distance_bias:
         scratch_ptr = 0
         if n_splits > 1:
@@ -310,7 +342,7 @@ def run(ctx, plan: AttentionPlan, q: torch.Tensor, out: torch.Tensor, cache: Cac
             ctx.seq_kv_len.data_ptr(), tile_seq.data_ptr(), tile_index.data_ptr(), n_tiles, rows_per_tile, n_splits,
             scratch_ptr, plan.heads, scale, window, ctx.stream), "attention_mma (distance bias)")
         return
-    if dec_splits and plan.decode_usable(cache):
+    def decode(seqs: int, indices: int, n, splits, half):
         from . import gemm
         library = plan.decode_half if half else plan.decode
         pool_map, box_rows = plan.decode_map(cache, library)
@@ -318,14 +350,19 @@ def run(ctx, plan: AttentionPlan, q: torch.Tensor, out: torch.Tensor, cache: Cac
             ctypes.addressof(pool_map), cache.pool_ptr, cache.pool_elems // plan.head_dim, box_rows, q.data_ptr(),
             out.data_ptr(), cache.k_ptr, cache.v_ptr, cache.block_table.data_ptr(), cache.page_stride,
             cache.table_stride, cache.page_tokens, cache.kv_heads, cache.head_dim, ctx.seq_q_start.data_ptr(),
-            ctx.seq_q_len.data_ptr(), ctx.seq_kv_len.data_ptr(), tile_seq.data_ptr(), tile_index.data_ptr(), n_tiles,
-            dec_splits, dec_slots, plan.heads, scale, window, *more, gemm.error_word(q.device).data_ptr(), ctx.stream),
-            "attention_decode")
+            ctx.seq_q_len.data_ptr(), ctx.seq_kv_len.data_ptr(), seqs, indices, n,
+            splits, 1, plan.heads, scale, window, *more, gemm.error_word(q.device).data_ptr(), ctx.stream), "attention_decode")
+
+    if dec_splits and plan.decode_usable(cache):
+        decode(tile_seq.data_ptr(), tile_index.data_ptr(), n_tiles, dec_splits, half)
         return
     if plan.tc is not None and rows_per_tile != 16:
         if not plan.tc_usable(cache):
             raise KernelLaunchError(f"attention_tcgen05: cache pages of {cache.page_tokens} positions are not supported "
                                     "(the page size must share a factor of at least 8 with 128)")
+        if n_few:      # (pages that the one kernel takes, the other takes)
+            behind = tile_seq.data_ptr() + 4 * 2 * n_tiles      # the second list lies behind the first (see step_tiles)
+            decode(behind, behind + 4 * n_few, n_few, few_splits, few_half)
         from . import gemm
         pool_map, box_rows = plan.pool_map(cache)
         _check(plan.tc.llm_attention_tcgen05(
