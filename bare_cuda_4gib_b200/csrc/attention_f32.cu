@@ -10,9 +10,9 @@
 // `join` are the only code that does this arithmetic, and both ways of dealing out the work call them:
 //   walk   (more than eight rows of a request): a block takes 64 rows, eight a warp; spans come through
 //          shared memory two at a time, once for all warps, and every warp joins as it goes.
-//   few    (a decoding request): the spans are dealt out to the eight blocks of a cluster and there to
-//          SLOTS warps, the states stay in shared memory, and block r joins them for row r through
-//          distributed shared memory.
+//   few    (a decoding request): the spans are dealt out to the eight blocks of a cluster, warp r makes the states of
+//          row r, they stay in shared memory, and block r joins them for row r through distributed shared memory.
+//          (One warp for all eight rows of a span: 19.3 us a layer for 4 requests of up to 300 keys, a warp a row 13.7.)
 // What bounds it: shared-memory wavefronts in the walk (24 of them for 32 packed FMAs), latency with few rows.
 //
 // A key that no row of a tile sees, or whose page is not held, is zero in shared memory; in a span that some
@@ -101,13 +101,14 @@ struct Join {
   }
 };
 
-// One warp: the state of keys [64 span, 64 span + 64) for eight rows.  Row i sees keys first[i] .. last[i].
+// One warp: the state of keys [64 span, 64 span + 64) for NR rows.  Row i sees keys first[i] .. last[i].
+template <int NR>
 __device__ __forceinline__ void span_state(uint32_t q, uint32_t keys, uint32_t values, uint32_t p, const int* held, int span,
-                                           const int (&first)[ROWS], const int (&last)[ROWS], float scale, int lane,
-                                           float (&m)[ROWS], float (&l)[ROWS], pair32 (&o)[ROWS][PAIRS]) {
-  pair32 dot[ROWS][2];
+                                           const int (&first)[NR], const int (&last)[NR], float scale, int lane,
+                                           float (&m)[NR], float (&l)[NR], pair32 (&o)[NR][PAIRS]) {
+  pair32 dot[NR][2];
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i) dot[i][0] = dot[i][1] = 0ull;
+  for (int i = 0; i < NR; ++i) dot[i][0] = dot[i][1] = 0ull;
   const uint32_t low = lane & 7, key = keys + lane * D * 4;
 #pragma unroll 4
   for (uint32_t c = 0; c < D / 4; ++c) {
@@ -115,7 +116,7 @@ __device__ __forceinline__ void span_state(uint32_t q, uint32_t keys, uint32_t v
     pairs_load(ax, ay, key + ((c ^ low) << 4));
     pairs_load(bx, by, key + 32 * D * 4 + ((c ^ low) << 4));
 #pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
+    for (int i = 0; i < NR; ++i) {
       pair32 qx, qy;
       pairs_load(qx, qy, q + i * D * 4 + (c << 4));
       fma_pair(dot[i][0], qx, ax);
@@ -128,7 +129,7 @@ __device__ __forceinline__ void span_state(uint32_t q, uint32_t keys, uint32_t v
   const bool held0 = held[lane] != 0, held1 = held[lane + 32] != 0;
   bool whole = true;
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i) {
+  for (int i = 0; i < NR; ++i) {
     whole = whole && first[i] <= span * SPAN && last[i] >= span * SPAN + SPAN - 1;
     const float2 d0 = unpack(dot[i][0]), d1 = unpack(dot[i][1]);
     const float s0 = held0 && j0 >= first[i] && j0 <= last[i] ? __fmul_rn(__fadd_rn(d0.x, d0.y), scale) : -INFINITY;
@@ -142,7 +143,7 @@ __device__ __forceinline__ void span_state(uint32_t q, uint32_t keys, uint32_t v
   }
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i)
+  for (int i = 0; i < NR; ++i)
 #pragma unroll
     for (int c = 0; c < PAIRS; ++c) o[i][c] = 0ull;
   const uint32_t value = values + lane * (PAIRS * 8);
@@ -155,7 +156,7 @@ __device__ __forceinline__ void span_state(uint32_t q, uint32_t keys, uint32_t v
       for (int c = 0; c < PAIRS; ++c)
         asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v[u][c]) : "r"(value + (j + u) * D * 4 + c * 8));
 #pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
+    for (int i = 0; i < NR; ++i) {
       float w[4];
       asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                    : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]) : "r"(p + (i * SPAN + j) * 4));
@@ -208,16 +209,16 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
   const int tile_last = base_pos + (min(r0 + TILE_ROWS, rows) - 1) / G;
   const int tile_first = a.window > 0 ? max(0, base_pos + r0 / G - a.window + 1) : 0;
   const int span_first = tile_first / SPAN, n_spans = tile_last / SPAN - span_first + 1;
-  int first[ROWS], last[ROWS];
-#pragma unroll
-  for (int i = 0; i < ROWS; ++i) {
-    const int r = r0 + (few ? 0 : warp * ROWS) + i, pos = base_pos + r / G;
-    last[i] = r < rows ? pos : -1;                                   // a row that does not exist sees nothing
-    first[i] = a.window > 0 ? max(0, pos - a.window + 1) : 0;
-  }
   const uint32_t spans = base + Shared::SPANS, p = base + Shared::P + warp * (ROWS * SPAN * 4);
 
   if (!few) {
+    int first[ROWS], last[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const int r = r0 + warp * ROWS + i, pos = base_pos + r / G;
+      last[i] = r < rows ? pos : -1;                                   // a row that does not exist sees nothing
+      first[i] = a.window > 0 ? max(0, pos - a.window + 1) : 0;
+    }
     float M[ROWS], L[ROWS];
     float2 O[ROWS][PAIRS];
 #pragma unroll
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
       float m[ROWS], l[ROWS];
       pair32 o[ROWS][PAIRS];
       const uint32_t at = spans + slot * 2 * SPAN_BYTES;
-      span_state(base + Shared::Q + warp * ROWS * D * 4, at, at + SPAN_BYTES, p, held + slot * SPAN, span, first, last, a.scale, lane, m, l, o);
+      span_state<ROWS>(base + Shared::Q + warp * ROWS * D * 4, at, at + SPAN_BYTES, p, held + slot * SPAN, span, first, last, a.scale, lane, m, l, o);
 #pragma unroll
       for (int i = 0; i < ROWS; ++i) {
         if (m[i] == -INFINITY) continue;
@@ -271,6 +272,8 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
     return;
   }
 
+  const int few_pos = base_pos + warp / G, few_last = warp < rows ? few_pos : -1;
+  const int few_first = a.window > 0 ? max(0, few_pos - a.window + 1) : 0;
   const int rank = blockIdx.x;          // grid.x is a multiple of the cluster, and only its first one has few rows
   float M = -INFINITY, L = 0.0f, O = 0.0f;     // row `rank`, output column threadIdx.x
   for (int s0 = 0; s0 < n_spans; s0 += CLUSTER * SLOTS) {
@@ -282,18 +285,20 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
     copies_commit();
     copies_wait_all();
     __syncthreads();
-    if (warp < SLOTS && s0 + warp * CLUSTER + rank < n_spans) {
-      float m[ROWS], l[ROWS];
-      pair32 o[ROWS][PAIRS];
-      const uint32_t at = spans + warp * 2 * SPAN_BYTES;
-      span_state(base + Shared::Q, at, at + SPAN_BYTES, p, held + warp * SPAN, span_first + s0 + warp * CLUSTER + rank, first, last, a.scale, lane, m, l, o);
-      float* state = reinterpret_cast<float*>(smem + Shared::STATES) + warp * STATE_FLOATS;
-#pragma unroll
-      for (int i = 0; i < ROWS; ++i) {
-        if (lane == 0) state[i] = m[i], state[ROWS + i] = l[i];
+    if (warp < rows) {                // row `warp` of every span that is here
+      const int row_first[1] = {few_first}, row_last[1] = {few_last};
+#pragma unroll 1
+      for (int slot = 0; slot < SLOTS && s0 + slot * CLUSTER + rank < n_spans; ++slot) {
+        float m[1], l[1];
+        pair32 o[1][PAIRS];
+        const uint32_t at = spans + slot * 2 * SPAN_BYTES;
+        span_state<1>(base + Shared::Q + warp * D * 4, at, at + SPAN_BYTES, p, held + slot * SPAN, span_first + s0 + slot * CLUSTER + rank,
+                      row_first, row_last, a.scale, lane, m, l, o);
+        float* state = reinterpret_cast<float*>(smem + Shared::STATES) + slot * STATE_FLOATS;
+        if (lane == 0) state[warp] = m[0], state[ROWS + warp] = l[0];
 #pragma unroll
         for (int c = 0; c < PAIRS; ++c)
-          *reinterpret_cast<float2*>(state + 2 * ROWS + i * D + lane * (PAIRS * 2) + 2 * c) = unpack(o[i][c]);
+          *reinterpret_cast<float2*>(state + 2 * ROWS + warp * D + lane * (PAIRS * 2) + 2 * c) = unpack(o[0][c]);
       }
     }
     cluster_sync();
