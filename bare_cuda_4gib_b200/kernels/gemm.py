@@ -335,6 +335,7 @@ CLUSTER_MAX_ROWS = 64
 # a large one is bound by its weights, which the split product's deeper ring streams faster (8 rows x 4,096 x 14,336, 117 MB:
 # 18.0 us and a norm kernel of 4.3 against 23.5).
 CLUSTER_FEW_ROWS, CLUSTER_FEW_BYTES = 24, 64 << 20
+CLUSTER_MIN_K = 8 * BK      # shorter sums are too short to share: a block of the cluster would have no K block to itself
 
 
 def cluster_size(n_tiles: int, k: int) -> int:
@@ -347,7 +348,7 @@ def cluster_size(n_tiles: int, k: int) -> int:
 
 def cluster_kind(plan: GemmPlan, rows: int, out_dtype, swiglu: bool, epilogue) -> Optional[int]:
     """Which of the cluster product's ends a call asks for, None where the kernel does not take it."""
-    if not 0 < rows <= CLUSTER_MAX_ROWS or plan.n % 8 or (rows <= CLUSTER_FEW_ROWS and 2 * plan.n * plan.k > CLUSTER_FEW_BYTES):
+    if plan.k < CLUSTER_MIN_K or not 0 < rows <= CLUSTER_MAX_ROWS or plan.n % 8 or (rows <= CLUSTER_FEW_ROWS and 2 * plan.n * plan.k > CLUSTER_FEW_BYTES):
         return None
     if swiglu:
         return CL_SWIGLU

@@ -376,7 +376,7 @@ def test_gemm_tcgen05_swiglu(m, inter, k):
 
 
 @pytest.mark.parametrize("rows,n,k", [(1, 128, 64), (16, 136, 72), (17, 2048, 2048), (33, 2560, 200), (48, 320, 5632), (63, 1000, 1024),
-                                      (64, 2048, 5632), (8, 2048, 14336), (25, 72, 1088)])
+                                      (64, 2048, 5632), (8, 2048, 14336), (8, 4096, 14336), (25, 72, 1088)])
 @pytest.mark.parametrize("prenormed", [False, True])
 def test_gemm_cluster_adds_prepares_and_gates(rows, n, k, prenormed):
     """The product whose blocks exchange their parts through distributed shared memory: into the residual stream with the
@@ -398,8 +398,9 @@ def test_gemm_cluster_adds_prepares_and_gates(rows, n, k, prenormed):
     residual, norm = torch.randn(rows + 2, n, device=DEV), _RowNorm(1 + 0.3 * torch.randn(n, device=DEV), eps)
     before = residual.double().clone()
     kind = gemm.cluster_kind(plan, rows, torch.float32, False, K.AddTo(residual, norm))
-    assert kind == gemm.CL_ADD
-    assert gemm.run_cluster(ctx, plan, kind, x, rows, torch.float32, "out", K.AddTo(residual, norm)) is None
+    few_and_large = rows <= gemm.CLUSTER_FEW_ROWS and 2 * n * k > gemm.CLUSTER_FEW_BYTES
+    assert kind == (None if k < gemm.CLUSTER_MIN_K or few_and_large else gemm.CL_ADD)
+    assert gemm.run_cluster(ctx, plan, gemm.CL_ADD, x, rows, torch.float32, "out", K.AddTo(residual, norm)) is None
     gemm.check_errors()
     before[:rows] += full
     _close(residual, before, 1e-5, 2 ** -20 * size)        # float32 sums in the tensor core: 2^-22 a step, a few steps deep
@@ -408,15 +409,14 @@ def test_gemm_cluster_adds_prepares_and_gates(rows, n, k, prenormed):
     _close(pre.sq[: pre.items, :rows].double().sum(0), now.square().sum(-1), 1e-5, 1e-5)
     inter = n // 2
     if inter % 8 == 0:
-        kind = gemm.cluster_kind(plan, rows, torch.bfloat16, True, None)
-        got = gemm.run_cluster(ctx, plan, kind, x, rows, torch.bfloat16, "act").tensor
+        got = gemm.run_cluster(ctx, plan, gemm.CL_SWIGLU, x, rows, torch.bfloat16, "act").tensor
         gemm.check_errors()
         gate, up = full[:, :inter], full[:, inter:]
         _close(got, gate / (1 + torch.exp(-gate)) * up, 2 ** -8, 1e-4 + 2 ** -18 * size)
 
 
 @pytest.mark.parametrize("rows,heads,kv_heads,d,rotate", [(25, 8, 2, 64, True), (64, 3, 1, 128, True), (40, 5, 2, 32, True), (33, 2, 1, 8, False)])
-def test_gemm_cluster_rotates_and_writes_the_cache(rows, heads, kv_heads, d, rotate):
+def test_gemm_cluster_rotates_and_writes_the_cache(rows, heads, kv_heads, d, rotate, monkeypatch):
     from bare_cuda_4gib_b200.kernels import gemm
     from bare_cuda_4gib_b200.kernels import lib as K
     torch.manual_seed(rows + d)
@@ -434,9 +434,9 @@ def test_gemm_cluster_rotates_and_writes_the_cache(rows, heads, kv_heads, d, rot
     q = torch.full((rows, heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
     end = K.RotateAndCache(q, view, pos, seq, inv, heads, True)
     plan = gemm.plan_for(w)
-    kind = gemm.cluster_kind(plan, rows, torch.float32, False, end)
-    assert kind == gemm.CL_ROPE
-    assert gemm.run_cluster(ctx, plan, kind, a, rows, torch.float32, "qkv", end) is None
+    monkeypatch.setattr(gemm, "CLUSTER_MIN_K", 0)           # whatever the length of the sums
+    assert gemm.cluster_kind(plan, rows, torch.float32, False, end) == gemm.CL_ROPE
+    assert gemm.run_cluster(ctx, plan, gemm.CL_ROPE, a, rows, torch.float32, "qkv", end) is None
     gemm.check_errors()
     full = (a.double() @ w.double().t()).view(rows, heads + 2 * kv_heads, d)
     turned = _rope_ref(full[:, : heads + kv_heads], pos, inv) if rotate else full[:, : heads + kv_heads]
