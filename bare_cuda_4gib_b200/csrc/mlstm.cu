@@ -20,13 +20,14 @@
 #define GATE_CHUNK 1024
 
 // Grid (sequence, head).  coef[row][head] = (a, b, exp(-m), m) for every new token of the sequence;
-// m_state[slot][head] is read at the start and written at the end.  The gates of a chunk of tokens
+// m_state[slot][head] is read at the start and written at the end.  `log_decay` and `weight` [row][head] (or both null)
+// receive log a and b for the walk in chunks.  The gates of a chunk of tokens
 // are computed side by side, m is walked through the chunk as a scan, then a and b side by side.
 template <typename TW>
 __global__ void __launch_bounds__(GATE_THREADS)
 mlstm_gates_kernel(const float* __restrict__ z, long long z_stride, int i_col, int f_col, const TW* __restrict__ i_bias,
                    const TW* __restrict__ f_bias, float cap, float* __restrict__ m_state, float4* __restrict__ coef,
-                   const int32_t* __restrict__ seq_slot, const int32_t* __restrict__ seq_q_start,
+                   float* __restrict__ log_decay, float* __restrict__ weight, const int32_t* __restrict__ seq_slot, const int32_t* __restrict__ seq_q_start,
                    const int32_t* __restrict__ seq_q_len, int heads) {
   pdl_launch_dependents();
   pdl_wait();
@@ -94,7 +95,10 @@ mlstm_gates_kernel(const float* __restrict__ z, long long z_stride, int i_col, i
     __syncthreads();
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
       const float m = mm[t + 1];
-      coef[(start + c0 + t) * heads + h] = make_float4(expf(gf[t] + mm[t] - m), expf(gi[t] - m), expf(-m), m);
+      const long long at = (start + c0 + t) * heads + h;
+      const float la = gf[t] + mm[t] - m, b = expf(gi[t] - m);
+      coef[at] = make_float4(expf(la), b, expf(-m), m);
+      if (log_decay) log_decay[at] = la, weight[at] = b;
     }
     m_prev = mm[n];
     __syncthreads();
@@ -103,19 +107,19 @@ mlstm_gates_kernel(const float* __restrict__ z, long long z_stride, int i_col, i
 }
 
 extern "C" int llm_mlstm_gates(const float* z, long long z_stride, int i_col, int f_col, const void* i_bias,
-                               const void* f_bias, int bias_dtype, float cap, float* m_state, float* coef,
-                               const int32_t* seq_slot, const int32_t* seq_q_start, const int32_t* seq_q_len, int n_seqs,
+                               const void* f_bias, int bias_dtype, float cap, float* m_state, float* coef, float* log_decay,
+                               float* weight, const int32_t* seq_slot, const int32_t* seq_q_start, const int32_t* seq_q_len, int n_seqs,
                                int heads, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
   LLM_HOST_CHECK(heads >= 1 && heads <= 65535 && cap > 0.0f, ERR_BAD_SIZE);
   dim3 grid(n_seqs, heads);
   if (bias_dtype == DT_F32)
     launch_kernel(mlstm_gates_kernel<float>, grid, GATE_THREADS, 0, stream, z, z_stride, i_col, f_col,
-                  (const float*)i_bias, (const float*)f_bias, cap, m_state, (float4*)coef, seq_slot, seq_q_start,
+                  (const float*)i_bias, (const float*)f_bias, cap, m_state, (float4*)coef, log_decay, weight, seq_slot, seq_q_start,
                   seq_q_len, heads);
   else if (bias_dtype == DT_BF16)
     launch_kernel(mlstm_gates_kernel<__nv_bfloat16>, grid, GATE_THREADS, 0, stream, z, z_stride, i_col, f_col,
-                  (const __nv_bfloat16*)i_bias, (const __nv_bfloat16*)f_bias, cap, m_state, (float4*)coef, seq_slot,
+                  (const __nv_bfloat16*)i_bias, (const __nv_bfloat16*)f_bias, cap, m_state, (float4*)coef, log_decay, weight, seq_slot,
                   seq_q_start, seq_q_len, heads);
   else
     return ERR_BAD_DTYPE;

@@ -4,11 +4,12 @@ operands for the state scan, and the quotient, unit norm and gate after it."""
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from typing import Optional
 
 import torch
 
 from . import build
-from .lib import _check, _dev, dtype_code
+from .lib import _check, _dev, _ptr, dtype_code
 
 _lib = None
 
@@ -18,7 +19,7 @@ def lib():
     if _lib is None:
         l = build.load_library("mlstm.cu")
         P, I, L, F = c_void_p, c_int, c_longlong, c_float
-        l.llm_mlstm_gates.argtypes = [P, L, I, I, P, P, I, F, P, P, P, P, P, I, I, P]
+        l.llm_mlstm_gates.argtypes = [P, L, I, I, P, P, I, F, P, P, P, P, P, P, P, I, I, P]
         l.llm_mlstm_operands.argtypes = [P, I, L, I, I, I, P, P, P, P, P, I, I, I, I, I, P]
         l.llm_mlstm_finish.argtypes = [P, P, P, P, L, P, L, I, I, I, I, I, F, P]
         l.llm_mlstm_step.argtypes = [P, I, L, I, I, I, I, P, L, I, I, P, P, F, P, P, P, P, L, P, P, P, I, I, I, I, I, F, F, P]
@@ -29,15 +30,17 @@ def lib():
 
 
 def gates(ctx, z: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor, f_bias: torch.Tensor, cap: float,
-          m_state: torch.Tensor, coef: torch.Tensor, heads: int) -> None:
+          m_state: torch.Tensor, coef: torch.Tensor, heads: int, log_decay: Optional[torch.Tensor] = None,
+          weight: Optional[torch.Tensor] = None) -> None:
     """z [rows, columns] float32 holds the gates' projections (input gate of head h at column
     i_col + h, forget gate at f_col + h); coef [rows, heads, 4] float32 receives (decay, input
-    weight, exp(-m), m) per new token; m_state [slots + 1, heads] carries m between steps."""
+    weight, exp(-m), m) per new token; m_state [slots + 1, heads] carries m between steps.  `log_decay` and `weight` [rows,
+    heads] float32 (both or neither) receive the decay's logarithm and the input weight for `chunked`."""
     _dev(z, i_bias, f_bias, m_state, coef)
     if z.dtype != torch.float32 or m_state.dtype != torch.float32 or coef.dtype != torch.float32:
         raise TypeError("mlstm gates: projections, state and coefficients must be float32")
     _check(lib().llm_mlstm_gates(z.data_ptr(), z.stride(0), i_col, f_col, i_bias.data_ptr(), f_bias.data_ptr(),
-                                 dtype_code(i_bias.dtype), float(cap), m_state.data_ptr(), coef.data_ptr(),
+                                 dtype_code(i_bias.dtype), float(cap), m_state.data_ptr(), coef.data_ptr(), _ptr(log_decay), _ptr(weight),
                                  ctx.seq_slot.data_ptr(), ctx.seq_q_start.data_ptr(), ctx.seq_q_len.data_ptr(),
                                  ctx.n_seqs, heads, ctx.stream), "mlstm_gates")
 
@@ -56,6 +59,33 @@ def finish(ctx, scanned: torch.Tensor, coef: torch.Tensor, norm_w: torch.Tensor,
     _check(lib().llm_mlstm_finish(scanned.data_ptr(), coef.data_ptr(), norm_w.data_ptr(), gate.data_ptr(),
                                   gate.stride(0), out.data_ptr(), out.stride(0), dtype_code(out.dtype), ctx.n_tokens,
                                   heads, dv, dvp, float(eps), ctx.stream), "mlstm_finish")
+
+
+def chunked_takes(dk: int, dv: int) -> bool:
+    """Sizes the walk in chunks on the tensor cores is built for (csrc/mamba2_chunked.cu, a library per pair)."""
+    return dk % 16 == 0 and 16 <= dk <= 256 and dv % 16 == 0 and 16 <= dv <= 1024
+
+
+def chunked_columns(dk: int) -> int:
+    """Value columns of a block: 16, so that a few heads put a block on most SMs (16 heads of 128 values: 144 blocks)."""
+    return 16
+
+
+def chunked(ctx, u: torch.Tensor, q_col: int, k_col: int, v_col: int, log_decay: torch.Tensor, weight: torch.Tensor,
+            state: torch.Tensor, out: torch.Tensor, heads: int, dk: int, dv: int, q_scale: float) -> None:
+    """Every request's portion in chunks of 64 tokens: q, k and v are read from the bfloat16 projection u; [S | n] float32
+    [slots, heads, dk, dv + 4] is read and left as after the portion; out [rows, heads * (dv + 4)] float32 = [S^T q | n . q | 0]
+    * q_scale."""
+    from . import mamba2
+    _dev(u, log_decay, weight, state, out)
+    if (u.dtype != torch.bfloat16 or state.dtype != torch.float32 or out.dtype != torch.float32 or not out.is_contiguous()
+            or state.shape[-1] != dv + 4 or out.shape[-1] != heads * (dv + 4)):
+        raise TypeError("mlstm chunked: element types or layout not as the kernel needs")
+    base = u.data_ptr()
+    _check(mamba2.chunked_lib(dk, dv, chunked_columns(dk), True).llm_mamba2_chunked(
+        base + 2 * v_col, base + 2 * k_col, base + 2 * q_col, u.stride(0), weight.data_ptr(), log_decay.data_ptr(),
+        state.data_ptr(), out.data_ptr(), float(q_scale), ctx.seq_slot.data_ptr(), ctx.seq_q_start.data_ptr(),
+        ctx.seq_q_len.data_ptr(), ctx.n_seqs, heads, heads, dk, dv, ctx.stream), "mlstm_chunked")
 
 
 STEP_MAX_VALUE_COLUMNS = 288      # vdim + pad the one-token kernel keeps per warp

@@ -10,7 +10,8 @@ Every head's o is divided by its root mean square, the heads are concatenated, m
 and by sigmoid(Wg h), then projected.  A request keeps S and n together as one float32 state
 [heads, dim, vdim + pad] (n is the column behind the values) and m as a second one [heads].  The
 walk over a step's tokens is the engine's state scan (`kernels.linear_attention.scan`), fed with
-float32 operands; the kernels of csrc/mlstm.cu come before and after it.
+float32 operands, or, for portions of a bfloat16 step, a walk in chunks on the tensor cores
+(`kernels.mlstm.chunked`); the kernels of csrc/mlstm.cu come before and after it.
 
 params: `hidden`, `heads`, `dim`, `vdim`, `gate_cap`, `eps`.
 tensors: `q`, `k` [heads * dim, hidden], `v`, `g` [heads * vdim, hidden], `o` [hidden, heads * vdim],
@@ -27,6 +28,9 @@ from .base import Part, StateRequest
 from .linear import Linear
 from .registry import register_mixer
 from ..weights.loader import fused_rows
+
+
+CHUNKED_MIN_TOKENS = 32      # steps whose longest portion has at least this many tokens walk in chunks on the tensor cores
 
 
 @register_mixer("mlstm")
@@ -70,6 +74,10 @@ class MLSTM(Part):
             lin.prepare(dtype)
         self.i_bias, self.f_bias = t["i_bias"].to(dtype).contiguous(), t["f_bias"].to(dtype).contiguous()
         self.norm_w = t["norm"].to(dtype).contiguous()
+        self.chunked = device.type == "cuda" and dtype == torch.bfloat16 and MK.chunked_takes(self.dim, self.vdim)
+        if self.chunked:
+            from ..kernels import mamba2
+            mamba2.chunked_lib(self.dim, self.vdim, MK.chunked_columns(self.dim), True)   # compiled with the model, not at its first portion
 
     def forward(self, ctx, call, h):
         n, H, dk, dv, dvp = ctx.n_tokens, self.heads, self.dim, self.vdim, self.vpad
@@ -83,13 +91,20 @@ class MLSTM(Part):
                     call.states[1], self.norm_w, out, H, dk, dv, dvp, dk ** -0.5, self.eps)
             return self.o.forward(ctx, out, n, torch.float32, "mixer_out", allow_partials=True)
         coef = ctx.ws.get("mlstm_coef", (n, H * 4), torch.float32)
+        scanned = ctx.ws.get("mlstm_scan", (n, H * dvp), torch.float32)
+        if self.chunked and ctx.use_fast_attention and ctx.max_q_len >= CHUNKED_MIN_TOKENS and u.stride(0) % 8 == 0 and u.data_ptr() % 16 == 0:
+            log_decay = ctx.ws.get("mlstm_log_decay", (n, H), torch.float32)
+            weight = ctx.ws.get("mlstm_weight", (n, H), torch.float32)
+            MK.gates(ctx, z, 0, H, self.i_bias, self.f_bias, self.cap, call.states[1], coef, H, log_decay, weight)
+            MK.chunked(ctx, u, 0, kd, 2 * kd, log_decay, weight, call.states[0], scanned, H, dk, dv, dk ** -0.5)
+            MK.finish(ctx, scanned, coef, self.norm_w, u[:, 2 * kd + vd:], out, H, dv, dvp, self.eps)
+            return self.o.forward(ctx, out, n, torch.float32, "mixer_out", allow_partials=True)
         MK.gates(ctx, z, 0, H, self.i_bias, self.f_bias, self.cap, call.states[1], coef, H)
         qf = ctx.ws.get("mlstm_q", (n, kd), torch.float32)
         kf = ctx.ws.get("mlstm_k", (n, kd), torch.float32)
         decay = ctx.ws.get("mlstm_decay", (n, H), torch.float32)
         vf = ctx.ws.get("mlstm_v", (n, H * dvp), torch.float32)
         MK.operands(ctx, u, 0, kd, 2 * kd, coef, qf, kf, decay, vf, H, dk, dv, dvp)
-        scanned = ctx.ws.get("mlstm_scan", (n, H * dvp), torch.float32)
         LA.scan(ctx, qf, kf, vf, decay, "token", call.states[0], scanned, H, dk, dvp, dk ** -0.5)
         MK.finish(ctx, scanned, coef, self.norm_w, u[:, 2 * kd + vd:], out, H, dv, dvp, self.eps)
         return self.o.forward(ctx, out, n, torch.float32, "mixer_out", allow_partials=True)

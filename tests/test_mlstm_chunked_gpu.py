@@ -1,0 +1,73 @@
+"""The walk of an mLSTM's matrix memory in chunks on the tensor cores against the recurrence in float64, beside the scan in
+float32 products that it stands in for."""
+
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _recurrence(q, k, v, a, b, S, n):
+    """All float64, one head: q, k [t, dk], v [t, dv], a, b [t]; returns [t, dv + 1] and the state after the last token."""
+    out = []
+    for t in range(q.shape[0]):
+        S = a[t] * S + b[t] * torch.outer(k[t], v[t])
+        n = a[t] * n + b[t] * k[t]
+        out.append(torch.cat([S.T @ q[t], (n @ q[t])[None]]))
+    return torch.stack(out), S, n
+
+
+@pytest.mark.parametrize("heads,dk,dv,lens,forget", [(2, 128, 128, [130, 64, 1], 2.0), (3, 16, 32, [65, 33, 200], 0.0), (1, 64, 16, [300], -4.0),
+                                                     (1, 256, 48, [100, 63], 6.0)])
+def test_mlstm_chunked(heads, dk, dv, lens, forget):
+    from bare_cuda_4gib_b200.kernels import lib as K, linear_attention as LA, mlstm as MK
+    torch.manual_seed(dk + dv)
+    rows, slots, dvp, cap = sum(lens), len(lens) + 2, dv + 4, 15.0
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    ctx = types.SimpleNamespace(seq_slot=ints([i + 1 for i in range(len(lens))]), seq_q_start=ints([sum(lens[:i]) for i in range(len(lens))]),
+                                seq_q_len=ints(lens), n_seqs=len(lens), n_tokens=rows, max_q_len=max(lens), stream=K.stream_handle(),
+                                dtype=torch.float32)
+    kd, vd = heads * dk, heads * dv
+    u = torch.randn(rows, 2 * kd + 2 * vd, device=DEV).to(torch.bfloat16)
+    z = torch.randn(rows, 2 * heads, device=DEV)
+    bias = [torch.randn(heads, device=DEV), forget + torch.randn(heads, device=DEV)]
+    m0 = torch.randn(slots, heads, device=DEV)
+    coef = torch.empty(rows, heads * 4, device=DEV)
+    la, b = torch.empty(rows, heads, device=DEV), torch.empty(rows, heads, device=DEV)
+    MK.gates(ctx, z, 0, heads, bias[0], bias[1], cap, m0.clone(), coef, heads, la, b)
+    assert torch.equal(coef.view(rows, heads, 4)[..., 1], b) and torch.allclose(coef.view(rows, heads, 4)[..., 0], la.exp(), rtol=1e-6, atol=0)
+    start = torch.randn(slots, heads, dk, dvp, device=DEV)
+    start[..., dv + 1:] = 0.0
+    state, out = start.clone(), torch.full((rows, heads * dvp), float("nan"), device=DEV)
+    MK.chunked(ctx, u, 0, kd, 2 * kd, la, b, state, out, heads, dk, dv, dk ** -0.5)
+    # the scan, in float32
+    qf, kf, vf = torch.empty(rows, kd, device=DEV), torch.empty(rows, kd, device=DEV), torch.empty(rows, heads * dvp, device=DEV)
+    decay, scanned, walked = torch.empty(rows, heads, device=DEV), torch.empty(rows, heads * dvp, device=DEV), start.clone()
+    MK.operands(ctx, u, 0, kd, 2 * kd, coef, qf, kf, decay, vf, heads, dk, dv, dvp)
+    LA.scan(ctx, qf, kf, vf, decay, "token", walked, scanned, heads, dk, dvp, dk ** -0.5)
+    far = {"chunked": 0.0, "scan": 0.0}
+    at = 0
+    for i, n in enumerate(lens):
+        for h in range(heads):
+            part = lambda col, d: u[at: at + n, col + h * d: col + (h + 1) * d].double().cpu()
+            q, k, v = part(0, dk) * dk ** -0.5, part(kd, dk), part(2 * kd, dv)
+            a64, b64 = la[at: at + n, h].double().exp().cpu(), b[at: at + n, h].double().cpu()
+            S0 = start[i + 1, h].double().cpu()
+            want, S, norm = _recurrence(q, k, v, a64, b64, S0[:, :dv], S0[:, dv])
+            size, _, _ = _recurrence(q.abs(), k.abs(), v.abs(), a64, b64, S0[:, :dv].abs(), S0[:, dv].abs())
+            for name, got, left in (("chunked", out, state), ("scan", scanned, walked)):
+                mine = got.view(rows, heads, dvp)[at: at + n, h].double().cpu()
+                far[name] = max(far[name], ((mine[:, : dv + 1] - want).abs() / size).max().item())
+                end = left[i + 1, h].double().cpu()
+                assert (end[:, :dv] - S).abs().max() <= 1e-5 * S.abs().max() and (end[:, dv] - norm).abs().max() <= 1e-5 * norm.abs().max()
+                assert not end[:, dv + 1:].any() and not mine[:, dv + 1:].any()
+        at += n
+    assert torch.equal(state[0], start[0]) and torch.equal(state[-1], start[-1])        # slots that no request of the step holds
+    # relative to the sum of the sizes of a result's terms: operands of 24 bits, exponentials of 2 units, and float32 sums of at
+    # most dk / 16 + 64 / 16 steps of three products each in the tensor core (2^-23 a step)
+    bound = (3 * (dk / 16 + 4) + 8) * 2.0 ** -23
+    assert far["chunked"] <= bound, (far, bound)
+    print(f"mlstm heads {heads} dk {dk} dv {dv}: chunked {far['chunked']:.2e} scan {far['scan']:.2e} bound {bound:.2e}")
