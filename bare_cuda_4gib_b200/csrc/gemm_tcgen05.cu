@@ -953,7 +953,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
 // product - exchange - stores, which is why eight warps share the epilogue.  (Storing the slices straight from registers into
 // the other blocks' shared memory, 16 bytes a lane, measured slower: 9.5 against 8.0 us for 64 tokens x 2,048 x 2,048.)
 enum { CL_STORE = 0, CL_ADD = 1, CL_SWIGLU = 2, CL_ROPE = 3 };
-constexpr int CL_MAX_TOKENS = 64;
+constexpr int CL_MAX_TOKENS = 64;         // of a tile; more tokens are more tiles, which read the weights again, from L2
 constexpr int CL_EPI_WARPS = 8, CL_EPI = CL_EPI_WARPS * 32, CL_THREADS = 64 + CL_EPI;
 constexpr int ERR_TIMEOUT_CLUSTER = 4;
 
@@ -1041,6 +1041,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
   const int rank = blockIdx.x % C, tile = blockIdx.x / C;
   constexpr int TILE_OUT = EPI == CL_SWIGLU ? BM / 2 : BM;
   const int f0 = tile * TILE_OUT;
+  const int t0 = blockIdx.y * a.bn, n_tokens = min(a.bn, a.n_tokens - t0);      // this block's tokens: rows t0 .. of everything
   const int kb_begin = rank * a.k_per_block, n_kb = max(0, min(a.k_blocks, kb_begin + a.k_per_block) - kb_begin);
 
   auto issue_weights = [&](int i, int s) {
@@ -1051,7 +1052,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     if (EPI == CL_SWIGLU) tma_load_2d(stage + A_BYTES / 2, &map_w, &full_bar[s], k0, a.up_row_offset + f0);
   };
   auto issue_activations = [&](int i, int s) {
-    tma_load_2d(smem + s * a.stage_bytes + A_BYTES, &map_a, &full_bar[s], (kb_begin + i) * BK, 0);
+    tma_load_2d(smem + s * a.stage_bytes + A_BYTES, &map_a, &full_bar[s], (kb_begin + i) * BK, t0);
   };
   const int n_early = min(n_kb, a.stages);
 
@@ -1066,7 +1067,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(received_bar, (uint32_t)(C * a.n_tokens * ROWS * 4));
+    mbar_expect_tx(received_bar, (uint32_t)(C * n_tokens * ROWS * 4));
     for (int i = 0; i < n_early; ++i) issue_weights(i, i);   // overlaps the tail of the kernel before
     pdl_wait();
     for (int i = 0; i < n_early; ++i) issue_activations(i, i);
@@ -1151,12 +1152,12 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
       for (int i = ew; i < a.sq_items; i += CL_EPI_WARPS)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-          if (lane + 32 * j < a.n_tokens) sq[j] += a.sq_in[(long long)i * a.sq_stride + lane + 32 * j];
+          if (lane + 32 * j < n_tokens) sq[j] += a.sq_in[(long long)i * a.sq_stride + t0 + lane + 32 * j];
 #pragma unroll
       for (int j = 0; j < 2; ++j)
-        if (lane + 32 * j < a.n_tokens) sq_part[ew * a.bn + lane + 32 * j] = sq[j];
+        if (lane + 32 * j < n_tokens) sq_part[ew * a.bn + lane + 32 * j] = sq[j];
       asm volatile("bar.sync 1, %0;" ::"n"(CL_EPI) : "memory");
-      if (e < a.n_tokens) {
+      if (e < n_tokens) {
         float total = 0.0f;
 #pragma unroll
         for (int i = 0; i < CL_EPI_WARPS; ++i) total += sq_part[i * a.bn + e];
@@ -1177,8 +1178,8 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     const int head = first_pair / span, entry = first_pair % span;       // CL_ROPE: of [q; k; v]
     const bool turned = EPI == CL_ROPE && a.inv_freq && head < a.q_heads + a.cache.kv_heads;
     if (EPI == CL_ADD && f_plain + 4 <= a.n_features) {
-      if (first_token < a.n_tokens) {
-        const float4 o = *reinterpret_cast<const float4*>(static_cast<const float*>(a.out) + (long long)first_token * a.ld_out + f_plain);
+      if (first_token < n_tokens) {
+        const float4 o = *reinterpret_cast<const float4*>(static_cast<const float*>(a.out) + (long long)(t0 + first_token) * a.ld_out + f_plain);
         old[0] = o.x, old[1] = o.y, old[2] = o.z, old[3] = o.w;
       }
       if (a.pre_x) {
@@ -1188,9 +1189,9 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
                                               : static_cast<const float*>(a.pre_w)[f_plain + j];
       }
     }
-    if (turned && first_token < a.n_tokens)
+    if (turned && first_token < n_tokens)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) sincosf((float)a.positions[first_token] * a.inv_freq[entry + j], &rot_s[j], &rot_c[j]);
+      for (int j = 0; j < 2; ++j) sincosf((float)a.positions[t0 + first_token] * a.inv_freq[entry + j], &rot_s[j], &rot_c[j]);
 
     bool ok = mbar_wait(acc_bar, 0, abort_flag, a.wait_ns);
     if (!ok) {
@@ -1201,7 +1202,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     // Two groups of four warps take half of the tokens each: the accumulator, cut into slices, into the pipeline's
     // stages (idle by now), then one bulk copy to every block of the cluster.
     const int part = ew / 4, part_tokens = (a.bn / 2 + 15) / 16 * 16, t_begin = part * part_tokens;
-    const int t_end = min(a.n_tokens, t_begin + part_tokens);
+    const int t_end = min(n_tokens, t_begin + part_tokens);
     float* outgoing = reinterpret_cast<float*>(smem);
     if (ok) {
       const int row = quad * 32 + lane, in_group = row % (2 * a.pair_span);
@@ -1255,16 +1256,16 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
           for (int j = 0; j < RUN; ++j) v[j] *= f;
         }
       };
-      const int rounds = (a.n_tokens + TOKEN_STEP - 1) / TOKEN_STEP;
+      const int rounds = (n_tokens + TOKEN_STEP - 1) / TOKEN_STEP;
 #pragma unroll 1
       for (int i = 0; i < rounds; ++i) {
-        const int t = first_token + i * TOKEN_STEP;
-        const bool there = t < a.n_tokens;
+        const int mine = first_token + i * TOKEN_STEP, t = t0 + mine;
+        const bool there = mine < n_tokens;
         float v[RUN];
         if (EPI == CL_ADD || EPI == CL_STORE) {
           float sq = 0.0f;
           if (there && f_plain + 4 <= a.n_features) {         // (the width is a multiple of four)
-            summed(t, at, v);
+            summed(mine, at, v);
             const long long where = (long long)t * a.ld_out + f_plain;
             if (EPI == CL_STORE) {
               if (a.out_is_f32) store_run(static_cast<float*>(a.out) + where, v);
@@ -1293,8 +1294,8 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
           }
         } else if (there) {
           float u[RUN];
-          summed(t, at, v);
-          summed(t, HALF + at, u);
+          summed(mine, at, v);
+          summed(mine, HALF + at, u);
           if (EPI == CL_SWIGLU) {
             const int f = f0 + rank * HALF + at;
             if (f + RUN > a.n_features) continue;
@@ -1429,7 +1430,7 @@ int launch_cluster(const ClusterArgs& a, size_t smem, int tiles, const CUtensorM
     configured = smem;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * C);
+  cfg.gridDim = dim3(tiles * C, (a.n_tokens + a.bn - 1) / a.bn);
   cfg.blockDim = dim3(CL_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -1660,8 +1661,8 @@ extern "C" int llm_turn_table(const int32_t* positions, const float* inv_freq, f
 }
 
 // The product of a few dozen tokens with its ends fused in (see gemm_cluster_kernel): `cluster` (1, 2, 4 or 8)
-// blocks share a tile of 128 weight rows.  map_w's box has 128 rows (64 for CL_SWIGLU), map_a's bn rows, bn the
-// tokens rounded up to a multiple of 16.  `pair_span` (CL_ROPE: head_dim / 2).  CL_ADD: out is the float32 residual
+// blocks share a tile of 128 weight rows and bn tokens (a multiple of 16, at most 64).  map_w's box has 128 rows (64 for
+// CL_SWIGLU), map_a's bn rows.  `pair_span` (CL_ROPE: head_dim / 2).  CL_ADD: out is the float32 residual
 // stream; pre_x, pre_w, pre_sq as for llm_gemm_bf16, with one row of parts per slice of 128 / cluster rows.
 extern "C" int llm_gemm_cluster(const void* map_w, const void* map_a, int epi, int cluster, int bn, int n_tokens, int n_features,
                                 int K, void* out, int out_dtype, long long ld_out, int up_row_offset, const float* sq_in,
@@ -1671,7 +1672,7 @@ extern "C" int llm_gemm_cluster(const void* map_w, const void* map_a, int epi, i
                                 int page_tokens, int kv_heads, int head_dim, const int32_t* positions, const int32_t* row_seq,
                                 const float* inv_freq, int q_heads, int write_cache, int* error_word, cudaStream_t stream) {
   if (n_tokens <= 0 || n_features <= 0) return 0;
-  if (n_tokens > CL_MAX_TOKENS || bn < 16 || bn > CL_MAX_TOKENS || bn % 16 || n_tokens > bn || K <= 0 || n_features % 4) return ERR_BAD_SIZE;
+  if (bn < 16 || bn > CL_MAX_TOKENS || bn % 16 || (n_tokens + bn - 1) / bn > 65535 || K <= 0 || n_features % 4) return ERR_BAD_SIZE;
   if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ERR_BAD_SIZE;
   if (out_dtype != DT_F32 && out_dtype != DT_BF16) return ERR_BAD_DTYPE;
   if ((reinterpret_cast<uintptr_t>(out) & 15) || ld_out % 4) return ERR_BAD_ALIGN;

@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
       split_store(Xt + r * LDP + c, L * LDP, __bfloat162float(Xs[r * LDP + c]) * (expf(between(cum_last, rest_last, r)) * dts[r]));
     }
 
-    // ---- this warp's 16 tokens i, 16 tokens j <= i at a time: G = C B^T, the weights (C_i . B_j) exp(cum_i - cum_j) dt_j as A
+    // ---- this warp's 16 tokens i against the tokens j <= i: G = C B^T, the weights (C_i . B_j) exp(cum_i - cum_j) dt_j as A
     // fragments, split, and their product with x
     uint32_t cf[N / 16][4];
 #pragma unroll
@@ -286,45 +286,94 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
       o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.0f;
       y2[nt][0] = y2[nt][1] = y2[nt][2] = y2[nt][3] = 0.0f;
     }
-#pragma unroll (TERMS < 3 ? L / 16 : 1)
-    for (int kk = 0; kk < L / 16; ++kk) {
-      if (kk > warp) break;
-      float s[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+    if constexpr (TERMS < 3) {
+      // all of the chunk's tokens j at once: more products in flight than 16 at a time (2.17 against 2.20 ms a prompt of the
+      // 4-layer Gurolix model)
+      float s[L / 8][4];
+#pragma unroll
+      for (int nt = 0; nt < L / 8; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
 #pragma unroll
       for (int ks = 0; ks < N / 16; ++ks) {
-        uint32_t bf[4];
-        ldmatrix_x4(bf, Bs + (kk * 16 + (mid >> 1) * 8 + (lane & 7)) * LDN + ks * 16 + (mid & 1) * 8);
-        const auto c_of = [&](int) -> const uint32_t(&)[4] { return cf[ks]; };
-        mma_split<1>(s[0], c_of, [&](int, int half) { return bf[half]; });
-        mma_split<1>(s[1], c_of, [&](int, int half) { return bf[2 + half]; });
-      }
-      uint32_t wt[TERMS][4];
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
+        for (int nt = 0; nt < L / 8; nt += 2) {
+          uint32_t bf[4];
+          ldmatrix_x4(bf, Bs + ((nt + (mid >> 1)) * 8 + (lane & 7)) * LDN + ks * 16 + (mid & 1) * 8);
+          mma_bf16(s[nt], cf[ks], bf[0], bf[1]);
+          mma_bf16(s[nt + 1], cf[ks], bf[2], bf[3]);
+        }
+      }
+      uint32_t wt[TERMS][L / 16][4];
+#pragma unroll
+      for (int nt = 0; nt < L / 8; ++nt) {
         float w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int i = (e >> 1) ? i1 : i0, j = kk * 16 + nt * 8 + tq * 2 + (e & 1);
-          w[e] = j <= i ? s[nt][e] * expf(between((e >> 1) ? ci1 : ci0, (e >> 1) ? ri1 : ri0, j)) * dts[j] : 0.0f;
+          const int i = (e >> 1) ? i1 : i0, j = nt * 8 + tq * 2 + (e & 1);
+          w[e] = j <= i ? s[nt][e] * expf(((e >> 1) ? ci1 : ci0) - cum[j]) * dts[j] : 0.0f;
         }
 #pragma unroll
         for (int t = 0; t < TERMS; ++t) {
-          wt[t][nt * 2 + 0] = pack_bf16(w[0], w[1]);
-          wt[t][nt * 2 + 1] = pack_bf16(w[2], w[3]);
+          wt[t][nt / 2][(nt & 1) * 2 + 0] = pack_bf16(w[0], w[1]);
+          wt[t][nt / 2][(nt & 1) * 2 + 1] = pack_bf16(w[2], w[3]);
 #pragma unroll
           for (int e = 0; e < 4; ++e) w[e] -= rounded(w[e]);
         }
       }
+      __syncthreads();      // Xt is complete (the state's product below reads it)
 #pragma unroll
-      for (int nt = 0; nt < NT; nt += 2) {
-        uint32_t xf[4];
-        ldmatrix_x4_trans(xf, Xs + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
-        const auto w_of = [&](int t) -> const uint32_t(&)[4] { return wt[t]; };
-        mma_split<TERMS>(o[nt], w_of, [&](int, int half) { return xf[half]; });
-        mma_split<TERMS>(o[nt + 1], w_of, [&](int, int half) { return xf[2 + half]; });
+      for (int kk = 0; kk < L / 16; ++kk) {
+#pragma unroll
+        for (int nt = 0; nt < NT; nt += 2) {
+          uint32_t xf[4];
+          ldmatrix_x4_trans(xf, Xs + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
+#pragma unroll
+          for (int t = 0; t < TERMS; ++t) {
+            mma_bf16(o[nt], wt[t][kk], xf[0], xf[1]);
+            mma_bf16(o[nt + 1], wt[t][kk], xf[2], xf[3]);
+          }
+        }
       }
+    } else {
+      // 16 tokens j at a time
+#pragma unroll 1
+      for (int kk = 0; kk <= warp; ++kk) {
+        float s[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+#pragma unroll
+        for (int ks = 0; ks < N / 16; ++ks) {
+          uint32_t bf[4];
+          ldmatrix_x4(bf, Bs + (kk * 16 + (mid >> 1) * 8 + (lane & 7)) * LDN + ks * 16 + (mid & 1) * 8);
+          const auto c_of = [&](int) -> const uint32_t(&)[4] { return cf[ks]; };
+          mma_split<1>(s[0], c_of, [&](int, int half) { return bf[half]; });
+          mma_split<1>(s[1], c_of, [&](int, int half) { return bf[2 + half]; });
+        }
+        uint32_t wt[TERMS][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          float w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = (e >> 1) ? i1 : i0, j = kk * 16 + nt * 8 + tq * 2 + (e & 1);
+            w[e] = j <= i ? s[nt][e] * expf(between((e >> 1) ? ci1 : ci0, (e >> 1) ? ri1 : ri0, j)) * dts[j] : 0.0f;
+          }
+#pragma unroll
+          for (int t = 0; t < TERMS; ++t) {
+            wt[t][nt * 2 + 0] = pack_bf16(w[0], w[1]);
+            wt[t][nt * 2 + 1] = pack_bf16(w[2], w[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] -= rounded(w[e]);
+          }
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; nt += 2) {
+          uint32_t xf[4];
+          ldmatrix_x4_trans(xf, Xs + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
+          const auto w_of = [&](int t) -> const uint32_t(&)[4] { return wt[t]; };
+          mma_split<TERMS>(o[nt], w_of, [&](int, int half) { return xf[half]; });
+          mma_split<TERMS>(o[nt + 1], w_of, [&](int, int half) { return xf[2 + half]; });
+        }
+      }
+      __syncthreads();      // Xt is complete (the state's product below reads it)
     }
-    __syncthreads();      // Xt is complete (the state's product below reads it)
     // ---- y = weights x  +  exp(cum_i) C S
 #pragma unroll
     for (int ks = 0; ks < N / 16; ++ks) {

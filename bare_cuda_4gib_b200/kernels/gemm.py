@@ -327,15 +327,30 @@ def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
 # ------------------------------------------------------------------ a few dozen tokens, ends fused in
 CL_STORE, CL_ADD, CL_SWIGLU, CL_ROPE = 0, 1, 2, 3
 # Measured, a whole step of TinyLlama's 22 layers, product + norm + rotation kernels against this: 25 rows 1,187 -> 989 us,
-# 32 rows 1,221 -> 1,011, 48 rows 1,338 -> 1,141, 64 rows 1,379 -> 1,245; with a tile of 96 or 128 tokens a block's shared
-# memory fills an SM and the step is slower (96 rows 1,513 -> 1,971, 128 rows 1,600 -> 3,084).
-CLUSTER_MAX_ROWS = 64
+# 32 rows 1,208 -> 1,009, 48 rows 1,330 -> 1,125, 64 rows 1,376 -> 1,129, 96 rows 1,502 -> 1,218, 128 rows 1,599 -> 1,286,
+# 192 rows 1,955 -> 1,546, 240 rows 2,148 -> 1,591; eight layers of the Llama-3-8B sizes: 32 rows 1,067 -> 1,012, 64 rows
+# 1,191 -> 1,148, 128 rows 1,306 -> 1,243, 240 rows 1,900 -> 1,735.  Above, tokens are on the MMA rows.
+CLUSTER_MAX_ROWS = TOKENS_ON_ROWS_ABOVE
+# A tile of 96 or 128 tokens would fill an SM's shared memory with one block (96 rows 1,971 us, 128 rows 3,084).
+CLUSTER_TILE_ROWS = 64
+# A gated product has enough tiles; with more rows than a tile's it runs with tokens on the MMA rows (16.3 us up to 128 rows).
+CLUSTER_GATED_ROWS = 64
 # With so few rows that the few-token product (gemv.py) takes the layer's other products, what comes here is a down
 # projection whose input does not fit beside its ring.  A small one gains (12 rows x 2,048 x 5,632, 23 MB: the step 904 -> 873 us),
 # a large one is bound by its weights, which the split product's deeper ring streams faster (8 rows x 4,096 x 14,336, 117 MB:
 # 18.0 us and a norm kernel of 4.3 against 23.5).
 CLUSTER_FEW_ROWS, CLUSTER_FEW_BYTES = 24, 64 << 20
 CLUSTER_MIN_K = 8 * BK      # shorter sums are too short to share: a block of the cluster would have no K block to itself
+
+
+def cluster_tile(rows: int, n_tiles: int) -> int:
+    """Tokens of a tile: the rows dealt out evenly over as few tiles as hold them, in steps of 16.  With few tiles of weight
+    rows 49 to 64 rows go in two tiles of 32: the exchange is what a block's tokens lengthen, and SMs are free
+    (TinyLlama, 16 and 20 tiles, 61 rows: 1,226 -> 1,127 us; with 32 to 48 tiles there is no room for twice the blocks)."""
+    tiles = -(-rows // CLUSTER_TILE_ROWS)
+    if 48 < rows <= 64 and 14 * n_tiles <= 2 * sm_count():
+        tiles = 2
+    return -(-rows // (16 * tiles)) * 16
 
 
 def cluster_size(n_tiles: int, k: int) -> int:
@@ -351,7 +366,7 @@ def cluster_kind(plan: GemmPlan, rows: int, out_dtype, swiglu: bool, epilogue) -
     if plan.k < CLUSTER_MIN_K or not 0 < rows <= CLUSTER_MAX_ROWS or plan.n % 8 or (rows <= CLUSTER_FEW_ROWS and 2 * plan.n * plan.k > CLUSTER_FEW_BYTES):
         return None
     if swiglu:
-        return CL_SWIGLU
+        return CL_SWIGLU if rows <= CLUSTER_GATED_ROWS else None      # (more rows: tokens on the MMA rows, one tile for 128 of them)
     if isinstance(epilogue, AddTo):
         r = epilogue.residual
         fits = (r.dtype == torch.float32 and r.shape[-1] == plan.n and r.stride(-1) == 1 and r.stride(0) % 4 == 0
@@ -382,8 +397,8 @@ def run_cluster(ctx, plan: GemmPlan, kind: int, a, rows: int, out_dtype: torch.d
         raise KernelLaunchError(f"gemm_cluster: activations {tuple(a.shape)} {a.dtype} do not fit weight [{plan.n}, {plan.k}]")
     n_out = plan.n // 2 if kind == CL_SWIGLU else plan.n
     tiles = -(-n_out // (BM // 2 if kind == CL_SWIGLU else BM))
-    cluster = cluster_size(tiles, plan.k)
-    bn = -(-rows // 16) * 16
+    bn = cluster_tile(rows, tiles)
+    cluster = cluster_size(tiles * -(-rows // bn), plan.k)
     pre = None
     extra_out, rope = (0, 0, 0, 0, 0, 0), (0, 0, 0, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0)
     if kind == CL_ADD:

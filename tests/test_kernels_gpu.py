@@ -376,7 +376,8 @@ def test_gemm_tcgen05_swiglu(m, inter, k):
 
 
 @pytest.mark.parametrize("rows,n,k", [(1, 128, 64), (16, 136, 72), (17, 2048, 2048), (33, 2560, 200), (48, 320, 5632), (63, 1000, 1024),
-                                      (64, 2048, 5632), (8, 2048, 14336), (8, 4096, 14336), (25, 72, 1088)])
+                                      (64, 2048, 5632), (8, 2048, 14336), (8, 4096, 14336), (25, 72, 1088), (65, 2048, 2048), (100, 136, 600),
+                                      (129, 2048, 1024), (240, 256, 2048)])
 @pytest.mark.parametrize("prenormed", [False, True])
 def test_gemm_cluster_adds_prepares_and_gates(rows, n, k, prenormed):
     """The product whose blocks exchange their parts through distributed shared memory: into the residual stream with the
@@ -415,7 +416,7 @@ def test_gemm_cluster_adds_prepares_and_gates(rows, n, k, prenormed):
         _close(got, gate / (1 + torch.exp(-gate)) * up, 2 ** -8, 1e-4 + 2 ** -18 * size)
 
 
-@pytest.mark.parametrize("rows,heads,kv_heads,d,rotate", [(25, 8, 2, 64, True), (64, 3, 1, 128, True), (40, 5, 2, 32, True), (33, 2, 1, 8, False)])
+@pytest.mark.parametrize("rows,heads,kv_heads,d,rotate", [(25, 8, 2, 64, True), (64, 3, 1, 128, True), (40, 5, 2, 32, True), (33, 2, 1, 8, False), (80, 8, 2, 64, True)])
 def test_gemm_cluster_rotates_and_writes_the_cache(rows, heads, kv_heads, d, rotate, monkeypatch):
     from bare_cuda_4gib_b200.kernels import gemm
     from bare_cuda_4gib_b200.kernels import lib as K
