@@ -344,11 +344,11 @@ CLUSTER_MIN_K = 8 * BK      # shorter sums are too short to share: a block of th
 
 
 def cluster_tile(rows: int, n_tiles: int) -> int:
-    """Tokens of a tile: the rows dealt out evenly over as few tiles as hold them, in steps of 16.  With few tiles of weight
-    rows 49 to 64 rows go in two tiles of 32: the exchange is what a block's tokens lengthen, and SMs are free
-    (TinyLlama, 16 and 20 tiles, 61 rows: 1,226 -> 1,127 us; with 32 to 48 tiles there is no room for twice the blocks)."""
+    """Tokens of a tile: the rows dealt out evenly over as few tiles as hold them, in steps of 16.  49 to 64 rows go in two
+    tiles where the twice as many blocks still fit two to an SM: the exchange at a tile's end lengthens with its tokens
+    (TinyLlama, 61 rows: 1,226 -> 1,127 us; the 224 tiles of the Llama-3-8B gate/up would queue, 64 rows 1,148 -> 1,349)."""
     tiles = -(-rows // CLUSTER_TILE_ROWS)
-    if 48 < rows <= 64 and 14 * n_tiles <= 2 * sm_count():
+    if 48 < rows <= 64 and n_tiles <= sm_count():
         tiles = 2
     return -(-rows // (16 * tiles)) * 16
 
