@@ -941,7 +941,6 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
 // layer, 4 to 6 us each).  Here the blocks that share a tile's K range are a cluster: each turns its
 // accumulator over to the others in slices (bulk copies through distributed shared memory), so block r
 // ends up with all parts of slice r, adds them in the order of the blocks and finishes the outputs:
-//   CL_STORE   plain store
 //   CL_ADD     residual[t, f] += result, and what the next norm's product needs (see RowsExtra)
 //   CL_SWIGLU  w = [gate; up]: act(gate) * up
 //   CL_ROPE    w = [Wq; Wk; Wv]: q and k rotated by position, q to `out`, k and v into the paged cache
@@ -952,7 +951,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
 // the kernel before it still runs on the other half.  What bounds it: the chain wait for the input - first tile - last
 // product - exchange - stores, which is why eight warps share the epilogue.  (Storing the slices straight from registers into
 // the other blocks' shared memory, 16 bytes a lane, measured slower: 9.5 against 8.0 us for 64 tokens x 2,048 x 2,048.)
-enum { CL_STORE = 0, CL_ADD = 1, CL_SWIGLU = 2, CL_ROPE = 3 };
+enum { CL_ADD = 1, CL_SWIGLU = 2, CL_ROPE = 3 };
 constexpr int CL_MAX_TOKENS = 64;         // of a tile; more tokens are more tiles, which read the weights again, from L2
 constexpr int CL_EPI_WARPS = 8, CL_EPI = CL_EPI_WARPS * 32, CL_THREADS = 64 + CL_EPI;
 constexpr int ERR_TIMEOUT_CLUSTER = 4;
@@ -1171,7 +1170,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     constexpr int RUN = EPI == CL_ROPE ? 2 : 4, PER_TOKEN = (PAIRED ? HALF : ROWS) / RUN, TOKEN_STEP = CL_EPI / PER_TOKEN;
     static_assert(PER_TOKEN <= 32, "a token's threads lie in one warp");
     const int at = e % PER_TOKEN * RUN, first_token = e / PER_TOKEN;     // first row of the slice that the thread owns
-    const int f_plain = f0 + rank * ROWS + at;                           // CL_ADD, CL_STORE: its feature
+    const int f_plain = f0 + rank * ROWS + at;                           // CL_ADD: its feature
     float old[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pre_w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     float rot_c[2] = {1.0f, 1.0f}, rot_s[2] = {0.0f, 0.0f};
     const int dim = a.cache.head_dim, span = max(dim / 2, 1), first_pair = tile * 64 + rank * HALF + at;
@@ -1262,32 +1261,27 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
         const int mine = first_token + i * TOKEN_STEP, t = t0 + mine;
         const bool there = mine < n_tokens;
         float v[RUN];
-        if (EPI == CL_ADD || EPI == CL_STORE) {
+        if (EPI == CL_ADD) {
           float sq = 0.0f;
           if (there && f_plain + 4 <= a.n_features) {         // (the width is a multiple of four)
             summed(mine, at, v);
             const long long where = (long long)t * a.ld_out + f_plain;
-            if (EPI == CL_STORE) {
-              if (a.out_is_f32) store_run(static_cast<float*>(a.out) + where, v);
-              else store_run(static_cast<__nv_bfloat16*>(a.out) + where, v);
-            } else {
-              float* res = static_cast<float*>(a.out) + where;
-              if (i > 0) {
-                const float4 o = *reinterpret_cast<const float4*>(res);
-                old[0] = o.x, old[1] = o.y, old[2] = o.z, old[3] = o.w;
-              }
+            float* res = static_cast<float*>(a.out) + where;
+            if (i > 0) {
+              const float4 o = *reinterpret_cast<const float4*>(res);
+              old[0] = o.x, old[1] = o.y, old[2] = o.z, old[3] = o.w;
+            }
 #pragma unroll
-              for (int j = 0; j < RUN; ++j) v[j] += old[j];
-              store_run(res, v);
-              if (a.pre_x) {
-                float w[RUN];
+            for (int j = 0; j < RUN; ++j) v[j] += old[j];
+            store_run(res, v);
+            if (a.pre_x) {
+              float w[RUN];
 #pragma unroll
-                for (int j = 0; j < RUN; ++j) w[j] = v[j] * pre_w[j], sq += v[j] * v[j];
-                store_run(a.pre_x + (long long)t * a.pre_x_stride + f_plain, w);
-              }
+              for (int j = 0; j < RUN; ++j) w[j] = v[j] * pre_w[j], sq += v[j] * v[j];
+              store_run(a.pre_x + (long long)t * a.pre_x_stride + f_plain, w);
             }
           }
-          if (EPI == CL_ADD && a.pre_x) {
+          if (a.pre_x) {
 #pragma unroll
             for (int o = 1; o < PER_TOKEN; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
             if (at == 0 && there) a.pre_sq[(long long)(tile * C + rank) * a.pre_sq_stride + t] = sq;
@@ -1699,8 +1693,6 @@ extern "C" int llm_gemm_cluster(const void* map_w, const void* map_a, int epi, i
   memcpy(&ma, map_a, sizeof(CUtensorMap));
   int rows = n_features;
   switch (epi) {
-    case CL_STORE:
-      return launch_cluster_of<CL_STORE>(cluster, a, smem, (rows + BM - 1) / BM, mw, ma, stream);
     case CL_ADD:
       if (out_dtype != DT_F32) return ERR_BAD_DTYPE;
       if (pre_x) {

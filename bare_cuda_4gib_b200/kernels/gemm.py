@@ -325,7 +325,7 @@ def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
 
 
 # ------------------------------------------------------------------ a few dozen tokens, ends fused in
-CL_STORE, CL_ADD, CL_SWIGLU, CL_ROPE = 0, 1, 2, 3
+CL_ADD, CL_SWIGLU, CL_ROPE = 1, 2, 3
 # Measured, a whole step of TinyLlama's 22 layers, product + norm + rotation kernels against this: 25 rows 1,187 -> 989 us,
 # 32 rows 1,208 -> 1,009, 48 rows 1,330 -> 1,125, 64 rows 1,376 -> 1,129, 96 rows 1,502 -> 1,218, 128 rows 1,599 -> 1,286,
 # 192 rows 1,955 -> 1,546, 240 rows 2,148 -> 1,591; eight layers of the Llama-3-8B sizes: 32 rows 1,067 -> 1,012, 64 rows
