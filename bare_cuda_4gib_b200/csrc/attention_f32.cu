@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
       span_state<ROWS>(base + Shared::Q + warp * ROWS * D * 4, at, at + SPAN_BYTES, p, held + slot * SPAN, span, first, last, a.scale, lane, m, l, o);
 #pragma unroll
       for (int i = 0; i < ROWS; ++i) {
-        if (m[i] == -INFINITY) continue;
+        if (l[i] == 0.0f) continue;          // nothing seen (a score of NaN is seen: it makes l NaN, whatever m is)
         const Join join(M[i], m[i]);
         M[i] = join.m;
         L[i] = join(L[i], l[i]);
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
         const uint32_t at = base + Shared::STATES + (s / CLUSTER) * (STATE_FLOATS * 4);
         const float m = peer_float(at + rank * 4, s % CLUSTER), l = peer_float(at + (ROWS + rank) * 4, s % CLUSTER);
         const float o = peer_float(at + (2 * ROWS + rank * D + threadIdx.x) * 4, s % CLUSTER);
-        if (m == -INFINITY) continue;
+        if (l == 0.0f) continue;
         const Join join(M, m);
         M = join.m;
         L = join(L, l);

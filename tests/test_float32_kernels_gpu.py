@@ -125,3 +125,18 @@ def test_add_rmsnorm_f32(rows, hidden, partials):
     assert ((residual.double() - want).abs() <= (partials + 1) * 2 * EPS * (x.abs() + delta.abs().sum(0)).double()).all()
     # the sum of squares adds up at most 16 terms a thread and 10 levels of the block, the factor rounds four times more
     assert ((out.double() - normed).abs() <= ((16 + 10) / 2 + 6 + 2 * partials) * 2 * EPS * normed.abs() + 1e-6).all()
+
+
+def test_attention_f32_keeps_nan_in_its_row():
+    """A query of NaN gives a row of NaN, whether its keys fill a span or not, and no other row changes."""
+    torch.manual_seed(9)
+    seqs = [(1, 10), (1, 300), (2, 128), (70, 70), (66, 200)]
+    case = _Attention(64, 1, 4, seqs, 0, 32)
+    parts = [(s, 0, n) for s, (n, _) in enumerate(seqs)]
+    clean = case.run(parts)
+    bad = [0, 1, 3, case.at[3], case.at[3] + 64, case.at[4] + 5]
+    case.q[bad] = float("nan")
+    got = case.run(parts)
+    assert got[bad].isnan().all()
+    others = [r for r in range(clean.shape[0]) if r not in bad]
+    assert torch.equal(got[others], clean[others])
