@@ -15,8 +15,9 @@
 //          (One warp for all eight rows of a span: 19.3 us a layer for 4 requests of up to 300 keys, a warp a row 13.7.)
 // What bounds it: shared-memory wavefronts in the walk (24 of them for 32 packed FMAs), latency with few rows.
 //
-// A key that no row of a tile sees, or whose page is not held, is zero in shared memory; in a span that some
-// row of a warp sees in part only, a weight of zero skips the value (which may be anything).
+// A key that no row of a tile sees, or whose page is not held, is zero in shared memory.  A weight of zero (the key is not
+// seen, or its weight underflows beside the span's largest) skips the value, which may be anything, infinity or NaN
+// too; so does a span that underflows beside the rest of a row.
 #include "common.cuh"
 
 #ifndef HEAD_DIM
@@ -96,6 +97,7 @@ struct Join {
     before = m_before == -INFINITY ? 0.0f : expf(m_before - m);
     now = m_span == -INFINITY ? 0.0f : expf(m_span - m);
   }
+  __device__ __forceinline__ bool underflows(float m_span) const { return now == 0.0f && m_span != -INFINITY; }
   __device__ __forceinline__ float operator()(float x_before, float x_span) const {
     return __fmaf_rn(x_before, before, __fmul_rn(x_span, now));
   }
@@ -127,21 +129,21 @@ __device__ __forceinline__ void span_state(uint32_t q, uint32_t keys, uint32_t v
   }
   const int j0 = span * SPAN + lane, j1 = j0 + 32;
   const bool held0 = held[lane] != 0, held1 = held[lane + 32] != 0;
-  bool whole = true;
+  bool none_zero = true;
 #pragma unroll
   for (int i = 0; i < NR; ++i) {
-    whole = whole && first[i] <= span * SPAN && last[i] >= span * SPAN + SPAN - 1;
     const float2 d0 = unpack(dot[i][0]), d1 = unpack(dot[i][1]);
     const float s0 = held0 && j0 >= first[i] && j0 <= last[i] ? __fmul_rn(__fadd_rn(d0.x, d0.y), scale) : -INFINITY;
     const float s1 = held1 && j1 >= first[i] && j1 <= last[i] ? __fmul_rn(__fadd_rn(d1.x, d1.y), scale) : -INFINITY;
     m[i] = warp_max(fmaxf(s0, s1));
     const float p0 = s0 == -INFINITY ? 0.0f : expf(s0 - m[i]);
     const float p1 = s1 == -INFINITY ? 0.0f : expf(s1 - m[i]);
+    none_zero = none_zero && p0 != 0.0f && p1 != 0.0f;
     l[i] = warp_sum(__fadd_rn(p0, p1));
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(p + (i * SPAN + lane) * 4), "f"(p0));
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(p + (i * SPAN + lane + 32) * 4), "f"(p1));
   }
-  __syncwarp();
+  none_zero = __all_sync(0xffffffffu, none_zero);       // then no weight has to be looked at below
 #pragma unroll
   for (int i = 0; i < NR; ++i)
 #pragma unroll
@@ -162,7 +164,7 @@ __device__ __forceinline__ void span_state(uint32_t q, uint32_t keys, uint32_t v
                    : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]) : "r"(p + (i * SPAN + j) * 4));
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (whole || w[u] != 0.0f)
+        if (none_zero || w[u] != 0.0f)
 #pragma unroll
           for (int c = 0; c < PAIRS; ++c) fma_pair(o[i][c], pack(w[u], w[u]), v[u][c]);
     }
@@ -250,6 +252,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
       for (int i = 0; i < ROWS; ++i) {
         if (l[i] == 0.0f) continue;          // nothing seen (a score of NaN is seen: it makes l NaN, whatever m is)
         const Join join(M[i], m[i]);
+        if (join.underflows(m[i])) continue;
         M[i] = join.m;
         L[i] = join(L[i], l[i]);
 #pragma unroll
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
         const float o = peer_float(at + (2 * ROWS + rank * D + threadIdx.x) * 4, s % CLUSTER);
         if (l == 0.0f) continue;
         const Join join(M, m);
+        if (join.underflows(m)) continue;
         M = join.m;
         L = join(L, l);
         O = join(O, o);

@@ -140,3 +140,29 @@ def test_attention_f32_keeps_nan_in_its_row():
     assert got[bad].isnan().all()
     others = [r for r in range(clean.shape[0]) if r not in bad]
     assert torch.equal(got[others], clean[others])
+
+
+def test_attention_f32_of_infinite_values_hangs_on_the_row_alone():
+    """Values of infinity behind keys whose weights underflow to zero: a row comes out finite or not by what it sees, not by
+    the rows beside it in a step, and finite here, as the plain kernel has it."""
+    from bare_cuda_4gib_b200.kernels import lib as K
+    torch.manual_seed(10)
+    seqs = [(1, 200), (70, 200), (130, 130)]
+    case = _Attention(64, 1, 2, seqs, 0, 32)
+    case.q.view(-1, 2, 64)[:, :, 0] = 8.0          # scores (8 k[0] / 8 and about 1 from the rest): 150 at key 5, -100 and -130 at two
+    for s, (_, kv) in enumerate(seqs):
+        for key in range(kv):
+            page = case.pool[case.table[s, key // 32].long()].view(2, 32, 64)
+            page[0, key % 32, 0] = {5: 150.0, 7: -100.0, 75: -130.0}.get(key, 0.0)
+            if key in (7, 75, 80):                 # beside key 5; beside the keys of its own span; a span that key 5 puts out
+                page[1, key % 32] = float("inf")
+    parts = [(s, 0, n) for s, (n, _) in enumerate(seqs)]
+    whole = case.run(parts)
+    for first, n in ((129, 1), (100, 3), (70, 40)):
+        assert torch.equal(case.run([(2, first, n)]), whole[case.at[2] + first: case.at[2] + first + n])
+    plain = torch.empty_like(case.q)
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    view = K.CacheView(case.pool.data_ptr(), case.pool.data_ptr() + case.elems // 2 * 4, case.table, case.elems, case.table.stride(0), 32, 1, 64, torch.float32)
+    K.attention_plain(case.q, plain, view, ints([kv - n + i for n, kv in seqs for i in range(n)]), ints([s for s, (n, _) in enumerate(seqs) for _ in range(n)]),
+                      2, case.q.shape[0], 64 ** -0.5, 0)
+    assert torch.isfinite(plain).all() and torch.isfinite(whole).all()
