@@ -461,7 +461,8 @@ constexpr int A_BYTES = BM * BK * 2;
 constexpr int MAX_STAGES = 8;
 
 // Set by llm_gemm_test_hooks: the wait limit of the launches that follow, and a k block whose copies
-// the producer of the non-persistent kernel leaves out, so that a test can watch a bounded wait run out.
+// the producer of the non-persistent kernel leaves out (in the cluster kernel, whose barrier waits for more than
+// they bring), so that a test can watch a bounded wait run out.
 static unsigned long long g_wait_ns = WAIT_LIMIT_NS;
 static int g_drop_k_block = -1;
 
@@ -960,6 +961,7 @@ struct ClusterArgs {
   int bn, stages, stage_bytes, tmem_cols;
   uint32_t idesc;
   unsigned long long wait_ns;
+  int drop_k_block;             // tests only (llm_gemm_test_hooks): this k block's barrier waits for 16 bytes more than its copies bring
   int pair_span;                // a row's partner lies this far behind it, rows come in groups of twice this many
   int n_tokens, n_features, k_blocks, k_per_block, up_row_offset;
   const float* sq_in;           // parts of the input rows' sums of squares (null: the input is what it is)
@@ -1045,7 +1047,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
 
   auto issue_weights = [&](int i, int s) {
     uint8_t* stage = smem + s * a.stage_bytes;
-    mbar_expect_tx(&full_bar[s], a.stage_bytes);
+    mbar_expect_tx(&full_bar[s], a.stage_bytes + (kb_begin + i == a.drop_k_block ? 16 : 0));
     const int k0 = (kb_begin + i) * BK;
     tma_load_2d(stage, &map_w, &full_bar[s], k0, f0);      // CL_SWIGLU: the box has 64 rows
     if (EPI == CL_SWIGLU) tma_load_2d(stage + A_BYTES / 2, &map_w, &full_bar[s], k0, a.up_row_offset + f0);
@@ -1225,6 +1227,9 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     }
     cluster_wait();          // the others have their barriers
     asm volatile("bar.sync %0, 128;" ::"r"(2 + part) : "memory");
+    // A role that gave up leaves an accumulator that is complete by its barrier and wrong: the flag, which every warp of this
+    // group has set by now if it did, says so.  Nothing is sent then, and the others' waits for it run out.
+    ok = ok && !*abort_flag;
     if (ok && t_end > t_begin && ew % 4 == 0 && lane < C) {      // a lane per receiver
       const uint32_t bytes = (uint32_t)(t_end - t_begin) * ROWS * 4;
       const uint32_t to = peer_address(smem_u32(received + rank * slot + t_begin * ROWS), lane);
@@ -1516,9 +1521,9 @@ extern "C" int llm_gemm_grouped_bf16(const void* map_w, const void* map_a, void*
 
 // For tests of the bounded waits: the launches that follow give up on an mbarrier after `wait_ns`
 // nanoseconds (0: the default of one second), and the producer of the non-persistent kernel arms
-// the barrier of k block `drop_k_block` of every tile without issuing its copies (-1: none), so the
-// MMA issuer's wait for it runs out: the kernel reports "MMA issuer" in the error word, releases its
-// tensor memory and returns.  Call with (0, -1) to put things back.
+// the barrier of k block `drop_k_block` of every tile without issuing its copies (the cluster kernel's, for 16 bytes more than
+// its copies bring; -1: none), so the MMA issuer's wait for it runs out: the kernel reports "MMA issuer" in the error
+// word (a cluster's other blocks, which wait for the slices, may come first), releases its tensor memory and returns.  Call with (0, -1) to put things back.
 extern "C" void llm_gemm_test_hooks(long long wait_ns, int drop_k_block) {
   g_wait_ns = wait_ns > 0 ? (unsigned long long)wait_ns : WAIT_LIMIT_NS;
   g_drop_k_block = drop_k_block;
@@ -1677,6 +1682,7 @@ extern "C" int llm_gemm_cluster(const void* map_w, const void* map_a, int epi, i
   while (a.tmem_cols < bn) a.tmem_cols *= 2;
   a.idesc = instr_desc_bf16(BM, bn);
   a.wait_ns = g_wait_ns;
+  a.drop_k_block = g_drop_k_block;
   a.k_blocks = (K + BK - 1) / BK;
   a.k_per_block = (a.k_blocks + cluster - 1) / cluster;
   size_t smem = 0;

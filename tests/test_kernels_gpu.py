@@ -533,6 +533,41 @@ def test_a_bounded_wait_runs_out_and_the_kernel_returns():
     _close(res.tensor, want, 1e-5, 2e-3)
 
 
+@pytest.mark.parametrize("k,drop", [(512, 0), (512, 7), (2048, 30), (5632, 9)])
+def test_a_block_of_a_cluster_gives_up_and_no_block_writes(k, drop):
+    """The cluster product when one block of a tile's cluster never gets a k block (in the ring's first round, or in a later
+    one): the block sends nothing, the others' waits for its slices run out too, all return, the residual stream and what
+    the next norm would be given stay untouched, the error word says so, and the next launch is right."""
+    from ctypes import c_int, c_longlong
+    from bare_cuda_4gib_b200.errors import KernelLaunchError
+    from bare_cuda_4gib_b200.kernels import gemm
+    from bare_cuda_4gib_b200.kernels import lib as K
+    torch.manual_seed(k + drop)
+    rows, n, ctx = 40, 256, _ctx()
+    a = ctx.ws.get("a", (rows, k), torch.bfloat16)
+    a.copy_(torch.randn(rows, k, device=DEV))
+    w = (torch.randn(n, k, device=DEV) / math.sqrt(k)).to(torch.bfloat16)
+    plan, residual = gemm.plan_for(w), torch.randn(rows, n, device=DEV)
+    before, norm = residual.clone(), _RowNorm(torch.ones(n, device=DEV), 1e-5)
+    end = K.AddTo(residual, norm)
+    assert gemm.cluster_kind(plan, rows, torch.float32, False, end) == gemm.CL_ADD
+    gemm.check_errors()
+    hooks = gemm.lib().llm_gemm_test_hooks
+    hooks.argtypes, hooks.restype = [c_longlong, c_int], None
+    hooks(2_000_000, drop)
+    try:
+        gemm.run_cluster(ctx, plan, gemm.CL_ADD, a, rows, torch.float32, "out", end)
+        torch.cuda.synchronize()               # returns: nothing waits for ever
+        with pytest.raises(KernelLaunchError, match="gemm MMA issuer|gemm cluster exchange"):
+            gemm.check_errors()
+    finally:
+        hooks(0, -1)
+    assert torch.equal(residual, before)
+    gemm.run_cluster(ctx, plan, gemm.CL_ADD, a, rows, torch.float32, "out", end)
+    gemm.check_errors()
+    _close(residual, before.double() + a.double() @ w.double().t(), 1e-5, 2e-3)
+
+
 # ------------------------------------------------------------------------------ tensor-core attention
 
 def _attention_case(seqs, heads, kv_heads, d, page, window, seed, far_key=False, drop_passed=False,
