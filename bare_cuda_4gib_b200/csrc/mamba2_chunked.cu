@@ -5,7 +5,7 @@
 //   y_i = sum_{j <= i} (C_i . B_j) exp(cum_i - cum_j) dt_j x_j  +  exp(cum_i) S^T C_i
 //   S  <- exp(cum_last) S + sum_j B_j (exp(cum_last - cum_j) dt_j x_j)^T
 //
-// which is S_t = a_t S_(t-1) + dt_t B_t x_t^T, y_t = S_t^T C_t written out over a chunk of 64 (or 128) tokens.  A block owns
+// which is S_t = a_t S_(t-1) + dt_t B_t x_t^T, y_t = S_t^T C_t written out over a chunk of 64 tokens.  A block owns
 // one request, one head and 32 (or 16) value columns and walks the request's chunks in order: the state's
 // columns are independent, so blocks never wait on one another.  B, C and x arrive as bfloat16 (activations of
 // the convolution); step sizes, decays, their exponentials and the state are float32.  Wherever a float32
@@ -17,20 +17,10 @@
 //
 // Built per model with -DSSD_N (state size) and -DSSD_P (value size of a head), multiples of 16, and
 // optionally -DSSD_PC (value columns of a block).
-//
-// The matrix memory of xLSTM is the same recurrence with q for C, k for B, v for x, the input gate's weight for dt
-// and every head a group of its own, plus a row sum n_t = a_t n_(t-1) + b_t k_t, which is one more value column
-// whose x is 1 (-DSSD_ONES): the state and the result then have P + 4 columns (three of padding), and one block
-// more per head walks with the ones.  -DSSD_TERMS=3 splits operands into three bfloat16 numbers (24 significant
-// bits, all that float32 has) where a walk in float32 products is replaced: 16 heads of 128 x 128, 2,048 tokens:
-// 177 us, where operands, scan in stretches, carry and correction took 491, at the same distance from float64 (1.0e-7 of the
-// result's norm beside 0.9e-7 to 1.5e-7).  The longest warp's share of the causal triangle bounds a chunk (barrier
-// stalls lead, the tensor pipe is 16 % busy); chunks of 64 tokens and four warps took 203 us.
 
 #include "common.cuh"
 
 #include <math.h>
-#include <type_traits>
 
 #ifndef SSD_N
 #define SSD_N 128
@@ -44,27 +34,15 @@ namespace {
 constexpr int N = SSD_N, P = SSD_P;
 static_assert(N % 16 == 0 && N >= 16 && N <= 256, "SSD_N must be a multiple of 16 up to 256");
 static_assert(P % 16 == 0 && P >= 16, "SSD_P must be a multiple of 16");
-#ifndef SSD_L
-#define SSD_L 64
-#endif
-constexpr int L = SSD_L;                      // tokens of a chunk, 16 to a warp
-static_assert(L == 64 || L == 128, "SSD_L must be 64 or 128");
+constexpr int L = 64;                         // tokens of a chunk
 #ifndef SSD_PC
 #define SSD_PC (SSD_P % 32 == 0 ? 32 : 16)
 #endif
-#ifndef SSD_ONES
-#define SSD_ONES 0
-#endif
-#ifndef SSD_TERMS
-#define SSD_TERMS 2
-#endif
-constexpr int SP = P + (SSD_ONES ? 4 : 0);    // columns of the state and of the result
-constexpr int TERMS = SSD_TERMS;              // bfloat16 numbers a float32 operand is split into
 constexpr int PC = SSD_PC;                    // value columns of a block: 32, or 16 where the model's heads alone
                                               // would leave most SMs without a block
 static_assert((PC == 16 || PC == 32) && P % PC == 0, "SSD_PC must be 16 or 32 and divide SSD_P");
 constexpr int LDN = N + 8, LDP = PC + 8;      // padded rows (conflict-free ldmatrix)
-constexpr int WARPS = L / 16, THREADS = WARPS * 32;
+constexpr int WARPS = 4, THREADS = WARPS * 32;
 constexpr int MT_N = N / 16;                  // row tiles of the state
 constexpr int MTW = (MT_N + WARPS - 1) / WARPS;   // of which a warp owns at most this many
 constexpr int NT = PC / 8;                    // column tiles of a block's columns
@@ -99,37 +77,12 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// c += a b for TERMS operands on one side, a(t) and b(t, half).  With three terms the smallest comes first, the three are summed
-// by themselves and that sum is added in float32: the tensor core cuts off what it adds to a running sum instead of rounding it.
-template <int COUNT, typename A, typename B>
-__device__ __forceinline__ void mma_split(float (&c)[4], const A& a, const B& b) {
-  if (TERMS < 3) {
-#pragma unroll
-    for (int t = 0; t < COUNT; ++t) mma_bf16(c, a(t), b(t, 0), b(t, 1));
-  } else {
-    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int t = COUNT - 1; t >= 0; --t) mma_bf16(sum, a(t), b(t, 0), b(t, 1));
-#pragma unroll
-    for (int e = 0; e < 4; ++e) c[e] += sum[e];
-  }
-}
-
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
 __device__ __forceinline__ float rounded(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
-// v as TERMS bfloat16 numbers, each rounding what the ones before it left, `stride` apart
-__device__ __forceinline__ void split_store(__nv_bfloat16* to, int stride, float v) {
-#pragma unroll
-  for (int t = 0; t < TERMS; ++t) {
-    to[t * stride] = __float2bfloat16_rn(v);
-    v -= rounded(v);
-  }
-}
 
 struct SsdArgs {
   const __nv_bfloat16* x;      // [rows, heads * P]    after convolution and silu; rows `in_stride` apart, like b and c
@@ -138,9 +91,8 @@ struct SsdArgs {
   long long in_stride;
   const float* dt;             // [rows, heads]
   const float* la;             // [rows, heads]   logarithm of the token's decay
-  float* state;                // [slots][heads][N][SP]
-  float* out;                  // [rows, heads * SP]   S_t^T C_t * out_scale
-  float out_scale;
+  float* state;                // [slots][heads][N][P]
+  float* out;                  // [rows, heads * P]   S_t^T C_t
   const int32_t* seq_slot;
   const int32_t* seq_q_start;
   const int32_t* seq_q_len;
@@ -153,12 +105,13 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
   __nv_bfloat16* Bs0 = reinterpret_cast<__nv_bfloat16*>(smem_raw);  // [2][L][LDN]
   __nv_bfloat16* Cs0 = Bs0 + 2 * L * LDN;                           // [2][L][LDN]
   __nv_bfloat16* Xs0 = Cs0 + 2 * L * LDN;                           // [2][L][LDP]  x
-  __nv_bfloat16* Xt = Xs0 + 2 * L * LDP;                            // [TERMS][L][LDP]  x times its decay to the chunk's end and dt, split
-  __nv_bfloat16* St = Xt + TERMS * L * LDP;                         // [TERMS][N][LDP]  the state at the chunk's start, likewise
-  float* cum = reinterpret_cast<float*>(St + TERMS * N * LDP);      // [L]
+  __nv_bfloat16* Xh = Xs0 + 2 * L * LDP;                            // [L][LDP]  x times its decay to the chunk's end and dt: rounded ...
+  __nv_bfloat16* Xl = Xh + L * LDP;                                 // ... and what the rounding left
+  __nv_bfloat16* Sh = Xl + L * LDP;                                 // [N][LDP]  the state at the chunk's start, likewise
+  __nv_bfloat16* Sl = Sh + N * LDP;
+  float* cum = reinterpret_cast<float*>(Sl + N * LDP);              // [L]
   float* dts0 = cum + L;                                            // [2][L] step sizes
   float* las0 = dts0 + 2 * L;                                       // [2][L] logarithms of the decays
-  float* cum_rest = las0 + 2 * L;                                   // [L] (three terms)
 
   pdl_launch_dependents();
   pdl_wait();
@@ -170,10 +123,8 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;      // a thread's row within eight and its column pair
   const int mid = lane >> 3;
-  const long long x_stride = a.in_stride, bc_stride = a.in_stride, out_stride = (long long)H * SP;
-  float* S_g = a.state + (((long long)slot * H + h) * N) * SP + col0;
-  const bool ones = SSD_ONES && col0 == P;         // this block walks the column whose x is 1
-  const int cols = SSD_ONES ? min(PC, SP - col0) : PC;
+  const long long x_stride = a.in_stride, bc_stride = a.in_stride, out_stride = (long long)H * P;
+  float* S_g = a.state + (((long long)slot * H + h) * N) * P + col0;
 
   // the state's tiles this warp owns, float32, for the whole walk
   float sreg[MTW][NT][4];
@@ -185,9 +136,13 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int n = mt * 16 + gq + (e >> 1) * 8, col = nt * 8 + tq * 2 + (e & 1);
-        const float v = mt < MT_N && col < cols ? S_g[(long long)n * SP + col] : 0.0f;
+        const float v = mt < MT_N ? S_g[(long long)n * P + col] : 0.0f;
         sreg[i][nt][e] = v;
-        if (mt < MT_N) split_store(St + n * LDP + col, N * LDP, v);
+        if (mt < MT_N) {
+          const float hi = rounded(v);
+          Sh[n * LDP + col] = __float2bfloat16_rn(v);
+          Sl[n * LDP + col] = __float2bfloat16_rn(v - hi);
+        }
       }
   }
 
@@ -211,10 +166,6 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
       for (int i = threadIdx.x; i < L * CP; i += THREADS) {
         const int r = i / CP, c8 = i % CP;
         const bool valid = r < count;
-        if (ones) {
-          *reinterpret_cast<uint4*>(Xd + r * LDP + c8 * 8) = make_uint4(valid && c8 == 0 ? 0x3f80u : 0u, 0u, 0u, 0u);
-          continue;
-        }
         cp_async16(Xd + r * LDP + c8 * 8, a.x + (valid ? (row0 + r) * x_stride + h * P + col0 + c8 * 8 : 0), valid);
       }
       if (threadIdx.x < L) {
@@ -239,167 +190,107 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
     load_chunk(ch + 1);      // into the other set, which every warp left at the last chunk's end
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();         // chunk `ch` has landed
-    if (warp == 0) {      // the running sum over the chunk's tokens: a lane takes L / 32 neighbours.  With three terms in 64
-      // bits, kept as a float32 and what its rounding left: a difference of large sums has to be as exact as the decays between
-      typedef typename std::conditional<TERMS == 3, double, float>::type Sum;
-      constexpr int EACH = L / 32;
-      Sum v[EACH], run = 0;
-#pragma unroll
-      for (int j = 0; j < EACH; ++j) v[j] = las[EACH * lane + j], run += v[j];
+    if (warp == 0) {      // the running sum over the chunk's 64 tokens: a lane takes two neighbours
+      const float v0 = las[2 * lane], v1 = las[2 * lane + 1];
+      float run = v0 + v1;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const Sum up = __shfl_up_sync(0xffffffffu, run, o);
+        const float up = __shfl_up_sync(0xffffffffu, run, o);
         if (lane >= o) run += up;
       }
-#pragma unroll
-      for (int j = EACH - 1; j >= 0; --j) {
-        cum[EACH * lane + j] = (float)run;
-        if (TERMS == 3) cum_rest[EACH * lane + j] = (float)(run - (Sum)(float)run);
-        run -= v[j];
-      }
+      cum[2 * lane] = run - v1;
+      cum[2 * lane + 1] = run;
     }
     __syncthreads();
     const float cum_last = cum[L - 1];
-    // the sum of the logarithms between tokens j and i
-    auto between = [&](float cum_i, float rest_i, int j) {
-      return TERMS == 3 ? (cum_i - cum[j]) + (rest_i - cum_rest[j]) : cum_i - cum[j];
-    };
-    const float rest_last = TERMS == 3 ? cum_rest[L - 1] : 0.0f;
-    // x times exp(cum_last - cum_j) dt_j, split
+    // x times exp(cum_last - cum_j) dt_j, as a rounded number and the rest
     for (int i = threadIdx.x; i < L * PC; i += THREADS) {
       const int r = i / PC, c = i % PC;
-      split_store(Xt + r * LDP + c, L * LDP, __bfloat162float(Xs[r * LDP + c]) * (expf(between(cum_last, rest_last, r)) * dts[r]));
+      const float v = __bfloat162float(Xs[r * LDP + c]) * (expf(cum_last - cum[r]) * dts[r]);
+      const float hi = rounded(v);
+      Xh[r * LDP + c] = __float2bfloat16_rn(v);
+      Xl[r * LDP + c] = __float2bfloat16_rn(v - hi);
     }
 
-    // ---- this warp's 16 tokens i against the tokens j <= i: G = C B^T, the weights (C_i . B_j) exp(cum_i - cum_j) dt_j as A
-    // fragments, split, and their product with x
-    uint32_t cf[N / 16][4];
+    // ---- G = C B^T for this warp's 16 tokens against all 64
+    float s[L / 8][4];
 #pragma unroll
-    for (int ks = 0; ks < N / 16; ++ks)
-      ldmatrix_x4(cf[ks], Cs + (warp * 16 + (lane & 15)) * LDN + ks * 16 + (lane >> 4) * 8);
+    for (int nt = 0; nt < L / 8; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
+#pragma unroll
+    for (int ks = 0; ks < N / 16; ++ks) {
+      uint32_t cf[4];
+      ldmatrix_x4(cf, Cs + (warp * 16 + (lane & 15)) * LDN + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int nt = 0; nt < L / 8; nt += 2) {
+        uint32_t bf[4];
+        ldmatrix_x4(bf, Bs + ((nt + (mid >> 1)) * 8 + (lane & 7)) * LDN + ks * 16 + (mid & 1) * 8);
+        mma_bf16(s[nt], cf, bf[0], bf[1]);
+        mma_bf16(s[nt + 1], cf, bf[2], bf[3]);
+      }
+    }
+    // ---- the weights (C_i . B_j) exp(cum_i - cum_j) dt_j for j <= i, as A fragments: rounded, and the rest
+    uint32_t wh[L / 16][4], wl[L / 16][4];
     const int i0 = warp * 16 + gq, i1 = i0 + 8;
     const float ci0 = cum[i0], ci1 = cum[i1];
-    const float ri0 = TERMS == 3 ? cum_rest[i0] : 0.0f, ri1 = TERMS == 3 ? cum_rest[i1] : 0.0f;
+#pragma unroll
+    for (int nt = 0; nt < L / 8; ++nt) {
+      float w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = (e >> 1) ? i1 : i0, j = nt * 8 + tq * 2 + (e & 1);
+        w[e] = j <= i ? s[nt][e] * expf(((e >> 1) ? ci1 : ci0) - cum[j]) * dts[j] : 0.0f;
+      }
+      wh[nt / 2][(nt & 1) * 2 + 0] = pack_bf16(w[0], w[1]);
+      wh[nt / 2][(nt & 1) * 2 + 1] = pack_bf16(w[2], w[3]);
+      wl[nt / 2][(nt & 1) * 2 + 0] = pack_bf16(w[0] - rounded(w[0]), w[1] - rounded(w[1]));
+      wl[nt / 2][(nt & 1) * 2 + 1] = pack_bf16(w[2] - rounded(w[2]), w[3] - rounded(w[3]));
+    }
+    __syncthreads();      // Xh and Xl are complete (the state's product below reads them)
+    // ---- y = weights x  +  exp(cum_i) C S
     float o[NT][4], y2[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
       o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.0f;
       y2[nt][0] = y2[nt][1] = y2[nt][2] = y2[nt][3] = 0.0f;
     }
-    if constexpr (TERMS < 3) {
-      // all of the chunk's tokens j at once: more products in flight than 16 at a time (2.17 against 2.20 ms a prompt of the
-      // 4-layer Gurolix model)
-      float s[L / 8][4];
 #pragma unroll
-      for (int nt = 0; nt < L / 8; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
-#pragma unroll
-      for (int ks = 0; ks < N / 16; ++ks) {
-#pragma unroll
-        for (int nt = 0; nt < L / 8; nt += 2) {
-          uint32_t bf[4];
-          ldmatrix_x4(bf, Bs + ((nt + (mid >> 1)) * 8 + (lane & 7)) * LDN + ks * 16 + (mid & 1) * 8);
-          mma_bf16(s[nt], cf[ks], bf[0], bf[1]);
-          mma_bf16(s[nt + 1], cf[ks], bf[2], bf[3]);
-        }
-      }
-      uint32_t wt[TERMS][L / 16][4];
-#pragma unroll
-      for (int nt = 0; nt < L / 8; ++nt) {
-        float w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = (e >> 1) ? i1 : i0, j = nt * 8 + tq * 2 + (e & 1);
-          w[e] = j <= i ? s[nt][e] * expf(((e >> 1) ? ci1 : ci0) - cum[j]) * dts[j] : 0.0f;
-        }
-#pragma unroll
-        for (int t = 0; t < TERMS; ++t) {
-          wt[t][nt / 2][(nt & 1) * 2 + 0] = pack_bf16(w[0], w[1]);
-          wt[t][nt / 2][(nt & 1) * 2 + 1] = pack_bf16(w[2], w[3]);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) w[e] -= rounded(w[e]);
-        }
-      }
-      __syncthreads();      // Xt is complete (the state's product below reads it)
-#pragma unroll
-      for (int kk = 0; kk < L / 16; ++kk) {
-#pragma unroll
-        for (int nt = 0; nt < NT; nt += 2) {
-          uint32_t xf[4];
-          ldmatrix_x4_trans(xf, Xs + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
-#pragma unroll
-          for (int t = 0; t < TERMS; ++t) {
-            mma_bf16(o[nt], wt[t][kk], xf[0], xf[1]);
-            mma_bf16(o[nt + 1], wt[t][kk], xf[2], xf[3]);
-          }
-        }
-      }
-    } else {
-      // 16 tokens j at a time
-#pragma unroll 1
-      for (int kk = 0; kk <= warp; ++kk) {
-        float s[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
-#pragma unroll
-        for (int ks = 0; ks < N / 16; ++ks) {
-          uint32_t bf[4];
-          ldmatrix_x4(bf, Bs + (kk * 16 + (mid >> 1) * 8 + (lane & 7)) * LDN + ks * 16 + (mid & 1) * 8);
-          const auto c_of = [&](int) -> const uint32_t(&)[4] { return cf[ks]; };
-          mma_split<1>(s[0], c_of, [&](int, int half) { return bf[half]; });
-          mma_split<1>(s[1], c_of, [&](int, int half) { return bf[2 + half]; });
-        }
-        uint32_t wt[TERMS][4];
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          float w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = (e >> 1) ? i1 : i0, j = kk * 16 + nt * 8 + tq * 2 + (e & 1);
-            w[e] = j <= i ? s[nt][e] * expf(between((e >> 1) ? ci1 : ci0, (e >> 1) ? ri1 : ri0, j)) * dts[j] : 0.0f;
-          }
-#pragma unroll
-          for (int t = 0; t < TERMS; ++t) {
-            wt[t][nt * 2 + 0] = pack_bf16(w[0], w[1]);
-            wt[t][nt * 2 + 1] = pack_bf16(w[2], w[3]);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) w[e] -= rounded(w[e]);
-          }
-        }
-#pragma unroll
-        for (int nt = 0; nt < NT; nt += 2) {
-          uint32_t xf[4];
-          ldmatrix_x4_trans(xf, Xs + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
-          const auto w_of = [&](int t) -> const uint32_t(&)[4] { return wt[t]; };
-          mma_split<TERMS>(o[nt], w_of, [&](int, int half) { return xf[half]; });
-          mma_split<TERMS>(o[nt + 1], w_of, [&](int, int half) { return xf[2 + half]; });
-        }
-      }
-      __syncthreads();      // Xt is complete (the state's product below reads it)
-    }
-    // ---- y = weights x  +  exp(cum_i) C S
-#pragma unroll
-    for (int ks = 0; ks < N / 16; ++ks) {
+    for (int kk = 0; kk < L / 16; ++kk) {
 #pragma unroll
       for (int nt = 0; nt < NT; nt += 2) {
-        uint32_t sf[TERMS][4];
+        uint32_t xf[4];
+        ldmatrix_x4_trans(xf, Xs + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
+        mma_bf16(o[nt], wh[kk], xf[0], xf[1]);
+        mma_bf16(o[nt + 1], wh[kk], xf[2], xf[3]);
+        mma_bf16(o[nt], wl[kk], xf[0], xf[1]);
+        mma_bf16(o[nt + 1], wl[kk], xf[2], xf[3]);
+      }
+    }
 #pragma unroll
-        for (int t = 0; t < TERMS; ++t)
-          ldmatrix_x4_trans(sf[t], St + t * N * LDP + (ks * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
-        const auto c_of = [&](int) -> const uint32_t(&)[4] { return cf[ks]; };
-        mma_split<TERMS>(y2[nt], c_of, [&](int t, int half) { return sf[t][half]; });
-        mma_split<TERMS>(y2[nt + 1], c_of, [&](int t, int half) { return sf[t][2 + half]; });
+    for (int ks = 0; ks < N / 16; ++ks) {
+      uint32_t cf[4];
+      ldmatrix_x4(cf, Cs + (warp * 16 + (lane & 15)) * LDN + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+      for (int nt = 0; nt < NT; nt += 2) {
+        uint32_t sf[4];
+        ldmatrix_x4_trans(sf, Sh + (ks * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
+        mma_bf16(y2[nt], cf, sf[0], sf[1]);
+        mma_bf16(y2[nt + 1], cf, sf[2], sf[3]);
+        ldmatrix_x4_trans(sf, Sl + (ks * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
+        mma_bf16(y2[nt], cf, sf[0], sf[1]);
+        mma_bf16(y2[nt + 1], cf, sf[2], sf[3]);
       }
     }
     {
       const float f0 = expf(ci0), f1 = expf(ci1);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {
-        if (nt * 8 + tq * 2 >= cols) continue;
-        const int col = h * SP + col0 + nt * 8 + tq * 2;
+        const int col = h * P + col0 + nt * 8 + tq * 2;
         if (i0 < count)
           *reinterpret_cast<float2*>(a.out + (row0 + i0) * out_stride + col) =
-              make_float2(fmaf(f0, y2[nt][0], o[nt][0]) * a.out_scale, fmaf(f0, y2[nt][1], o[nt][1]) * a.out_scale);
+              make_float2(fmaf(f0, y2[nt][0], o[nt][0]), fmaf(f0, y2[nt][1], o[nt][1]));
         if (i1 < count)
           *reinterpret_cast<float2*>(a.out + (row0 + i1) * out_stride + col) =
-              make_float2(fmaf(f1, y2[nt][2], o[nt][2]) * a.out_scale, fmaf(f1, y2[nt][3], o[nt][3]) * a.out_scale);
+              make_float2(fmaf(f1, y2[nt][2], o[nt][2]), fmaf(f1, y2[nt][3], o[nt][3]));
       }
     }
     // ---- the state: S <- exp(cum_last) S + B^T (x exp(cum_last - cum_j) dt_j), this warp's row tiles
@@ -418,13 +309,13 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
         ldmatrix_x4_trans(bt, Bs + (kk * 16 + (mid >> 1) * 8 + (lane & 7)) * LDN + mt * 16 + (mid & 1) * 8);
 #pragma unroll
         for (int nt = 0; nt < NT; nt += 2) {
-          uint32_t xf[TERMS][4];
-#pragma unroll
-          for (int t = 0; t < TERMS; ++t)
-            ldmatrix_x4_trans(xf[t], Xt + t * L * LDP + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
-          const auto b_of = [&](int) -> const uint32_t(&)[4] { return bt; };
-          mma_split<TERMS>(sreg[i][nt], b_of, [&](int t, int half) { return xf[t][half]; });
-          mma_split<TERMS>(sreg[i][nt + 1], b_of, [&](int t, int half) { return xf[t][2 + half]; });
+          uint32_t xf[4];
+          ldmatrix_x4_trans(xf, Xh + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
+          mma_bf16(sreg[i][nt], bt, xf[0], xf[1]);
+          mma_bf16(sreg[i][nt + 1], bt, xf[2], xf[3]);
+          ldmatrix_x4_trans(xf, Xl + (kk * 16 + (mid & 1) * 8 + (lane & 7)) * LDP + (nt + (mid >> 1)) * 8);
+          mma_bf16(sreg[i][nt], bt, xf[0], xf[1]);
+          mma_bf16(sreg[i][nt + 1], bt, xf[2], xf[3]);
         }
       }
     }
@@ -438,7 +329,9 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int n = mt * 16 + gq + (e >> 1) * 8, col = nt * 8 + tq * 2 + (e & 1);
-          split_store(St + n * LDP + col, N * LDP, sreg[i][nt][e]);
+          const float v = sreg[i][nt][e];
+          Sh[n * LDP + col] = __float2bfloat16_rn(v);
+          Sl[n * LDP + col] = __float2bfloat16_rn(v - rounded(v));
         }
     }
     // (the next chunk's barriers come before anything reads the state again)
@@ -452,13 +345,12 @@ __global__ void __launch_bounds__(THREADS) mamba2_chunked_kernel(SsdArgs a) {
 #pragma unroll
       for (int e = 0; e < 4; e += 2) {
         const int n = mt * 16 + gq + (e >> 1) * 8, col = nt * 8 + tq * 2;
-        if (col < cols) *reinterpret_cast<float2*>(S_g + (long long)n * SP + col) = make_float2(sreg[i][nt][e], sreg[i][nt][e + 1]);
+        *reinterpret_cast<float2*>(S_g + (long long)n * P + col) = make_float2(sreg[i][nt][e], sreg[i][nt][e + 1]);
       }
   }
 }
 
-constexpr size_t SMEM = (size_t)(4 * L * LDN + (2 + TERMS) * L * LDP + TERMS * N * LDP) * 2 + 6 * L * 4;
-static_assert(SMEM <= 227 * 1024, "a block's tiles fit in shared memory");
+constexpr size_t SMEM = (size_t)(4 * L * LDN + 4 * L * LDP + 2 * N * LDP) * 2 + 5 * L * 4;
 
 }  // namespace
 
@@ -466,7 +358,7 @@ extern "C" int llm_mamba2_chunked_columns() { return PC; }
 
 extern "C" int llm_mamba2_chunked(const void* x, const void* b, const void* c, long long in_stride, const float* dt,
                                   const float* la, float* state,
-                                  float* out, float out_scale, const int32_t* seq_slot, const int32_t* seq_q_start, const int32_t* seq_q_len,
+                                  float* out, const int32_t* seq_slot, const int32_t* seq_q_start, const int32_t* seq_q_len,
                                   int n_seqs, int heads, int groups, int state_size, int vdim, cudaStream_t stream) {
   if (n_seqs <= 0) return 0;
   LLM_HOST_CHECK(state_size == N && vdim == P && groups >= 1 && heads % groups == 0, ERR_BAD_SIZE);
@@ -481,8 +373,8 @@ extern "C" int llm_mamba2_chunked(const void* x, const void* b, const void* c, l
       return launch_status();
     configured = true;
   }
-  SsdArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)b, (const __nv_bfloat16*)c, in_stride, dt, la, state, out, out_scale,
+  SsdArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)b, (const __nv_bfloat16*)c, in_stride, dt, la, state, out,
             seq_slot, seq_q_start, seq_q_len, heads, groups};
-  launch_kernel(mamba2_chunked_kernel, dim3(P / PC + (SSD_ONES ? 1 : 0), heads, n_seqs), THREADS, SMEM, stream, a);
+  launch_kernel(mamba2_chunked_kernel, dim3(P / PC, heads, n_seqs), THREADS, SMEM, stream, a);
   return launch_status();
 }

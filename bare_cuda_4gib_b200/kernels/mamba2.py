@@ -118,22 +118,15 @@ def chunked_columns(heads: int, vdim: int) -> int:
     return 32 if vdim % 32 == 0 and heads * (vdim // 32) >= sm_count() else 16
 
 
-def ones_flags(state: int):
-    """... of 128 tokens where their tiles fit in shared memory: eight warps walk half as many chunks."""
-    return ("-DSSD_ONES=1", "-DSSD_TERMS=3") + (("-DSSD_L=128",) if state <= 128 else ())
-
-
-def chunked_lib(state: int, vdim: int, columns: int = 0, ones: bool = False):
-    """`ones`: the walk of a matrix memory with its row sums (one more value column whose x is 1, operands in three terms)."""
+def chunked_lib(state: int, vdim: int, columns: int = 0):
     columns = columns or (32 if vdim % 32 == 0 else 16)
-    l = _chunked_libs.get((state, vdim, columns, ones))
+    l = _chunked_libs.get((state, vdim, columns))
     if l is None:
-        flags = (f"-DSSD_N={state}", f"-DSSD_P={vdim}", f"-DSSD_PC={columns}") + (ones_flags(state) if ones else ())
-        l = build.load_library("mamba2_chunked.cu", flags)
-        P, I, L, F = c_void_p, c_int, c_longlong, c_float
-        l.llm_mamba2_chunked.argtypes = [P, P, P, L, P, P, P, P, F, P, P, P, I, I, I, I, I, P]
+        l = build.load_library("mamba2_chunked.cu", (f"-DSSD_N={state}", f"-DSSD_P={vdim}", f"-DSSD_PC={columns}"))
+        P, I, L = c_void_p, c_int, c_longlong
+        l.llm_mamba2_chunked.argtypes = [P, P, P, L, P, P, P, P, P, P, P, I, I, I, I, I, P]
         l.llm_mamba2_chunked.restype = c_int
-        _chunked_libs[(state, vdim, columns, ones)] = l
+        _chunked_libs[(state, vdim, columns)] = l
     return l
 
 
@@ -150,5 +143,5 @@ def chunked(ctx, compact: torch.Tensor, dt: torch.Tensor, la: torch.Tensor, stat
     base, esize = compact.data_ptr(), 2
     _check(chunked_lib(state_size, vdim, columns).llm_mamba2_chunked(
         base, base + inner * esize, base + (inner + groups * state_size) * esize, compact.stride(0), dt.data_ptr(),
-        la.data_ptr(), state.data_ptr(), out.data_ptr(), 1.0, ctx.seq_slot.data_ptr(), ctx.seq_q_start.data_ptr(),
+        la.data_ptr(), state.data_ptr(), out.data_ptr(), ctx.seq_slot.data_ptr(), ctx.seq_q_start.data_ptr(),
         ctx.seq_q_len.data_ptr(), ctx.n_seqs, heads, groups, state_size, vdim, ctx.stream), "mamba2_chunked")

@@ -62,30 +62,38 @@ def finish(ctx, scanned: torch.Tensor, coef: torch.Tensor, norm_w: torch.Tensor,
 
 
 def chunked_takes(dk: int, dv: int) -> bool:
-    """Sizes the walk in chunks on the tensor cores is built for (csrc/mamba2_chunked.cu, a library per pair)."""
+    """Sizes the walk in chunks on the tensor cores is built for (csrc/mlstm_chunked.cu, a library per pair)."""
     return dk % 16 == 0 and 16 <= dk <= 256 and dv % 16 == 0 and 16 <= dv <= 1024
 
 
-def chunked_columns(dk: int) -> int:
-    """Value columns of a block: 16, so that a few heads put a block on most SMs (16 heads of 128 values: 144 blocks)."""
-    return 16
+_chunked_libs = {}
+
+
+def chunked_lib(dk: int, dv: int):
+    l = _chunked_libs.get((dk, dv))
+    if l is None:
+        l = build.load_library("mlstm_chunked.cu", (f"-DML_DK={dk}", f"-DML_DV={dv}"))
+        P, I, L, F = c_void_p, c_int, c_longlong, c_float
+        l.llm_mlstm_chunked.argtypes = [P, P, P, L, P, P, P, P, F, P, P, P, I, I, I, I, P]
+        l.llm_mlstm_chunked.restype = c_int
+        _chunked_libs[(dk, dv)] = l
+    return l
 
 
 def chunked(ctx, u: torch.Tensor, q_col: int, k_col: int, v_col: int, log_decay: torch.Tensor, weight: torch.Tensor,
             state: torch.Tensor, out: torch.Tensor, heads: int, dk: int, dv: int, q_scale: float) -> None:
-    """Every request's portion in chunks of 64 tokens: q, k and v are read from the bfloat16 projection u; [S | n] float32
-    [slots, heads, dk, dv + 4] is read and left as after the portion; out [rows, heads * (dv + 4)] float32 = [S^T q | n . q | 0]
-    * q_scale."""
-    from . import mamba2
+    """Every request's portion in chunks (of 128 tokens, 64 for keys of more than 128 entries): q, k and v are read from the
+    bfloat16 projection u; [S | n] float32 [slots, heads, dk, dv + 4] is read and left as after the portion; out [rows, heads *
+    (dv + 4)] float32 = [S^T q | n . q | 0] * q_scale."""
     _dev(u, log_decay, weight, state, out)
     if (u.dtype != torch.bfloat16 or state.dtype != torch.float32 or out.dtype != torch.float32 or not out.is_contiguous()
             or state.shape[-1] != dv + 4 or out.shape[-1] != heads * (dv + 4)):
         raise TypeError("mlstm chunked: element types or layout not as the kernel needs")
     base = u.data_ptr()
-    _check(mamba2.chunked_lib(dk, dv, chunked_columns(dk), True).llm_mamba2_chunked(
-        base + 2 * v_col, base + 2 * k_col, base + 2 * q_col, u.stride(0), weight.data_ptr(), log_decay.data_ptr(),
+    _check(chunked_lib(dk, dv).llm_mlstm_chunked(
+        base + 2 * q_col, base + 2 * k_col, base + 2 * v_col, u.stride(0), weight.data_ptr(), log_decay.data_ptr(),
         state.data_ptr(), out.data_ptr(), float(q_scale), ctx.seq_slot.data_ptr(), ctx.seq_q_start.data_ptr(),
-        ctx.seq_q_len.data_ptr(), ctx.n_seqs, heads, heads, dk, dv, ctx.stream), "mlstm_chunked")
+        ctx.seq_q_len.data_ptr(), ctx.n_seqs, heads, dk, dv, ctx.stream), "mlstm_chunked")
 
 
 STEP_MAX_VALUE_COLUMNS = 288      # vdim + pad the one-token kernel keeps per warp

@@ -14,9 +14,8 @@ def all_libraries():
             ("gated_sandwich.cu", ()), ("mamba2.cu", ()),
             ("mamba2_chunked.cu", ("-DSSD_N=128", "-DSSD_P=64", "-DSSD_PC=16")),
             ("mamba2_chunked.cu", ("-DSSD_N=128", "-DSSD_P=64", "-DSSD_PC=32")),
-            ("mamba2_chunked.cu", ("-DSSD_N=16", "-DSSD_P=16", "-DSSD_PC=16", "-DSSD_ONES=1", "-DSSD_TERMS=3", "-DSSD_L=128")),
-            ("mamba2_chunked.cu", ("-DSSD_N=128", "-DSSD_P=128", "-DSSD_PC=16", "-DSSD_ONES=1", "-DSSD_TERMS=3", "-DSSD_L=128")),
-            ("mamba2_chunked.cu", ("-DSSD_N=256", "-DSSD_P=256", "-DSSD_PC=16", "-DSSD_ONES=1", "-DSSD_TERMS=3")),
+            ("mlstm_chunked.cu", ("-DML_DK=16", "-DML_DV=16")), ("mlstm_chunked.cu", ("-DML_DK=128", "-DML_DV=128")),
+            ("mlstm_chunked.cu", ("-DML_DK=256", "-DML_DV=256")),
             ("gated_delta.cu", ()), ("gated_delta_chunked.cu", ("-DGD_DK=16",)), ("gated_delta_chunked.cu", ("-DGD_DK=128",))]
     jobs += [("gemm_tcgen05.cu", ("-DGLU_GELU_TANH",)), ("gemv_fused.cu", ("-DGLU_GELU_TANH",)),
              ("gemm_tcgen05.cu", ("-DGROUPED_UP_RELU2",))]

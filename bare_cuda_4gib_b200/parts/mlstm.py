@@ -76,8 +76,7 @@ class MLSTM(Part):
         self.norm_w = t["norm"].to(dtype).contiguous()
         self.chunked = device.type == "cuda" and dtype == torch.bfloat16 and MK.chunked_takes(self.dim, self.vdim)
         if self.chunked:
-            from ..kernels import mamba2
-            mamba2.chunked_lib(self.dim, self.vdim, MK.chunked_columns(self.dim), True)   # compiled with the model, not at its first portion
+            MK.chunked_lib(self.dim, self.vdim)      # compiled with the model, not at its first portion
 
     def forward(self, ctx, call, h):
         n, H, dk, dv, dvp = ctx.n_tokens, self.heads, self.dim, self.vdim, self.vpad

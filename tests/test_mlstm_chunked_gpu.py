@@ -71,3 +71,72 @@ def test_mlstm_chunked(heads, dk, dv, lens, forget):
     bound = (3 * (dk / 16 + 4) + 8) * 2.0 ** -23
     assert far["chunked"] <= bound, (far, bound)
     print(f"mlstm heads {heads} dk {dk} dv {dv}: chunked {far['chunked']:.2e} scan {far['scan']:.2e} bound {bound:.2e}")
+
+
+class _Walks:
+    """One request's portion through the walk in chunks and through the scan, from a zero memory."""
+
+    def __init__(self, heads, d, n, forget, seed):
+        from bare_cuda_4gib_b200.engine.step import Workspace
+        from bare_cuda_4gib_b200.kernels import lib as K, mlstm as MK
+        torch.manual_seed(seed)
+        self.heads, self.d, self.n = heads, d, n
+        ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+        self.ctx = types.SimpleNamespace(seq_slot=ints([0]), seq_q_start=ints([0]), seq_q_len=ints([n]), n_seqs=1, n_tokens=n, max_q_len=n,
+                                         stream=K.stream_handle(), dtype=torch.bfloat16, ws=Workspace(DEV, 2048))
+        self.u = (0.9 * torch.randn(n, 4 * heads * d, device=DEV)).to(torch.bfloat16)
+        self.coef = torch.empty(n, heads * 4, device=DEV)
+        self.la, self.b = torch.empty(n, heads, device=DEV), torch.empty(n, heads, device=DEV)
+        MK.gates(self.ctx, 0.9 * torch.randn(n, 2 * heads, device=DEV), 0, heads, torch.randn(heads, device=DEV), forget + torch.randn(heads, device=DEV),
+                 15.0, torch.zeros(1, heads, device=DEV), self.coef, heads, self.la, self.b)
+
+    def run(self, chunked):
+        """(results [n, heads, d + 1], memory [heads, d, d + 1])"""
+        from bare_cuda_4gib_b200.kernels import linear_attention as LA, mlstm as MK
+        heads, d, n, wide = self.heads, self.d, self.n, self.heads * self.d
+        state, out = torch.zeros(1, heads, d, d + 4, device=DEV), torch.empty(n, heads * (d + 4), device=DEV)
+        if chunked:
+            MK.chunked(self.ctx, self.u, 0, wide, 2 * wide, self.la, self.b, state, out, heads, d, d, d ** -0.5)
+        else:
+            qf, kf, vf = torch.empty(n, wide, device=DEV), torch.empty(n, wide, device=DEV), torch.empty(n, heads * (d + 4), device=DEV)
+            decay = torch.empty(n, heads, device=DEV)
+            MK.operands(self.ctx, self.u, 0, wide, 2 * wide, self.coef, qf, kf, decay, vf, heads, d, d, d + 4)
+            LA.scan(self.ctx, qf, kf, vf, decay, "token", state, out, heads, d, d + 4, d ** -0.5)
+        return out.view(n, heads, d + 4)[..., : d + 1], state[0, ..., : d + 1]
+
+    def exact(self, size=False):
+        """The recurrence in 64 bits; with `size` the sum of its terms' sizes."""
+        f = (lambda x: x.abs()) if size else (lambda x: x)
+        q, k, v = (f(self.u[:, i * self.heads * self.d: (i + 1) * self.heads * self.d].double().view(self.n, self.heads, self.d)) for i in range(3))
+        v = torch.cat([v, torch.ones_like(v[..., :1])], -1)
+        a, b = self.la.double().exp(), self.b.double()
+        S, out = torch.zeros(self.heads, self.d, self.d + 1, dtype=torch.float64, device=DEV), []
+        for t in range(self.n):
+            S = a[t, :, None, None] * S + b[t, :, None, None] * k[t, :, :, None] * v[t, :, None]
+            out.append(torch.einsum("hkv,hk->hv", S, q[t] * self.d ** -0.5))
+        return torch.stack(out), S
+
+
+@pytest.mark.parametrize("d,n,forget", [(128, 40, 0.0), (128, 300, 0.0), (128, 700, 3.0), (16, 200, 0.0)])
+def test_mlstm_chunked_is_no_further_from_64_bits_than_the_scan(d, n, forget):
+    """By the norm of the results, by their worst element and by the norm of the memory left behind (three inputs each)."""
+    far = []
+    for seed in range(3):
+        walks = _Walks(16, d, n, forget, seed)
+        (want, memory), (size, _) = walks.exact(), walks.exact(True)
+        far.append([[((y - want).norm() / want.norm()).item(), ((y - want).abs() / size).max().item(), ((s - memory).norm() / memory.norm()).item()]
+                    for y, s in (walks.run(True), walks.run(False))])
+    chunked, scan = torch.tensor(far).mean(0)
+    assert (chunked <= scan).all(), (chunked, scan)
+
+
+def test_mlstm_chunked_keeps_infinity_and_nan_from_earlier_tokens():
+    walks = _Walks(2, 128, 200, 0.0, 5)
+    clean, _ = walks.run(True)
+    for col, token, value in ((0, 37, float("nan")), (256, 70, float("inf")), (512, 105, float("nan")), (512 + 130, 150, float("inf"))):      # q, k, v, v
+        walks.u[token, col] = value
+    got, scanned = walks.run(True)[0], walks.run(False)[0]
+    assert torch.equal(got[:37], clean[:37]) and torch.equal(got[38:70, 0], clean[38:70, 0])
+    assert torch.equal(got[:150, 1, 1:], clean[:150, 1, 1:]) and torch.equal(got[:150, 1, 0], clean[:150, 1, 0])
+    assert not torch.isfinite(got[37, 0]).any() and not torch.isfinite(got[105:, 0, 0]).any() and not torch.isfinite(got[150:, 1, 2]).any()
+    assert (torch.isfinite(got) >= torch.isfinite(scanned)).all()
