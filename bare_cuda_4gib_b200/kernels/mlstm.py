@@ -9,7 +9,7 @@ from typing import Optional
 import torch
 
 from . import build
-from .lib import _check, _dev, _ptr, dtype_code
+from .lib import _check, _dev, _ptr, dtype_code, sm_count
 
 _lib = None
 
@@ -64,6 +64,22 @@ def finish(ctx, scanned: torch.Tensor, coef: torch.Tensor, norm_w: torch.Tensor,
 def chunked_takes(dk: int, dv: int) -> bool:
     """Sizes the walk in chunks on the tensor cores is built for (csrc/mlstm_chunked.cu, a library per pair)."""
     return dk % 16 == 0 and 16 <= dk <= 256 and dv % 16 == 0 and 16 <= dv <= 1024
+
+
+def chunks_pay(q_len, heads: int, dk: int, dv: int) -> bool:
+    """Whether the walk in chunks takes less time than operands and scan for portions of these lengths (microseconds on one B200).
+
+    A request's blocks (one per head and 16 value columns, and one more) take about 14 a chunk however few tokens it holds,
+    a block an SM, so many short portions, and single tokens beside a portion, are better off with the scan, which takes
+    about 0.145 a token at 16 heads of 128 x 128, 0.16 for every step of the longest chain and 1 a request.  Measured at that size,
+    chunks / scan: one portion of 24 tokens 15.2 / 16.7, of 64 15.6 / 30.6, of 2,048 214 / 487; two of 32 29.7 / 21.5, two of 64
+    29.9 / 35.0; eight of 32 114 / 51, of 64 115 / 90, of 128 118 / 167; 256 tokens beside four single ones 85 / 120, beside eight
+    141 / 123, beside 24 365 / 141; 1,024 beside eight 220 / 295, beside 24 445 / 342."""
+    blocks, tokens = heads * (-(-dv // 16) + 1), 128 if dk <= 128 else 64
+    chunks = [-(-n // tokens) for n in q_len]
+    walk = 2.0 + 14.0 * max(max(chunks), -(-sum(chunks) * blocks // sm_count()))
+    scan = 8.0 + 0.145 * sum(q_len) * (heads * dk * dv) / (16 * 128 * 128) + 0.16 * max(q_len) + 1.0 * len(q_len)
+    return walk < 0.95 * scan
 
 
 _chunked_libs = {}

@@ -30,9 +30,6 @@ from .registry import register_mixer
 from ..weights.loader import fused_rows
 
 
-CHUNKED_MIN_TOKENS = 32      # steps whose longest portion has at least this many tokens walk in chunks on the tensor cores
-
-
 @register_mixer("mlstm")
 class MLSTM(Part):
     takes_lazy_input = False
@@ -78,6 +75,15 @@ class MLSTM(Part):
         if self.chunked:
             MK.chunked_lib(self.dim, self.vdim)      # compiled with the model, not at its first portion
 
+    def _in_chunks(self, ctx) -> bool:
+        """Whether this step's portions walk in chunks: asked once per step for all layers of a size."""
+        if not (self.chunked and ctx.use_fast_attention):
+            return False
+        key = ("mlstm_chunks", self.heads, self.dim, self.vdim)
+        if key not in ctx.extras:
+            ctx.extras[key] = MK.chunks_pay(ctx.host_q_len, self.heads, self.dim, self.vdim)
+        return ctx.extras[key]
+
     def forward(self, ctx, call, h):
         n, H, dk, dv, dvp = ctx.n_tokens, self.heads, self.dim, self.vdim, self.vpad
         kd, vd = H * dk, H * dv
@@ -91,7 +97,7 @@ class MLSTM(Part):
             return self.o.forward(ctx, out, n, torch.float32, "mixer_out", allow_partials=True)
         coef = ctx.ws.get("mlstm_coef", (n, H * 4), torch.float32)
         scanned = ctx.ws.get("mlstm_scan", (n, H * dvp), torch.float32)
-        if self.chunked and ctx.use_fast_attention and ctx.max_q_len >= CHUNKED_MIN_TOKENS and u.stride(0) % 8 == 0 and u.data_ptr() % 16 == 0:
+        if self._in_chunks(ctx) and u.stride(0) % 8 == 0 and u.data_ptr() % 16 == 0:
             log_decay = ctx.ws.get("mlstm_log_decay", (n, H), torch.float32)
             weight = ctx.ws.get("mlstm_weight", (n, H), torch.float32)
             MK.gates(ctx, z, 0, H, self.i_bias, self.f_bias, self.cap, call.states[1], coef, H, log_decay, weight)

@@ -104,3 +104,15 @@ def test_random_weights_of_a_preset():
     tensors = random_tensors(expected, 5)
     assert set(tensors) == set(expected)
     assert abs(float(tensors["l0.norm1b"].float().mean()) - 1.0) < 0.05
+
+
+@pytest.mark.parametrize("lens,heads,d,pays", [
+    ([24], 16, 128, False), ([64], 16, 128, True), ([2048], 16, 128, True), ([32] * 2, 16, 128, False), ([32] * 8, 16, 128, False),
+    ([64] * 8, 16, 128, False), ([128] * 8, 16, 128, True), ([32] * 16, 16, 128, False), ([256] * 8, 16, 128, True),
+    ([64] + [1] * 4, 16, 128, False), ([256] + [1] * 8, 16, 128, False), ([256] + [1] * 24, 16, 128, False), ([1024] + [1] * 8, 16, 128, True),
+    ([1024] + [1] * 24, 16, 128, False), ([60, 30, 20], 16, 128, False), ([600, 300, 200], 16, 128, True), ([256], 4, 128, True),
+    ([32] * 8, 4, 128, False), ([64] + [1] * 24, 4, 128, False), ([400] * 2, 4, 128, True), ([256], 16, 256, True), ([32] * 8, 16, 256, False),
+    ([64] + [1] * 8, 16, 256, False), ([256] * 8, 16, 256, True)])
+def test_matrix_memories_walk_in_chunks_where_that_measured_faster(lens, heads, d, pays):
+    from bare_cuda_4gib_b200.kernels import mlstm as MK
+    assert MK.chunks_pay(lens, heads, d, d) == pays
