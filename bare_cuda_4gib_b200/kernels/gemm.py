@@ -353,9 +353,12 @@ def cluster_tile(rows: int, n_tiles: int) -> int:
     return -(-rows // (16 * tiles)) * 16
 
 
+CLUSTER_MAX_SIZE = 8
+
+
 def cluster_size(n_tiles: int, k: int) -> int:
     """Blocks that share a tile's K range: as many (1, 2, 4, 8) as two blocks an SM and two 64-wide K blocks each allow."""
-    c = 8
+    c = CLUSTER_MAX_SIZE
     while c > 1 and (n_tiles * c > 2 * sm_count() or -(-k // BK) < 2 * c):
         c //= 2
     return c
@@ -407,7 +410,8 @@ def run_cluster(ctx, plan: GemmPlan, kind: int, a, rows: int, out_dtype: torch.d
         if then is not None and then.tensors["weight"].data_ptr() % 16 == 0 and then.tensors["weight"].dtype in (torch.float32, torch.bfloat16):
             w, slices = then.tensors["weight"], tiles * cluster
             pre_x = ctx.ws.get("prenormed.cluster.x", (rows, n_out), torch.bfloat16, max_rows=CLUSTER_MAX_ROWS)
-            pre_sq = ctx.ws.get("prenormed.cluster.sq", (slices, CLUSTER_MAX_ROWS), torch.float32, max_rows=slices)
+            # one row of parts per slice; fewer rows are shared by larger clusters, so more slices
+            pre_sq = ctx.ws.get("prenormed.cluster.sq", (slices, CLUSTER_MAX_ROWS), torch.float32, max_rows=tiles * CLUSTER_MAX_SIZE)
             extra_out = (pre_x.data_ptr(), pre_x.stride(0), w.data_ptr(), DT_BF16 if w.dtype == torch.bfloat16 else DT_F32,
                          pre_sq.data_ptr(), pre_sq.stride(0))
             pre = Prenormed(then, pre_x, pre_sq, slices)

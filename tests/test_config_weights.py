@@ -299,3 +299,28 @@ def test_large_tensor_goes_through_the_staging_buffer_in_pieces(tmp_path, monkey
     assert got["w"].dtype == torch.bfloat16 and torch.equal(got["w"], t["w"].to(torch.bfloat16))
     assert got["i"].dtype == torch.int32 and torch.equal(got["i"], t["i"].to(torch.int32))
     assert got["f"].dtype == torch.float32 and torch.equal(got["f"], t["f"])
+
+
+def test_the_cluster_product_outgrows_no_buffer_of_the_workspace(monkeypatch):
+    """Fewer rows are shared by larger clusters, whose parts of the sums of squares are more: the buffer of a step of 240 rows holds
+    what any later step leaves."""
+    import ctypes
+    import types
+    from bare_cuda_4gib_b200.engine.step import Workspace
+    from bare_cuda_4gib_b200.kernels import gemm, lib as K
+
+    class Plan:
+        n, k = 2048, 5632
+        weight_map = act_map = lambda self, *sizes: ctypes.c_int()
+
+    calls = []
+    monkeypatch.setattr(gemm, "lib", lambda activation: types.SimpleNamespace(llm_gemm_cluster=lambda *a: calls.append(a) or 0))
+    monkeypatch.setattr(gemm, "error_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    ctx = types.SimpleNamespace(ws=Workspace("cpu", 2048), stream=0)
+    norm = types.SimpleNamespace(prenormable=True, tensors={"weight": torch.ones(2048)})
+    residual = torch.zeros(240, 2048)
+    for rows in (240, 128, 64, 32, 25, 12):
+        gemm.run_cluster(ctx, Plan(), gemm.CL_ADD, torch.zeros(rows, 5632, dtype=torch.bfloat16), rows, torch.float32, "out", K.AddTo(residual, norm))
+        pre = ctx.prenormed
+        assert pre.sq.shape[0] == pre.items and pre.sq.stride(0) >= rows
+    assert len(calls) == 6 and not ctx.ws.retired
