@@ -138,11 +138,13 @@ class AttentionPlan:
         self._pool_maps = {}
         self._decode_maps = {}
 
-    def key_blocks(self, kv_len: int, q_len: int, block: int) -> int:
-        """The most blocks of `block` keys that one tile of a request reads: `kv_len` keys, `q_len` tokens."""
+    def key_blocks(self, kv_len: int, q_len: int, block: int, window: int = 0) -> int:
+        """The most blocks of `block` keys that one tile of a request reads: `kv_len` keys, `q_len` tokens, `window` (or the
+        plan's)."""
         n = -(-kv_len // block)
-        if self.window:
-            n = min(n, -(-(self.window + q_len - 2) // block) + 1)
+        window = self.window or window
+        if window:
+            n = min(n, -(-(window + q_len - 2) // block) + 1)
         if self.chunk:
             whole = q_len == 1 and self.chunk % block == 0      # blocks of positions that begin with a block of keys
             n = min(n, self.chunk // block if whole else -(-(self.chunk + q_len - 2) // block) + 1)
@@ -216,7 +218,7 @@ def plan_for(head_dim: int, heads: int, kv_heads: int, distance_bias: bool = Fal
     return AttentionPlan(head_dim, heads, kv_heads, distance_bias, v_dim, softcap, window, chunk)
 
 
-def few_beside_prompts(plan: AttentionPlan, q_len, kv_len) -> list:
+def few_beside_prompts(plan: AttentionPlan, q_len, kv_len, window: int = 0) -> list:
     """In a step with prompt portions: the requests (at most 16 packed rows each) that a launch of the decode kernel takes,
     if that pays.  In the prefill kernel such a request's tile of 128 rows walks through all of its keys alone, so long
     contexts beside short portions make the launch as long as the longest of them; the decode kernel deals a
@@ -229,7 +231,7 @@ def few_beside_prompts(plan: AttentionPlan, q_len, kv_len) -> list:
     if not few or len(few) == len(q_len) or len(few) * plan.kv_heads > DECODE_MAX_TILES:
         return []
     tiles = [-(-q * plan.group // plan.prefill_rows) for q in q_len]
-    blocks = [plan.key_blocks(kv, q, 128) for q, kv in zip(q_len, kv_len)]
+    blocks = [plan.key_blocks(kv, q, 128, window) for q, kv in zip(q_len, kv_len)]
     chosen = set(few)
 
     def launch(which):
@@ -260,17 +262,21 @@ def decode_blocks(plan: AttentionPlan, n_tiles: int, max_q_len: int) -> Tuple[in
     return splits, 0
 
 
-def step_tiles(ctx, plan: AttentionPlan):
-    """The step's row tiles for this head grouping: built once per step and shared by all layers."""
-    key = ("attention_tiles", plan.group, plan.kv_heads, plan.head_dim, plan.distance_bias, plan.prefill_rows,
-           plan.decode is not None, plan.window, plan.chunk)
+def step_tiles(ctx, plan: AttentionPlan, window: int = 0):
+    """The step's row tiles for this head grouping: built once per step and shared by all layers.  `window`: the calls' (0: none),
+    where the plan was made without; it decides only whether a mixed step's few rows go apart."""
+    g = plan.group
+    rows_per_tile = 16 if ctx.max_q_len * g <= 16 else plan.prefill_rows
+    mixed = rows_per_tile != 16 and plan.tc is not None and plan.decode is not None and min(ctx.host_q_len) * g <= 16
+    if plan.window or not mixed:
+        window = 0
+    key = ("attention_tiles", g, plan.kv_heads, plan.head_dim, plan.distance_bias, plan.prefill_rows,
+           plan.decode is not None, plan.window, plan.chunk, window)
     cached = ctx.extras.get(key)
     if cached is not None:
         return cached
-    g = plan.group
-    rows_per_tile = 16 if ctx.max_q_len * g <= 16 else plan.prefill_rows
     # requests whose rows the decode kernel takes although others of the step bring a prompt
-    few = few_beside_prompts(plan, ctx.host_q_len, ctx.host_kv_len) if rows_per_tile != 16 else []
+    few = few_beside_prompts(plan, ctx.host_q_len, ctx.host_kv_len, window) if mixed else []
     apart = set(few)
     counts = [0 if s in apart else -(-q * g // rows_per_tile) for s, q in enumerate(ctx.host_q_len)]
     pad = ctx.pad_seqs if rows_per_tile == 16 else 0     # padded decode steps keep a fixed grid
@@ -329,7 +335,7 @@ def run(ctx, plan: AttentionPlan, q: torch.Tensor, out: torch.Tensor, cache: Cac
     more = (extras or AttentionExtras()).arguments(plan.heads, q.dtype)
     if plan.distance_bias and extras:
         raise KernelLaunchError("attention_mma (distance bias): the variant takes no blocks of positions, sink or gate")
-    tile_seq, tile_index, n_tiles, rows_per_tile, n_splits, dec_splits, half, n_few, few_splits, few_half = step_tiles(ctx, plan)
+    tile_seq, tile_index, n_tiles, rows_per_tile, n_splits, dec_splits, half, n_few, few_splits, few_half = step_tiles(ctx, plan, window)
     if plan.distance_bias:
         scratch_ptr = 0
         if n_splits > 1:

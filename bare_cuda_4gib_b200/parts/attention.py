@@ -71,7 +71,7 @@ class Attention(Part):
     def plan_step(self, ctx) -> None:
         if self.fast is not None and ctx.use_fast_attention:
             from ..kernels import attention as fast
-            fast.step_tiles(ctx, self.fast)
+            fast.step_tiles(ctx, self.fast, int(self.window or 0))
 
     takes_lazy_input = True
 
@@ -185,7 +185,7 @@ class GatedAttention(Part):
     def plan_step(self, ctx) -> None:
         if self.fast is not None and ctx.use_fast_attention:
             from ..kernels import attention as fast
-            fast.step_tiles(ctx, self.fast)
+            fast.step_tiles(ctx, self.fast, int(self.window or 0))
 
     def forward(self, ctx, call, h):
         from ..kernels import head_prepare as HP

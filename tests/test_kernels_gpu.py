@@ -872,13 +872,14 @@ def test_attention_decode_half_key_blocks(heads, kv_heads, page, window, count):
     _close(got, want, 2 ** -7, 1e-2)
 
 
-@pytest.mark.parametrize("heads,kv_heads,d,window", [(32, 4, 64, 0), (8, 8, 128, 0), (16, 4, 64, 300)])
-def test_attention_of_few_rows_beside_prompts(heads, kv_heads, d, window):
-    """Requests of a token or two with long contexts beside prompt portions: a launch each, together every row."""
+@pytest.mark.parametrize("heads,kv_heads,d,window,apart", [(32, 4, 64, 0, 5), (8, 8, 128, 0, 5), (16, 4, 64, 1500, 5), (16, 4, 64, 300, 0)])
+def test_attention_of_few_rows_beside_prompts(heads, kv_heads, d, window, apart):
+    """Requests of a token or two with long contexts beside prompt portions: a launch each, together every row.  (With a window of
+    300 positions no request reads more than four blocks of 128 keys, and one launch has them all.)"""
     seqs = [(1, 2000), (90, 90), (1, 1), (2, 1500), (1, 640), (130, 200), (1, 1024)]
     got, want, ctx = _attention_case(seqs, heads, kv_heads, d, 64, window, 5)
     tiles = [v for k, v in ctx.extras.items() if isinstance(k, tuple) and k[0] == "attention_tiles"]
-    assert tiles[0][7] == 5
+    assert tiles[0][7] == apart
     _close(got, want, 2 ** -7, 1e-2)
     seqs = [(1, 300), (90, 90), (260, 700)]             # short contexts stay in the prompts' launch
     got, want, ctx = _attention_case(seqs, heads, kv_heads, d, 64, window, 5)
