@@ -4,6 +4,7 @@ the token tile and of the K split, and the device error word that bounded waits 
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Dict, Optional, Tuple
@@ -178,6 +179,12 @@ def feature_tile(rows: int, n_out: int, swiglu: bool, multiple: int = 0) -> int:
     forced = os.environ.get("BARE_CUDA_B200_GEMM_BN")     # experiments only
     if forced and not multiple:
         return int(forced)
+    return _feature_tile(rows, n_out, swiglu, multiple)
+
+
+@functools.lru_cache(maxsize=4096)
+def _feature_tile(rows: int, n_out: int, swiglu: bool, multiple: int) -> int:
+    """The search itself, once for the same sizes: it takes 3.4 us on the host, and a layer of a step asks up to six times."""
     step = 32 if swiglu else 16
     best, best_cost = 256, None
     for bn in range(256, 63, -step):

@@ -324,3 +324,17 @@ def test_the_cluster_product_outgrows_no_buffer_of_the_workspace(monkeypatch):
         pre = ctx.prenormed
         assert pre.sq.shape[0] == pre.items and pre.sq.stride(0) >= rows
     assert len(calls) == 6 and not ctx.ws.retired
+
+
+def test_the_tile_of_a_product_is_searched_for_once(monkeypatch):
+    """Every layer of a step asks for the same tiles; only the first one pays for the search."""
+    from bare_cuda_4gib_b200.kernels import gemm
+    asked = []
+    cost = gemm.tile_cost
+    monkeypatch.setattr(gemm, "tile_cost", lambda *sizes: asked.append(sizes) or cost(*sizes))
+    sizes = [(851, 2560, False, 0), (851, 2560, False, 64), (851, 5632, True, 0)]
+    first = [gemm.feature_tile(*s) for s in sizes]
+    searched = len(asked)
+    assert searched and [gemm.feature_tile(*s) for s in sizes * 22] == first * 22 and len(asked) == searched
+    monkeypatch.setenv("BARE_CUDA_B200_GEMM_BN", "96")
+    assert gemm.feature_tile(851, 2560, False) == 96 and gemm.feature_tile(851, 2560, False, 64) == first[1]
