@@ -15,6 +15,7 @@ from that block, so a step of the same padded shape can be replayed as a CUDA gr
 from __future__ import annotations
 
 import gc
+import math
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -62,7 +63,7 @@ class Workspace:
         full[rows_axis] = max(min(self.max_rows, max_rows) if max_rows else self.max_rows, shape[rows_axis])
         if rows_axis == 1 and max_lead:
             full[0] = max(full[0], int(max_lead))
-        need = int(np.prod(full))
+        need = math.prod(full)      # (a step without a graph asks some 180 times)
         key = (name, dtype)
         buf = self._buffers.get(key)
         if buf is None or buf.numel() < need:
@@ -75,7 +76,7 @@ class Workspace:
             return buf[:need].view(full)[: shape[0]]
         # the stride of the leading axis follows from the rows axis and the width only, so it is
         # the same whatever `lead` a call asks for
-        per = full[1] * int(np.prod(full[2:]))
+        per = math.prod(full[1:])
         return buf[: shape[0] * per].view([shape[0]] + full[1:])[:, : shape[1]]
 
     def bytes(self) -> int:
