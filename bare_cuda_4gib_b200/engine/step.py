@@ -188,6 +188,8 @@ class StepRunner:
                 views.append(cache.cache_view(i, self._tables[where[0]][1], j) if where is not None else None)
                 states.append(cache.state_of(i, j))
             c.calls.append(CallContext(i, views, call.cache_from is None, states))
+        for part in model.all_parts():
+            getattr(part, "reserve", lambda ctx: None)(c)
 
     def _row_views(self, rows: int):
         """token ids, positions, batch sequence of a row, wanted rows: four arrays of `rows` entries at

@@ -318,8 +318,7 @@ def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
         return Partials(out)
     splits = choose_splits(rows, plan.n, plan.k, bn) if (allow_partials and out_dtype == torch.float32) else 1
     if splits > 1:
-        out = ctx.ws.get(buffer + ".partials", (splits, rows, plan.n), torch.float32, max_rows=SPLIT_MAX_ROWS,
-                         max_lead=max_splits(plan.n, plan.k))
+        out = _partials(ctx.ws, plan, buffer, splits, rows)
         stride = out.stride(0)
     else:
         out = ctx.ws.get(buffer, (rows, plan.n), out_dtype)
@@ -369,6 +368,23 @@ def cluster_size(n_tiles: int, k: int) -> int:
     while c > 1 and (n_tiles * c > 2 * sm_count() or -(-k // BK) < 2 * c):
         c //= 2
     return c
+
+
+def reserve_partials(ws, plan: GemmPlan, buffer: str, taken) -> None:
+    """Asks for the buffer of partial results that a step of a few rows will need of a product that more rows send to the cluster
+    product: otherwise no step before the first decode step asks for it (36 MB for 4,096 x 14,336).  `taken(rows)`: whether the
+    few-token product runs that many rows."""
+    if plan.k < CLUSTER_MIN_K or plan.n % 8 or 2 * plan.n * plan.k <= CLUSTER_FEW_BYTES:
+        return
+    few = [rows for rows in (8, 16, CLUSTER_FEW_ROWS) if not taken(rows)]
+    if any(choose_splits(rows, plan.n, plan.k, token_tile(rows)) > 1 for rows in few):
+        _partials(ws, plan, buffer, 1, 1)
+
+
+def _partials(ws, plan: GemmPlan, buffer: str, splits: int, rows: int) -> torch.Tensor:
+    """The [splits, rows, features] buffer for a product that splits K."""
+    return ws.get(buffer + ".partials", (splits, rows, plan.n), torch.float32, max_rows=SPLIT_MAX_ROWS,
+                  max_lead=max_splits(plan.n, plan.k))
 
 
 def cluster_kind(plan: GemmPlan, rows: int, out_dtype, swiglu: bool, epilogue) -> Optional[int]:

@@ -75,6 +75,9 @@ class Attention(Part):
 
     takes_lazy_input = True
 
+    def reserve(self, ctx) -> None:
+        self.o.reserve(ctx, "attn_proj")
+
     def forward(self, ctx, call, h):
         n = ctx.n_tokens
         qd = self.heads * self.head_dim

@@ -100,6 +100,9 @@ class Part:
     def prepare(self, dtype: torch.dtype, device: torch.device) -> None:
         """Called once after binding, on the device: fuse tensors, build tables, compile kernels."""
 
+    def reserve(self, ctx) -> None:
+        """Called once per step runner, before its first step: asks `ctx.ws` for buffers that only some later step would allocate."""
+
     # A part that must look at the batch on the host before its kernels run (to build work lists
     # and upload them) defines `plan_step(ctx)`; it is called once per step before `forward`, and
     # is NOT part of a captured CUDA graph, while `forward` may be.

@@ -31,6 +31,13 @@ class Linear:
             from ..kernels import gemv
             self.few = gemv.supports(self.weight)
 
+    def reserve(self, ctx, buffer: str) -> None:
+        """For a product whose result is added into the residual stream: asks the workspace for what a step of a few rows will leave
+        in `buffer`, so that the first such step does not have to allocate it."""
+        if self.fast is not None and ctx.use_fast_gemm:
+            from ..kernels import gemm, gemv
+            gemm.reserve_partials(ctx.ws, self.fast, buffer, lambda rows: self.few and gemv.takes(rows, self.in_features))
+
     def forward(self, ctx, a, rows: int, out_dtype: torch.dtype, buffer: str,
                 allow_partials: bool = False, swiglu: bool = False, epilogue=None,
                 glu: Optional[str] = None) -> Optional[K.Partials]:

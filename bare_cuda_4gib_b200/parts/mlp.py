@@ -35,6 +35,9 @@ class SwiGLUFeedForward(Part):
 
     takes_lazy_input = True
 
+    def reserve(self, ctx) -> None:
+        self.down.reserve(ctx, "ffn_out")
+
     def forward(self, ctx, h):
         n = ctx.n_tokens
         act = self.gate_up.forward(ctx, h, n, ctx.dtype, "ffn_act", swiglu=True)

@@ -338,3 +338,24 @@ def test_the_tile_of_a_product_is_searched_for_once(monkeypatch):
     assert searched and [gemm.feature_tile(*s) for s in sizes * 22] == first * 22 and len(asked) == searched
     monkeypatch.setenv("BARE_CUDA_B200_GEMM_BN", "96")
     assert gemm.feature_tile(851, 2560, False) == 96 and gemm.feature_tile(851, 2560, False, 64) == first[1]
+
+
+@pytest.mark.parametrize("n,k,asked", [(4096, 14336, True), (4096, 11008, True), (2048, 5632, False), (4096, 4096, False), (12288, 4096, True)])
+def test_the_workspace_is_asked_for_split_products_before_any_step(n, k, asked, monkeypatch):
+    """A product that more rows send elsewhere leaves no allocation of its partial results to the first decode step; one that never
+    splits at a few rows asks for nothing.  (The few-token product takes up to 24 rows of 2,048, 16 of 4,096, 8 of 5,632.)"""
+    import types
+    from bare_cuda_4gib_b200.engine.step import Workspace
+    from bare_cuda_4gib_b200.kernels import gemm, gemv
+    from bare_cuda_4gib_b200.parts.linear import Linear
+    monkeypatch.setattr(gemv, "smem_bytes", lambda rows, k: 1 if rows * k <= 16 * 4096 else 0)
+    linear = Linear(torch.empty(n, k, dtype=torch.bfloat16, device="meta"), "down")
+    linear.fast, linear.few = types.SimpleNamespace(n=n, k=k), True
+    ctx = types.SimpleNamespace(ws=Workspace("meta", 4096), use_fast_gemm=True)
+    linear.reserve(ctx, "ffn_out")
+    assert list(ctx.ws._buffers) == ([("ffn_out.partials", torch.float32)] if asked else [])
+    if asked:       # what any later call asks for fits
+        held = ctx.ws._buffers["ffn_out.partials", torch.float32]
+        for rows in (1, 8, 24, 200, 256):
+            gemm._partials(ctx.ws, linear.fast, "ffn_out", max(1, gemm.choose_splits(rows, n, k, gemm.token_tile(rows))), rows)
+        assert ctx.ws._buffers["ffn_out.partials", torch.float32] is held and not ctx.ws.retired
