@@ -332,10 +332,11 @@ def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
 
 # ------------------------------------------------------------------ a few dozen tokens, ends fused in
 CL_ADD, CL_SWIGLU, CL_ROPE = 1, 2, 3
-# Measured, a whole step of TinyLlama's 22 layers, product + norm + rotation kernels against this: 25 rows 1,187 -> 989 us,
-# 32 rows 1,208 -> 1,009, 48 rows 1,330 -> 1,125, 64 rows 1,376 -> 1,129, 96 rows 1,502 -> 1,218, 128 rows 1,599 -> 1,286,
-# 192 rows 1,955 -> 1,546, 240 rows 2,148 -> 1,591; eight layers of the Llama-3-8B sizes: 32 rows 1,067 -> 1,012, 64 rows
-# 1,191 -> 1,148, 128 rows 1,306 -> 1,243, 240 rows 1,900 -> 1,735.  Above, tokens are on the MMA rows.
+# Measured, a whole step of TinyLlama's 22 layers, product + norm + rotation kernels against this: 30 rows 1,230 -> 1,003 us,
+# 40 rows 1,314 -> 1,118, 64 rows 1,396 -> 1,119, 96 rows 1,513 -> 1,232, 130 rows 1,741 -> 1,458, 180 rows 1,951 -> 1,544, 240
+# rows 2,168 -> 1,607; four layers of the Llama-3-8B sizes: 30 rows 634 -> 597, 64 rows 691 -> 659, 112 rows 747 -> 710, 144 rows
+# 830 -> 810, 180 rows 1,022 -> 896, 240 rows 1,056 -> 981; of the Llama-2-7B sizes: 30 rows 488 -> 488, 64 rows 524 -> 534, 112 rows
+# 591 -> 588, 144 rows 648 -> 647, 180 rows 849 -> 751, 240 rows 886 -> 848.  Above, tokens are on the MMA rows.
 CLUSTER_MAX_ROWS = TOKENS_ON_ROWS_ABOVE
 # A tile of 96 or 128 tokens would fill an SM's shared memory with one block (96 rows 1,971 us, 128 rows 3,084).
 CLUSTER_TILE_ROWS = 64
@@ -349,16 +350,6 @@ CLUSTER_FEW_ROWS, CLUSTER_FEW_BYTES = 24, 64 << 20
 CLUSTER_MIN_K = 8 * BK      # shorter sums are too short to share: a block of the cluster would have no K block to itself
 
 
-def cluster_tile(rows: int, n_tiles: int) -> int:
-    """Tokens of a tile: the rows dealt out evenly over as few tiles as hold them, in steps of 16.  49 to 64 rows go in two
-    tiles where the twice as many blocks still fit two to an SM: the exchange at a tile's end lengthens with its tokens
-    (TinyLlama, 61 rows: 1,226 -> 1,127 us; the 224 tiles of the Llama-3-8B gate/up would queue, 64 rows 1,148 -> 1,349)."""
-    tiles = -(-rows // CLUSTER_TILE_ROWS)
-    if 48 < rows <= 64 and n_tiles <= sm_count():
-        tiles = 2
-    return -(-rows // (16 * tiles)) * 16
-
-
 CLUSTER_MAX_SIZE = 8
 
 
@@ -368,6 +359,42 @@ def cluster_size(n_tiles: int, k: int) -> int:
     while c > 1 and (n_tiles * c > 2 * sm_count() or -(-k // BK) < 2 * c):
         c //= 2
     return c
+
+
+@functools.lru_cache(maxsize=4096)
+def cluster_tile(rows: int, n_tiles: int, k: int) -> int:
+    """Tokens of a tile: the rows dealt out evenly over as few tiles as hold them, in steps of 16.  49 to 64 rows go in two
+    tiles where the blocks of a cluster still walk through at most 12 K blocks each: the exchange at a tile's end lengthens with
+    its tokens (TinyLlama, 61 rows: 1,226 -> 1,127 us a step).  With longer walks the larger cluster of one tile wins: 64 rows, one
+    tile / two: 4,096 x 4,096 (16 K blocks in two tiles) 12.1 / 12.2 us, 6,144 x 4,096 (32) 17.7 / 18.7, 4,096 x 11,008 (43) 21.7 / 23.8."""
+    tiles = -(-rows // CLUSTER_TILE_ROWS)
+    if 48 < rows <= 64 and cluster_walk(2 * n_tiles, k) <= 12:
+        tiles = 2
+    return -(-rows // (16 * tiles)) * 16
+
+
+def cluster_walk(n_tiles: int, k: int) -> int:
+    """The 64-wide K blocks that a block of a cluster goes through."""
+    return -(--(-k // BK) // cluster_size(n_tiles, k))
+
+
+CLUSTER_LONG_WALK = 48
+
+
+@functools.lru_cache(maxsize=4096)
+def cluster_pays(rows: int, n_tiles: int, k: int) -> bool:
+    """Whether the cluster product beats the split product and the kernel behind it, for `n_tiles` tiles of weight rows.  It does while
+    its blocks walk through K quickly.  With wide layers and several token tiles the clusters are small and the walks
+    long, and then the other product, whose one tile holds all tokens, is faster, until that tile leaves its ring too few
+    stages (more than 160 tokens).  Microseconds with the kernel behind it, cluster / other: 12,288 x 4,096 (32 K blocks a walk) 64
+    rows 27.5 / 28.9, (64) 128 rows 41.8 / 37.8, 192 rows 42.5 / 55.5, (64, and more blocks than two to an SM) 240 rows 74.5 / 63.7;
+    4,096 x 11,008 (43) 128 rows 28.3 / 30.5, (86) 144 rows 42.9 / 31.6, 192 rows 45.3 / 49.5; 4,096 x 14,336 (56) 96 rows 33.5 / 33.0,
+    (112) 144 rows 53.9 / 37.1, 192 rows 56.2 / 54.8, 240 rows 56.1 / 61.6."""
+    tiles = n_tiles * -(-rows // cluster_tile(rows, n_tiles, k))
+    walk = cluster_walk(tiles, k)
+    if tiles > 2 * sm_count():
+        return walk <= CLUSTER_LONG_WALK // 2
+    return walk <= CLUSTER_LONG_WALK or (rows > 160 and walk <= 2 * CLUSTER_LONG_WALK) or rows > 200
 
 
 def reserve_partials(ws, plan: GemmPlan, buffer: str, taken) -> None:
@@ -396,13 +423,13 @@ def cluster_kind(plan: GemmPlan, rows: int, out_dtype, swiglu: bool, epilogue) -
     if isinstance(epilogue, AddTo):
         r = epilogue.residual
         fits = (r.dtype == torch.float32 and r.shape[-1] == plan.n and r.stride(-1) == 1 and r.stride(0) % 4 == 0
-                and r.data_ptr() % 16 == 0)
+                and r.data_ptr() % 16 == 0 and cluster_pays(rows, -(-plan.n // BM), plan.k))
         return CL_ADD if fits else None
     if isinstance(epilogue, RotateAndCache):
         c, q = epilogue.cache, epilogue.q_out
         fits = (c.dtype == q.dtype == torch.bfloat16 and c.v_dim == c.head_dim and c.head_dim % 8 == 0 and 128 % c.head_dim == 0
                 and (epilogue.q_heads + 2 * c.kv_heads) * c.head_dim == plan.n and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0
-                and (c.k_ptr | c.v_ptr) % 8 == 0 and c.page_stride % 4 == 0)
+                and (c.k_ptr | c.v_ptr) % 8 == 0 and c.page_stride % 4 == 0 and cluster_pays(rows, -(-plan.n // BM), plan.k))
         return CL_ROPE if fits else None
     return None
 
@@ -423,7 +450,7 @@ def run_cluster(ctx, plan: GemmPlan, kind: int, a, rows: int, out_dtype: torch.d
         raise KernelLaunchError(f"gemm_cluster: activations {tuple(a.shape)} {a.dtype} do not fit weight [{plan.n}, {plan.k}]")
     n_out = plan.n // 2 if kind == CL_SWIGLU else plan.n
     tiles = -(-n_out // (BM // 2 if kind == CL_SWIGLU else BM))
-    bn = cluster_tile(rows, tiles)
+    bn = cluster_tile(rows, tiles, plan.k)
     cluster = cluster_size(tiles * -(-rows // bn), plan.k)
     pre = None
     extra_out, rope = (0, 0, 0, 0, 0, 0), (0, 0, 0, 0, 0, 1, 0, 0, 0, 0, 0, 0, 0)

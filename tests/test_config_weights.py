@@ -359,3 +359,18 @@ def test_the_workspace_is_asked_for_split_products_before_any_step(n, k, asked, 
         for rows in (1, 8, 24, 200, 256):
             gemm._partials(ctx.ws, linear.fast, "ffn_out", max(1, gemm.choose_splits(rows, n, k, gemm.token_tile(rows))), rows)
         assert ctx.ws._buffers["ffn_out.partials", torch.float32] is held and not ctx.ws.retired
+
+
+@pytest.mark.parametrize("n,k,rows_and_choice", [
+    (12288, 4096, {32: 1, 48: 1, 64: 1, 72: 0, 96: 0, 128: 0, 144: 0, 160: 0, 176: 1, 192: 1, 208: 0, 240: 0}),
+    (4096, 11008, {32: 1, 64: 1, 80: 1, 128: 1, 130: 0, 144: 0, 160: 0, 176: 1, 192: 1, 240: 1}),
+    (4096, 14336, {32: 1, 48: 1, 64: 1, 72: 0, 96: 0, 130: 0, 160: 0, 208: 1, 240: 1}),
+    (6144, 4096, {32: 1, 64: 1, 128: 1, 160: 1, 192: 1, 208: 1, 240: 1}),
+    (4096, 4096, {32: 1, 64: 1, 128: 1, 176: 1, 240: 1}), (2560, 2048, {32: 1, 64: 1, 128: 1, 240: 1}),
+    (2048, 2048, {32: 1, 64: 1, 130: 1, 240: 1}), (2048, 5632, {12: 1, 32: 1, 64: 1, 130: 1, 160: 1, 240: 1})])
+def test_the_cluster_product_runs_where_it_measured_faster(n, k, rows_and_choice):
+    from bare_cuda_4gib_b200.kernels import gemm
+    got = {rows: int(gemm.cluster_pays(rows, -(-n // 128), k)) for rows in rows_and_choice}
+    assert got == rows_and_choice
+    # 49 to 64 rows go in two tiles only with short walks through K
+    assert gemm.cluster_tile(64, -(-n // 128), k) == (32 if n <= 2560 else 64)
