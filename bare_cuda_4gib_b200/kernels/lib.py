@@ -250,6 +250,7 @@ def add_rmsnorm(residual: torch.Tensor, delta: Optional[Partials], weight: torch
 
 
 _matmul_f32 = None
+MATMUL_F32_MAX_FEATURES = 65535 * 64      # its blocks of weight rows (64 at least) are counted in a grid's second or third axis
 
 
 def _matmul_f32_lib():
@@ -270,7 +271,7 @@ def matmul_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, m: int, st
     n, k = w.shape
     if a.shape[-1] != k or out.shape[-1] != n or a.stride(-1) != 1 or out.stride(-1) != 1 or not w.is_contiguous():
         raise KernelLaunchError(f"matmul_plain: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)}")
-    if (a.dtype == w.dtype == out.dtype == torch.float32 and k > 0 and k % 4 == 0 and a.stride(-2) % 4 == 0
+    if (a.dtype == w.dtype == out.dtype == torch.float32 and k > 0 and k % 4 == 0 and a.stride(-2) % 4 == 0 and n <= MATMUL_F32_MAX_FEATURES
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         _check(_matmul_f32_lib().llm_matmul_f32(a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k, a.stride(-2),
                                                 out.stride(-2), sm_count(), stream if stream is not None else stream_handle()),

@@ -374,3 +374,19 @@ def test_the_cluster_product_runs_where_it_measured_faster(n, k, rows_and_choice
     assert got == rows_and_choice
     # 49 to 64 rows go in two tiles only with short walks through K
     assert gemm.cluster_tile(64, -(-n // 128), k) == (32 if n <= 2560 else 64)
+
+
+@pytest.mark.parametrize("n,general", [(65535 * 64, False), (65535 * 64 + 1, True), (9_000_000, True)])
+@pytest.mark.parametrize("rows", [1, 40, 600])
+def test_float32_products_of_very_many_features_keep_the_general_kernel(n, general, rows, monkeypatch):
+    """The float32 product counts its blocks of weight rows in a grid axis of 65,535; the general kernel takes any number.  Which
+    one runs must not hang on the number of rows (a result would then change its bits with the cut of a step)."""
+    import types
+    from bare_cuda_4gib_b200.kernels import lib as K
+    ran = []
+    monkeypatch.setattr(K, "_dev", lambda *tensors: None)
+    monkeypatch.setattr(K, "_matmul_f32_lib", lambda: types.SimpleNamespace(llm_matmul_f32=lambda *a: ran.append("float32") or 0))
+    monkeypatch.setattr(K, "plain", lambda: types.SimpleNamespace(lib=types.SimpleNamespace(llm_matmul_plain=lambda *a: ran.append("general") or 0)))
+    meta = lambda *shape: torch.empty(*shape, device="meta")
+    K.matmul_plain(meta(rows, 4), meta(n, 4), meta(rows, n), rows, stream=0)
+    assert ran == ["general" if general else "float32"]
