@@ -23,7 +23,8 @@ class RotaryPositions(Part):
         d, theta = int(self.params["head_dim"]), float(self.params["theta"])
         exponent = torch.arange(d // 2, dtype=torch.float32) * 2.0 / d
         self.inv_freq = (1.0 / (theta ** exponent)).to(device)
-        self.angles = ("rope", theta, d)      # layers that agree in these have the same angles
+        # layers that agree in these have the same angles (a subclass may make others of the same parameters)
+        self.angles = ("rope", theta, d) if type(self) is RotaryPositions else None
 
     def fused_rotation(self):
         """Inverse frequencies for kernels that rotate q and k themselves."""

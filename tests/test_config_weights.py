@@ -390,3 +390,25 @@ def test_float32_products_of_very_many_features_keep_the_general_kernel(n, gener
     meta = lambda *shape: torch.empty(*shape, device="meta")
     K.matmul_plain(meta(rows, 4), meta(n, 4), meta(rows, n), rows, stream=0)
     assert ran == ["general" if general else "float32"]
+
+
+def test_only_layers_with_the_same_frequencies_share_a_table_of_angles():
+    """A position encoding derived from the rotary one may scale its frequencies: its layers must not be handed the table of cosines
+    and sines of a layer that has the same parameters."""
+    from bare_cuda_4gib_b200.parts.base import PartSpec
+    from bare_cuda_4gib_b200.parts.rope import RotaryPositions
+
+    class Scaled(RotaryPositions):
+        def prepare(self, dtype, device):
+            super().prepare(dtype, device)
+            self.inv_freq = self.inv_freq / self.params["factor"]
+
+    made = [RotaryPositions(PartSpec("rope", {"head_dim": 64, "theta": theta})) for theta in (1e4, 1e4, 5e5)]
+    made += [Scaled(PartSpec("rope", {"head_dim": 64, "theta": 1e4, "factor": factor})) for factor in (1.0, 4.0)]
+    for position in made:
+        position.prepare(torch.bfloat16, torch.device("cpu"))
+    for a in made:
+        for b in made:
+            if a.angles is not None and a.angles == b.angles:
+                assert torch.equal(a.fused_rotation(), b.fused_rotation())
+    assert made[0].angles is not None and made[0].angles == made[1].angles
