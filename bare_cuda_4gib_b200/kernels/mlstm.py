@@ -66,6 +66,9 @@ def chunked_takes(dk: int, dv: int) -> bool:
     return dk % 16 == 0 and 16 <= dk <= 256 and dv % 16 == 0 and 16 <= dv <= 1024
 
 
+MAX_REQUESTS = 65535      # of the walk in chunks: they are a grid's third axis (the scan's first)
+
+
 def chunks_pay(q_len, heads: int, dk: int, dv: int) -> bool:
     """Whether the walk in chunks takes less time than operands and scan for portions of these lengths (microseconds on one B200).
 
@@ -75,6 +78,8 @@ def chunks_pay(q_len, heads: int, dk: int, dv: int) -> bool:
     chunks / scan: one portion of 24 tokens 15.2 / 16.7, of 64 15.6 / 30.6, of 2,048 214 / 487; two of 32 29.7 / 21.5, two of 64
     29.9 / 35.0; eight of 32 114 / 51, of 64 115 / 90, of 128 118 / 167; 256 tokens beside four single ones 85 / 120, beside eight
     141 / 123, beside 24 365 / 141; 1,024 beside eight 220 / 295, beside 24 445 / 342."""
+    if len(q_len) > MAX_REQUESTS:
+        return False
     blocks, tokens = heads * (-(-dv // 16) + 1), 128 if dk <= 128 else 64
     chunks = [-(-n // tokens) for n in q_len]
     walk = 2.0 + 14.0 * max(max(chunks), -(-sum(chunks) * blocks // sm_count()))

@@ -116,3 +116,8 @@ def test_random_weights_of_a_preset():
 def test_matrix_memories_walk_in_chunks_where_that_measured_faster(lens, heads, d, pays):
     from bare_cuda_4gib_b200.kernels import mlstm as MK
     assert MK.chunks_pay(lens, heads, d, d) == pays
+
+
+def test_matrix_memories_of_more_requests_than_a_grid_has_layers_keep_the_scan():
+    from bare_cuda_4gib_b200.kernels import mlstm as MK
+    assert MK.chunks_pay([64] * 65535, 1, 16, 16) and not MK.chunks_pay([64] * 65536, 1, 16, 16)
