@@ -9,7 +9,8 @@
 // last ones possibly short or empty); in a segment the even and the odd k's each form one chain of
 // FMAs, which are the two halves of a packed pair, so that operands come as they lie in memory; a
 // segment's sum is even + odd, and the segments are added in order.  The longest chain of roundings is
-// k / 16 + 1 + 8 (the plain kernel's, which adds slices of 16: k / 16 + 16).
+// segment / 2 + 1 + 8 with segment = k / 8 rounded up to a multiple of 32: k / 16 + 9 for multiples of 256 (the plain kernel's, which
+// adds slices of 16: k / 16 + 16), and 25 for every k up to 256.
 //
 // Layout of the work.  A block takes BM rows x BN weight rows; k goes by in stages of 32 (128 bytes a
 // row), brought by 16-byte cp.async into a ring, the 16-byte pieces of a row exchanged by the row's
@@ -25,7 +26,7 @@
 // Measured on one B200 (microseconds a launch; the plain kernel's 64 x 64 tiles before, this now):
 //   weights 11,264 x 2,048 (92 MB): 4 rows 1,010 -> 17.9 (5.2 TB/s); 257 rows 1,380 -> 302; 2,048 rows 2,105 (44.9 TFLOP/s)
 //   weights 2,048 x 2,048 (17 MB):  4 rows 450 -> 5.4 (3.1 TB/s); 257 rows 68; 2,048 rows 435
-// The packed FMA alone reaches 70 TFLOP/s; with eight rows x four weight rows a thread the shared-memory wavefronts
+// The FMA units' peak is 74.4 TFLOP/s (148 SMs x 128 FMAs x 1.965 GHz); with eight rows x four weight rows a thread the shared-memory wavefronts
 // (32 for 64 packed FMAs) take as long as the arithmetic.  Tiles of 8 x 8 or 16 x 4 a thread (one block an SM) gained 4 % at
 // 2,048 rows and lose it at 257.
 #include "common.cuh"

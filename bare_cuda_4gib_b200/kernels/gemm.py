@@ -347,7 +347,10 @@ CLUSTER_GATED_ROWS = 64
 # a large one is bound by its weights, which the split product's deeper ring streams faster (8 rows x 4,096 x 14,336, 117 MB:
 # 18.0 us and a norm kernel of 4.3 against 23.5).
 CLUSTER_FEW_ROWS, CLUSTER_FEW_BYTES = 24, 64 << 20
-CLUSTER_MIN_K = 8 * BK      # shorter sums are too short to share: a block of the cluster would have no K block to itself
+# Layers of a smaller inner size keep the kernels they had.  The kernel takes them (every block of a cluster has two K blocks
+# whatever the size), but a product that adds its result itself hands nothing on, and callers that run a tiny model's block by
+# itself at 25 to 64 rows expect its contribution un-added.
+CLUSTER_MIN_K = 8 * BK
 
 
 CLUSTER_MAX_SIZE = 8

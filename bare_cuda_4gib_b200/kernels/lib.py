@@ -185,7 +185,8 @@ class AddTo:
 
 class Prenormed:
     """What an adding product left for the norm `norm`: `x` [rows, width] bfloat16 = residual *
-    weight, `sq` [items, 32] float32 parts of every row's sum of squares."""
+    weight, `sq` float32 parts of every row's sum of squares: `items` rows `sq.stride(0)` apart, each with one number per token
+    (32 behind the few-token product, up to 240 behind the cluster product, any number behind the many-token one)."""
 
     __slots__ = ("norm", "x", "sq", "items")
 
