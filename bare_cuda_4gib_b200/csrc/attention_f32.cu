@@ -33,6 +33,7 @@ constexpr int CLUSTER = 8;                       // blocks that share a decoding
 constexpr int SLOTS = D == 64 ? 4 : 2;           // spans a block holds at once with few rows
 constexpr int PAIRS = D / 64;                    // pairs of output columns a lane owns
 constexpr int SPAN_BYTES = SPAN * D * 4;         // keys or values of a span
+constexpr int GRID_MAX = 65535;                  // of a grid's second and third axis
 constexpr int STATE_FLOATS = ROWS * (D + 2);     // m [ROWS], l [ROWS], o [ROWS][D]
 
 typedef unsigned long long pair32;
@@ -336,14 +337,12 @@ extern "C" int llm_attention_f32(const float* q, float* out, float* k_base, floa
                                  const int32_t* q_start, const int32_t* q_len, const int32_t* kv_len, int n_seqs, int max_q_len,
                                  int any_few, int q_heads, float scale, int window, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q_len <= 0) return 0;
-  if (head_dim != D || kv_heads < 1 || q_heads % kv_heads || n_seqs > 65535 || kv_heads > 65535) return ERR_BAD_SIZE;
+  if (head_dim != D || kv_heads < 1 || q_heads % kv_heads || kv_heads > GRID_MAX) return ERR_BAD_SIZE;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(k_base) |
        reinterpret_cast<uintptr_t>(v_base)) & 15 || page_stride % 4)
     return ERR_BAD_ALIGN;
   Args a;
   a.q = q, a.out = out;
-  a.cache = PagedCache{k_base, v_base, block_table, page_stride, table_stride, page_tokens, kv_heads, head_dim};
-  a.q_start = q_start, a.q_len = q_len, a.kv_len = kv_len;
   a.q_heads = q_heads, a.group = q_heads / kv_heads, a.window = window, a.scale = scale;
   const int smem = any_few ? Shared::TOTAL_FEW : Shared::TOTAL_WALK;
   static bool raised = false;
@@ -355,7 +354,7 @@ extern "C" int llm_attention_f32(const float* q, float* out, float* k_base, floa
   const long long tiles = ((long long)max_q_len * a.group + TILE_ROWS - 1) / TILE_ROWS;
   cudaLaunchConfig_t cfg = {};
   // clusters only where some request needs one: they leave a few SMs of each group idle
-  cfg.gridDim = dim3((unsigned)(any_few ? (tiles + CLUSTER - 1) / CLUSTER * CLUSTER : tiles), kv_heads, n_seqs);
+  cfg.gridDim = dim3((unsigned)(any_few ? (tiles + CLUSTER - 1) / CLUSTER * CLUSTER : tiles), kv_heads);
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -375,6 +374,11 @@ extern "C" int llm_attention_f32(const float* q, float* out, float* k_base, floa
   }
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  cudaLaunchKernelEx(&cfg, attention_f32_kernel, a);
+  for (int s = 0; s < n_seqs; s += GRID_MAX) {        // (one launch unless a step has more requests than a grid has layers)
+    a.cache = PagedCache{k_base, v_base, block_table + (long long)s * table_stride, page_stride, table_stride, page_tokens, kv_heads, head_dim};
+    a.q_start = q_start + s, a.q_len = q_len + s, a.kv_len = kv_len + s;
+    cfg.gridDim.z = n_seqs - s < GRID_MAX ? n_seqs - s : GRID_MAX;
+    if (cudaLaunchKernelEx(&cfg, attention_f32_kernel, a) != cudaSuccess) break;
+  }
   return launch_status();
 }

@@ -28,7 +28,7 @@ def _lib(head_dim: int):
 def takes(q: torch.Tensor, out: torch.Tensor, cache: K.CacheView) -> bool:
     """All float32, a head size the kernel is built for, and everything on 16-byte boundaries."""
     return (q.dtype == out.dtype == cache.dtype == torch.float32 and cache.head_dim in ATTENTION_F32_HEAD_DIMS
-            and cache.v_dim == cache.head_dim and cache.page_stride % 4 == 0 and q.is_contiguous() and out.is_contiguous()
+            and cache.v_dim == cache.head_dim and cache.kv_heads <= 65535 and cache.page_stride % 4 == 0 and q.is_contiguous() and out.is_contiguous()
             and (q.data_ptr() | out.data_ptr() | cache.k_ptr | cache.v_ptr) % 16 == 0)
 
 

@@ -166,3 +166,23 @@ def test_attention_f32_of_infinite_values_hangs_on_the_row_alone():
     K.attention_plain(case.q, plain, view, ints([kv - n + i for n, kv in seqs for i in range(n)]), ints([s for s, (n, _) in enumerate(seqs) for _ in range(n)]),
                       2, case.q.shape[0], 64 ** -0.5, 0)
     assert torch.isfinite(plain).all() and torch.isfinite(whole).all()
+
+
+def test_attention_f32_of_more_requests_than_a_grid_has_layers():
+    from bare_cuda_4gib_b200.kernels import attention_f32, lib as K
+    torch.manual_seed(12)
+    n, page, held = 65535 + 9, 16, 40
+    pool, q = torch.randn(held, 2, page, 64, device=DEV), torch.randn(n, 64, device=DEV)
+    ints = lambda x: x.to(device=DEV, dtype=torch.int32)
+    pages, kv = torch.randint(held, (n,)), torch.randint(1, page + 1, (n,))
+    table, ctx = ints(pages)[:, None].contiguous(), types.SimpleNamespace()
+    ctx.host_q_len, ctx.n_seqs, ctx.max_q_len, ctx.n_tokens, ctx.stream = [1] * n, n, 1, n, K.stream_handle()
+    ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len = ints(torch.arange(n)), ints(torch.ones(n)), ints(kv)
+    view = K.CacheView(pool.data_ptr(), pool[0, 1].data_ptr(), table, 2 * page * 64, 1, page, 1, 64, torch.float32)
+    out = torch.full_like(q, float("nan"))
+    attention_f32.run(ctx, q, out, view, 1, 0.125, 0)
+    keys = pool[pages.to(DEV)].double()
+    hidden = torch.arange(page, device=DEV)[None] >= kv.to(DEV)[:, None]
+    w = (torch.einsum("nd,njd->nj", q.double(), keys[:, 0]) * 0.125).masked_fill(hidden, -float("inf")).softmax(-1)
+    want = torch.einsum("nj,njd->nd", w, keys[:, 1])
+    assert ((out.double() - want).abs() <= (4 * 34 + 2 * 64 + 6) * EPS * want.abs().max()).all()
