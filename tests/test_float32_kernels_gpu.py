@@ -24,9 +24,10 @@ def test_matmul_f32(n, k):
     a, w = torch.randn(600, k, device=DEV), torch.randn(n, k, device=DEV)
     want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
     whole = _product(a, w, 600)
-    # chains of k / 16 + 32 packed FMAs at most, then the pair and the eight segments: each rounds once, relative to at most
-    # the sum of the sizes
-    assert ((whole.double() - want).abs() <= (k / 16 + 32 + 9) * EPS * size).all()
+    # a segment's chains of packed FMAs, then the pair and the eight segments: each rounds once, relative to at most the sum of
+    # the sizes
+    segment = -(--(-k // 8) // 32) * 32
+    assert ((whole.double() - want).abs() <= (segment / 2 + 1 + 8) * EPS * size).all()
     for rows in (1, 2, 3, 4, 5, 8, 9, 16, 17, 24, 25, 33, 64, 65, 100, 257):
         assert torch.equal(_product(a, w, rows), whole[:rows]), rows
 
@@ -78,7 +79,8 @@ class _Attention:
         attention_f32.run(ctx, q, out, view, self.kv_heads * self.group, self.dim ** -0.5, self.window)
         return out
 
-    def want(self):
+    def want(self, absent=()):
+        """In 64 bits; `absent`: (request, page of it) whose keys count as not there."""
         rows = []
         for s, (n, kv) in enumerate(self.seqs):
             held = self.table[s, : -(-kv // self.page)].long()
@@ -87,6 +89,8 @@ class _Attention:
             q = self.q[self.at[s]: self.at[s] + n].double().view(n, self.kv_heads, self.group, self.dim)
             i, j = (kv - n + torch.arange(n, device=DEV))[:, None], torch.arange(kv, device=DEV)[None]
             hidden = (j > i) | (i - j >= self.window) if self.window else j > i
+            for r, b in absent:
+                hidden = hidden | (r == s) & (j // self.page == b)
             w = (torch.einsum("tkgd,kjd->kgtj", q, k) * self.dim ** -0.5).masked_fill(hidden, -float("inf")).softmax(-1)
             rows.append(torch.einsum("kgtj,kjd->tkgd", w, v).reshape(n, -1))
         return torch.cat(rows)
@@ -166,6 +170,28 @@ def test_attention_f32_of_infinite_values_hangs_on_the_row_alone():
     K.attention_plain(case.q, plain, view, ints([kv - n + i for n, kv in seqs for i in range(n)]), ints([s for s, (n, _) in enumerate(seqs) for _ in range(n)]),
                       2, case.q.shape[0], 64 ** -0.5, 0)
     assert torch.isfinite(plain).all() and torch.isfinite(whole).all()
+
+
+@pytest.mark.parametrize("dim,kv_heads,group,page,window", [(64, 2, 2, 16, 40), (64, 1, 8, 64, 100), (128, 1, 4, 32, 0), (64, 2, 1, 32, 300)])
+def test_attention_f32_of_pages_that_are_not_held(dim, kv_heads, group, page, window):
+    """Pages behind the window of all of a request's rows are given back (no entry in the table, and NaN where they were), and a
+    page inside the window that is not held counts as absent: in the walk and in the cluster's form, at every cut."""
+    torch.manual_seed(dim + page)
+    seqs = [(1, 500), (2, 300), (70, 400), (33, 333)]            # (one or two tokens: the cluster's form; over eight rows: the walk)
+    case = _Attention(dim, kv_heads, group, seqs, window, page)
+    absent = [(s, (kv - 5) // page - 1) for s, (_, kv) in enumerate(seqs)]       # seen by the last rows, not held
+    want = case.want(absent)
+    gone = absent + [(s, b) for s, (n, kv) in enumerate(seqs) if window for b in range(max(0, kv - n - window + 1) // page)]
+    assert len(gone) > len(absent) + 5 or not window
+    for s, b in gone:
+        case.pool[case.table[s, b].long()] = float("nan")
+        case.table[s, b] = -1
+    whole = case.run([(s, 0, n) for s, (n, _) in enumerate(seqs)])
+    bound = (4 * (dim / 2 + 2) + 2 * 64 + 3 * (500 / 64 + 1)) * EPS          # as in test_attention_f32
+    assert ((whole.double() - want).abs() <= bound * want.abs().max()).all()
+    for tail in (1, 30):
+        parts = [(s, max(0, n - tail), min(n, tail)) for s, (n, _) in enumerate(seqs)]
+        assert torch.equal(case.run(parts), torch.cat([whole[case.at[s] + f: case.at[s] + f + n] for s, f, n in parts])), tail
 
 
 def test_attention_f32_of_more_requests_than_a_grid_has_layers():

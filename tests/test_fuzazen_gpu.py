@@ -178,6 +178,19 @@ def test_attention_kernels_with_blocks_sinks_and_gates(heads, kv_heads, d, dv, p
         _close(got, want, 1.5e-2)
 
 
+@pytest.mark.parametrize("heads,kv_heads,d", [(16, 4, 64), (8, 8, 128), (8, 1, 64)])
+@pytest.mark.parametrize("options", [dict(sink=2.0), dict(gate=True), dict(chunk=700), dict(chunk=1024, sink=1.0, gate=True),
+                                     dict(window=900, sink=200.0, gate=True)])
+def test_few_rows_beside_prompts_with_blocks_sinks_and_gates(heads, kv_heads, d, options):
+    """Requests of a token or two whose long contexts go to a launch of their own beside prompt portions: both launches are given
+    the options."""
+    seqs = [(1, 2000), (90, 90), (1, 1), (2, 1690), (1, 1300), (130, 200), (1, 1024)]
+    got, want, ctx = _attention_case(seqs, heads, kv_heads, d, d, 64, torch.bfloat16, seed=heads + d, **options)
+    (plan,) = [v for k, v in ctx.extras.items() if k[0] == "attention_tiles"]
+    assert plan[7] == 5
+    _close(got, want, 1.5e-2)
+
+
 @pytest.mark.parametrize("options", [dict(chunk=50, sink=2.0, gate=True), dict(chunk=100, window=30, sink=3.0), dict(gate=True),
                                      dict(chunk=7, sink=200.0, gate=True)])
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 1.5e-2)])

@@ -497,6 +497,42 @@ def test_gemm_many_tokens_rotates_and_writes_the_cache(rows, heads, kv_heads, d,
     assert not storage[~used].any()
 
 
+@pytest.mark.parametrize("rows,kv_heads,d", [(25, 2, 64), (64, 1, 128), (80, 2, 32), (241, 1, 64), (300, 2, 128)])
+def test_heads_turned_in_a_product_leave_a_borrowed_cache_alone(rows, kv_heads, d, monkeypatch):
+    """Both products whose end turns heads, asked not to write the cache (a layer that reads another layer's): the queries are
+    those of the writing call, bit by bit, and no element of the cache changes."""
+    from bare_cuda_4gib_b200.kernels import gemm
+    from bare_cuda_4gib_b200.kernels import lib as K
+    monkeypatch.setattr(gemm, "whole_heads_pay", lambda *sizes: True)
+    torch.manual_seed(rows + d)
+    ctx, k, heads, page, pages = _ctx(), 576, 4, 32, 16
+    ctx.extras = {}
+    a = ctx.ws.get("a", (rows, k), torch.bfloat16)
+    a.copy_(torch.randn(rows, k, device=DEV))
+    w = (torch.randn((heads + 2 * kv_heads) * d, k, device=DEV) / math.sqrt(k)).to(torch.bfloat16)
+    storage, table, view = _paged_cache(kv_heads, d, page, pages, torch.bfloat16)
+    table[0, :12] = torch.randperm(pages, device=DEV)[:12].int()
+    storage.copy_(torch.randn_like(storage.float()))
+    before = storage.clone()
+    seq, pos = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.arange(rows, dtype=torch.int32, device=DEV)
+    inv = 1.0 / 10000.0 ** (torch.arange(d // 2, device=DEV).float() * 2 / d)
+    plan, got = gemm.plan_for(w), []
+    for write in (False, True):
+        ctx.extras.clear()
+        q = torch.full((rows, heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+        end = K.RotateAndCache(q, view, pos, seq, inv, heads, write, ("rope", 10000.0, d))
+        if rows <= gemm.CLUSTER_MAX_ROWS:
+            assert gemm.cluster_kind(plan, rows, torch.float32, False, end) == gemm.CL_ROPE
+            assert gemm.run_cluster(ctx, plan, gemm.CL_ROPE, a, rows, torch.float32, "qkv", end) is None
+        else:
+            assert gemm.turns(end, plan.n)
+            assert gemm.run(ctx, plan, a, rows, torch.bfloat16, "qkv", True, False, end) is None
+        gemm.check_errors()
+        assert torch.equal(storage, before) == (not write)
+        got.append(q)
+    assert torch.equal(got[0], got[1]) and torch.isfinite(got[0].float()).all()
+
+
 def test_a_bounded_wait_runs_out_and_the_kernel_returns():
     """Every wait inside the pipelined kernels has a limit.  Here one is seen to run out: with the
     test hooks of the GEMM library the producer arms one stage's barrier and issues no copy for it,

@@ -66,9 +66,10 @@ def test_mlstm_chunked(heads, dk, dv, lens, forget):
                 assert not end[:, dv + 1:].any() and not mine[:, dv + 1:].any()
         at += n
     assert torch.equal(state[0], start[0]) and torch.equal(state[-1], start[-1])        # slots that no request of the step holds
-    # relative to the sum of the sizes of a result's terms: operands of 24 bits, exponentials of 2 units, and float32 sums of at
-    # most dk / 16 + 64 / 16 steps of three products each in the tensor core (2^-23 a step)
-    bound = (3 * (dk / 16 + 4) + 8) * 2.0 ** -23
+    # relative to the sum of the sizes of a result's terms: q . k is exact products, 16 at a time in the tensor core (which cuts
+    # off each of them, 2^-23 at most), those sums added pairwise in fours and then in order in float32 (2^-24 an addition); the
+    # rest is 64-bit numbers and one rounding of the result
+    bound = (16 + (2 + dk / 64) / 2 + 0.5) * 2.0 ** -23
     assert far["chunked"] <= bound, (far, bound)
     print(f"mlstm heads {heads} dk {dk} dv {dv}: chunked {far['chunked']:.2e} scan {far['scan']:.2e} bound {bound:.2e}")
 
