@@ -400,6 +400,15 @@ def cluster_pays(rows: int, n_tiles: int, k: int) -> bool:
     return walk <= CLUSTER_LONG_WALK or (rows > 160 and walk <= 2 * CLUSTER_LONG_WALK) or rows > 200
 
 
+def cluster_pays_gated(rows: int, n_tiles: int, k: int) -> bool:
+    """The same for a gated product of `n_tiles` tiles of 64 outputs, against tokens on the MMA rows (which run it from 61 rows on).
+    With long walks a block an SM and a few SMs with two take as long as two everywhere: it has to fill two thirds of the places.  Four
+    layers, 61 to 64 rows, cluster / tokens on rows: 11,008 x 4,096 (172 of 296 places) 539 / 520 us, 14,336 x 4,096 (224) 656 / 681; all of
+    TinyLlama's (5,632 x 2,048, 16 K blocks a walk) 1,112 / 1,147."""
+    tiles = n_tiles * -(-rows // cluster_tile(rows, n_tiles, k))
+    return rows <= SWIGLU_TOKENS_ON_ROWS_ABOVE or cluster_walk(tiles, k) <= CLUSTER_LONG_WALK or 3 * tiles >= 4 * sm_count()
+
+
 def reserve_partials(ws, plan: GemmPlan, buffer: str, taken) -> None:
     """Asks for the buffer of partial results that a step of a few rows will need of a product that more rows send to the cluster
     product: otherwise no step before the first decode step asks for it (36 MB for 4,096 x 14,336).  `taken(rows)`: whether the
@@ -422,7 +431,8 @@ def cluster_kind(plan: GemmPlan, rows: int, out_dtype, swiglu: bool, epilogue) -
     if plan.k < CLUSTER_MIN_K or not 0 < rows <= CLUSTER_MAX_ROWS or plan.n % 8 or (rows <= CLUSTER_FEW_ROWS and 2 * plan.n * plan.k > CLUSTER_FEW_BYTES):
         return None
     if swiglu:
-        return CL_SWIGLU if rows <= CLUSTER_GATED_ROWS else None      # (more rows: tokens on the MMA rows, one tile for 128 of them)
+        # (more rows: tokens on the MMA rows, one tile for 128 of them)
+        return CL_SWIGLU if rows <= CLUSTER_GATED_ROWS and cluster_pays_gated(rows, -(-plan.n // BM), plan.k) else None
     if isinstance(epilogue, AddTo):
         r = epilogue.residual
         fits = (r.dtype == torch.float32 and r.shape[-1] == plan.n and r.stride(-1) == 1 and r.stride(0) % 4 == 0

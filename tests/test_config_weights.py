@@ -412,3 +412,12 @@ def test_only_layers_with_the_same_frequencies_share_a_table_of_angles():
             if a.angles is not None and a.angles == b.angles:
                 assert torch.equal(a.fused_rotation(), b.fused_rotation())
     assert made[0].angles is not None and made[0].angles == made[1].angles
+
+
+@pytest.mark.parametrize("inter,k,choice", [(5632, 2048, 1), (11008, 4096, 0), (14336, 4096, 1)])
+def test_gated_products_of_61_to_64_rows_run_where_they_measured_faster(inter, k, choice):
+    import types
+    from bare_cuda_4gib_b200.kernels import gemm
+    plan = types.SimpleNamespace(n=2 * inter, k=k)
+    kinds = [gemm.cluster_kind(plan, rows, torch.bfloat16, True, None) for rows in (25, 60, 61, 64, 65)]
+    assert kinds == [gemm.CL_SWIGLU] * 2 + [gemm.CL_SWIGLU if choice else None] * 2 + [None]
