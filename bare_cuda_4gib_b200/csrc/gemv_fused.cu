@@ -32,9 +32,16 @@
 // producer warp streams the block's items through a ring of shared-memory stages (16 row pieces
 // of up to `kc` values each, one bulk copy per piece, landing on an mbarrier); it starts before
 // the kernel has waited for its predecessor in the stream, since weights are never written.
-// Eight consumer warps split each stage's k range, multiply out of shared memory, and at the end
-// of an item add their partial sums in warp order, so a result depends neither on the batch nor
-// on the grid.  x for all tokens sits in shared memory for the whole kernel.  Every
+// Eight consumer warps split each stage's k range, multiply out of shared memory, and leave their
+// sums of an item to the finishing warps, one for every eight tokens, which add them in warp order (so a
+// result depends neither on the number of tokens in a group of eight nor on the grid) and run the
+// item's end while the consumers are at the next item.  x for all tokens sits in shared memory for the
+// whole kernel.
+//
+// What bounds it: HBM for the wide products (gate and up of 5,632 x 2,048: 46 MB in 6.8 us from the wait of the kernel
+// before), the chain of memory trips for the others.  So nothing stands on that chain that need not: metadata,
+// angles and weights of norms are fetched before the wait, and the norm's factor per token is the finishers' business, beside the
+// products.  One decode step of TinyLlama's 22 layers: 1 token 714 -> 612 us, 8 tokens 781 -> 723 us.  Every
 // wait on an mbarrier is bounded: after about a second without progress the thread records an
 // error code, and from then on every wait of the block returns at once, so the block still
 // reaches its barriers and returns (its results are then invalid, which the error word tells).
@@ -44,7 +51,7 @@ namespace {
 
 constexpr int WARPS = 8;                       // consumer warps
 constexpr int CONSUMERS = WARPS * 32;
-constexpr int THREADS = CONSUMERS + 32;        // plus the producer warp
+constexpr int threads_of(int nt) { return CONSUMERS + 32 + 32 * nt; }   // plus the producer and a finishing warp per eight tokens
 constexpr int MAX_STAGES = 12;
 constexpr int ROW_PAD = 64;                    // bytes between row pieces of a stage beyond their data:
                                                // keeps the 16-byte reads of a quarter warp on distinct banks
@@ -55,6 +62,7 @@ constexpr int ERR_GEMV_PRODUCER = 21, ERR_GEMV_CONSUMER = 22;
 
 enum { PRO_BF16 = 0, PRO_NORM = 1, PRO_PRENORMED = 2 };
 constexpr int SQ_SLOTS = 32;                  // token slots per item in the sums-of-squares parts
+constexpr int SQ_BATCH = 32;                  // parts of a token that a lane asks for at once
 enum { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2, EPI_ROPE = 3 };
 
 
@@ -62,6 +70,7 @@ struct GemvArgs {
   const __nv_bfloat16* w;   // [w_rows, k] row-major
   int w_rows, k, n_items, tokens;
   int x_ld;                 // shared-memory row stride of x in elements
+  int x_rows;               // its rows: one per token, and one of zeros for all token slots beyond (PRO_NORM: a row per slot)
   int kc, stages;           // k values per stage of the ring, number of stages
   int norm_rows;            // PRO_NORM: residual rows staged in shared memory at a time
   int first_aliased;        // PRO_NORM: stages from this one on double as that staging area (else = stages)
@@ -155,6 +164,11 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+// Named barriers: 1 the consumers; 2 and 3: an item's sums lie in half 0 or 1 of `red`; 4 and 5: that half has been read.
+template <int NT>
+__device__ __forceinline__ void barrier_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(CONSUMERS + 32 * NT) : "memory"); }
+template <int NT>
+__device__ __forceinline__ void barrier_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(CONSUMERS + 32 * NT) : "memory"); }
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMERS) : "memory"); }
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -183,14 +197,13 @@ __device__ __forceinline__ void item_rows(const GemvArgs& a, int item, int g, in
 }
 
 template <int NT, int PRO, int EPI>
-__global__ void __launch_bounds__(THREADS, PRO == PRO_NORM ? 1 : 2) gemv_fused_kernel(const GemvArgs a) {
+__global__ void __launch_bounds__(threads_of(NT), PRO == PRO_NORM || NT > 1 ? 1 : 2) gemv_fused_kernel(const GemvArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int row_stride = a.kc * 2 + ROW_PAD, stage_bytes = 16 * row_stride;
   uint8_t* ring = smem;                                                              // [stages][16][row_stride]
-  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(ring + (size_t)a.stages * stage_bytes);   // [8 * NT][x_ld]
-  float* red = reinterpret_cast<float*>(xs + (size_t)8 * NT * a.x_ld);               // [2][WARPS][NT * 4][32]
-  float* scale_s = red + 2 * WARPS * NT * 4 * 32;                                    // PRO_PRENORMED: [SQ_SLOTS]
-  float* norm_ws = scale_s + SQ_SLOTS;                                               // PRO_NORM: [k]
+  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(ring + (size_t)a.stages * stage_bytes);   // [x_rows][x_ld]
+  float* red = reinterpret_cast<float*>(xs + (size_t)a.x_rows * a.x_ld);               // [2][WARPS][NT * 4][32]
+  float* norm_ws = red + 2 * WARPS * NT * 4 * 32;                                               // PRO_NORM: [k]
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(norm_ws + (PRO == PRO_NORM ? a.k : 0));
   uint64_t* empty_bar = full_bar + MAX_STAGES;
   uint64_t* x_bar = empty_bar + MAX_STAGES;
@@ -256,6 +269,171 @@ __global__ void __launch_bounds__(THREADS, PRO == PRO_NORM ? 1 : 2) gemv_fused_k
           const unsigned long long start = global_timer();
           while (!mbar_try_wait(&full_bar[s], (in_flight_parity >> s) & 1u) && global_timer() - start < WAIT_LIMIT_NS) {}
         }
+    return;
+  }
+
+  if (warp > WARPS) {
+    // ---- finishers: warp n adds up and finishes the sums of token group n while the consumers go on to the next item.  (As
+    // part of a consumer's work an item's end took as long as its products, 0.4 us.)
+    const int n = warp - WARPS - 1;
+    // What an item's epilogue reads that no kernel of the step writes: the next norm's weights; positions, angles and the
+    // places in the cache, a chain of three loads and a sine (1 us).  The first item's is fetched before the wait.
+    float rot_sin[2], rot_cos[2], pre_lo = 0.0f, pre_hi = 0.0f;
+    long long cache_at[2];
+    auto fetch_constant = [&](int item) {
+      if (EPI == EPI_ADD && a.pre_x) {
+        const int lo = item * 16 + g, hi = lo + 8;
+        const bool half = a.pre_w_dtype == DT_BF16;
+        const __nv_bfloat16* w16 = static_cast<const __nv_bfloat16*>(a.pre_w);
+        const float* w32 = static_cast<const float*>(a.pre_w);
+        if (lo < a.n_out) pre_lo = half ? __bfloat162float(w16[lo]) : w32[lo];
+        if (hi < a.n_out) pre_hi = half ? __bfloat162float(w16[hi]) : w32[hi];
+      }
+      if (EPI == EPI_ROPE) {
+        const int groups = a.cache.head_dim / 16, h = item / groups, i = (item % groups) * 8 + g;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          rot_sin[j] = 0.0f, rot_cos[j] = 1.0f, cache_at[j] = -1;
+          const int tok = n * 8 + 2 * t + j;
+          if (tok >= a.tokens) continue;
+          const int pos = a.positions[tok];
+          if (h < a.q_heads + a.cache.kv_heads && a.inv_freq) sincosf((float)pos * a.inv_freq[i], &rot_sin[j], &rot_cos[j]);
+          if (h >= a.q_heads && a.write_cache) {
+            const bool is_v = h >= a.q_heads + a.cache.kv_heads;
+            cache_at[j] = cache_offset(a.cache, a.row_seq[tok], pos, h - a.q_heads - (is_v ? a.cache.kv_heads : 0));
+          }
+        }
+      }
+    };
+    fetch_constant(blockIdx.x);
+    pdl_wait();
+    float scale[2] = {1.0f, 1.0f};
+    if (PRO == PRO_PRENORMED) {
+      // The norm's factor per token from the parts of its row's sum of squares: lane (p, j) takes parts p, p + 4, ... of token j,
+      // a batch of loads on its way at once, in eight sums (parts 32 apart), which meet in pairs as the four lanes then do (the
+      // same order whatever the batch).  Lanes as parts, one token after the other, took 2.1 us for one token and 3.1 us for
+      // eight, longer than the first item.
+      const int tok = n * 8 + (lane & 7);
+      float part[8];
+#pragma unroll
+      for (int m = 0; m < 8; ++m) part[m] = 0.0f;
+      if (tok < a.tokens) {
+        const float* from = a.sq_in + (a.row_index ? a.row_index[tok] : tok);
+        for (int i0 = lane >> 3; i0 < a.sq_items; i0 += 4 * SQ_BATCH) {
+          float v[SQ_BATCH];
+#pragma unroll
+          for (int b = 0; b < SQ_BATCH; ++b) v[b] = i0 + 4 * b < a.sq_items ? from[(long long)(i0 + 4 * b) * a.sq_stride] : 0.0f;
+#pragma unroll
+          for (int b = 0; b < SQ_BATCH; ++b) part[b & 7] += v[b];
+        }
+      }
+#pragma unroll
+      for (int half = 4; half > 0; half >>= 1)
+#pragma unroll
+        for (int m = 0; m < half; ++m) part[m] += part[m + half];
+      float sq = part[0];
+      sq += __shfl_xor_sync(0xffffffffu, sq, 16);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 8);
+      const float mine = 1.0f / sqrtf(sq / (float)a.k + a.eps);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) scale[j] = __shfl_sync(0xffffffffu, mine, 2 * t + j);
+    }
+    int buf = 0;
+    for (int item = blockIdx.x; item < a.n_items; item += gridDim.x) {
+      if (item != (int)blockIdx.x) fetch_constant(item);
+      float old_lo[2] = {0.0f, 0.0f}, old_hi[2] = {0.0f, 0.0f};
+      if (EPI == EPI_ADD) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int tok = n * 8 + 2 * t + j;
+          if (tok >= a.tokens) continue;
+          const float* res = static_cast<const float*>(a.out) + (long long)tok * a.out_stride;
+          if (item * 16 + g < a.n_out) old_lo[j] = res[item * 16 + g];
+          if (item * 16 + g + 8 < a.n_out) old_hi[j] = res[item * 16 + g + 8];
+        }
+      }
+      // Sums over the warps in index order.  v[0], v[1]: row "lo" for tokens 2t and 2t + 1; v[2], v[3]: row "hi".
+      barrier_sync<NT>(2 + buf);
+      float v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float s = 0.0f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) s += red[((size_t)(buf * WARPS + w) * NT * 4 + n * 4 + i) * 32 + lane];
+        v[i] = s;
+      }
+      if (item + 2 * (int)gridDim.x < a.n_items) barrier_arrive<NT>(4 + buf);
+      buf ^= 1;
+      float sq_mine[2] = {0.0f, 0.0f};   // EPI_ADD with pre outputs: this thread's share of its two tokens' sums of squares
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int tok = n * 8 + 2 * t + j;
+        if (tok >= a.tokens) continue;
+        float lo_v = v[j], hi_v = v[2 + j];
+        if (PRO == PRO_PRENORMED) {
+          lo_v *= scale[j];
+          hi_v *= scale[j];
+        }
+        if (EPI == EPI_STORE || EPI == EPI_ADD) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int row = item * 16 + g + 8 * half;
+            if (row >= a.n_out) continue;
+            const float val = half ? hi_v : lo_v;
+            const long long at = (long long)tok * a.out_stride + row;
+            if (EPI == EPI_ADD) {
+              const float now = (half ? old_hi[j] : old_lo[j]) + val;
+              static_cast<float*>(a.out)[at] = now;
+              if (a.pre_x) {
+                a.pre_x[(long long)tok * a.pre_x_stride + row] = __float2bfloat16_rn(now * (half ? pre_hi : pre_lo));
+                sq_mine[j] += now * now;
+              }
+            }
+            else if (a.out_dtype == DT_F32) static_cast<float*>(a.out)[at] = val;
+            else static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(val);
+          }
+        } else if (EPI == EPI_SWIGLU) {
+          const int col = item * 8 + g;
+          if (col >= a.n_out) continue;
+          const float val = glu_pair(lo_v, hi_v);
+          const long long at = (long long)tok * a.out_stride + col;
+          if (a.out_dtype == DT_F32) static_cast<float*>(a.out)[at] = val;
+          else static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(val);
+        } else {  // EPI_ROPE
+          const int d = a.cache.head_dim, groups = d / 16, half = d / 2;
+          const int h = item / groups, i = (item % groups) * 8 + g;   // head of [q; k; v], feature in the lower half
+          const float first = lo_v * rot_cos[j] - hi_v * rot_sin[j];  // v heads keep cos 1, sin 0
+          const float second = hi_v * rot_cos[j] + lo_v * rot_sin[j];
+          if (h < a.q_heads) {
+            const long long at = (long long)tok * a.out_stride + (long long)h * d + i;
+            if (a.out_dtype == DT_F32) {
+              static_cast<float*>(a.out)[at] = first;
+              static_cast<float*>(a.out)[at + half] = second;
+            } else {
+              static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(first);
+              static_cast<__nv_bfloat16*>(a.out)[at + half] = __float2bfloat16_rn(second);
+            }
+          } else if (cache_at[j] >= 0) {
+            const bool is_v = h >= a.q_heads + a.cache.kv_heads;
+            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(is_v ? a.cache.v : a.cache.k) + cache_at[j] + i;
+            dst[0] = __float2bfloat16_rn(first);
+            dst[half] = __float2bfloat16_rn(second);
+          }
+        }
+      }
+      if (EPI == EPI_ADD && a.pre_x) {
+        // the item's 16 rows are spread over the 8 lanes that share t: add them up, lane g = 0 writes
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float part = sq_mine[j];
+          part += __shfl_xor_sync(0xffffffffu, part, 4);
+          part += __shfl_xor_sync(0xffffffffu, part, 8);
+          part += __shfl_xor_sync(0xffffffffu, part, 16);
+          const int tok = n * 8 + 2 * t + j;
+          if (g == 0 && tok < a.tokens) a.pre_sq[(size_t)item * SQ_SLOTS + tok] = part;
+        }
+      }
+    }
     return;
   }
 
@@ -327,26 +505,16 @@ __global__ void __launch_bounds__(THREADS, PRO == PRO_NORM ? 1 : 2) gemv_fused_k
         bulk_load(xs + (size_t)r * a.x_ld, x + (long long)(a.row_index ? a.row_index[r] : r) * a.x_stride,
                   (uint32_t)a.k * 2u, x_bar);
     }
-    const int per_row = a.k / 8;
-    for (int r = a.tokens; r < 8 * NT; ++r)
-      for (int c = threadIdx.x; c < per_row; c += CONSUMERS)
+    for (int r = a.tokens; r < a.x_rows; ++r)
+      for (int c = threadIdx.x; c < a.k / 8; c += CONSUMERS)
         *reinterpret_cast<uint4*>(xs + (size_t)r * a.x_ld + c * 8) = make_uint4(0u, 0u, 0u, 0u);
-    if (PRO == PRO_PRENORMED) {
-      // the norm's factor per token from the parts of its row's sum of squares: lanes take items
-      // lane, lane + 32, ..., then the warp adds up (the same order whatever the batch)
-      for (int tok = warp; tok < a.tokens; tok += WARPS) {
-        const int src = a.row_index ? a.row_index[tok] : tok;
-        float sq = 0.0f;
-        for (int i = lane; i < a.sq_items; i += 32) sq += a.sq_in[(long long)i * a.sq_stride + src];
-        sq = warp_sum(sq);
-        if (lane == 0) scale_s[tok] = 1.0f / sqrtf(sq / (float)a.k + a.eps);
-      }
-    }
     mbar_wait(x_bar, 0, gave_up, a.error_word, ERR_GEMV_CONSUMER);
   }
   consumer_barrier();
   if (PRO == PRO_NORM && threadIdx.x == 0) mbar_arrive(norm_done);
-
+  const __nv_bfloat16* x_row[NT];      // this thread's token slot in each group of eight
+#pragma unroll
+  for (int n = 0; n < NT; ++n) x_row[n] = xs + (size_t)min(n * 8 + g, a.x_rows - 1) * a.x_ld + 8 * t;
   int buf = 0, stage = 0;
   uint32_t phase = 0;
   for (int item = blockIdx.x; item < a.n_items; item += gridDim.x) {
@@ -355,32 +523,6 @@ __global__ void __launch_bounds__(THREADS, PRO == PRO_NORM ? 1 : 2) gemv_fused_k
     for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[n][i] = 0.0f;
-
-    // What the epilogue needs from memory does not depend on the sums: fetch it before the
-    // barrier (old residual values; positions, angles and cache addresses).
-    float old_lo[2] = {0.0f, 0.0f}, old_hi[2] = {0.0f, 0.0f}, rot_sin[2] = {0.0f, 0.0f}, rot_cos[2] = {1.0f, 1.0f};
-    long long cache_at[2] = {-1, -1};
-    if (warp < NT) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int tok = warp * 8 + 2 * t + j;
-        if (tok >= a.tokens) continue;
-        if (EPI == EPI_ADD) {
-          const float* res = static_cast<const float*>(a.out) + (long long)tok * a.out_stride;
-          if (item * 16 + g < a.n_out) old_lo[j] = res[item * 16 + g];
-          if (item * 16 + g + 8 < a.n_out) old_hi[j] = res[item * 16 + g + 8];
-        } else if (EPI == EPI_ROPE) {
-          const int d = a.cache.head_dim, groups = d / 16;
-          const int h = item / groups, i = (item % groups) * 8 + g;
-          const int pos = a.positions[tok];
-          if (h < a.q_heads + a.cache.kv_heads && a.inv_freq) sincosf((float)pos * a.inv_freq[i], &rot_sin[j], &rot_cos[j]);
-          if (h >= a.q_heads && a.write_cache) {
-            const bool is_v = h >= a.q_heads + a.cache.kv_heads;
-            cache_at[j] = cache_offset(a.cache, a.row_seq[tok], pos, h - a.q_heads - (is_v ? a.cache.kv_heads : 0));
-          }
-        }
-      }
-    }
 
     for (int k0 = 0; k0 < a.k; k0 += a.kc) {
       const int n_steps = min(a.kc, a.k - k0) / 32;
@@ -394,7 +536,7 @@ __global__ void __launch_bounds__(THREADS, PRO == PRO_NORM ? 1 : 2) gemv_fused_k
         const uint4 hi = *reinterpret_cast<const uint4*>(hi_row + s * 64);
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-          const uint4 b = *reinterpret_cast<const uint4*>(xs + (size_t)(n * 8 + g) * a.x_ld + k0 + s * 32 + 8 * t);
+          const uint4 b = *reinterpret_cast<const uint4*>(x_row[n] + k0 + s * 32);
           mma_bf16(acc[n], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
           mma_bf16(acc[n], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
         }
@@ -407,96 +549,13 @@ __global__ void __launch_bounds__(THREADS, PRO == PRO_NORM ? 1 : 2) gemv_fused_k
       }
     }
 
+    if (item >= (int)(blockIdx.x + 2 * gridDim.x)) barrier_sync<NT>(4 + buf);
     float* mine = red + ((size_t)(buf * WARPS + warp) * NT * 4) * 32;
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int i = 0; i < 4; ++i) mine[(n * 4 + i) * 32 + lane] = acc[n][i];
-    consumer_barrier();
-    // Warp n of the first NT warps finishes token group n: sums over the warps in index order,
-    // then the epilogue.  v[0], v[1]: row "lo" for tokens 2t and 2t + 1; v[2], v[3]: row "hi".
-    if (warp < NT) {
-      const int n = warp;
-      float v[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float s = 0.0f;
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) s += red[((size_t)(buf * WARPS + w) * NT * 4 + n * 4 + i) * 32 + lane];
-        v[i] = s;
-      }
-      float sq_mine[2] = {0.0f, 0.0f};   // EPI_ADD with pre outputs: this thread's share of its two tokens' sums of squares
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int tok = n * 8 + 2 * t + j;
-        if (tok >= a.tokens) continue;
-        float lo_v = v[j], hi_v = v[2 + j];
-        if (PRO == PRO_PRENORMED) {
-          lo_v *= scale_s[tok];
-          hi_v *= scale_s[tok];
-        }
-        if (EPI == EPI_STORE || EPI == EPI_ADD) {
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int row = item * 16 + g + 8 * half;
-            if (row >= a.n_out) continue;
-            const float val = half ? hi_v : lo_v;
-            const long long at = (long long)tok * a.out_stride + row;
-            if (EPI == EPI_ADD) {
-              const float now = (half ? old_hi[j] : old_lo[j]) + val;
-              static_cast<float*>(a.out)[at] = now;
-              if (a.pre_x) {
-                const float w = a.pre_w_dtype == DT_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.pre_w)[row])
-                                                         : static_cast<const float*>(a.pre_w)[row];
-                a.pre_x[(long long)tok * a.pre_x_stride + row] = __float2bfloat16_rn(now * w);
-                sq_mine[j] += now * now;
-              }
-            }
-            else if (a.out_dtype == DT_F32) static_cast<float*>(a.out)[at] = val;
-            else static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(val);
-          }
-        } else if (EPI == EPI_SWIGLU) {
-          const int col = item * 8 + g;
-          if (col >= a.n_out) continue;
-          const float val = glu_pair(lo_v, hi_v);
-          const long long at = (long long)tok * a.out_stride + col;
-          if (a.out_dtype == DT_F32) static_cast<float*>(a.out)[at] = val;
-          else static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(val);
-        } else {  // EPI_ROPE
-          const int d = a.cache.head_dim, groups = d / 16, half = d / 2;
-          const int h = item / groups, i = (item % groups) * 8 + g;   // head of [q; k; v], feature in the lower half
-          const float first = lo_v * rot_cos[j] - hi_v * rot_sin[j];  // v heads keep cos 1, sin 0
-          const float second = hi_v * rot_cos[j] + lo_v * rot_sin[j];
-          if (h < a.q_heads) {
-            const long long at = (long long)tok * a.out_stride + (long long)h * d + i;
-            if (a.out_dtype == DT_F32) {
-              static_cast<float*>(a.out)[at] = first;
-              static_cast<float*>(a.out)[at + half] = second;
-            } else {
-              static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16_rn(first);
-              static_cast<__nv_bfloat16*>(a.out)[at + half] = __float2bfloat16_rn(second);
-            }
-          } else if (cache_at[j] >= 0) {
-            const bool is_v = h >= a.q_heads + a.cache.kv_heads;
-            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(is_v ? a.cache.v : a.cache.k) + cache_at[j] + i;
-            dst[0] = __float2bfloat16_rn(first);
-            dst[half] = __float2bfloat16_rn(second);
-          }
-        }
-      }
-      if (EPI == EPI_ADD && a.pre_x) {
-        // the item's 16 rows are spread over the 8 lanes that share t: add them up, lane g = 0 writes
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          float part = sq_mine[j];
-          part += __shfl_xor_sync(0xffffffffu, part, 4);
-          part += __shfl_xor_sync(0xffffffffu, part, 8);
-          part += __shfl_xor_sync(0xffffffffu, part, 16);
-          const int tok = n * 8 + 2 * t + j;
-          if (g == 0 && tok < a.tokens) a.pre_sq[(size_t)item * SQ_SLOTS + tok] = part;
-        }
-      }
-    }
+    barrier_arrive<NT>(2 + buf);
     buf ^= 1;
   }
 }
@@ -510,7 +569,7 @@ int launch(const GemvArgs& a, size_t smem, int grid, cudaStream_t stream) {
       return launch_status();
     raised = true;
   }
-  launch_kernel(kern, grid, THREADS, smem, stream, a);
+  launch_kernel(kern, grid, threads_of(NT), smem, stream, a);
   return launch_status();
 }
 
@@ -536,7 +595,7 @@ int launch_pro(int pro, int epi, const GemvArgs& a, size_t smem, int grid, cudaS
 // How a launch lays out shared memory: the stage size kc (k values), the number of stages, the
 // residual rows staged at a time, and the total.  Returns false if x and two stages do not fit.
 struct SmemPlan {
-  int x_ld, kc, stages, norm_rows, first_aliased;
+  int x_ld, x_rows, kc, stages, norm_rows, first_aliased;
   size_t bytes;
 };
 
@@ -544,8 +603,11 @@ static bool plan_smem(int tokens, int k, int pro, size_t budget, int min_stages,
   if (tokens < 1 || tokens > 32 || k < 32 || k % 32) return false;
   const int nt = (tokens + 7) / 8;
   p.x_ld = k + ((k * 2) % 128 == 64 ? 0 : 32);
+  p.x_rows = pro == PRO_NORM || tokens == 8 * nt ? 8 * nt : tokens + 1;
   constexpr int kc_wish = 2048;   // the longest row piece of a stage: 4 KB per bulk copy (the copy unit's cost is per copy)
-  const size_t fixed = (size_t)8 * nt * p.x_ld * 2 + (size_t)2 * WARPS * nt * 4 * 32 * 4 + SQ_SLOTS * 4 +
+  // (the stage's size is that of a whole group of eight tokens, so that the order of a sum is; fewer tokens get more stages)
+  const size_t spare = (size_t)(8 * nt - p.x_rows) * p.x_ld * 2;
+  const size_t fixed = (size_t)8 * nt * p.x_ld * 2 + (size_t)2 * WARPS * nt * 4 * 32 * 4 +
                        (pro == PRO_NORM ? (size_t)k * 4 : 0) + (2 * MAX_STAGES + 2) * 8 + 16;
   // the stage size: the longest piece of a row (k / n values, a multiple of 32, at most kc_wish)
   // of which two stages fit; longer pieces mean fewer copies per byte
@@ -555,9 +617,9 @@ static bool plan_smem(int tokens, int k, int pro, size_t budget, int min_stages,
     if (use < 128 && n > 1) break;
     const size_t stage = (size_t)16 * (use * 2 + ROW_PAD);
     if (fixed + min_stages * stage > budget) continue;
-    size_t stages = (budget - fixed) / stage;
+    size_t stages = (budget - fixed + spare) / stage;
     if (stages > MAX_STAGES) stages = MAX_STAGES;
-    p.kc = use, p.stages = (int)stages, p.bytes = fixed + stages * stage;
+    p.kc = use, p.stages = (int)stages, p.bytes = fixed - spare + stages * stage;
     p.norm_rows = 0, p.first_aliased = (int)stages;
     if (pro == PRO_NORM) {
       // the staging area takes the ring's last stages; all eight rows of a token group at once if
@@ -606,7 +668,7 @@ extern "C" int llm_gemv_fused(const void* w, int w_rows, int k, int tokens, int 
   GemvArgs a = {};
   a.w = static_cast<const __nv_bfloat16*>(w);
   a.w_rows = w_rows, a.k = k, a.tokens = tokens;
-  a.x_ld = plan.x_ld, a.kc = plan.kc, a.stages = plan.stages, a.norm_rows = plan.norm_rows, a.first_aliased = plan.first_aliased, a.error_word = error_word;
+  a.x_ld = plan.x_ld, a.x_rows = plan.x_rows, a.kc = plan.kc, a.stages = plan.stages, a.norm_rows = plan.norm_rows, a.first_aliased = plan.first_aliased, a.error_word = error_word;
   a.x = x, a.x_stride = x_stride, a.norm_w = norm_w, a.norm_w_dtype = norm_w_dtype, a.eps = eps, a.row_index = row_index;
   a.out = out, a.out_dtype = out_dtype, a.out_stride = out_stride, a.n_out = n_out, a.up_offset = up_offset;
   a.cache = PagedCache{k_base, v_base, block_table, page_stride, table_stride, page_tokens, kv_heads, head_dim};

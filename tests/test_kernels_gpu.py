@@ -813,6 +813,36 @@ def test_gemv_fused_plain_and_add(tokens, n, k, norm):
     _close(target, before + want, 1e-5, 2e-4 * math.sqrt(k))
 
 
+def test_gemv_fused_many_items_and_parts():
+    """More items to a block than sums have halves, more parts of the sums of squares than a lane asks for at once, token slots
+    that share the row of zeros; and a token's result is the same bits in any batch of up to eight."""
+    import types as _types
+    from bare_cuda_4gib_b200.kernels import gemm, gemv
+    from bare_cuda_4gib_b200.kernels import lib as K
+    torch.manual_seed(4)
+    n, hidden = 16 * 700 + 5, 2112                    # 701 items over at most 148 blocks; 132 parts
+    ctx = _ctx()
+    ctx.dtype = torch.bfloat16
+    norm = _types.SimpleNamespace(prenormable=True, params={"eps": 1e-6, "size": hidden},
+                                  tensors={"weight": (1.0 + 0.2 * torch.randn(hidden, device=DEV)).to(torch.bfloat16)})
+    w_add = (torch.randn(hidden, 64, device=DEV) * 0.3).to(torch.bfloat16)
+    w = (torch.randn(n, hidden, device=DEV) * 0.1).to(torch.bfloat16)
+    act, stream = torch.randn(24, 64, device=DEV).to(torch.bfloat16), torch.randn(24, hidden, device=DEV)
+    results = {}
+    for tokens in (1, 8, 9, 24):
+        residual = stream[:tokens].clone()
+        assert gemv.run(ctx, w_add, act[:tokens], tokens, torch.float32, "out", False, K.AddTo(residual, norm)) is None
+        lazy = K.LazyNorm(ctx, residual, norm.tensors["weight"], 1e-6, tokens, None, "normed", ctx.prenormed)
+        results[tokens] = gemv.run(ctx, w, lazy, tokens, torch.float32, "out2", False, None).tensor.clone()
+    gemm.check_errors()
+    r = stream.double() + act.double() @ w_add.double().t()
+    x = r / torch.sqrt((r * r).mean(-1, keepdim=True) + 1e-6) * norm.tensors["weight"].double()
+    # the input is rounded to bfloat16 once, see test_gemv_fused_add_then_prenormed_input: sigma = 2^-9 / sqrt(3) * sqrt(hidden) * 0.1,
+    # and the bound is 8 sigma
+    _close(results[24], x @ w.double().t(), 0.0, 8 * 2.0 ** -9 / math.sqrt(3.0) * math.sqrt(hidden) * 0.1)
+    assert torch.equal(results[1], results[8][:1])
+
+
 @pytest.mark.parametrize("tokens,inter,k", [(2, 176, 64), (8, 100, 96), (16, 5632, 2048), (7, 13, 160)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_gemv_fused_swiglu(tokens, inter, k, norm):
