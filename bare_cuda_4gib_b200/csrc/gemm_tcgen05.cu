@@ -950,7 +950,10 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
 // members are simply neighbouring runs.
 // Two blocks share an SM (112 KB of shared memory each), so that a kernel's weights are on their way while
 // the kernel before it still runs on the other half.  What bounds it: the chain wait for the input - first tile - last
-// product - exchange - stores, which is why eight warps share the epilogue.  (Storing the slices straight from registers into
+// product - exchange - stores, which is why eight warps share the epilogue, why every role waits for the kernel before by itself,
+// and why metadata, angles and the next norm's weights are read before that wait (a step of 22 layers of TinyLlama's sizes: 26 rows
+// 992 -> 908 us, 61 rows 1,094 -> 987, 128 rows 1,289 -> 1,196, 240 rows 1,587 -> 1,476).  An arrival at the cluster's barrier that
+// releases costs about 0.5 us each time, waiting for the thread's own accesses.  (Storing the slices straight from registers into
 // the other blocks' shared memory, 16 bytes a lane, measured slower: 9.5 against 8.0 us for 64 tokens x 2,048 x 2,048.)
 enum { CL_ADD = 1, CL_SWIGLU = 2, CL_ROPE = 3 };
 constexpr int CL_MAX_TOKENS = 64;         // of a tile; more tokens are more tiles, which read the weights again, from L2
@@ -985,8 +988,9 @@ struct ClusterArgs {
   int* error_word;
 };
 
-// The cluster's barrier in two halves: a thread arrives, later waits, then may arrive again.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+// The cluster's barrier in two halves: a thread arrives, later waits, then may arrive again.  An arrival says only that this block
+// has its barriers (which fence.mbarrier_init has made visible) or has received its slices; data go by the copies' own barriers.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t peer_address(uint32_t smem_addr, int rank) {
@@ -1031,7 +1035,8 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
   float* received = reinterpret_cast<float*>(smem + a.stages * a.stage_bytes);      // [C][bn][ROWS], a slice `slot` apart
   float* sq_part = received + C * slot;                                             // [CL_EPI_WARPS][bn]
   float* scale_s = sq_part + CL_EPI_WARPS * a.bn;                                   // [bn]
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(scale_s + a.bn);
+  long long* place = reinterpret_cast<long long*>(scale_s + a.bn);                  // CL_ROPE: [bn], where a token's first key head goes in the cache
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(place + a.bn);
   uint64_t* empty_bar = full_bar + a.stages;
   uint64_t* acc_bar = empty_bar + a.stages;
   uint64_t* received_bar = acc_bar + 1;
@@ -1070,8 +1075,6 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(received_bar, (uint32_t)(C * n_tokens * ROWS * 4));
     for (int i = 0; i < n_early; ++i) issue_weights(i, i);   // overlaps the tail of the kernel before
-    pdl_wait();
-    for (int i = 0; i < n_early; ++i) issue_activations(i, i);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)),
@@ -1079,15 +1082,18 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_wait();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   cluster_arrive();        // this block has its barriers
   const uint32_t tmem_base = *tmem_base_slot;
+  // Every role that reads what other kernels write waits for them by itself: with a barrier of the block behind one thread's wait
+  // and copies the others began 0.9 us later.
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer (two lanes share a stage's copies)
+    pdl_wait();
+    if (lane < n_early) issue_activations(lane, lane);
     if (lane < 2) {
       int armed = n_early;
       int s = n_early == a.stages ? 0 : n_early;
@@ -1146,7 +1152,53 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
   } else {
     // ---------------------------------------------------------------- epilogue (warps 2..9)
     const int e = threadIdx.x - 64, ew = warp - 2, quad = warp & 3;   // quad: the tensor-memory lanes 32 quad .. of this warp
-    // What does not depend on the accumulator comes first: the norm's factor per token ...
+    // What does not depend on the accumulator comes first, before the wait what no kernel of the step writes: the next norm's
+    // weights; a token's place in the cache and its angles.  A thread owns RUN neighbouring features of a token, with pairs
+    // their partners too; a token's threads are neighbouring lanes.
+    constexpr bool PAIRED = EPI == CL_SWIGLU || EPI == CL_ROPE;
+    constexpr int RUN = EPI == CL_ROPE ? 2 : 4, PER_TOKEN = (PAIRED ? HALF : ROWS) / RUN, TOKEN_STEP = CL_EPI / PER_TOKEN;
+    static_assert(PER_TOKEN <= 32, "a token's threads lie in one warp");
+    const int at = e % PER_TOKEN * RUN, first_token = e / PER_TOKEN;     // first row of the slice that the thread owns
+    const int f_plain = f0 + rank * ROWS + at;                           // CL_ADD: its feature
+    // The residual values and angles of the thread's next two tokens.
+    float old[2][4], pre_w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float rot_c[2][2], rot_s[2][2];
+    const int dim = a.cache.head_dim, span = max(dim / 2, 1), first_pair = tile * 64 + rank * HALF + at;
+    const int head = first_pair / span, entry = first_pair % span;       // CL_ROPE: of [q; k; v]
+    const bool turned = EPI == CL_ROPE && a.inv_freq && head < a.q_heads + a.cache.kv_heads;
+    auto fetch_old = [&](int round, float (&o)[4]) {
+      const int mine = first_token + round * TOKEN_STEP;
+      if (mine < n_tokens && f_plain + 4 <= a.n_features) {
+        const float4 x = *reinterpret_cast<const float4*>(static_cast<const float*>(a.out) + (long long)(t0 + mine) * a.ld_out + f_plain);
+        o[0] = x.x, o[1] = x.y, o[2] = x.z, o[3] = x.w;
+      }
+    };
+    auto fetch_angles = [&](int round, float (&c)[2], float (&s)[2]) {
+      const int mine = first_token + round * TOKEN_STEP;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        c[j] = 1.0f, s[j] = 0.0f;
+        if (turned && mine < n_tokens) sincosf((float)a.positions[t0 + mine] * a.inv_freq[entry + j], &s[j], &c[j]);
+      }
+    };
+    if (EPI == CL_ADD && a.pre_x && f_plain + 4 <= a.n_features) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        pre_w[j] = a.pre_w_dtype == DT_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.pre_w)[f_plain + j])
+                                            : static_cast<const float*>(a.pre_w)[f_plain + j];
+    }
+    if (EPI == CL_ROPE) {
+      if (e < n_tokens) place[e] = a.write_cache ? cache_offset(a.cache, a.row_seq[t0 + e], a.positions[t0 + e], 0) : -1;
+      fetch_angles(0, rot_c[0], rot_s[0]);
+      fetch_angles(1, rot_c[1], rot_s[1]);
+      asm volatile("bar.sync 1, %0;" ::"n"(CL_EPI) : "memory");
+    }
+    pdl_wait();
+    if (EPI == CL_ADD) {
+      fetch_old(0, old[0]);
+      fetch_old(1, old[1]);
+    }
+    // The norm's factor per token.
     if (a.sq_in) {
       float sq[2] = {0.0f, 0.0f};
 #pragma unroll 16
@@ -1166,33 +1218,6 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
       }
       asm volatile("bar.sync 1, %0;" ::"n"(CL_EPI) : "memory");
     }
-    // ... and what the thread's first output needs.  A thread owns RUN neighbouring features of a token, with pairs their
-    // partners too; a token's threads are neighbouring lanes.
-    constexpr bool PAIRED = EPI == CL_SWIGLU || EPI == CL_ROPE;
-    constexpr int RUN = EPI == CL_ROPE ? 2 : 4, PER_TOKEN = (PAIRED ? HALF : ROWS) / RUN, TOKEN_STEP = CL_EPI / PER_TOKEN;
-    static_assert(PER_TOKEN <= 32, "a token's threads lie in one warp");
-    const int at = e % PER_TOKEN * RUN, first_token = e / PER_TOKEN;     // first row of the slice that the thread owns
-    const int f_plain = f0 + rank * ROWS + at;                           // CL_ADD: its feature
-    float old[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pre_w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    float rot_c[2] = {1.0f, 1.0f}, rot_s[2] = {0.0f, 0.0f};
-    const int dim = a.cache.head_dim, span = max(dim / 2, 1), first_pair = tile * 64 + rank * HALF + at;
-    const int head = first_pair / span, entry = first_pair % span;       // CL_ROPE: of [q; k; v]
-    const bool turned = EPI == CL_ROPE && a.inv_freq && head < a.q_heads + a.cache.kv_heads;
-    if (EPI == CL_ADD && f_plain + 4 <= a.n_features) {
-      if (first_token < n_tokens) {
-        const float4 o = *reinterpret_cast<const float4*>(static_cast<const float*>(a.out) + (long long)(t0 + first_token) * a.ld_out + f_plain);
-        old[0] = o.x, old[1] = o.y, old[2] = o.z, old[3] = o.w;
-      }
-      if (a.pre_x) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          pre_w[j] = a.pre_w_dtype == DT_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.pre_w)[f_plain + j])
-                                              : static_cast<const float*>(a.pre_w)[f_plain + j];
-      }
-    }
-    if (turned && first_token < n_tokens)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) sincosf((float)a.positions[t0 + first_token] * a.inv_freq[entry + j], &rot_s[j], &rot_c[j]);
 
     bool ok = mbar_wait(acc_bar, 0, abort_flag, a.wait_ns);
     if (!ok) {
@@ -1210,19 +1235,22 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
       const int pair = row / (2 * a.pair_span) * a.pair_span + in_group % a.pair_span;
       float* mine = outgoing + pair / HALF * slot + pair % HALF + (in_group >= a.pair_span ? HALF : 0);
       const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-#pragma unroll 1
-      for (int c0 = t_begin; c0 < t_end; c0 += 16) {
-        uint32_t v[16];
-        if (n_kb > 0) {
-          tmem_load16(lane_base + c0, v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      uint32_t v[2][16];       // at most 32 tokens
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (n_kb > 0 && t_begin + 16 * c < t_end) {
+          tmem_load16(lane_base + t_begin + 16 * c, v[c]);
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0u;
+          for (int j = 0; j < 16; ++j) v[c][j] = 0u;
         }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) mine[(c0 + j) * ROWS] = __uint_as_float(v[j]);
       }
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (t_begin + 16 * c < t_end)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) mine[(t_begin + 16 * c + j) * ROWS] = __uint_as_float(v[c][j]);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     cluster_wait();          // the others have their barriers
@@ -1272,12 +1300,8 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
             summed(mine, at, v);
             const long long where = (long long)t * a.ld_out + f_plain;
             float* res = static_cast<float*>(a.out) + where;
-            if (i > 0) {
-              const float4 o = *reinterpret_cast<const float4*>(res);
-              old[0] = o.x, old[1] = o.y, old[2] = o.z, old[3] = o.w;
-            }
 #pragma unroll
-            for (int j = 0; j < RUN; ++j) v[j] += old[j];
+            for (int j = 0; j < RUN; ++j) v[j] += old[0][j];
             store_run(res, v);
             if (a.pre_x) {
               float w[RUN];
@@ -1291,6 +1315,9 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
             for (int o = 1; o < PER_TOKEN; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
             if (at == 0 && there) a.pre_sq[(long long)(tile * C + rank) * a.pre_sq_stride + t] = sq;
           }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) old[0][j] = old[1][j];
+          fetch_old(i + 2, old[1]);
         } else if (there) {
           float u[RUN];
           summed(mine, at, v);
@@ -1303,28 +1330,29 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
             if (a.out_is_f32) store_run(static_cast<float*>(a.out) + (long long)t * a.ld_out + f, v);
             else store_run(static_cast<__nv_bfloat16*>(a.out) + (long long)t * a.ld_out + f, v);
           } else if (head < a.q_heads + 2 * a.cache.kv_heads) {     // CL_ROPE: RUN pairs of one head
-            const int pos = a.positions[t];
             if (turned) {
 #pragma unroll
               for (int j = 0; j < RUN; ++j) {
-                if (i > 0) sincosf((float)pos * a.inv_freq[entry + j], &rot_s[j], &rot_c[j]);
                 const float lo = v[j], hi = u[j];
-                v[j] = lo * rot_c[j] - hi * rot_s[j];
-                u[j] = hi * rot_c[j] + lo * rot_s[j];
+                v[j] = lo * rot_c[0][j] - hi * rot_s[0][j];
+                u[j] = hi * rot_c[0][j] + lo * rot_s[0][j];
               }
             }
             __nv_bfloat16* to = nullptr;
             if (head < a.q_heads) {
               to = static_cast<__nv_bfloat16*>(a.out) + (long long)t * a.ld_out + (long long)head * dim;
-            } else if (a.write_cache) {
+            } else if (place[mine] >= 0) {
               const bool is_v = head >= a.q_heads + a.cache.kv_heads;
-              const long long off = cache_offset(a.cache, a.row_seq[t], pos, head - a.q_heads - (is_v ? a.cache.kv_heads : 0));
-              if (off >= 0) to = static_cast<__nv_bfloat16*>(is_v ? a.cache.v : a.cache.k) + off;
+              const long long kvh = head - a.q_heads - (is_v ? a.cache.kv_heads : 0);
+              to = static_cast<__nv_bfloat16*>(is_v ? a.cache.v : a.cache.k) + place[mine] + kvh * a.cache.page_tokens * dim;
             }
             if (to) {
               store_run(to + entry, v);
               store_run(to + entry + span, u);
             }
+#pragma unroll
+            for (int j = 0; j < RUN; ++j) rot_c[0][j] = rot_c[1][j], rot_s[0][j] = rot_s[1][j];
+            if (i + 2 < rounds) fetch_angles(i + 2, rot_c[1], rot_s[1]);
           }
         }
       }
@@ -1408,7 +1436,7 @@ int launch_persistent(int bn, const CUtensorMap* map_w, const CUtensorMap* map_a
 
 // How a cluster product lays out a block: as many stages as let two blocks share an SM.
 static bool cluster_layout(int bn, int k_per_block, int& stages, size_t& smem) {
-  const size_t fixed = (size_t)(128 * bn + 8 * 8) * 4 + (size_t)(CL_EPI_WARPS + 1) * bn * 4 + (2 * MAX_STAGES + 2) * 8 + 16 + 1024;
+  const size_t fixed = (size_t)(128 * bn + 8 * 8) * 4 + (size_t)(CL_EPI_WARPS + 1) * bn * 4 + (size_t)bn * 8 + (2 * MAX_STAGES + 2) * 8 + 16 + 1024;
   const size_t stage = A_BYTES + (size_t)bn * BK * 2, budget = 112 * 1024;
   stages = (int)((budget - fixed) / stage);
   if (stages > k_per_block) stages = k_per_block;
