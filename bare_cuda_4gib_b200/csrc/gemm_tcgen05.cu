@@ -57,6 +57,16 @@ __device__ __forceinline__ unsigned long long global_timer() {
   return t;
 }
 
+// True in one thread of the (converged) warp.  The compiler knows that of elect.sync, and not of a test of the lane: behind `lane ==
+// 0` every tensor-core instruction and every copy, whose operands have to be uniform, becomes a loop over the threads that might
+// be there, about 110 cycles each: a k block's four products and two copies took 590 and 455 cycles, whatever the tile (2,048 x
+// 5,632, 300 rows 31.2 -> 19.5 us, 900 rows 34.7 -> 22.9; 11,264 x 2,048 gated, 900 rows 48.9 -> 43.3).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+  return elected != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
@@ -535,19 +545,19 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
   // One stage's loads, in two halves: the weight tiles depend on no other kernel and may be
   // fetched before pdl_wait(); the activation tile is another kernel's output and may not.
   // The first half arms the stage's barrier with the bytes of both.
-  auto issue_weights = [&](int i, int s, int which) {   // which: 0 = arm + first tile, 1 = second tile, 2 = both
+  auto issue_weights = [&](int i, int s) {
     uint8_t* stage = smem + s * geo.stage_bytes;
-    if (which != 1) mbar_expect_tx(&full_bar[s], geo.stage_bytes);
+    mbar_expect_tx(&full_bar[s], geo.stage_bytes);
     if (i == geo.drop_k_block) return;   // a test's way to leave a barrier waiting (never set otherwise)
     const int k0 = (kb_begin + i) * BK;
     if (ORIENT == 0) {
-      if (which != 1) tma_load_2d(stage, &map_w, &full_bar[s], k0, f0);   // MODE 1: map_w's box has 64 rows
-      if (MODE == 1 && which != 0) tma_load_2d(stage + A_BYTES / 2, &map_w, &full_bar[s], k0, up_row_offset + f0);
+      tma_load_2d(stage, &map_w, &full_bar[s], k0, f0);   // MODE 1: map_w's box has 64 rows
+      if (MODE == 1) tma_load_2d(stage + A_BYTES / 2, &map_w, &full_bar[s], k0, up_row_offset + f0);
     } else {
       uint8_t* b_tile = stage + A_BYTES;
-      if (which != 1) tma_load_2d(b_tile, &map_w, &full_bar[s], k0, w_row0 + f0);
+      tma_load_2d(b_tile, &map_w, &full_bar[s], k0, w_row0 + f0);
       // MODE 1: map_w's box has BN/2 rows: gate rows above, the matching up rows below
-      if (MODE == 1 && which != 0)
+      if (MODE == 1)
         tma_load_2d(b_tile + geo.b_bytes / 2, &map_w, &full_bar[s], k0, w_row0 + up_row_offset + f0);
     }
   };
@@ -561,7 +571,7 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
   const int n_early = min(n_kb, geo.stages);  // stages that are free from the start
 
   pdl_launch_dependents();
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
     for (int s = 0; s < geo.stages; ++s) {
@@ -572,9 +582,7 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    for (int i = 0; i < n_early; ++i) issue_weights(i, i, 2);   // overlaps the tail of the kernel before
-    pdl_wait();
-    for (int i = 0; i < n_early; ++i) issue_activations(i, i);
+    for (int i = 0; i < n_early; ++i) issue_weights(i, i);   // overlaps the tail of the kernel before
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_slot)),
@@ -582,7 +590,6 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_wait();  // every thread: nothing below may run ahead of the kernels before this one
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -590,10 +597,9 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    // Issuing a TMA copy costs the issuing thread a few hundred cycles, so a stage's copies are
-    // shared: lane 0 arms the barrier and fetches the weight tile(s), lane 1 the activations.
-    // (A third lane for the second weight tile of a SwiGLU product measured slower.)
-    if (lane < 2) {
+    if (elect_one()) {
+      pdl_wait();
+      for (int i = 0; i < n_early; ++i) issue_activations(i, i);
       int armed = n_early;
       // stage and phase advance by counting: a division per k block would slow the issue down
       int s = n_early == geo.stages ? 0 : n_early;
@@ -604,12 +610,12 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
           atomicCAS(error_word, 0, ERR_TIMEOUT_PRODUCER);
           break;
         }
-        if (lane == 1) issue_activations(i, s);
-        else issue_weights(i, s, 2);
+        issue_weights(i, s);
+        issue_activations(i, s);
         armed = i + 1;
         if (++s == geo.stages) { s = 0; phase ^= 1; }
       }
-      if (lane == 0 && *abort_flag) {
+      if (*abort_flag) {
         // copies already issued still land in shared memory: wait for them (bounded) before leaving
         for (int i = max(0, armed - geo.stages); i < armed; ++i) {
           const unsigned long long start = global_timer();
@@ -621,7 +627,7 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = geo.idesc;
       bool ok = true;
       int s = 0;
@@ -652,6 +658,7 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
     }
   } else {
     // ---------------------------------------------------------------- epilogue (warps 2..5)
+    pdl_wait();
     const int quad = warp & 3;  // tensor-memory lanes 32 * quad .. + 31 belong to this warp
     auto wait_acc = [&]() -> bool {
       bool ok = mbar_wait(tmem_full_bar, 0, abort_flag, geo.wait_ns);
@@ -786,7 +793,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
   const int n_tiles = f_tiles * t_tiles;
 
   pdl_launch_dependents();
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
     for (int s = 0; s < geo.stages; ++s) {
@@ -806,7 +813,6 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_wait();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -814,19 +820,14 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    // Issuing a copy costs its thread a few hundred cycles, about what the tensor core needs for
-    // a stage of a narrow tile.  So four lanes issue: lanes 0 and 1 take the even k blocks of the
-    // block's sequence (weights and barrier / activations), lanes 2 and 3 the odd ones.
-    if (lane < 4) {
-      const int role = lane & 1, turn = lane >> 1;
-      int s = turn % geo.stages, armed = 0;
+    if (elect_one()) {
+      pdl_wait();
+      int s = 0, armed = 0;
       uint32_t phase = 0;
-      int q = 0;   // k blocks of this thread block so far, over all its tiles
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         const int f0 = (tile / t_tiles) * F_TILE, t0 = (tile % t_tiles) * BM;
-        for (int i = 0; i < n_kb; ++i, ++q) {
-          if ((q & 1) != turn) continue;
+        for (int i = 0; i < n_kb; ++i) {
           if (!mbar_wait(&empty_bar[s], phase ^ 1, abort_flag, geo.wait_ns)) {
             *abort_flag = 1;
             atomicCAS(error_word, 0, ERR_TIMEOUT_PRODUCER);
@@ -834,22 +835,17 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
             break;
           }
           uint8_t* stage = smem + s * geo.stage_bytes;
+          uint8_t* b_tile = stage + A_BYTES;
           const int k0 = i * BK;
-          if (role == 0) {
-            mbar_expect_tx(&full_bar[s], geo.stage_bytes);
-            uint8_t* b_tile = stage + A_BYTES;
-            tma_load_2d(b_tile, &map_w, &full_bar[s], k0, f0);
-            if (MODE == 1) tma_load_2d(b_tile + geo.b_bytes / 2, &map_w, &full_bar[s], k0, up_row_offset + f0);
-          } else {
-            tma_load_2d(stage, &map_a, &full_bar[s], k0, t0);
-          }
-          armed = q + 1;
-          s += 2;
-          if (s >= geo.stages) { s -= geo.stages; phase ^= 1; }
+          mbar_expect_tx(&full_bar[s], geo.stage_bytes);
+          tma_load_2d(b_tile, &map_w, &full_bar[s], k0, f0);
+          if (MODE == 1) tma_load_2d(b_tile + geo.b_bytes / 2, &map_w, &full_bar[s], k0, up_row_offset + f0);
+          tma_load_2d(stage, &map_a, &full_bar[s], k0, t0);
+          ++armed;
+          if (++s == geo.stages) { s = 0; phase ^= 1; }
         }
       }
-      armed = max(armed, __shfl_sync(0xfu, armed, 2));
-      if (lane == 0 && *abort_flag) {
+      if (*abort_flag) {
         // copies already issued still land in shared memory: wait for them (bounded) before leaving
         for (int i = max(0, armed - geo.stages); i < armed; ++i) {
           const unsigned long long start = global_timer();
@@ -861,7 +857,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = geo.idesc, smem_base = smem_u32(smem);
       int s = 0, j = 0;
       uint32_t phase = 0;
@@ -898,6 +894,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
     }
   } else {
     // ---------------------------------------------------------------- epilogue (warps 2..5)
+    pdl_wait();
     const int quad = warp & 3;
     int j = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++j) {
@@ -1063,7 +1060,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
   const int n_early = min(n_kb, a.stages);
 
   pdl_launch_dependents();
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < a.stages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
@@ -1091,10 +1088,10 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
   // and copies the others began 0.9 us later.
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer (two lanes share a stage's copies)
-    pdl_wait();
-    if (lane < n_early) issue_activations(lane, lane);
-    if (lane < 2) {
+    // ---------------------------------------------------------------- TMA producer
+    if (elect_one()) {
+      pdl_wait();
+      for (int i = 0; i < n_early; ++i) issue_activations(i, i);
       int armed = n_early;
       int s = n_early == a.stages ? 0 : n_early;
       uint32_t phase = n_early == a.stages ? 1 : 0;
@@ -1104,12 +1101,12 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
           atomicCAS(a.error_word, 0, ERR_TIMEOUT_PRODUCER);
           break;
         }
-        if (lane == 1) issue_activations(i, s);
-        else issue_weights(i, s);
+        issue_weights(i, s);
+        issue_activations(i, s);
         armed = i + 1;
         if (++s == a.stages) { s = 0; phase ^= 1; }
       }
-      if (lane == 0 && *abort_flag) {
+      if (*abort_flag) {
         // copies already issued still land in shared memory: wait for them (bounded) before leaving
         for (int i = max(0, armed - a.stages); i < armed; ++i) {
           const unsigned long long start = global_timer();
@@ -1123,7 +1120,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     cluster_arrive();
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0;
       uint32_t phase = 0;
       const uint32_t smem_base = smem_u32(smem);
