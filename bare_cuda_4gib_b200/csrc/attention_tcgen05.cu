@@ -308,11 +308,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap pool_map, AttnArgs 
                  "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_wait();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  if (warp != MMA_WARP) pdl_wait();      // (the MMA issuer reads shared and tensor memory only)
   if (warp > MMA_WARP) {
     // ------------------------------------------------------------------ loader warp
     // Tile n of the ring is the keys (n even) or the values (n odd) of key block n / 2: one TMA box
@@ -322,7 +322,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap pool_map, AttnArgs 
     // reach P V.
     const int page_tokens = a.cache.page_tokens;
     const int32_t* table_row = a.cache.block_table + (long long)max(seq, 0) * a.cache.table_stride;
-    const int pieces = BN / a.box_rows;   // at most 16: lane p looks piece p up, lanes 0 and 1 issue the copies
+    const int pieces = BN / a.box_rows;   // at most 16: lane p looks piece p up, one thread issues the copies
     const uint32_t piece_mask = (pieces < 32) ? ((1u << pieces) - 1u) : 0xffffffffu;
     const int page_shift = (page_tokens & (page_tokens - 1)) == 0 ? __ffs(page_tokens) - 1 : -1;
     long long my_row = -1;     // lane p: the pool row (without the cache's K or V offset) of piece p, or -1
@@ -356,11 +356,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap pool_map, AttnArgs 
       if (lane == 0) mbar_expect_tx(&tile_full[slot], (uint32_t)__popc(held) * KA * a.box_rows * 128u);   // also the one arrival
       __syncwarp();
       const long long row0_of_cache = values ? a.v_row0 : a.k_row0;
-      for (int piece = 0; piece < pieces; ++piece) {     // lanes 0 and 1 take the pieces in turn: issuing is what takes the time
+      for (int piece = 0; piece < pieces; ++piece) {
         const long long row = __shfl_sync(0xffffffffu, my_row, piece);
-        if (lane != (piece & 1) || row < 0) continue;
-        for (int at = 0; at < KA; ++at)
-          tma_load_2d(base + at * SUB + piece * a.box_rows * 128, &pool_map, &tile_full[slot], at * 64, (int)(row + row0_of_cache));
+        if (row >= 0 && elect_one())
+          for (int at = 0; at < KA; ++at)
+            tma_load_2d(base + at * SUB + piece * a.box_rows * 128, &pool_map, &tile_full[slot], at * 64, (int)(row + row0_of_cache));
+        __syncwarp();
       }
     };
     bool ok = true;
@@ -395,7 +396,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap pool_map, AttnArgs 
     mbar_arrive(v_clean);      // in every case: the MMA thread must not wait in vain
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_kb > 0) {
+    if (n_kb > 0 && elect_one()) {
       constexpr uint32_t idesc_s = instr_desc(BM, BN, 0);
       constexpr uint32_t idesc_o = instr_desc(BM, 64, 1);
       auto active = [&](int g, int jj) { return kb_lo + jj >= g_lo[g] && kb_lo + jj < g_hi[g]; };

@@ -57,16 +57,6 @@ __device__ __forceinline__ unsigned long long global_timer() {
   return t;
 }
 
-// True in one thread of the (converged) warp.  The compiler knows that of elect.sync, and not of a test of the lane: behind `lane ==
-// 0` every tensor-core instruction and every copy, whose operands have to be uniform, becomes a loop over the threads that might
-// be there, about 110 cycles each: a k block's four products and two copies took 590 and 455 cycles, whatever the tile (2,048 x
-// 5,632, 300 rows 31.2 -> 19.5 us, 900 rows 34.7 -> 22.9; 11,264 x 2,048 gated, 900 rows 48.9 -> 43.3).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t elected;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
-  return elected != 0;
-}
-
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
