@@ -62,6 +62,10 @@ __device__ __forceinline__ void copies_wait_all() { asm volatile("cp.async.wait_
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same where nothing written has to be seen.
+__device__ __forceinline__ void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 __device__ __forceinline__ float peer_float(uint32_t smem_addr, uint32_t rank) {
   uint32_t at;
   float v;
@@ -195,25 +199,38 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
   const int kvh = blockIdx.y, seq = blockIdx.z, G = a.group;
   int* held = reinterpret_cast<int*>(smem + Shared::HELD);
   pdl_launch_dependents();
-  pdl_wait();
+  // the step's metadata is written by the host before the step's first kernel and by no kernel: it is read ahead of the wait
   const int q_len = a.q_len[seq], q_start = a.q_start[seq];
   const int rows = q_len * G, base_pos = a.kv_len[seq] - q_len;
   const bool few = rows <= ROWS;
   const int tiles = (rows + TILE_ROWS - 1) / TILE_ROWS;
-  if (rows == 0 || (!few && (int)blockIdx.x >= tiles) || (few && blockIdx.x >= CLUSTER)) return;   // whole clusters, or blocks of a walk
+  if (rows == 0 || (!few && (int)blockIdx.x >= tiles) || (few && blockIdx.x >= CLUSTER)) {         // whole clusters, or blocks of a walk
+    pdl_wait();
+    return;
+  }
   // the last tile sees the most keys: it starts first
   const int r0 = few ? 0 : (tiles - 1 - (int)blockIdx.x) * TILE_ROWS;
+  const int tile_last = base_pos + (min(r0 + TILE_ROWS, rows) - 1) / G;
+  const int tile_first = a.window > 0 ? max(0, base_pos + r0 / G - a.window + 1) : 0;
+  const int span_first = tile_first / SPAN, n_spans = tile_last / SPAN - span_first + 1;
+  const uint32_t spans = base + Shared::SPANS, p = base + Shared::P + warp * (ROWS * SPAN * 4);
+  // A few rows' first spans that lie below the step's first new position hold what earlier steps wrote: they too are asked for
+  // ahead of the wait.
+  auto early = [&](int s) { return s < n_spans && (span_first + s + 1) * SPAN <= base_pos; };
+  if (few) {
+#pragma unroll
+    for (int slot = 0; slot < SLOTS; ++slot) {
+      const int s = slot * CLUSTER + (int)blockIdx.x;
+      if (early(s)) stage_span(a, seq, kvh, span_first + s, tile_first, tile_last, spans + slot * 2 * SPAN_BYTES, held + slot * SPAN);
+    }
+  }
+  pdl_wait();
   for (int e = threadIdx.x; e < (few ? ROWS : TILE_ROWS) * (D / 4); e += THREADS) {
     const int r = r0 + e / (D / 4), c = (e % (D / 4)) * 4;
     float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (r < rows) v = *reinterpret_cast<const float4*>(a.q + ((long long)(q_start + r / G) * a.q_heads + kvh * G + r % G) * D + c);
     reinterpret_cast<float4*>(smem + Shared::Q)[e] = v;
   }
-  const int tile_last = base_pos + (min(r0 + TILE_ROWS, rows) - 1) / G;
-  const int tile_first = a.window > 0 ? max(0, base_pos + r0 / G - a.window + 1) : 0;
-  const int span_first = tile_first / SPAN, n_spans = tile_last / SPAN - span_first + 1;
-  const uint32_t spans = base + Shared::SPANS, p = base + Shared::P + warp * (ROWS * SPAN * 4);
-
   if (!few) {
     int first[ROWS], last[ROWS];
 #pragma unroll
@@ -284,7 +301,8 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
 #pragma unroll
     for (int slot = 0; slot < SLOTS; ++slot) {
       const int s = s0 + slot * CLUSTER + rank;
-      if (s < n_spans) stage_span(a, seq, kvh, span_first + s, tile_first, tile_last, spans + slot * 2 * SPAN_BYTES, held + slot * SPAN);
+      if (s < n_spans && !(s0 == 0 && early(s)))
+        stage_span(a, seq, kvh, span_first + s, tile_first, tile_last, spans + slot * 2 * SPAN_BYTES, held + slot * SPAN);
     }
     copies_commit();
     copies_wait_all();
@@ -321,7 +339,7 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
         O = join(O, o);
       }
     }
-    cluster_sync();                     // the states may be written again, and no block leaves while they are read
+    cluster_sync_relaxed();             // the states may be written again, and no block leaves while they are read
   }
   if (rank < rows && threadIdx.x < D) {
     const float inv = L > 0.0f ? 1.0f / L : 0.0f;

@@ -411,15 +411,20 @@ rope_cache_write_kernel(const TI* __restrict__ qkv, int n_partials, long long pa
                         const int32_t* __restrict__ row_seq, const float* __restrict__ inv_freq, int q_heads,
                         int write_cache) {
   pdl_launch_dependents();
-  pdl_wait();
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31;
   const int h = blockIdx.y * ROPE_HEADS_PER_BLOCK + (threadIdx.x >> 5);
   const int d = cache.head_dim, half = d / 2;
   const int kvh_n = cache.kv_heads;
   const int n_heads = q_heads + 2 * kvh_n;
-  if (h >= n_heads || (h >= q_heads && !write_cache)) return;
+  const bool none = h >= n_heads || (h >= q_heads && !write_cache);
+  // positions, angles and places in the cache are no kernel's results: fetched ahead of the wait
   const int pos = positions[t];
+  const long long off = !none && h >= q_heads ? cache_offset(cache, row_seq[t], pos, h - q_heads - (h >= q_heads + kvh_n ? kvh_n : 0)) : 0;
+  float c0 = 1.0f, s0 = 0.0f;
+  if (!none && h < q_heads + kvh_n && inv_freq && lane < half) sincosf((float)pos * inv_freq[lane], &s0, &c0);
+  pdl_wait();
+  if (none || off < 0) return;
   const TI* row = qkv + (long long)t * n_heads * d + (long long)h * d;
   auto load = [&](int i) {
     float v = 0.0f;
@@ -431,20 +436,16 @@ rope_cache_write_kernel(const TI* __restrict__ qkv, int n_partials, long long pa
     if (h < q_heads) {
       dst = q_out + ((long long)t * q_heads + h) * d;
     } else {
-      const long long off = cache_offset(cache, row_seq[t], pos, h - q_heads);
-      if (off < 0) return;
       dst = (TO*)cache.k + off;
     }
     for (int p = lane; p < half; p += 32) {
       const float lo = load(p), hi = load(p + half);
-      float c = 1.0f, s = 0.0f;
-      if (inv_freq) sincosf((float)pos * inv_freq[p], &s, &c);
+      float c = c0, s = s0;
+      if (inv_freq && p != lane) sincosf((float)pos * inv_freq[p], &s, &c);
       dst[p] = from_float<TO>(lo * c - hi * s);
       dst[p + half] = from_float<TO>(hi * c + lo * s);
     }
   } else {
-    const long long off = cache_offset(cache, row_seq[t], pos, h - q_heads - kvh_n);
-    if (off < 0) return;
     TO* dst = (TO*)cache.v + off;
     for (int i = lane; i < d; i += 32) dst[i] = from_float<TO>(load(i));
   }
