@@ -41,6 +41,11 @@ constexpr int BM = 128;      // features per block (MMA M)
 constexpr int BK = 64;       // k elements per stage (one 128-byte swizzle row)
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;
+// The gated end of tokens on the MMA rows, one block to an SM, is arithmetic (an exponential and a division an output) that nothing
+// hides: eight warps share it instead of four, half of the tile's columns each (300 tokens x 11,264 x 2,048: 23.4 -> 19.8 us).  The
+// adding end, which memory bounds, gets slower with eight (2,048 x 2,048 x 5,632: 44.4 -> 47.9).
+constexpr int epilogue_warps(int mode, int orient, int blocks_per_sm) { return mode == 1 && orient == 1 && blocks_per_sm == 1 ? 8 : 4; }
+constexpr int threads_of(int mode, int orient, int blocks_per_sm) { return 64 + 32 * epilogue_warps(mode, orient, blocks_per_sm); }
 constexpr unsigned long long WAIT_LIMIT_NS = 1000000000ull;
 
 constexpr int ERR_TIMEOUT_PRODUCER = 1;
@@ -203,12 +208,14 @@ __device__ __forceinline__ float row_scale(const RowsExtra& ex, int t, int n_tok
 // the tensor-memory address of the warp's lanes at the accumulator's first column; `have_acc`
 // false means an empty K range (zeros).  MODE 1: gate in column c, up in column BN/2 + c.
 // `wait_acc()` waits until the accumulator is complete (false: the block has given up, nothing is
-// stored); what does not depend on the accumulator is requested from memory before it is called.
+// stored); what does not depend on the accumulator is requested from memory before it is called.  Modes 0 (but for the adding end)
+// and 1 take the columns [c_begin, c_end) of the tile's F_TILE (multiples of 16).
 template <int MODE, int DEPTH, typename Wait>
 __device__ __forceinline__ void epilogue_tokens_on_rows(uint32_t lane_base, int BN, int F_TILE, int f0, int f_tile_index,
                                                         int t_first, int lane, bool have_acc, void* out, int out_is_f32,
                                                         long long ld_out, int n_tokens, int n_features,
-                                                        const RowsExtra& ex, const HeadsExtra& hx, float* staging, Wait&& wait_acc) {
+                                                        const RowsExtra& ex, const HeadsExtra& hx, float* staging, int c_begin, int c_end,
+                                                        Wait&& wait_acc) {
   float* out_f32 = reinterpret_cast<float*>(out);
   __nv_bfloat16* out_bf16 = reinterpret_cast<__nv_bfloat16*>(out);
   if (MODE == 0 && out_is_f32 == 2 && ex.pre_x) {
@@ -378,8 +385,8 @@ __device__ __forceinline__ void epilogue_tokens_on_rows(uint32_t lane_base, int 
   const bool vec_ok = out_is_f32 ? (ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out_f32) & 15) == 0)
                                  : (ld_out % 8 == 0 && (reinterpret_cast<uintptr_t>(out_bf16) & 15) == 0);
 #pragma unroll 1
-  for (int c0 = 0; c0 < F_TILE; c0 += 16) {
-    if (f0 + c0 >= n_features) break;  // uniform across the block
+  for (int c0 = c_begin; c0 < c_end; c0 += 16) {
+    if (f0 + c0 >= n_features) break;  // uniform across the warp
     uint32_t g[16], u[16];
     if (have_acc) {
       tmem_load16(lane_base + c0, g);
@@ -499,7 +506,7 @@ static int sm_count() {
 static size_t smem_bytes(const Geometry& g) { return (size_t)g.stages * g.stage_bytes + 1024 + 256; }
 
 template <int MODE, int ORIENT, int BLOCKS_PER_SM>
-__global__ void __launch_bounds__(NUM_THREADS, BLOCKS_PER_SM)
+__global__ void __launch_bounds__(threads_of(MODE, ORIENT, BLOCKS_PER_SM), BLOCKS_PER_SM)
 gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                     void* __restrict__ out, int out_is_f32, int n_tokens, int n_features, int k_blocks,
                     int k_blocks_per_split, long long ld_out, long long partial_stride, int up_row_offset,
@@ -647,7 +654,8 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
       umma_commit(tmem_full_bar);    // accumulator complete (or, after giving up, releases the epilogue)
     }
   } else {
-    // ---------------------------------------------------------------- epilogue (warps 2..5)
+    // ---------------------------------------------------------------- epilogue (warps 2..5, or 2..9)
+    constexpr int EPI = epilogue_warps(MODE, ORIENT, BLOCKS_PER_SM);
     pdl_wait();
     const int quad = warp & 3;  // tensor-memory lanes 32 * quad .. + 31 belong to this warp
     auto wait_acc = [&]() -> bool {
@@ -656,7 +664,7 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
         *abort_flag = 1;
         atomicCAS(error_word, 0, ERR_TIMEOUT_EPILOGUE);
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");   // the four epilogue warps agree on whether to go on
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI) : "memory");   // the epilogue warps agree on whether to go on
       ok = !*abort_flag;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       return ok;
@@ -665,11 +673,12 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
     float* out_f32 = reinterpret_cast<float*>(out) + (long long)blockIdx.z * partial_stride;
     __nv_bfloat16* out_bf16 = reinterpret_cast<__nv_bfloat16*>(out) + (long long)blockIdx.z * partial_stride;
     if (ORIENT == 1) {
+      const int first_half = EPI == 8 ? (F_TILE + 31) / 32 * 16 : F_TILE, part = (warp - 2) / 4;
       // (the pipeline's stages are idle once the accumulator is complete: the adding epilogue passes its tiles through them)
       epilogue_tokens_on_rows<MODE, BLOCKS_PER_SM == 1 ? 4 : 1>(
           lane_base, BN, F_TILE, f0, blockIdx.x, t0 + quad * 32, lane, n_kb > 0,
           out_is_f32 ? static_cast<void*>(out_f32) : static_cast<void*>(out_bf16), out_is_f32, ld_out, n_tokens, n_features,
-          ex, hx, reinterpret_cast<float*>(smem) + quad * (32 * 32), wait_acc);
+          ex, hx, reinterpret_cast<float*>(smem) + quad * (32 * 32), part ? first_half : 0, part ? F_TILE : first_half, wait_acc);
     } else if (wait_acc()) {
       if (ORIENT == 0 && MODE == 1) {
         // lanes 0..63 hold gate, lanes 64..127 up, for the block's 64 output features: the up warps
@@ -904,7 +913,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
       epilogue_tokens_on_rows<MODE, 2>(lane_base, BN, F_TILE, f0, tile / t_tiles, t0 + quad * 32, lane, n_kb > 0, out, out_is_f32,
                                        ld_out, n_tokens, n_features, ex, hx,
                                        reinterpret_cast<float*>(smem + geo.stages * geo.stage_bytes + 256) + quad * (32 * 32),
-                                       wait_acc);
+                                       0, F_TILE, wait_acc);
       if (!ok) break;
       // this warp has read its lanes of the half out: the MMA warp may overwrite it
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1393,7 +1402,7 @@ int launch(int bn, const CUtensorMap* map_w, const CUtensorMap* map_a, void* out
   const int t_tile = ORIENT == 0 ? bn : BM;
   dim3 grid((n_features + f_tile - 1) / f_tile, (n_tokens + t_tile - 1) / t_tile, splits);
   if (grid.y > 65535 || grid.z > 65535) return ERR_BAD_SIZE;
-  launch_kernel(kern, grid, NUM_THREADS, smem, stream, g, *map_w, *map_a, out, out_is_f32, n_tokens, n_features,
+  launch_kernel(kern, grid, threads_of(MODE, ORIENT, BLOCKS_PER_SM), smem, stream, g, *map_w, *map_a, out, out_is_f32, n_tokens, n_features,
                 k_blocks, per_split, ld_out, partial_stride, up_row_offset, ex, hx, error_word);
   return launch_status();
 }
