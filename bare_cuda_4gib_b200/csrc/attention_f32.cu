@@ -62,10 +62,6 @@ __device__ __forceinline__ void copies_wait_all() { asm volatile("cp.async.wait_
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The same where nothing written has to be seen.
-__device__ __forceinline__ void cluster_sync_relaxed() {
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float peer_float(uint32_t smem_addr, uint32_t rank) {
   uint32_t at;
   float v;
@@ -339,7 +335,9 @@ __global__ void __launch_bounds__(THREADS) attention_f32_kernel(const Args a) {
         O = join(O, o);
       }
     }
-    cluster_sync_relaxed();             // the states may be written again, and no block leaves while they are read
+    // The states may be written again, and no block leaves while they are read.  The arrival has to release: a relaxed one would not
+    // order the reads of other blocks' states before their next writes.  No store to global memory lies ahead of it to wait for.
+    cluster_sync();
   }
   if (rank < rows && threadIdx.x < D) {
     const float inv = L > 0.0f ? 1.0f / L : 0.0f;

@@ -116,6 +116,21 @@ def test_attention_f32(dim, kv_heads, group, page, window, seqs):
         assert torch.equal(case.run(parts), rows), tail
 
 
+@pytest.mark.parametrize("dim,kv", [(64, 4200), (128, 3100)])
+def test_attention_f32_of_more_spans_than_the_cluster_holds_twice(dim, kv):
+    """A few rows over three rounds of the cluster's spans, whose states are written again each time: against 64 bits, and the
+    same bits every time and for the row alone."""
+    torch.manual_seed(dim)
+    case = _Attention(dim, 4, 2, [(1, kv), (3, kv - 70), (1, 2), (4, kv - 1)], 0, 64)
+    parts = [(s, 0, n) for s, (n, _) in enumerate(case.seqs)]
+    got, want = case.run(parts), case.want()
+    bound = (4 * (dim / 2 + 2) + 2 * 64 + 3 * (kv / 64 + 1)) * EPS          # as in test_attention_f32
+    assert ((got.double() - want).abs() <= bound * want.abs().max()).all()
+    for _ in range(20):
+        assert torch.equal(case.run(parts), got)
+    assert torch.equal(case.run([(3, 3, 1)]), got[-1:])
+
+
 @pytest.mark.parametrize("rows,hidden,partials", [(1, 64, 1), (3, 2048, 2), (300, 4100, 1), (2, 2050, 1)])
 def test_add_rmsnorm_f32(rows, hidden, partials):
     from bare_cuda_4gib_b200.kernels import lib as K
