@@ -56,15 +56,9 @@ __device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_
 template <int N>
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// The same where nothing written has to be seen: no block leaves before all have come here.  (A releasing arrival would wait for the
-// results' stores, 0.5 us.)
-__device__ __forceinline__ void cluster_sync_relaxed() {
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
+// The cluster's barrier: what a thread has written is seen, and what it has read may be written again or go, behind everyone's wait.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ float4 peer_load(uint32_t smem_addr, uint32_t rank) {
   uint32_t at;
@@ -231,20 +225,26 @@ matmul_f32_kernel(const Args p) {
 #pragma unroll
     for (int j = 0; j < TN; ++j)
       smem[(wm * TM + i) * S::BN + (wn * TN + j) * 32 + lane] = pair_sum(part[i][j]);
-  cluster_sync();
+  cluster_arrive();
+  cluster_wait();
   constexpr int PIECES = S::BM * S::BN / 4, EACH = PIECES / SEGMENTS, ROW_PIECES = S::BN / 4;
   static_assert(PIECES % SEGMENTS == 0, "every block of a cluster adds up the same number of pieces");
-  for (int e = tid; e < EACH; e += S::THREADS) {
-    const int piece = rank * EACH + e, r = piece / ROW_PIECES, c = (piece % ROW_PIECES) * 4;
-    const int m = m0 + r, n = n0 + c;
-    if (m >= m_end || n >= p.N) continue;
+  static_assert(EACH <= S::THREADS, "a thread adds up one piece at most");
+  const int piece = rank * EACH + tid, r = piece / ROW_PIECES, c = (piece % ROW_PIECES) * 4;
+  const int m = m0 + r, n = n0 + c;
+  const bool mine = tid < EACH && m < m_end && n < p.N;
+  float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (mine) {
     const uint32_t at = base + (uint32_t)(r * S::BN + c) * 4;
     float4 v[SEGMENTS];
 #pragma unroll
     for (int q = 0; q < SEGMENTS; ++q) v[q] = peer_load(at, q);
-    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
     for (int q = 0; q < SEGMENTS; ++q) sum.x += v[q].x, sum.y += v[q].y, sum.z += v[q].z, sum.w += v[q].w;
+  }
+  __syncwarp();
+  cluster_arrive();                  // this block's reads are done (ahead of the results' stores, which the arrival would wait for: 0.5 us)
+  if (mine) {
     float* to = p.out + (long long)m * p.ldo + n;
     to[0] = sum.x;
     if (n + 1 < p.N) to[1] = sum.y;
@@ -252,7 +252,7 @@ matmul_f32_kernel(const Args p) {
     if (n + 3 < p.N) to[3] = sum.w;
   }
   __syncwarp();
-  cluster_sync_relaxed();            // no block leaves while another reads its sums
+  cluster_wait();                    // no block leaves while another reads its sums
 }
 
 template <int TM, int TN, int WM, int WN, int STAGES, bool SPLIT>
