@@ -312,7 +312,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap pool_map, AttnArgs 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  if (warp != MMA_WARP) pdl_wait();      // (the MMA issuer reads shared and tensor memory only)
+  pdl_wait();      // (the MMA issuer too: the limit of its waits counts from here)
   if (warp > MMA_WARP) {
     // ------------------------------------------------------------------ loader warp
     // Tile n of the ring is the keys (n even) or the values (n odd) of key block n / 2: one TMA box

@@ -88,16 +88,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Waits for the phase with the given parity; gives up after limit_ns or when another role
-// has already given up.  Returns false on giving up.
+// has already given up.  Returns false on giving up.  The time of the kernels before does not count: a role comes here behind
+// pdl_wait(), or names a flag of the block that a role sets which did.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          unsigned long long limit_ns) {
+                                          unsigned long long limit_ns, const volatile int* past_wait = nullptr) {
   if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long start = global_timer();
+  unsigned long long start = global_timer();
   for (unsigned spins = 0;; ++spins) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((spins & 63u) == 63u) {
       if (*abort_flag) return false;
-      if (global_timer() - start > limit_ns) return false;
+      if (past_wait && !*past_wait) start = global_timer();
+      else if (global_timer() - start > limit_ns) return false;
     }
   }
 }
@@ -625,6 +627,7 @@ gemm_tcgen05_kernel(const Geometry geo, const __grid_constant__ CUtensorMap map_
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     if (elect_one()) {
+      pdl_wait();      // the limit of its waits counts from here: the kernels before have their own time
       const uint32_t idesc = geo.idesc;
       bool ok = true;
       int s = 0;
@@ -857,6 +860,7 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     if (elect_one()) {
+      pdl_wait();      // (the limit of its waits counts from here)
       const uint32_t idesc = geo.idesc, smem_base = smem_u32(smem);
       int s = 0, j = 0;
       uint32_t phase = 0;
@@ -1038,6 +1042,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
   uint64_t* received_bar = acc_bar + 1;
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(received_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+  volatile int* past_wait = reinterpret_cast<volatile int*>(tmem_base_slot + 2);   // the producer is behind its pdl_wait()
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % C, tile = blockIdx.x / C;
@@ -1067,6 +1072,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
     mbar_init(acc_bar, 1);
     mbar_init(received_bar, 1);
     *abort_flag = 0;
+    *past_wait = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(received_bar, (uint32_t)(C * n_tokens * ROWS * 4));
@@ -1083,13 +1089,14 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   cluster_arrive();        // this block has its barriers
   const uint32_t tmem_base = *tmem_base_slot;
-  // Every role that reads what other kernels write waits for them by itself: with a barrier of the block behind one thread's wait
-  // and copies the others began 0.9 us later.
+  // Every role that reads what other kernels write waits for them by itself: with a barrier of the block behind one thread's wait and
+  // copies the others began 0.9 us later.  The MMA issuer goes by the producer's wait.
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     if (elect_one()) {
       pdl_wait();
+      *past_wait = 1;
       for (int i = 0; i < n_early; ++i) issue_activations(i, i);
       int armed = n_early;
       int s = n_early == a.stages ? 0 : n_early;
@@ -1124,7 +1131,7 @@ gemm_cluster_kernel(const ClusterArgs a, const __grid_constant__ CUtensorMap map
       uint32_t phase = 0;
       const uint32_t smem_base = smem_u32(smem);
       for (int i = 0; i < n_kb; ++i) {
-        if (!mbar_wait(&full_bar[s], phase, abort_flag, a.wait_ns)) {
+        if (!mbar_wait(&full_bar[s], phase, abort_flag, a.wait_ns, past_wait)) {
           *abort_flag = 1;
           atomicCAS(a.error_word, 0, ERR_TIMEOUT_MMA);
           break;

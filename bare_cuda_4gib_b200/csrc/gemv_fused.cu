@@ -235,13 +235,14 @@ __global__ void __launch_bounds__(threads_of(NT), PRO == PRO_NORM || NT > 1 ? 1 
     int stage = 0;
     uint32_t phase = 0;
     uint32_t in_flight = 0, in_flight_parity = 0;   // per stage: a load was issued / with which parity
-    bool staging_free = false;
+    bool staging_free = false, ring_full = false;
     for (int item = blockIdx.x; item < a.n_items; item += gridDim.x) {
       int lo, hi, lo_last, hi_last;
       item_rows<EPI>(a, item, lo, hi, lo_last, hi_last);
       for (int k0 = 0; k0 < a.k; k0 += a.kc) {
         const int len = min(a.kc, a.k - k0);
         if (PRO == PRO_NORM && stage >= a.first_aliased && !staging_free) {
+          pdl_wait();      // (the limit of its waits counts from here)
           if (!mbar_wait(norm_done, 0, gave_up, a.error_word, ERR_GEMV_PRODUCER)) goto producer_done;
           staging_free = true;
         }
@@ -260,6 +261,8 @@ __global__ void __launch_bounds__(threads_of(NT), PRO == PRO_NORM || NT > 1 ? 1 
         in_flight |= 1u << stage;
         in_flight_parity = (in_flight_parity & ~(1u << stage)) | (phase << stage);
         if (++stage == a.stages) {
+          if (!ring_full) pdl_wait();      // from here on the consumers, who are behind that wait, have to free a stage first
+          ring_full = true;
           stage = 0;
           phase ^= 1u;
         }

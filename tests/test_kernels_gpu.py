@@ -604,6 +604,60 @@ def test_a_block_of_a_cluster_gives_up_and_no_block_writes(k, drop):
     _close(residual, before.double() + a.double() @ w.double().t(), 1e-5, 2e-3)
 
 
+@pytest.mark.parametrize("form,rows,n,k", [("weights on the rows", 40, 256, 256), ("tokens on the rows", 300, 256, 256),
+                                           ("persistent", 2048, 5120, 128), ("cluster", 40, 256, 1024)])
+def test_a_slow_kernel_ahead_does_not_use_up_a_products_wait_limit(form, rows, n, k, monkeypatch):
+    """A product starts while the kernel before it still runs, and its roles' waits have a limit.  The limit is for the product's own
+    progress: behind a kernel that takes many times as long as the limit it still gives the right result."""
+    from ctypes import c_int, c_longlong
+    from bare_cuda_4gib_b200.kernels import gemm
+    from bare_cuda_4gib_b200.kernels import lib as K
+    torch.manual_seed(rows + k)
+    if form == "persistent":
+        monkeypatch.setenv("BARE_CUDA_B200_GEMM_BN", "256")
+    ctx = _ctx()
+    a = ctx.ws.get("a", (rows, k), torch.bfloat16)
+    a.copy_(torch.randn(rows, k, device=DEV))
+    w = (torch.randn(n, k, device=DEV) / math.sqrt(k)).to(torch.bfloat16)
+    plan = gemm.plan_for(w)
+    residual = torch.zeros(rows, n, device=DEV)
+    end = K.AddTo(residual)
+    assert form != "cluster" or gemm.cluster_kind(plan, rows, torch.float32, False, end) == gemm.CL_ADD
+
+    def product():
+        if form == "cluster":
+            residual.zero_()
+            before()
+            gemm.run_cluster(ctx, plan, gemm.CL_ADD, a, rows, torch.float32, "out", end)
+            return residual
+        before()
+        return gemm.run(ctx, plan, a, rows, torch.float32, "out", allow_partials=False, swiglu=False).tensor
+
+    before = lambda: None
+    want = a.double() @ w.double().t()
+    _close(product(), want, 1e-5, 2e-3)                       # (and the kernel is loaded)
+    # one block walks over a long row: some 148 SMs are free for the product meanwhile
+    row, place = torch.zeros(1, 40_000_001, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    marks = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    before = lambda: K.argmax_rows(row, place, 1, ctx.stream)
+    before()
+    marks[0].record()
+    before()
+    marks[1].record()
+    torch.cuda.synchronize()
+    assert marks[0].elapsed_time(marks[1]) > 1.5              # ms: five times the limit below
+    hooks = gemm.lib().llm_gemm_test_hooks
+    hooks.argtypes, hooks.restype = [c_longlong, c_int], None
+    hooks(300_000, -1)
+    try:
+        got = product()
+        torch.cuda.synchronize()
+        gemm.check_errors()
+    finally:
+        hooks(0, -1)
+    _close(got, want, 1e-5, 2e-3)
+
+
 # ------------------------------------------------------------------------------ tensor-core attention
 
 def _attention_case(seqs, heads, kv_heads, d, page, window, seed, far_key=False, drop_passed=False,
