@@ -198,8 +198,9 @@ __device__ __forceinline__ void item_rows(const GemvArgs& a, int item, int& lo, 
   }
 }
 
+// (Two blocks' registers have to fit an SM wherever the launcher gives every item a block of its own.)
 template <int NT, int PRO, int EPI>
-__global__ void __launch_bounds__(threads_of(NT), PRO == PRO_NORM || NT > 1 ? 1 : 2) gemv_fused_kernel(const GemvArgs a) {
+__global__ void __launch_bounds__(threads_of(NT), PRO == PRO_NORM ? 1 : 2) gemv_fused_kernel(const GemvArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int row_stride = a.kc * 2 + ROW_PAD, stage_bytes = 16 * row_stride;
   uint8_t* ring = smem;                                                              // [stages][16][row_stride]
@@ -568,8 +569,9 @@ __global__ void __launch_bounds__(threads_of(NT), PRO == PRO_NORM || NT > 1 ? 1 
   }
 }
 
+// `resident`: not a launch but the question how many blocks of `smem` bytes an SM holds at once.
 template <int NT, int PRO, int EPI>
-int launch(const GemvArgs& a, size_t smem, int grid, cudaStream_t stream) {
+int launch(const GemvArgs& a, size_t smem, int grid, cudaStream_t stream, int* resident) {
   auto kern = gemv_fused_kernel<NT, PRO, EPI>;
   static bool raised = false;   // one instantiation, one attribute (per process; one device per process)
   if (!raised) {
@@ -577,26 +579,40 @@ int launch(const GemvArgs& a, size_t smem, int grid, cudaStream_t stream) {
       return launch_status();
     raised = true;
   }
+  if (resident) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(resident, kern, threads_of(NT), smem);
+    return launch_status();
+  }
   launch_kernel(kern, grid, threads_of(NT), smem, stream, a);
   return launch_status();
 }
 
 template <int NT, int PRO>
-int launch_epi(int epi, const GemvArgs& a, size_t smem, int grid, cudaStream_t stream) {
+int launch_epi(int epi, const GemvArgs& a, size_t smem, int grid, cudaStream_t stream, int* resident) {
   switch (epi) {
-    case EPI_STORE: return launch<NT, PRO, EPI_STORE>(a, smem, grid, stream);
-    case EPI_ADD: return launch<NT, PRO, EPI_ADD>(a, smem, grid, stream);
-    case EPI_SWIGLU: return launch<NT, PRO, EPI_SWIGLU>(a, smem, grid, stream);
-    case EPI_ROPE: return launch<NT, PRO, EPI_ROPE>(a, smem, grid, stream);
+    case EPI_STORE: return launch<NT, PRO, EPI_STORE>(a, smem, grid, stream, resident);
+    case EPI_ADD: return launch<NT, PRO, EPI_ADD>(a, smem, grid, stream, resident);
+    case EPI_SWIGLU: return launch<NT, PRO, EPI_SWIGLU>(a, smem, grid, stream, resident);
+    case EPI_ROPE: return launch<NT, PRO, EPI_ROPE>(a, smem, grid, stream, resident);
   }
   return ERR_BAD_SIZE;
 }
 
 template <int NT>
-int launch_pro(int pro, int epi, const GemvArgs& a, size_t smem, int grid, cudaStream_t stream) {
-  if (pro == PRO_BF16) return launch_epi<NT, PRO_BF16>(epi, a, smem, grid, stream);
-  if (pro == PRO_NORM) return launch_epi<NT, PRO_NORM>(epi, a, smem, grid, stream);
-  if (pro == PRO_PRENORMED) return launch_epi<NT, PRO_PRENORMED>(epi, a, smem, grid, stream);
+int launch_pro(int pro, int epi, const GemvArgs& a, size_t smem, int grid, cudaStream_t stream, int* resident) {
+  if (pro == PRO_BF16) return launch_epi<NT, PRO_BF16>(epi, a, smem, grid, stream, resident);
+  if (pro == PRO_NORM) return launch_epi<NT, PRO_NORM>(epi, a, smem, grid, stream, resident);
+  if (pro == PRO_PRENORMED) return launch_epi<NT, PRO_PRENORMED>(epi, a, smem, grid, stream, resident);
+  return ERR_BAD_SIZE;
+}
+
+int launch_tokens(int tokens, int pro, int epi, const GemvArgs& a, size_t smem, int grid, cudaStream_t stream, int* resident) {
+  switch ((tokens + 7) / 8) {
+    case 1: return launch_pro<1>(pro, epi, a, smem, grid, stream, resident);
+    case 2: return launch_pro<2>(pro, epi, a, smem, grid, stream, resident);
+    case 3: return launch_pro<3>(pro, epi, a, smem, grid, stream, resident);
+    case 4: return launch_pro<4>(pro, epi, a, smem, grid, stream, resident);
+  }
   return ERR_BAD_SIZE;
 }
 
@@ -655,6 +671,12 @@ extern "C" long long llm_gemv_fused_smem(int tokens, int k) {
   return plan_smem(tokens, k, PRO_NORM, SMEM_BUDGET, 2, p) ? (long long)p.bytes : 0;
 }
 
+// Blocks of the form for `tokens` tokens that an SM holds at once when each takes half of its shared memory (0: there is no such form).
+extern "C" int llm_gemv_fused_resident(int tokens, int pro, int epi) {
+  int blocks = 0;
+  return tokens >= 1 && launch_tokens(tokens, pro, epi, GemvArgs{}, SMEM_HALF, 0, nullptr, &blocks) == 0 ? blocks : 0;
+}
+
 extern "C" int llm_gemv_fused(const void* w, int w_rows, int k, int tokens, int pro, int epi,
                               const void* x, long long x_stride, const void* norm_w, int norm_w_dtype, float eps,
                               const int32_t* row_index, void* out, int out_dtype, long long out_stride, int n_out,
@@ -694,12 +716,12 @@ extern "C" int llm_gemv_fused(const void* w, int w_rows, int k, int tokens, int 
     if (n_out < 1 || n_out > w_rows) return ERR_BAD_SIZE;
     a.n_items = (n_out + 15) / 16;
   }
-  const int nt = (tokens + 7) / 8;
   int grid = a.n_items < max_blocks ? a.n_items : max_blocks;
   if (grid < 1) return ERR_BAD_SIZE;
   // A product with a few more items than SMs (one and a bit per block) would keep most SMs waiting
   // for the blocks that run two.  If a block with one whole-row stage fits twice on an SM, every
-  // item gets a block of its own instead and all of them stream at once.
+  // item gets a block of its own instead and all of them stream at once.  (The launch bounds see to it that its registers fit too: with
+  // rotation, 4,096 x 1,024, 9 and 24 tokens 6.5 and 7.2 us in two waves of one block an SM, 4.3 and 4.8 with two.)
   SmemPlan one;
   if (pro != PRO_NORM && a.n_items > max_blocks && a.n_items <= 2 * max_blocks &&
       plan_smem(tokens, k, pro, SMEM_HALF, 1, one) && one.kc == k) {
@@ -708,12 +730,5 @@ extern "C" int llm_gemv_fused(const void* w, int w_rows, int k, int tokens, int 
     a.kc = plan.kc, a.stages = 1, a.first_aliased = 1;
     grid = a.n_items;
   }
-  const size_t smem = plan.bytes;
-  switch (nt) {
-    case 1: return launch_pro<1>(pro, epi, a, smem, grid, stream);
-    case 2: return launch_pro<2>(pro, epi, a, smem, grid, stream);
-    case 3: return launch_pro<3>(pro, epi, a, smem, grid, stream);
-    case 4: return launch_pro<4>(pro, epi, a, smem, grid, stream);
-  }
-  return ERR_BAD_SIZE;
+  return launch_tokens(tokens, pro, epi, a, plan.bytes, grid, stream, nullptr);
 }

@@ -897,6 +897,18 @@ def test_gemv_fused_many_items_and_parts():
     assert torch.equal(results[1], results[8][:1])
 
 
+@pytest.mark.parametrize("tokens", [1, 8, 9, 16, 17, 24, 32])
+def test_gemv_fused_two_blocks_fit_an_sm(tokens):
+    """A product with up to two items an SM gives each item a block of its own, all running at once: every form that takes its input as
+    it is has to fit twice on an SM, registers and all."""
+    from bare_cuda_4gib_b200.kernels import gemv
+    for activation in ("silu", "gelu_tanh"):
+        resident = gemv.lib(activation).llm_gemv_fused_resident
+        for pro in (gemv.PRO_BF16, gemv.PRO_PRENORMED):
+            for epi in (gemv.EPI_STORE, gemv.EPI_ADD, gemv.EPI_SWIGLU, gemv.EPI_ROPE):
+                assert resident(tokens, pro, epi) >= 2, (activation, pro, epi)
+
+
 @pytest.mark.parametrize("tokens,inter,k", [(2, 176, 64), (8, 100, 96), (16, 5632, 2048), (7, 13, 160)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_gemv_fused_swiglu(tokens, inter, k, norm):
