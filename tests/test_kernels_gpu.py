@@ -869,7 +869,8 @@ def test_gemv_fused_plain_and_add(tokens, n, k, norm):
 
 def test_gemv_fused_many_items_and_parts():
     """More items to a block than sums have halves, more parts of the sums of squares than a lane asks for at once, token slots
-    that share the row of zeros; and a token's result is the same bits in any batch of up to eight."""
+    that share the row of zeros (in the first, second and third group of eight); and a token's result is the same bits whatever
+    tokens are with it in as many groups of eight."""
     import types as _types
     from bare_cuda_4gib_b200.kernels import gemm, gemv
     from bare_cuda_4gib_b200.kernels import lib as K
@@ -882,19 +883,22 @@ def test_gemv_fused_many_items_and_parts():
     w_add = (torch.randn(hidden, 64, device=DEV) * 0.3).to(torch.bfloat16)
     w = (torch.randn(n, hidden, device=DEV) * 0.1).to(torch.bfloat16)
     act, stream = torch.randn(24, 64, device=DEV).to(torch.bfloat16), torch.randn(24, hidden, device=DEV)
+    r = stream.double() + act.double() @ w_add.double().t()
+    x = r / torch.sqrt((r * r).mean(-1, keepdim=True) + 1e-6) * norm.tensors["weight"].double()
+    want = x @ w.double().t()
+    # the input is rounded to bfloat16 once, see test_gemv_fused_add_then_prenormed_input: sigma = 2^-9 / sqrt(3) * sqrt(hidden) * 0.1,
+    # and the bound is 8 sigma
+    bound = 8 * 2.0 ** -9 / math.sqrt(3.0) * math.sqrt(hidden) * 0.1
     results = {}
-    for tokens in (1, 8, 9, 24):
+    for tokens in (1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 16, 17, 23, 24):
         residual = stream[:tokens].clone()
         assert gemv.run(ctx, w_add, act[:tokens], tokens, torch.float32, "out", False, K.AddTo(residual, norm)) is None
         lazy = K.LazyNorm(ctx, residual, norm.tensors["weight"], 1e-6, tokens, None, "normed", ctx.prenormed)
         results[tokens] = gemv.run(ctx, w, lazy, tokens, torch.float32, "out2", False, None).tensor.clone()
     gemm.check_errors()
-    r = stream.double() + act.double() @ w_add.double().t()
-    x = r / torch.sqrt((r * r).mean(-1, keepdim=True) + 1e-6) * norm.tensors["weight"].double()
-    # the input is rounded to bfloat16 once, see test_gemv_fused_add_then_prenormed_input: sigma = 2^-9 / sqrt(3) * sqrt(hidden) * 0.1,
-    # and the bound is 8 sigma
-    _close(results[24], x @ w.double().t(), 0.0, 8 * 2.0 ** -9 / math.sqrt(3.0) * math.sqrt(hidden) * 0.1)
-    assert torch.equal(results[1], results[8][:1])
+    for tokens, got in results.items():
+        _close(got, want[:tokens], 0.0, bound)
+        assert torch.equal(got, results[-(-tokens // 8) * 8][:tokens]), tokens
 
 
 @pytest.mark.parametrize("tokens", [1, 8, 9, 16, 17, 24, 32])
