@@ -24,12 +24,24 @@
 #define ERR_BAD_ALIGN 3
 
 // Programmatic dependent launch.  Every kernel of the engine is launched with the attribute that
-// lets it start while the kernel before it in the stream is still running.  In return every
-// kernel calls pdl_wait() before it touches global memory that another kernel may have written
-// or may still read (it returns once all earlier kernels have finished and their writes are
-// visible), and pdl_launch_dependents() at its start, which lets the next kernel begin its own
-// preamble.  What runs before pdl_wait() may only touch shared memory, tensor memory, and global
-// memory that no kernel writes (weights).  Set BARE_CUDA_B200_NO_PDL=1 to launch without it.
+// lets it start while the kernel before it in the stream is still running, and calls
+// pdl_launch_dependents() at its start, which lets the next kernel begin its own preamble; so
+// several kernels before may still run.  In return a role that reads or writes global memory which
+// they write or read calls pdl_wait() first (it returns once all earlier kernels have finished and
+// their writes are visible).  Ahead of it only this may be touched:
+//  - shared memory and tensor memory;
+//  - weights and tables that were made with the model;
+//  - the step's metadata (positions, lengths, block tables): it is copied to the device ahead of the
+//    step's first kernel, and no kernel writes it;
+//  - cache positions below the step's first new one (read so by the two attentions of decoding requests): kernels of
+//    earlier steps wrote them.
+// The last two are safe because every step begins with that copy, an ordinary operation of the stream:
+// no kernel of the step starts before it, and it waits for all kernels of the step before.  A caller that
+// appends to a request's cache and attends over it, or writes metadata by a kernel, with nothing but
+// such kernels in between would race: it has to put a copy or a synchronisation there.
+// A role that touches no such memory (an MMA issuer) need not wait, but some thread of every block does,
+// because a kernel may not end before those before it; and the limit of a bounded wait counts from the end
+// of the kernels before.  Set BARE_CUDA_B200_NO_PDL=1 to launch without it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -63,10 +75,9 @@ static inline int launch_status() {
   return e == cudaSuccess ? 0 : 1000 + static_cast<int>(e);
 }
 
-// True in one thread of the (converged) warp.  The compiler knows that of elect.sync, and not of a test of the lane: behind `lane ==
-// 0` every tensor-core instruction and every copy, whose operands have to be uniform, becomes a loop over the threads that might
-// be there, about 110 cycles each: a k block's four products and two copies took 590 and 455 cycles, whatever the tile (2,048 x
-// 5,632, 300 rows 31.2 -> 19.5 us, 900 rows 34.7 -> 22.9; 11,264 x 2,048 gated, 900 rows 48.9 -> 43.3).
+// True in one thread of the (converged) warp.  Issuing copies and tensor-core instructions, whose operands are the same for a whole
+// warp, measured faster behind this than behind `lane == 0`, whatever the tile (2,048 x 5,632, 300 rows 31.2 -> 19.5 us, 900 rows
+// 34.7 -> 22.9; 11,264 x 2,048 gated, 900 rows 48.9 -> 43.3).
 __device__ __forceinline__ bool elect_one() {
   uint32_t elected;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
