@@ -42,7 +42,8 @@ constexpr int BK = 64;       // k elements per stage (one 128-byte swizzle row)
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;
 // The gated end of tokens on the MMA rows, one block to an SM, is arithmetic (an exponential and a division an output) that nothing
-// hides: eight warps share it instead of four, half of the tile's columns each (300 tokens x 11,264 x 2,048: 23.4 -> 19.8 us).  The
+// hides: eight warps share it instead of four, half of the tile's columns each (300 tokens x 11,264 x 2,048: 23.4 -> 19.8 us; 150 cases of 256 to
+// 5,632 outputs and 65 to 300 tokens: tiles of 64 rows 0.96 of the time, 128 0.90, 256 0.86, silu and gelu alike; experts' products 0.88).  The
 // adding end, which memory bounds, gets slower with eight (2,048 x 2,048 x 5,632: 44.4 -> 47.9).
 constexpr int epilogue_warps(int mode, int orient, int blocks_per_sm) { return mode == 1 && orient == 1 && blocks_per_sm == 1 ? 8 : 4; }
 constexpr int threads_of(int mode, int orient, int blocks_per_sm) { return 64 + 32 * epilogue_warps(mode, orient, blocks_per_sm); }
@@ -951,8 +952,8 @@ gemm_tcgen05_persistent_kernel(const Geometry geo, const __grid_constant__ CUten
 // Two blocks share an SM (112 KB of shared memory each), so that a kernel's weights are on their way while
 // the kernel before it still runs on the other half.  What bounds it: the chain wait for the input - first tile - last
 // product - exchange - stores, which is why eight warps share the epilogue, why every role waits for the kernel before by itself,
-// and why metadata, angles and the next norm's weights are read before that wait (a step of 22 layers of TinyLlama's sizes: 26 rows
-// 992 -> 908 us, 61 rows 1,094 -> 987, 128 rows 1,289 -> 1,196, 240 rows 1,587 -> 1,476).  An arrival at the cluster's barrier that
+// and why metadata, angles and the next norm's weights are read before that wait (a step of 22 layers of TinyLlama's sizes, with elected
+// issuers: 61 rows 1,094 -> 934 us, 128 rows 1,289 -> 1,089, 240 rows 1,587 -> 1,349).  An arrival at the cluster's barrier that
 // releases costs about 0.5 us each time, waiting for the thread's own accesses.  (Storing the slices straight from registers into
 // the other blocks' shared memory, 16 bytes a lane, measured slower: 9.5 against 8.0 us for 64 tokens x 2,048 x 2,048.)
 enum { CL_ADD = 1, CL_SWIGLU = 2, CL_ROPE = 3 };
@@ -1613,9 +1614,9 @@ static int gemm_bf16(const void* map_w, const void* map_a, void* out, int out_dt
   const bool pair = tiles > sm_count() && two.tmem_cols <= 256 && two.stages >= ((orient == 1 && mode == 1) ? 2 : 3);
   if (orient == 1 && splits == 1 && tiles > sm_count() && bn >= 192) {
     // More tiles than SMs: one block per SM walks over them (see the persistent kernel).  Only for
-    // wide tiles: a stage of a narrow tile is shorter on the tensor core than the one issuing
-    // thread's round of waiting for it, issuing its instructions and committing, and then two
-    // blocks per SM with an issuing thread each are faster.
+    // wide tiles, which do not fit twice on an SM.  Narrower ones, adding end, 2,048 rows, two blocks an SM / persistent: tiles of 128,
+    // 2,048 x 2,048 24.0 / 25.4 us, 2,048 x 5,632 47.9 / 48.4, 4,096 x 4,096 74.4 / 70.0; of 160, 27.1 / 29.5, 52.7 / 54.6, 79.9 /
+    // 66.1: only products for which tiles of 256 are the choice anyway (67.3) would gain by it.
     if (hx.dim) return launch_persistent<2>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, hx, error_word, stream);
     if (mode == 0) return launch_persistent<0>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, hx, error_word, stream);
     return launch_persistent<1>(bn, mw, ma, out, f32, n_tokens, n_features, K, ld_out, up_row_offset, ex, hx, error_word, stream);

@@ -24,8 +24,8 @@
 // SMs idle.
 //
 // Measured on one B200 (microseconds a launch; the plain kernel's 64 x 64 tiles before, this now):
-//   weights 11,264 x 2,048 (92 MB): 4 rows 1,010 -> 17.9 (5.2 TB/s); 257 rows 1,380 -> 302; 2,048 rows 2,105 (44.9 TFLOP/s)
-//   weights 2,048 x 2,048 (17 MB):  4 rows 450 -> 5.4 (3.1 TB/s); 257 rows 68; 2,048 rows 435
+//   weights 11,264 x 2,048 (92 MB): 4 rows 1,010 -> 19.2 (4.8 TB/s); 257 rows 1,380 -> 303; 2,048 rows 2,106 (44.9 TFLOP/s)
+//   weights 2,048 x 2,048 (17 MB):  4 rows 450 -> 6.0 (2.8 TB/s); 257 rows 69; 2,048 rows 436
 // The FMA units' peak is 74.4 TFLOP/s (148 SMs x 128 FMAs x 1.965 GHz); with eight rows x four weight rows a thread the shared-memory wavefronts
 // (32 for 64 packed FMAs) take as long as the arithmetic.  Tiles of 8 x 8 or 16 x 4 a thread (one block an SM) gained 4 % at
 // 2,048 rows and lose it at 257.

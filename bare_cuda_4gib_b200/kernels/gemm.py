@@ -145,12 +145,13 @@ def max_splits(n: int, k: int) -> int:
     return max(1, min(-(-k // BK) // 4, (2 * sm_count()) // -(-n // BM)))
 
 
-TOKENS_ON_ROWS_ABOVE = 240    # steps with more rows put 128 tokens on the MMA rows (orientation 1); measured: a step
-                              # of 256 rows takes 2.32 ms that way and 2.53 ms with the weights on the MMA rows, one of 224 rows 2.5 and 2.23
+TOKENS_ON_ROWS_ABOVE = 240    # steps with more rows put 128 tokens on the MMA rows (orientation 1); measured: a step of TinyLlama's sizes
+                              # with 256 rows takes 1,657 us that way and 2,249 with the weights on the MMA rows, one of 240 rows 1,653
+                              # that way and 1,349 with the cluster product
 # The SwiGLU product changes over earlier: with the weights on the MMA rows a block holds only 64
-# outputs, so from about a hundred tokens on the other orientation's wider tiles measured faster
-# (TinyLlama's feed-forward at 128 / 256 tokens: 16 / 19 us against 23 / 48 us; at 48 / 64 / 80 / 96 tokens 16.3 us
-# that way, whatever the count, against 14.9 / 16.8 / 18.5 / 20.2 us).
+# outputs, so from a few dozen tokens on the other orientation's wider tiles measured faster
+# (TinyLlama's feed-forward at 64 / 96 / 128 / 256 tokens: 13.3 / 13.2 / 13.4 / 16.2 us that way against 16.8 / 20.2 / 23.2 / 27.7;
+# 11,008 x 4,096 at 64 / 128: 35.7 / 36.4 against 42.5 / 53.0).  Up to here the cluster product takes it.
 SWIGLU_TOKENS_ON_ROWS_ABOVE = 60
 
 
@@ -173,8 +174,9 @@ def feature_tile(rows: int, n_out: int, swiglu: bool, multiple: int = 0) -> int:
     SwiGLU, whose tile is half gate rows and half up rows).  Every SM works through
     ceil(tiles / SMs) tiles and a tile's time grows with its width, so the product of the two is
     minimised; a small fixed cost per tile breaks ties towards wider tiles.  Wide tiles (192 rows
-    and more) of a product with more tiles than SMs run in the persistent kernel, whose tiles
-    measured about an eighth cheaper (no pipeline refill per tile, the epilogue off the critical path).
+    and more) of a product with more tiles than SMs run in the persistent kernel, whose tiles count an eighth
+    less (no pipeline refill per tile, the epilogue off the critical path).  Of 32 sizes (eight layers of 2,048 to 12,288 outputs, 300 to
+    2,048 rows) the tile this picks is within 8 % of the best one, but for 2,048 x 2,048 at 2,048 rows (256: 26.7 us, 128: 24.0).
     `multiple`: the tile has to be a multiple of this (whole heads)."""
     forced = os.environ.get("BARE_CUDA_B200_GEMM_BN")     # experiments only
     if forced and not multiple:
@@ -190,8 +192,9 @@ def _feature_tile(rows: int, n_out: int, swiglu: bool, multiple: int) -> int:
     for bn in range(256, 63, -step):
         if multiple and bn % multiple:
             continue
-        # between 160 and 256 a tile is too big for two blocks per SM with three stages each, yet
-        # more than one tile per SM needs that overlap: only SwiGLU tiles (two stages) use the range
+        # between 160 and 256 a tile is too big for two blocks per SM with three stages each: only SwiGLU tiles (two stages) use
+        # the range.  (2,048 rows, adding end, tiles of 128 / 192 / 256: 2,048 x 5,632 47.9 / 59.8 / 48.2 us, 4,096 x 4,096 74.4 / 69.8 /
+        # 67.3; one of the measured products would gain: 12,288 x 4,096 254 / 170 / 187.)
         if not swiglu and 160 < bn < 256:
             continue
         cost = tile_cost(rows, n_out, bn, swiglu)
@@ -332,20 +335,20 @@ def run(ctx, plan: GemmPlan, a, rows: int, out_dtype: torch.dtype, buffer: str,
 
 # ------------------------------------------------------------------ a few dozen tokens, ends fused in
 CL_ADD, CL_SWIGLU, CL_ROPE = 1, 2, 3
-# Measured, a whole step of TinyLlama's 22 layers, product + norm + rotation kernels against this: 30 rows 1,230 -> 1,003 us,
-# 40 rows 1,314 -> 1,118, 64 rows 1,396 -> 1,119, 96 rows 1,513 -> 1,232, 130 rows 1,741 -> 1,458, 180 rows 1,951 -> 1,544, 240
-# rows 2,168 -> 1,607; four layers of the Llama-3-8B sizes: 30 rows 634 -> 597, 64 rows 691 -> 659, 112 rows 747 -> 710, 144 rows
-# 830 -> 810, 180 rows 1,022 -> 896, 240 rows 1,056 -> 981; of the Llama-2-7B sizes: 30 rows 488 -> 488, 64 rows 524 -> 534, 112 rows
-# 591 -> 588, 144 rows 648 -> 647, 180 rows 849 -> 751, 240 rows 886 -> 848.  Above, tokens are on the MMA rows.
+# Measured, a whole step of TinyLlama's 22 layers, product + norm + rotation kernels against this: 30 rows 1,094 -> 881 us,
+# 40 rows 1,189 -> 959, 64 rows 1,207 -> 950, 96 rows 1,341 -> 1,013, 130 rows 1,570 -> 1,206, 180 rows 1,783 -> 1,298, 240
+# rows 2,037 -> 1,349; eight layers of the Llama-3-8B sizes: 30 rows 1,014 -> 936, 64 rows 1,121 -> 1,065, 112 rows 1,219 -> 1,135, 144 rows
+# 1,396 -> 1,338, 180 rows 1,789 -> 1,508, 240 rows 1,845 -> 1,612; of the Llama-2-7B sizes: 30 rows 848 -> 802, 64 rows 918 -> 877, 112 rows
+# 1,048 -> 1,003, 144 rows 1,167 -> 1,141, 180 rows 1,559 -> 1,250, 240 rows 1,642 -> 1,516.  Above, tokens are on the MMA rows.
 CLUSTER_MAX_ROWS = TOKENS_ON_ROWS_ABOVE
 # A tile of 96 or 128 tokens would fill an SM's shared memory with one block (96 rows 1,971 us, 128 rows 3,084).
 CLUSTER_TILE_ROWS = 64
-# A gated product has enough tiles; with more rows than a tile's it runs with tokens on the MMA rows (16.3 us up to 128 rows).
+# A gated product has enough tiles; with more rows than a tile's it runs with tokens on the MMA rows (TinyLlama's: 13.4 us up to 128 rows).
 CLUSTER_GATED_ROWS = 64
 # With so few rows that the few-token product (gemv.py) takes the layer's other products, what comes here is a down
-# projection whose input does not fit beside its ring.  A small one gains (12 rows x 2,048 x 5,632, 23 MB: the step 904 -> 873 us),
-# a large one is bound by its weights, which the split product's deeper ring streams faster (8 rows x 4,096 x 14,336, 117 MB:
-# 18.0 us and a norm kernel of 4.3 against 23.5).
+# projection whose input does not fit beside its ring.  A small one gains (12 rows x 2,048 x 5,632, 23 MB, with the norm: 10.1 -> 7.7 us);
+# for a large one, bound by its weights, the split product's deeper ring streamed them faster when the line was drawn (8 rows x 4,096 x
+# 14,336, 117 MB, with the norm: 22.3 against 23.5 us; with elected issuers it is 24.9 against 21.6, and the line stands where it stood).
 CLUSTER_FEW_ROWS, CLUSTER_FEW_BYTES = 24, 64 << 20
 # Layers of a smaller inner size keep the kernels they had.  The kernel takes them (every block of a cluster has two K blocks
 # whatever the size), but a product that adds its result itself hands nothing on, and callers that run a tiny model's block by
@@ -368,8 +371,8 @@ def cluster_size(n_tiles: int, k: int) -> int:
 def cluster_tile(rows: int, n_tiles: int, k: int) -> int:
     """Tokens of a tile: the rows dealt out evenly over as few tiles as hold them, in steps of 16.  49 to 64 rows go in two
     tiles where the blocks of a cluster still walk through at most 12 K blocks each: the exchange at a tile's end lengthens with
-    its tokens (TinyLlama, 61 rows: 1,226 -> 1,127 us a step).  With longer walks the larger cluster of one tile wins: 64 rows, one
-    tile / two: 4,096 x 4,096 (16 K blocks in two tiles) 12.1 / 12.2 us, 6,144 x 4,096 (32) 17.7 / 18.7, 4,096 x 11,008 (43) 21.7 / 23.8."""
+    its tokens (64 rows, one tile / two: 2,048 x 2,048 7.0 / 6.2 us, 2,048 x 5,632 10.6 / 9.3).  With longer walks the larger cluster of one tile wins:
+    4,096 x 4,096 (16 K blocks in two tiles) 11.5 / 12.0, 6,144 x 4,096 (32) 16.0 / 17.1, 4,096 x 11,008 (43) 20.7 / 22.7."""
     tiles = -(-rows // CLUSTER_TILE_ROWS)
     if 48 < rows <= 64 and cluster_walk(2 * n_tiles, k) <= 12:
         tiles = 2
@@ -390,9 +393,10 @@ def cluster_pays(rows: int, n_tiles: int, k: int) -> bool:
     its blocks walk through K quickly.  With wide layers and several token tiles the clusters are small and the walks
     long, and then the other product, whose one tile holds all tokens, is faster, until that tile leaves its ring too few
     stages (more than 160 tokens).  Microseconds with the kernel behind it, cluster / other: 12,288 x 4,096 (32 K blocks a walk) 64
-    rows 27.5 / 28.9, (64) 128 rows 41.8 / 37.8, 192 rows 42.5 / 55.5, (64, and more blocks than two to an SM) 240 rows 74.5 / 63.7;
-    4,096 x 11,008 (43) 128 rows 28.3 / 30.5, (86) 144 rows 42.9 / 31.6, 192 rows 45.3 / 49.5; 4,096 x 14,336 (56) 96 rows 33.5 / 33.0,
-    (112) 144 rows 53.9 / 37.1, 192 rows 56.2 / 54.8, 240 rows 56.1 / 61.6."""
+    rows 24.9 / 26.6, (64) 128 rows 35.7 / 36.2, 192 rows 36.0 / 56.2, (64, and more blocks than two to an SM) 240 rows 65.2 / 65.6;
+    4,096 x 11,008 (43) 128 rows 26.2 / 30.3, (86) 144 rows 37.7 / 31.2, 192 rows 40.4 / 49.1; 4,096 x 14,336 (56) 96 rows 29.7 / 32.7,
+    (112) 144 rows 47.3 / 36.6, 192 rows 49.8 / 54.4, 240 rows 49.9 / 61.0.  (Drawn before the products' issuers were elected, when walks of 56
+    and 64 K blocks were slower in a cluster: those now gain 1 to 9 % there.)"""
     tiles = n_tiles * -(-rows // cluster_tile(rows, n_tiles, k))
     walk = cluster_walk(tiles, k)
     if tiles > 2 * sm_count():
@@ -402,9 +406,9 @@ def cluster_pays(rows: int, n_tiles: int, k: int) -> bool:
 
 def cluster_pays_gated(rows: int, n_tiles: int, k: int) -> bool:
     """The same for a gated product of `n_tiles` tiles of 64 outputs, against tokens on the MMA rows (which run it from 61 rows on).
-    With long walks a block an SM and a few SMs with two take as long as two everywhere: it has to fill two thirds of the places.  Four
-    layers, 61 to 64 rows, cluster / tokens on rows: 11,008 x 4,096 (172 of 296 places) 539 / 520 us, 14,336 x 4,096 (224) 656 / 681; all of
-    TinyLlama's (5,632 x 2,048, 16 K blocks a walk) 1,112 / 1,147."""
+    With long walks a block an SM and a few SMs with two take as long as two everywhere: it has to fill two thirds of the places.  Eight
+    layers, 64 rows, cluster / tokens on rows: 11,008 x 4,096 (172 of 296 places) 923 / 873 us, 14,336 x 4,096 (224) 1,065 / 1,084; all of
+    TinyLlama's (5,632 x 2,048, 16 K blocks a walk) 952 / 936 (1,112 / 1,147 before the issuers were elected)."""
     tiles = n_tiles * -(-rows // cluster_tile(rows, n_tiles, k))
     return rows <= SWIGLU_TOKENS_ON_ROWS_ABOVE or cluster_walk(tiles, k) <= CLUSTER_LONG_WALK or 3 * tiles >= 4 * sm_count()
 
