@@ -38,7 +38,7 @@
 // item's end while the consumers are at the next item.  x for all tokens sits in shared memory for the
 // whole kernel.
 //
-// What bounds it: memory for the wide products (gate and up of 5,632 x 2,048, 8 tokens, one launch behind another: 46 MB in 9.7 us, 0.73
+// What bounds it: memory for the wide products (gate and up of 5,632 x 2,048, 8 tokens, one launch behind another: 46 MB in 8.7 us, 0.81
 // of the copy rate), the chain of memory trips for the others (2,048 x 2,048 3.5 us, 0.36).  So nothing stands on that chain that
 // need not: metadata, angles and weights of norms are fetched before the wait, and the norm's factor per token is the finishers' business,
 // beside the products.  One decode step of TinyLlama's 22 layers: 1 token 714 -> 616 us, 8 tokens 781 -> 716 us.  Every
